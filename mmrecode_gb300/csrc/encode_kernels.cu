@@ -3,9 +3,10 @@
 // transform.rs:111-134), byte-identical to it, for many frames per pass.
 //
 //   fdct_kernel        8 threads per 8x8 block: edge-replicated samples, fp32 row and
-//                      column passes, quantisation; a coefficient whose quotient lies
-//                      within its error bound of a half-integer is recomputed in
-//                      binary64 in the reference's operation order
+//                      column passes, quantisation; coefficients whose quotient lies
+//                      within the error bound of a half-integer are listed and
+//                      recomputed packed, a thread each, in binary64 in the
+//                      reference's operation order
 //   bits_kernel        thread per block: Huffman bit count (DC difference against the
 //                      previous block of the component in its restart interval)
 //   scan (3 kernels)   exclusive prefix of the bit counts, of the segment words and
@@ -109,67 +110,149 @@ __device__ __forceinline__ uint32_t segment_of_chunk(const EncLaunch &L, uint64_
 
 // ----------------------------------------------------------------- FDCT ---
 
-constexpr int kEncBlocksPerCta = 32;
+constexpr int kEncBlocksPerTile = 32;                    // blocks per CTA step, eight threads each
+constexpr int kEncThreads = 8 * kEncBlocksPerTile;
+constexpr int kTieQueue = kEncThreads;                   // packed binary64 work: a thread per entry
+constexpr int kRowStride = 12;                           // floats per row: 16-byte stores of 8 rows hit all banks
+constexpr int kTileStride = 8 * kRowStride + 8;          // per block: four blocks' column loads on distinct banks
 
-__global__ void __launch_bounds__(256) fdct_kernel(EncLaunch L) {
-    __shared__ float s_in[kEncBlocksPerCta][8][9];
-    __shared__ float s_row[kEncBlocksPerCta][8][9];
-    __shared__ float s_mag[kEncBlocksPerCta][8][9];  // sum_x |M[x][u]| |S[r][x]|
-    __shared__ uint8_t s_raw[kEncBlocksPerCta][64];
+// Where block blk's samples come from.
+struct BlockSource {
+    const uint8_t *plane;
+    size_t stride;
+    uint32_t x0, y0, pw, ph, tq;
+};
+
+__device__ __forceinline__ BlockSource block_source(const EncFrame &F, uint64_t blk) {
+    const uint32_t i = (uint32_t)(blk - F.block_base);
+    const uint32_t mcu = i / F.bpm, k = i - mcu * F.bpm;
+    const uint32_t c = F.sched_comp[k];
+    const uint32_t my = mcu / F.mcu_cols, mx = mcu - my * F.mcu_cols;
+    BlockSource B;
+    B.plane = F.plane[c];
+    B.stride = F.stride[c];
+    B.x0 = (mx * F.comp_h[c] + F.sched_bx[k]) * 8;
+    B.y0 = (my * F.comp_v[c] + F.sched_by[k]) * 8;
+    B.pw = F.pw[c];
+    B.ph = F.ph[c];
+    B.tq = F.comp_tq[c];
+    return B;
+}
+
+// Row r of the block's samples, byte x in bits 8x (read_block, encoder.rs:392-402:
+// rows and columns past the plane repeat its last).
+__device__ __forceinline__ uint2 source_row(const BlockSource &B, uint32_t r) {
+    const uint8_t *row = B.plane + (size_t)min(B.y0 + r, B.ph - 1) * B.stride;
+    if (B.x0 + 8 <= B.pw && (reinterpret_cast<uintptr_t>(row + B.x0) & 7) == 0)  // one 8-byte load
+        return *reinterpret_cast<const uint2 *>(row + B.x0);
+    uint2 w = make_uint2(0, 0);
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+        w.x |= (uint32_t)row[min(B.x0 + x, B.pw - 1)] << (8 * x);
+        w.y |= (uint32_t)row[min(B.x0 + 4 + x, B.pw - 1)] << (8 * x);
+    }
+    return w;
+}
+
+// Persistent CTAs, 32 blocks per step. Quotients too close to a half-integer (exact
+// ties of the DC and of the (0, 4), (4, 0), (4, 4) coefficients, a few per cent of
+// the blocks, and what the fp32 bound leaves open) are not recomputed where they
+// turn up: a binary64 warp instruction holds GB300's FP64 pipe for tens of cycles
+// whatever its active lanes, and one or two lanes per warp cost 5.6 of the 7.0 ms
+// of an encode of 60 1080p 4:2:2 frames of integer content. They are listed in
+// shared memory instead and recomputed a thread each once about 256 are waiting
+// (363k of 249 M coefficients): 0.73 ms against 5.67 ms, with the even/odd passes.
+__global__ void __launch_bounds__(kEncThreads) fdct_kernel(EncLaunch L, uint64_t n_tiles) {
+    __shared__ __align__(16) float s_t[kEncBlocksPerTile * kTileStride];
+    __shared__ __align__(16) int16_t s_out[kEncBlocksPerTile][64];  // blocks in zigzag order
+    __shared__ double s_m64[64];
+    __shared__ unsigned long long s_tie[kTieQueue + 64 * kEncBlocksPerTile];  // block << 6 | v * 8 + u
+    __shared__ uint32_t s_ties, s_frame;
     const int lb = threadIdx.x >> 3, r = threadIdx.x & 7;
-    const uint64_t blk = (uint64_t)blockIdx.x * kEncBlocksPerCta + lb;
-    const bool valid = blk < L.n_blocks;
-    uint32_t tq = 0;
-    if (valid) {
-        const EncFrame &F = L.frames[frame_of_block(L, blk)];
-        const uint64_t i = blk - F.block_base;
-        const uint32_t mcu = (uint32_t)(i / F.bpm), k = (uint32_t)(i % F.bpm);
-        const uint32_t c = F.sched_comp[k];
-        tq = F.comp_tq[c];
-        const uint32_t mx = mcu % F.mcu_cols, my = mcu / F.mcu_cols;
-        const uint32_t x0 = (mx * F.comp_h[c] + F.sched_bx[k]) * 8, y0 = (my * F.comp_v[c] + F.sched_by[k]) * 8;
-        // read_block (encoder.rs:392-402): rows and columns past the plane repeat its last
-        const uint32_t sy = min(y0 + r, F.ph[c] - 1);
-        const uint8_t *row = F.plane[c] + (size_t)sy * F.stride[c];
-        uint8_t px[8];
-        if (x0 + 8 <= F.pw[c] && (reinterpret_cast<uintptr_t>(row + x0) & 7) == 0) {  // one 8-byte load
-            const uint2 w = *reinterpret_cast<const uint2 *>(row + x0);
+    if (threadIdx.x < 64) s_m64[threadIdx.x] = c_m64[threadIdx.x];
+    if (threadIdx.x == 0) s_ties = 0;
+    uint32_t zzcol[2];  // zigzag positions of this thread's column, byte v of the pair
+    {
+        uint32_t w[2] = {0, 0};
 #pragma unroll
-            for (int xx = 0; xx < 8; xx++) px[xx] = (uint8_t)((xx < 4 ? w.x : w.y) >> (8 * (xx & 3)));
-        } else {
+        for (int v = 0; v < 8; v++) w[v >> 2] |= (uint32_t)L.nat2zz[v * 8 + r] << (8 * (v & 3));
+        zzcol[0] = w[0];
+        zzcol[1] = w[1];
+    }
+    for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        if (threadIdx.x == 0) s_frame = frame_of_block(L, tile * kEncBlocksPerTile);
+        __syncthreads();
+        const uint64_t blk = tile * kEncBlocksPerTile + lb;
+        const bool valid = blk < L.n_blocks;
+        float *tb = s_t + lb * kTileStride;
+        float mag = 0.0f;
+        uint32_t tq = 0;
+        if (valid) {  // row pass: t[r][u] = sum_x M[x][u] S[r][x]
+            uint32_t f = s_frame;
+            while (f + 1 < L.n_frames && L.frames[f + 1].block_base <= blk) f++;
+            const BlockSource B = block_source(L.frames[f], blk);
+            tq = B.tq;
+            const uint2 w = source_row(B, r);
+            float s[8], t[8];
 #pragma unroll
-            for (int xx = 0; xx < 8; xx++) px[xx] = row[min(x0 + xx, F.pw[c] - 1)];
+            for (int x = 0; x < 8; x++) {  // 2^23 + sample as a float, then centred
+                const uint32_t b = __byte_perm(x < 4 ? w.x : w.y, 0x4B00u, 0x5440 | (x & 3));
+                s[x] = __uint_as_float(b) - 8388736.0f;
+                mag += fabsf(s[x]);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) t[u] = fdct_row(s, u);
+            reinterpret_cast<float4 *>(tb + r * kRowStride)[0] = make_float4(t[0], t[1], t[2], t[3]);
+            reinterpret_cast<float4 *>(tb + r * kRowStride)[1] = make_float4(t[4], t[5], t[6], t[7]);
         }
 #pragma unroll
-        for (int xx = 0; xx < 8; xx++) {
-            s_raw[lb][r * 8 + xx] = px[xx];
-            s_in[lb][r][xx] = (float)px[xx] - 128.0f;
+        for (int o = 1; o < 8; o <<= 1) mag += __shfl_xor_sync(0xffffffffu, mag, o);
+        __syncwarp();  // a warp's blocks are its own
+        if (valid) {   // column pass of column u = r, quantisation
+            const int u = r;
+            const float *rq = L.rq + tq * 64;
+            const float b = mag * kFdctBound;
+            float t[8];
+#pragma unroll
+            for (int y = 0; y < 8; y++) t[y] = tb[y * kRowStride + u];
+            uint32_t open = 0;
+#pragma unroll
+            for (int v = 0; v < 8; v++) {
+                bool unsure;
+                int k = fdct_round(fdct_column(t, v), b, rq[v * 8 + u], unsure);
+                open |= (unsure ? 1u : 0u) << v;
+                if (v | u) k = min(max(k, -1023), 1023);  // encode_scan (encoder.rs:372-374)
+                s_out[lb][(zzcol[v >> 2] >> (8 * (v & 3))) & 63] = (int16_t)k;
+            }
+            if (open) {
+                uint32_t at = atomicAdd(&s_ties, (uint32_t)__popc(open));
+                for (; open; open &= open - 1) s_tie[at++] = blk << 6 | (uint32_t)((__ffs(open) - 1) * 8 + u);
+            }
+        }
+        __syncwarp();
+        if (valid)  // 16 bytes per thread: the block's 128 bytes in one coalesced row
+            reinterpret_cast<uint4 *>(L.coef + blk * 64)[r] = reinterpret_cast<const uint4 *>(s_out[lb])[r];
+        __syncthreads();  // the list is complete, the coefficients are written
+        const uint32_t n = s_ties;
+        const bool last = tile + gridDim.x >= n_tiles;
+        if (n < (uint32_t)kTieQueue && !(last && n)) continue;
+        for (uint32_t i = threadIdx.x; i < n; i += kEncThreads) {
+            const uint64_t eb = s_tie[i] >> 6;
+            const int nat = (int)(s_tie[i] & 63);
+            const BlockSource B = block_source(L.frames[frame_of_block(L, eb)], eb);
+            uint2 rows[8];
+#pragma unroll
+            for (int y = 0; y < 8; y++) rows[y] = source_row(B, y);
+            int k = exact_coefficient(s_m64, rows, nat & 7, nat >> 3, L.qt[B.tq * 64 + nat]);
+            if (nat) k = min(max(k, -1023), 1023);
+            L.coef[eb * 64 + L.nat2zz[nat]] = (int16_t)k;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (n) atomicAdd(L.exact, (unsigned long long)n);
+            s_ties = 0;
         }
     }
-    __syncthreads();
-    if (valid) {  // row pass: t[r][u] = sum_x M[x][u] S[r][x], and its magnitude sum
-#pragma unroll
-        for (int u = 0; u < 8; u++) fdct_row_pass(s_in[lb][r], u, s_row[lb][r][u], s_mag[lb][r][u]);
-    }
-    __syncthreads();
-    __shared__ __align__(16) int16_t s_out[kEncBlocksPerCta][64];  // the block in zigzag order
-    if (valid) {
-        const int u = r;  // column pass: this thread's column
-        const uint8_t *qt = L.qt + tq * 64;
-        const float *rq = L.rq + tq * 64;
-#pragma unroll
-        for (int v = 0; v < 8; v++) {
-            bool exact;
-            int k = fdct_quantise(&s_row[lb][0][0], &s_mag[lb][0][0], 9, s_raw[lb], u, v, qt[v * 8 + u],
-                                  rq[v * 8 + u], exact);
-            if (exact) atomicAdd(L.exact, 1ull);
-            if (v | u) k = min(max(k, -1023), 1023);  // encode_scan (encoder.rs:372-374)
-            s_out[lb][L.nat2zz[v * 8 + u]] = (int16_t)k;
-        }
-    }
-    __syncthreads();
-    if (valid)  // 16 bytes per thread: the block's 128 bytes in one coalesced row
-        reinterpret_cast<uint4 *>(L.coef + blk * 64)[r] = reinterpret_cast<const uint4 *>(s_out[lb])[r];
 }
 
 // ------------------------------------------------------------- Huffman ---
@@ -681,7 +764,9 @@ int32_t GpuJpegEncoder::encode(EncodeItem *items, size_t n, const JpegEncodeOpti
         L.exact = I.exact.as<unsigned long long>();
         cudaMemsetAsync(L.exact, 0, 8, I.s);
         const unsigned bgrid = (unsigned)((blocks + 255) / 256);
-        fdct_kernel<<<(unsigned)((blocks + kEncBlocksPerCta - 1) / kEncBlocksPerCta), 256, 0, I.s>>>(L);
+        const uint64_t tiles = (blocks + kEncBlocksPerTile - 1) / kEncBlocksPerTile;
+        // one wave of resident CTAs (64 registers: four per SM)
+        fdct_kernel<<<(unsigned)std::min<uint64_t>(tiles, 152 * 4), kEncThreads, 0, I.s>>>(L, tiles);
         bits_kernel<<<bgrid, 256, 0, I.s>>>(L);
         exclusive_scan(L.block_bits, blocks, L.bit_off, I.part.as<uint64_t>(), I.s);
         segment_kernel<<<(segs + 255) / 256, 256, 0, I.s>>>(L);
