@@ -617,7 +617,7 @@ Probe probe_packet(uint32_t codec, const uint8_t *data, size_t len) {
 struct Engine::Impl {
     DevBuf d_in, d_tok, d_blob, d_tile_tok, d_tile_rst, d_rsts, d_results, d_coef, d_dc, d_planes, d_out, d_dvcoef,
         d_modes, d_flags, d_segerr, d_vlc, d_fix, d_slot_item, d_ivs, d_sync, d_spec, d_prefix, d_events, d_ivkey,
-        d_own, d_match, d_redo, d_work, d_scratch, d_scratch_dc, d_blkmap,
+        d_ivpend, d_synclist,
         d_fixtab;  // fixed-point transform weights: MJPEG, DV 8-8, DV 2-4-8 (exact_fixed.h)
     PinBuf h_blob, h_back;
     std::vector<uint32_t> vlc;
@@ -749,6 +749,8 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         std::vector<JBlockRec> brecs;
         std::vector<JComp> comps;
         std::vector<HuffLut> luts;
+        std::vector<uint16_t> lut_sym, lut_sub;  // the chunked decoder's lookups of the same tables
+        std::vector<uint32_t> lut_skip, lut_sub_first;
         std::vector<uint8_t> symbols;
         std::vector<uint16_t> quant;
         std::vector<uint2> items_small, items_big;
@@ -862,15 +864,30 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                         symbols.insert(symbols.end(), key.begin() + 16, key.end() - 1);
                         f = lut_index.emplace(key, (uint32_t)luts.size()).first;
                         luts.push_back(L);
+                        lut_sub_first.push_back((uint32_t)lut_sub.size());
+                        lut_sym.resize(luts.size() << kHuffFastBits);
+                        lut_skip.resize(luts.size() << kHuffFastBits);
+                        build_sym(key.data(), key.size() - 1, s >= 4, lut_sym.data() + ((luts.size() - 1) << kHuffFastBits),
+                                  lut_skip.data() + ((luts.size() - 1) << kHuffFastBits), &lut_sub);
                     }
                     F.lut[s] = f->second;
                 }
+                // the scan's distinct tables, numbered within the frame
+                auto local_table = [](uint32_t *ids, uint32_t *count, uint32_t lut) {
+                    for (uint32_t t = 0; t < *count; t++)
+                        if (ids[t] == lut) return t;
+                    ids[*count] = lut;
+                    return (*count)++;
+                };
                 for (const JSched &e : p.sched) {
                     const JComp &C = p.comps[e.comp];
                     JBlockRec R;
                     memset(&R, 0, sizeof(R));
                     R.dc_lut = F.lut[e.dc];
                     R.ac_lut = F.lut[4 + e.ac];
+                    R.local = e.comp;  // (frames of more than four components take no slices)
+                    if (p.ncomp <= 4)
+                        R.local |= local_table(F.dc_id, &F.n_dc, R.dc_lut) << 8 | local_table(F.ac_id, &F.n_ac, R.ac_lut) << 16;
                     R.comp = e.comp;
                     R.q0 = p.quant[C.q][0];
                     if (p.interleaved) {
@@ -894,7 +911,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                     }
                     F.slice_bits = slice_bits;
                     F.slot_first = (uint32_t)n_slots;
-                    F.slot_count = (uint32_t)((8 * (uint64_t)it.len + slice_bits - 1) / slice_bits + 2 * (uint64_t)p.n_intervals);
+                    F.slot_count = (uint32_t)align_up((8 * (uint64_t)it.len + slice_bits - 1) / slice_bits + p.n_intervals, kSliceThreads);
                     n_slots += F.slot_count;
                 }
                 F.blk_off = blocks;
@@ -1050,8 +1067,9 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
 
         // ------------------------------------------------- device arenas
         I.d_in.ensure(std::max<size_t>(in_bytes, 256));
-        // +64: the entropy decoder's 32-bit word reader may read a few bytes past a frame's tokens
-        I.d_tok.ensure(std::max<size_t>(tok_bytes + 64, 256));
+        // +512: the entropy decoders' 32-bit word readers may read a few bytes, and the lean
+        // decode a block (at most 1,728 bits), past a frame's tokens
+        I.d_tok.ensure(tok_bytes + 512);
         I.d_tile_tok.ensure(std::max<size_t>(tile_first.back() * 4, 256));
         I.d_tile_rst.ensure(std::max<size_t>(tile_first.back() * 4, 256));
         I.d_rsts.ensure(std::max<size_t>(rst_total * sizeof(RstEntry), 256));
@@ -1077,17 +1095,9 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         I.d_events.ensure(std::max<size_t>(n_slots * sizeof(SliceEvent), 256));
         I.d_ivs.ensure(std::max<size_t>(items_small.size() * sizeof(IvInfo), 256));
         I.d_ivkey.ensure(std::max<size_t>(items_small.size() * 8, 256));
-        // levels the speculative decode stores: every block once, plus the unused
-        // tail of each slot's last chunk
-        const uint64_t scratch_blocks = blocks + n_slots * kOwnChunkBlocks;
-        if (scratch_blocks > 0xffffffffull) throw std::runtime_error("batch too large for the chunked entropy decoder");
-        I.d_own.ensure(std::max<size_t>(n_slots * sizeof(SliceOwn), 256));
-        I.d_match.ensure(std::max<size_t>(n_slots * sizeof(SliceMatch), 256));
-        I.d_redo.ensure(std::max<size_t>(n_slots * 4, 256));
-        I.d_work.ensure(std::max<size_t>(n_slots * 4, 256));
-        I.d_scratch.ensure(std::max<size_t>(scratch_blocks * 128, 256));
-        I.d_scratch_dc.ensure(std::max<size_t>(scratch_blocks * 2, 256));
-        I.d_blkmap.ensure(std::max<size_t>(blocks * 4, 256));
+        if (blocks > 0xffffffffull) throw std::runtime_error("batch too large for the chunked entropy decoder");
+        I.d_ivpend.ensure(std::max<size_t>(items_small.size() * 4, 256));
+        I.d_synclist.ensure(std::max<size_t>(2 * n_slots * 4, 256));
 
         uint8_t *d_in = I.d_in.as<uint8_t>();
         auto in_ptr = [&](size_t i) -> const uint8_t * { return items[i].dev_data ? items[i].dev_data : d_in + in_off[i]; };
@@ -1118,6 +1128,8 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         size_t o_jframes = blob.add_vec(jframes), o_jstates = blob.add_vec(jstates),
                o_tile_first = blob.add_vec(tile_first), o_sched = blob.add_vec(sched), o_brec = blob.add_vec(brecs), o_comps = blob.add_vec(comps),
                o_luts = blob.add_vec(luts), o_symbols = blob.add_vec(symbols), o_quant = blob.add_vec(quant);
+        size_t o_sym = blob.add_vec(lut_sym), o_skip = blob.add_vec(lut_skip), o_sub = blob.add_vec(lut_sub),
+               o_subfirst = blob.add_vec(lut_sub_first);
         std::vector<uint2> all_items(items_small);
         all_items.insert(all_items.end(), items_big.begin(), items_big.end());
         size_t o_items = blob.add_vec(all_items), o_ranges = blob.add_vec(ranges), o_idctcta = blob.add_vec(idct_cta), o_itemok = blob.add_vec(item_ok),
@@ -1130,14 +1142,12 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             o_fcta[v] = blob.add_vec(fcta[v]);
         }
 
-        // fixup entries, exact samples, slices redone, slices, short redos listed for
-        // the final decode, slices redone whole
+        // fixup entries, exact samples, slices decoded again, slices, unused, slices decoded
+        // again whole
         uint32_t zero_counters[8] = {};
         size_t o_fixcount = blob.add(zero_counters, sizeof(zero_counters));
-        uint32_t zero_dirty[2 * kSyncPasses] = {};  // changed-exit counts, then work counters
-        size_t o_dirty = blob.add(zero_dirty, sizeof(zero_dirty));
-        uint32_t zero_scratch[4] = {};  // scratch allocation counter
-        size_t o_scratch_next = blob.add(zero_scratch, sizeof(zero_scratch));
+        uint32_t zero_sync[kSyncCounters] = {};
+        size_t o_sync = blob.add(zero_sync, sizeof(zero_sync));
         size_t blob_size = std::max<size_t>(blob.bytes.size(), 256);
         I.d_blob.ensure(blob_size);
         I.h_blob.ensure(blob_size);
@@ -1205,20 +1215,15 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         JL.prefix = I.d_prefix.as<SlicePrefix>();
         JL.events = I.d_events.as<SliceEvent>();
         JL.iv_key = I.d_ivkey.as<unsigned long long>();
-        JL.sync_dirty = reinterpret_cast<uint32_t *>(db + o_dirty);
-        JL.own = I.d_own.as<SliceOwn>();
-        JL.match = I.d_match.as<SliceMatch>();
-        JL.redo = I.d_redo.as<uint32_t>();
-        JL.work = I.d_work.as<uint32_t>();
-        JL.scratch = I.d_scratch.as<int16_t>();
-        JL.scratch_dc = I.d_scratch_dc.as<int16_t>();
-        JL.scratch_blocks = (uint32_t)scratch_blocks;
-        JL.scratch_next = reinterpret_cast<unsigned long long *>(db + o_scratch_next);
-        JL.blk_map = I.d_blkmap.as<uint32_t>();
+        JL.iv_pend = I.d_ivpend.as<uint32_t>();
+        JL.sync_list = I.d_synclist.as<uint32_t>();
+        JL.sync_count = reinterpret_cast<uint32_t *>(db + o_sync);
+        JL.sym = reinterpret_cast<const uint16_t *>(db + o_sym);
+        JL.skip = reinterpret_cast<const uint32_t *>(db + o_skip);
+        JL.sub = reinterpret_cast<const uint16_t *>(db + o_sub);
+        JL.sub_first = reinterpret_cast<const uint32_t *>(db + o_subfirst);
         JL.fixw = I.d_fixtab.as<long long>();
         if (!jframes.empty()) {
-            if (n_slots) MMR_CUDA(cudaMemsetAsync(I.d_redo.ptr, 0, n_slots * 4, s));
-            if (blocks) MMR_CUDA(cudaMemsetAsync(I.d_blkmap.ptr, 0xff, blocks * 4, s));
             launch_jpeg_scan(JL, s);
             MMR_CUDA(record_event(I.ev[2], s, capturing));
             launch_jpeg_slices(JL, s, I.marks, capturing);
@@ -1316,7 +1321,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             // states them so that no change of shape can replay a stale graph
             for (uintptr_t v : {(uintptr_t)jframes.size(), (uintptr_t)tile_first.back(), (uintptr_t)luts.size(),
                                 (uintptr_t)items_small.size(), (uintptr_t)n_items, (uintptr_t)ranges.size(),
-                                (uintptr_t)idct_cta.back(), (uintptr_t)n_slots, (uintptr_t)scratch_blocks,
+                                (uintptr_t)idct_cta.back(), (uintptr_t)n_slots,
                                 (uintptr_t)blocks, (uintptr_t)dframes.size(), (uintptr_t)seg_first.back(),
                                 (uintptr_t)dif_first.back(), (uintptr_t)dv_blocks, (uintptr_t)rgbjobs.size(),
                                 (uintptr_t)rgbcta.back()})
@@ -1328,8 +1333,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             for (const DevBuf *b : {&I.d_in, &I.d_tok, &I.d_blob, &I.d_tile_tok, &I.d_tile_rst, &I.d_rsts,
                                     &I.d_results, &I.d_coef, &I.d_dc, &I.d_planes, &I.d_out, &I.d_dvcoef, &I.d_modes,
                                     &I.d_flags, &I.d_segerr, &I.d_vlc, &I.d_fix, &I.d_slot_item, &I.d_ivs, &I.d_sync,
-                                    &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_own, &I.d_match, &I.d_redo,
-                                    &I.d_work, &I.d_scratch, &I.d_scratch_dc, &I.d_blkmap})
+                                    &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_ivpend, &I.d_synclist})
                 key.push_back((uintptr_t)b->ptr);
             for (size_t i = 0; i < n; i++) {
                 const Item &it = items[i];

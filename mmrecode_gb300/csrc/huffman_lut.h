@@ -5,6 +5,8 @@
 
 #include <string.h>
 
+#include <vector>
+
 #include "plan.h"
 
 namespace mmr {
@@ -90,6 +92,61 @@ inline void build_lut(const uint8_t *key, size_t key_len, uint32_t sym_off, bool
     }
     lut->sym_off = sym_off;
     lut->nsym = (uint32_t)(key_len - 16);
+}
+
+// The chunked decoder's lookups of the same table (plan.h: sym, skip and its blocks of
+// `sub`, appended to *sub; skip only for AC tables). The table is not oversubscribed.
+inline void build_sym(const uint8_t *key, size_t key_len, bool ac, uint16_t *sym, uint32_t *skip,
+                      std::vector<uint16_t> *sub) {
+    constexpr uint32_t FB = kHuffFastBits;
+    for (uint32_t x = 0; x < (1u << FB); x++) sym[x] = (uint16_t)kSymInvalid;
+    const uint8_t *symbols = key + 16;
+    const size_t first_sub = sub->size();
+    uint32_t code = 0, k = 0;
+    for (uint32_t l = 1; l <= 16; l++, code <<= 1) {
+        for (uint32_t i = 0; i < key[l - 1] && k < key_len - 16; i++, code++, k++) {
+            const uint32_t s = symbols[k], size = ac ? s & 15 : s, run = s >> 4;
+            uint32_t adv = ac ? run + 1 : 1;
+            bool ok = size <= (ac ? 10u : 11u);
+            if (ac && size == 0) {
+                ok = run == 0 || run == 15;
+                if (run == 0) adv = kSymEob;
+            }
+            const uint32_t rest = (size << 4) | (adv << 8);
+            if (l <= FB) {
+                const uint16_t e = (uint16_t)(ok ? rest | l : kSymInvalid);
+                const uint32_t at = code << (FB - l), n = 1u << (FB - l);
+                for (uint32_t j = 0; j < n && at + j < (1u << FB); j++) sym[at + j] = e;
+                continue;
+            }
+            const uint32_t prefix = code >> (l - FB);
+            if (prefix >= (1u << FB)) continue;
+            if (sym[prefix] == kSymInvalid) {
+                sym[prefix] = (uint16_t)(kSymEscape | (uint32_t)((sub->size() - first_sub) / kSubEntries));
+                sub->insert(sub->end(), kSubEntries, (uint16_t)kSymInvalid);
+            }
+            uint16_t *block = sub->data() + first_sub + (size_t)(sym[prefix] & 0x7fffu) * kSubEntries;
+            const uint32_t low = (code << (16 - l)) & (kSubEntries - 1), n = 1u << (16 - l);
+            for (uint32_t j = 0; j < n && low + j < kSubEntries; j++)
+                block[low + j] = (uint16_t)(ok ? rest | (l - FB) : kSymInvalid);
+        }
+    }
+    if (!ac) return;
+    for (uint32_t x = 0; x < (1u << FB); x++) {
+        const uint32_t e = sym[x];
+        if (e & kSymEscape) {
+            skip[x] = kSkipEscape;
+            continue;
+        }
+        const uint32_t cl = e & 15, len = cl + ((e >> 4) & 15), adv = e >> 8;
+        uint32_t one = len | adv << 5, two = one;
+        if (adv < kSymEob && len < FB) {
+            const uint32_t e2 = sym[(x << len) & ((1u << FB) - 1)];
+            if (!(e2 & kSymEscape) && (e2 & 15) <= FB - len)  // (it depends on its code bits only)
+                two = (len + (e2 & 15) + ((e2 >> 4) & 15)) | (adv + (e2 >> 8)) << 5;
+        }
+        skip[x] = one | two << 12;
+    }
 }
 
 }  // namespace mmr

@@ -120,17 +120,6 @@ __device__ __forceinline__ void settle_samples(const long long *fixw, const int3
     }
 }
 
-// The 64 levels of block g: in the speculative decode's scratch arena when the
-// block map points there, else in the coefficient arena (any map value past the
-// arena, the reset value included, means in place).
-__device__ __forceinline__ const int16_t *block_levels(const JpegLaunch &L, uint64_t g) {
-    if (L.blk_map) {
-        const uint32_t v = L.blk_map[g];
-        if (v < L.scratch_blocks) return L.scratch + (uint64_t)v * 64;
-    }
-    return L.coef + g * 64;
-}
-
 // Dequantises block g (its levels at `levels`) into fp32 rows q and q+4 of `blk` (the product of an
 // int16 level and an 8-bit quantiser is exact in fp32; the DC is the decoder's
 // dequantised int32, rounded to fp32 like every c in the bound). Returns the

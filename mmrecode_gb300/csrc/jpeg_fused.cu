@@ -90,7 +90,7 @@ __device__ __forceinline__ void fused_tile(const JpegLaunch &L, const FusedLaunc
     }
     __syncthreads();  // q, n
     float *blk = S.f + lb * kFStride;
-    float l1 = valid ? stage_rows(block_levels(L, g), L.dc, g, q, S.q[comp], blk) : 0.0f;
+    float l1 = valid ? stage_rows(L.coef + g * 64, L.dc, g, q, S.q[comp], blk) : 0.0f;
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
     __syncwarp();
@@ -126,7 +126,7 @@ __device__ __forceinline__ void fused_tile(const JpegLaunch &L, const FusedLaunc
             const uint32_t bc = bi < HM * VM ? 0 : bi - HM * VM + 1;
             const uint64_t bg = S.blk[b];
             const uint16_t *Q = L.quant + F.quant_off + comps[bc].q * 64;
-            const int16_t *lv = block_levels(L, bg);
+            const int16_t *lv = L.coef + bg * 64;
             cx[lane] = lane == 0 ? L.dc[bg] : (int32_t)lv[lane] * (int32_t)Q[lane];
             cx[lane + 32] = (int32_t)lv[lane + 32] * (int32_t)Q[lane + 32];
             __syncwarp();

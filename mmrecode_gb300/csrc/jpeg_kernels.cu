@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kIdctThreads, 4) idct_kernel(JpegLaunch L) {
     const bool valid = local < nblk;
     const uint64_t g = R.first + local;
     float *blk = s_f + lb * kIdctStride;
-    float l1 = valid ? stage_rows(block_levels(L, g), L.dc, g, q, s_q, blk) : 0.0f;
+    float l1 = valid ? stage_rows(L.coef + g * 64, L.dc, g, q, s_q, blk) : 0.0f;
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
     __syncwarp();
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(256) idct_fixup_kernel(JpegLaunch L) {
         const JFrame *F = &L.frames[L.ranges[r].frame];
         const JComp *C = &L.comps[F->comp_off + L.ranges[r].comp];
         const uint16_t *Q = L.quant + F->quant_off + C->q * 64;
-        const int16_t *lv = block_levels(L, g);
+        const int16_t *lv = L.coef + g * 64;
         c[lane] = lane == 0 ? L.dc[g] : (int32_t)lv[lane] * (int32_t)Q[lane];
         c[lane + 32] = (int32_t)lv[lane + 32] * (int32_t)Q[lane + 32];
         __syncwarp();

@@ -5,37 +5,44 @@
 // thread per interval leaves a GB300 nearly idle (135 intervals per 1080p frame,
 // one per scan without DRI), so every interval is cut into fixed-size bit slices
 // that decode in parallel. Huffman codes resynchronise: a decode started at a
-// wrong bit or in a wrong coefficient state soon meets the true decode at a
-// symbol boundary with the same state, and from there both are identical.
+// wrong bit or in a wrong state soon meets the true decode at a block boundary
+// with the same position in the MCU, and from there both are identical.
+//
+// A slice owns the blocks that start inside it; its start state is the first block
+// boundary at or past its nominal start (bit position, block of the MCU), which is
+// its predecessor's exit state. Two decodes run over the bits: a lean one that only
+// finds the states (code lengths and coefficient advances, two symbols per lookup,
+// nothing stored), then one from the true states that writes the levels.
 //
 //   slice_plan     per frame: interval token ranges, slice counts, slot -> interval map
-//   slice_spec     every slice decoded from a guessed state spec_lead(S) bits before it
-//                  (the first slice from the true one) up to its end; keeps the state
-//                  at eight checkpoints (64 .. 2048 bits into the slice) and stores
-//                  the levels of the blocks it owns
-//   slice_sync     (kSyncPasses passes; one after a pass that changed nothing returns
-//                  at once) each slice whose start no longer equals its predecessor's
-//                  exit state re-decodes from that state, two symbols per lookup where
-//                  both end before the next checkpoint, until it meets one of its own
-//                  checkpoints (then the rest is known) or its end
-//   slice_fix      per interval, only when the last sync pass still changed a state:
-//                  walks the slices in order until every start equals the previous
-//                  exit. Then slice 0 starts in the true state and each exit is the
-//                  true state at that point, so every start is the true one.
+//   slice_spec     the lean decode of every slice from a guessed state spec_lead(S) bits
+//                  before it (the first slice from the true one) to its exit; keeps the
+//                  first block boundary past each of eight marks (checkpoints)
+//   slice_match    slices whose predecessor's exit is their own first boundary are
+//                  settled; the others are listed
+//   slice_sync     (kSyncPasses passes) listed slices decode again from their
+//                  predecessor's exit until they meet one of their checkpoints (then
+//                  the rest is known) or their end; a changed exit lists the next slice
+//   slice_fix      per interval with slices still listed: walks its slices in order
+//                  until every start equals the previous exit. Then slice 0 starts in
+//                  the true state and each exit is the true state at that point, so
+//                  every start is the true one.
 //   slice_prefix   per interval: block index and DC predictors at each slice start
-//   slice_place    the owned blocks past each slice's match point placed (DC
-//                  predictors, block map); the slots with short work listed
-//   slice_decode   the final decode from true states of what was not placed: quantised
-//                  AC levels, dequantised DC, and each slice's first event (an error,
-//                  or the interval's last block completed)
+//   slice_decode   from the true states: quantised AC levels, dequantised DC, and each
+//                  slice's first event (an error, or the interval's last block completed)
 //   slice_resolve  per interval: the earliest event in stream order becomes the
 //                  interval's result, or the restart-marker check (entropy.rs:111-134)
 //
-// A slice owns the blocks whose DC symbol starts between its start state and its
-// exit state; it decodes the block that straddles its end to completion, and skips
-// (decodes without output) the one straddling its start. Errors are reported only
-// by the owner of the block they occur in, so the earliest reported event is the
-// one the serial decoder stops at.
+// Errors are reported by the owner of the block they occur in, decoded a second time
+// with the reference's checks in its order, so the earliest reported event is the one
+// the serial decoder stops at.
+//
+// Both decodes are bound by the instructions per symbol and by how few lanes of a
+// warp take the same path: a block ends every 10 to 60 symbols, at a different step
+// in each lane, and what happens there (the next tables, the DC difference, 128
+// bytes of levels) costs more than a symbol. So lanes take kSteps symbols (or pairs)
+// at a time without a branch, a lane whose block has ended standing still (its table
+// entry reads as zero), and the block ends are handled once per kSteps.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -47,90 +54,124 @@
 namespace mmr {
 namespace {
 
-__constant__ uint8_t c_slice_zz[64] = MMR_ZIGZAG_INIT;
-
 constexpr unsigned long long kStErr = ~0ull;        // no state: the decode failed before this point
 constexpr unsigned long long kStGuess = ~0ull - 1;  // start not yet derived from the predecessor
-constexpr int kSliceThreads = 128;
-constexpr int kStride = 72;  // int16 per staged block (144 B: conflict-free 16 B rows)
+constexpr int kStride = 72;  // int16 per staged block: 64 levels, and 64.. for what EOB steps store
 constexpr int kKeyBits = 26;
-#ifndef MMR_SPEC_CTAS_PER_SM
-#define MMR_SPEC_CTAS_PER_SM 8
-#endif
+constexpr int kSpecSteps = 4;    // lookups between block-end checks, lean decode
+constexpr int kDecodeSteps = 4;  // and final decode
+constexpr uint32_t kTab = 1u << kHuffFastBits;
+__constant__ uint8_t c_slice_zz[64] = MMR_ZIGZAG_INIT;
+constexpr uint32_t kMostShared = 2;  // DC and AC tables a CTA keeps in shared memory, of each
 
-__device__ __forceinline__ unsigned long long pack_state(unsigned long long p, uint32_t si, uint32_t k) {
-    return (p << 16) | (si << 8) | k;
-}
-
-// Tables of MCU block si.
-struct BlockTabs {
-    const HuffLut *dc;
-    const HuffLut *ac;
-    uint32_t comp;
-};
-
-__device__ __forceinline__ BlockTabs block_tabs(const JpegLaunch &L, const JFrame &F, uint32_t si) {
-    const JBlockRec &R = L.brec[F.sched_off + si];
-    BlockTabs t;
-    t.comp = R.comp;
-    t.dc = L.luts + R.dc_lut;
-    t.ac = L.luts + R.ac_lut;
-    return t;
-}
+__device__ __forceinline__ unsigned long long pack_state(unsigned long long p, uint32_t si) { return (p << 8) | si; }
 
 // Bit offset of checkpoint q from the nominal slice start (UINT32_MAX past the slice).
-__constant__ uint32_t c_slice_marks[kSliceCheckpoints] = {64, 128, 256, 512, 768, 1024, 1536, 2048};
+__constant__ uint32_t c_slice_marks[kSliceCheckpoints] = {0, 64, 128, 256, 512, 768, 1024, 1536};
 
 __device__ __forceinline__ uint32_t mark_of(uint32_t q, uint32_t S) {
     const uint32_t m = q < (uint32_t)kSliceCheckpoints ? c_slice_marks[q] : 0xffffffffu;
     return m < S ? m : 0xffffffffu;
 }
 
-__device__ __forceinline__ void add_dc(int32_t (&dc)[4], uint32_t comp, int32_t v) {
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-        if (comp == (uint32_t)c) dc[c] += v;
-}
-
-__device__ __forceinline__ void add_dc_at(int32_t *dc, uint32_t comp, int32_t v) { dc[comp] += v; }
-
 struct SliceRef {
     uint32_t item, j;
     IvInfo v;
-    const JFrame *F;
     bool last;
 };
 
 __device__ __forceinline__ bool slice_ref(const JpegLaunch &L, uint32_t slot, SliceRef &s) {
-    if (slot >= L.n_slots) return false;
     s.item = L.slot_item[slot];
     if (s.item == 0xffffffffu) return false;
     s.v = L.ivs[s.item];
     s.j = slot - s.v.slot_first;
-    s.F = L.frames + L.items[s.item].x;
     s.last = s.j + 1 == s.v.n_slices;
     return true;
-}
-
-// Nominal start (bits from the interval's start) and length of a slice that is
-// not its interval's last.
-__device__ __forceinline__ void slice_span(const SliceRef &s, uint32_t S, unsigned long long &start, uint32_t &len) {
-    start = (unsigned long long)s.j * S;
-    len = S;
-    if (s.v.tail && s.j + 2 == s.v.n_slices)  // the next is the split-off last slice
-        len = (uint32_t)((unsigned long long)(s.v.barrier - s.v.start) * 8 - s.v.tail - start);
 }
 
 __device__ __forceinline__ uint32_t clamp_u32(unsigned long long x) {
     return x > 0xffffffffull ? 0xffffffffu : (uint32_t)x;
 }
 
+// ------------------------------------------------------------- reader ---
+//
+// The window is the 32 bits at offset `off` of two token words; the word after
+// them is loaded one refill ahead. A symbol takes at most 27 bits, a pair 21.
+
+struct Window {
+    const uint32_t *next;  // the word after pf
+    uint32_t w0, w1, pf;   // pf as stored (little-endian)
+    uint32_t off;          // 0..31
+};
+
+__device__ __forceinline__ void window_init(Window &r, const uint8_t *tok, unsigned long long bit) {
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(tok) + (bit >> 5);
+    r.w0 = bswap32(__ldg(w));
+    r.w1 = bswap32(__ldg(w + 1));
+    r.pf = __ldg(w + 2);
+    r.next = w + 3;
+    r.off = (uint32_t)bit & 31;
+}
+
+__device__ __forceinline__ uint32_t window_bits(const Window &r) { return __funnelshift_l(r.w1, r.w0, r.off); }
+
+__device__ __forceinline__ void window_take(Window &r, uint32_t n) {
+    r.off += n;
+    if (r.off >= 32) {
+        r.off -= 32;
+        r.w0 = r.w1;
+        r.w1 = bswap32(r.pf);
+        r.pf = __ldg(r.next);
+        r.next++;
+    }
+}
+
+// Bits taken since the reader stood at bit `bit0` of the token stream at `tok`
+// (modulo 2^32: a slice and its lead stay far below).
+__device__ __forceinline__ uint32_t window_pos(const Window &r, const uint8_t *tok, uint32_t bit0) {
+    return (uint32_t)(r.next - 3 - reinterpret_cast<const uint32_t *>(tok)) * 32 + r.off - bit0;
+}
+
+// The signed value of `size` magnitude bits at the top of t (receive_extend,
+// entropy.rs:168-182); 0 for size 0.
+__device__ __forceinline__ int32_t extend(uint32_t t, uint32_t size) {
+    const uint32_t neg = (uint32_t)((int32_t)~t >> 31);
+    uint32_t w;
+    asm("shr.u32 %0, %1, %2;" : "=r"(w) : "r"(t ^ neg), "r"(32 - size));  // (a shift by 32 gives 0)
+    return (int32_t)((w ^ neg) - neg);
+}
+
+// A code of more than kHuffFastBits bits: its entry (code bits past the first 11,
+// magnitude size, advance), or the invalid marker.
+__device__ __noinline__ uint32_t sub_entry(const JpegLaunch &L, uint32_t lut, uint32_t e, uint32_t window) {
+    if (e == kSymInvalid) return e;
+    return __ldg(L.sub + __ldg(L.sub_first + lut) + (e & 0x7fffu) * kSubEntries + ((window >> 16) & (kSubEntries - 1)));
+}
+
+// --------------------------------------------------------------- tables ---
+//
+// Lookup tables of the CTA's frame. Frames with at most two DC and two AC tables
+// (all but exotic ones) keep them in shared memory, where 32 lanes' lookups cost a
+// few bank conflicts instead of as many L1 lines; offsets count table entries from
+// s_tab. Others read the batch's tables.
+
+// What the lean decode needs of an MCU block: its component and tables (the frame's
+// own numbers where they are in shared memory, else the batch's).
+struct BlockTabs {
+    uint32_t comp, dc, ac;
+};
+
 // ------------------------------------------------------------------ plan ---
 
-__global__ void slice_plan_kernel(JpegLaunch L) {
-    const uint32_t f = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const uint32_t lane = threadIdx.x & 31;
-    if (f >= L.n_frames) return;
+constexpr int kPlanThreads = 512;
+constexpr int kPlanPer = 8;  // consecutive intervals per thread and step
+
+// CTA per frame: kPlanThreads * kPlanPer intervals per step, one prefix sum each (a
+// warp per frame with 32 intervals per step took 6.0 ms of the 17.1 ms of a mixed
+// batch whose 4:4:4 frames have up to 32k intervals).
+__global__ void __launch_bounds__(kPlanThreads) slice_plan_kernel(JpegLaunch L) {
+    __shared__ uint32_t s_warp[kPlanThreads / 32];
+    const uint32_t f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const JFrame &F = L.frames[f];
     if (!F.decode || F.ncomp > 4) return;
     const JState &st = L.states[f];
@@ -141,280 +182,344 @@ __global__ void slice_plan_kernel(JpegLaunch L) {
     const RstEntry *rst = L.rsts + F.rst_off;
     const uint32_t S = F.slice_bits;
     uint32_t used = 0;
-    for (uint32_t c = 0; c < n_int; c += 32) {
-        const uint32_t iv = c + lane;
-        uint32_t n_s = 0, start = 0, barrier = 0, flags = 0, blocks = 0, tail = 0;
-        if (iv < n_int) {
-            bool dec = scan_ok;
-            if (iv == 0) start = 0;
-            else if (iv - 1 < n_rst) start = rst[iv - 1].tok;
-            else dec = false;  // no RST precedes it: an earlier interval fails its restart check
-            if (dec) {
-                flags = iv < n_rst ? 1u : 0u;
-                barrier = flags ? rst[iv].tok : n_tok;
-                const unsigned long long lbits = (unsigned long long)(barrier - start) * 8;
-                n_s = (uint32_t)max(1ull, (lbits + S - 1) / S);
-                if (lbits - (unsigned long long)(n_s - 1) * S > kSliceTail) {  // split the end off
-                    n_s++;
-                    tail = kSliceTail;
-                }
-                const uint32_t mcu0 = iv * F.ri, mcu1 = min(mcu0 + F.ri, F.total_mcus);
-                blocks = (mcu1 - mcu0) * F.sched_len;
+    for (uint32_t c = 0; c < n_int; c += kPlanThreads * kPlanPer) {
+        const uint32_t iv0 = c + tid * kPlanPer;
+        uint32_t start[kPlanPer], barrier[kPlanPer], n_s[kPlanPer], sum = 0;
+        uint32_t prev = iv0 == 0 ? 0 : iv0 - 1 < n_rst ? rst[iv0 - 1].tok : 0xffffffffu;
+#pragma unroll
+        for (int i = 0; i < kPlanPer; i++) {
+            const uint32_t iv = iv0 + i;
+            n_s[i] = 0;
+            start[i] = prev;
+            barrier[i] = prev;
+            const uint32_t end = iv < n_rst ? rst[iv].tok : n_tok;
+            // an interval that no RST precedes: an earlier one fails its restart check
+            if (iv < n_int && scan_ok && prev != 0xffffffffu) {
+                barrier[i] = end;
+                n_s[i] = max(1u, (uint32_t)(((unsigned long long)(end - prev) * 8 + S - 1) / S));
             }
+            prev = iv < n_rst ? end : 0xffffffffu;
+            sum += n_s[i];
         }
-        uint32_t incl = n_s;
+        uint32_t incl = sum;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= (uint32_t)d) incl += o;
         }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        uint32_t first = used + incl - n_s;
-        if (used + total > F.slot_count) {  // cannot happen: slot_count bounds the token count
-            n_s = 0;
-            first = used;
+        __syncthreads();  // (the last step's sums are read)
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t first = used + incl - sum, total = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kPlanThreads / 32; w++) {
+            if (w < warp) first += s_warp[w];
+            total += s_warp[w];
         }
-        if (iv < n_int) {
-            IvInfo v;
-            v.start = start;
-            v.barrier = barrier;
-            v.slot_first = F.slot_first + first;
-            v.n_slices = n_s;
-            v.blocks = blocks;
-            v.flags = flags;
-            v.tail = tail;
-            v.pad = 0;
-            L.ivs[F.item_base + iv] = v;
-            L.iv_key[F.item_base + iv] = ~0ull;
+        const bool fits = used + total <= F.slot_count;  // always: slot_count bounds the token count
+#pragma unroll
+        for (int i = 0; i < kPlanPer; i++) {
+            const uint32_t iv = iv0 + i;
+            if (!fits) n_s[i] = 0;
+            if (iv < n_int) {
+                const uint32_t mcu0 = iv * F.ri, mcu1 = min(mcu0 + F.ri, F.total_mcus);
+                IvInfo v;
+                v.start = start[i];
+                v.barrier = barrier[i];
+                v.slot_first = F.slot_first + first;
+                v.n_slices = n_s[i];
+                v.blocks = n_s[i] ? (mcu1 - mcu0) * F.sched_len : 0;
+                v.flags = n_s[i] && iv < n_rst ? 1u : 0u;
+                v.frame = f;
+                v.pad = 0;
+                L.ivs[F.item_base + iv] = v;
+                L.iv_key[F.item_base + iv] = ~0ull;
+                L.iv_pend[F.item_base + iv] = 0xffffffffu;
+            }
+            const bool own = n_s[i] <= 8;
+            if (own)
+                for (uint32_t x = 0; x < n_s[i]; x++) L.slot_item[F.slot_first + first + x] = F.item_base + iv;
+            for (uint32_t m = __ballot_sync(0xffffffffu, !own); m; m &= m - 1) {  // the warp fills long ones
+                const int src = __ffs(m) - 1;
+                const uint32_t nt = __shfl_sync(0xffffffffu, n_s[i], src), ft = __shfl_sync(0xffffffffu, first, src);
+                const uint32_t it = __shfl_sync(0xffffffffu, F.item_base + iv, src);
+                for (uint32_t x = lane; x < nt; x += 32) L.slot_item[F.slot_first + ft + x] = it;
+            }
+            first += n_s[i];
         }
-        for (uint32_t t = 0; t < 32 && c + t < n_int; t++) {
-            const uint32_t nt = __shfl_sync(0xffffffffu, n_s, t), ft = __shfl_sync(0xffffffffu, first, t);
-            for (uint32_t x = lane; x < nt; x += 32) L.slot_item[F.slot_first + ft + x] = F.item_base + c + t;
-        }
-        if (used + total <= F.slot_count) used += total;
+        if (fits) used += total;
     }
-    for (uint32_t x = used + lane; x < F.slot_count; x += 32) L.slot_item[F.slot_first + x] = 0xffffffffu;
+    for (uint32_t x = used + tid; x < F.slot_count; x += kPlanThreads) L.slot_item[F.slot_first + x] = 0xffffffffu;
 }
 
-// ------------------------------------------------------ speculative pass ---
+// ------------------------------------------------------------ lean decode ---
 
-// Stores the staged block as owned block n of the slot (allocating a scratch
-// chunk at each chunk's first block) and clears the stage; false when the slot's
-// chunks or the arena are exhausted.
-__device__ __forceinline__ bool store_owned(const JpegLaunch &L, uint32_t slot, uint32_t n, uint32_t &chunk_base,
-                                            int4 *stage4, int32_t dc_diff) {
-    const uint32_t c = n / kOwnChunkBlocks, i = n % kOwnChunkBlocks;
-    if (i == 0) {
-        if (c >= (uint32_t)kOwnChunks) return false;
-        const unsigned long long first = atomicAdd(L.scratch_next, (unsigned long long)kOwnChunkBlocks);
-        if (first + kOwnChunkBlocks > L.scratch_blocks) return false;
-        chunk_base = (uint32_t)first;
-        L.own[slot].chunk[c] = chunk_base;
+// Tables as the lean decode reads them: kShared from the CTA's copies, else the batch's.
+template <bool kShared>
+struct LeanTabs {
+    const uint32_t *skip;  // AC: one or two symbols per entry (huffman_lut.h)
+    const uint16_t *sym;   // DC
+    const uint32_t *local;   // kShared: per MCU block JBlockRec::local
+    const uint32_t *ids;     // kShared: batch index of each of the frame's tables, DC then AC
+    const JBlockRec *recs;   // the frame's records
+    __device__ __forceinline__ uint32_t skip_at(uint32_t i) const { return kShared ? skip[i] : __ldg(skip + i); }
+    __device__ __forceinline__ uint32_t sym_at(uint32_t i) const { return kShared ? sym[i] : __ldg(sym + i); }
+    __device__ __forceinline__ uint32_t dc_lut(uint32_t t) const { return kShared ? ids[t] : t; }
+    __device__ __forceinline__ uint32_t ac_lut(uint32_t t) const { return kShared ? ids[kMostShared + t] : t; }
+    __device__ __forceinline__ BlockTabs block(uint32_t si) const {
+        if (kShared) {
+            const uint32_t p = local[si];
+            return BlockTabs{p & 0xff, (p >> 8) & 0xff, p >> 16};
+        }
+        const JBlockRec &R = recs[si];
+        return BlockTabs{R.comp, R.dc_lut, R.ac_lut};
     }
-    int4 *dst = reinterpret_cast<int4 *>(L.scratch + (uint64_t)(chunk_base + i) * 64);
+};
+
+// State of a lean decode between block boundaries.
+struct Lean {
+    Window r;
+    int k;           // next coefficient; 64 or 96 and more: the block is complete, 65..95: invalid
+    uint32_t si;     // block of the MCU
+    uint32_t tab;    // its AC table's first entry
+    uint32_t blocks; // blocks started
+};
+
+// kSpecSteps lookups (none for a lane whose block has ended).
+template <bool kShared>
+__device__ __forceinline__ void lean_steps(const JpegLaunch &L, const LeanTabs<kShared> &T, Lean &s) {
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-        dst[q] = stage4[q];
-        stage4[q] = make_int4(0, 0, 0, 0);
+    for (int u = 0; u < kSpecSteps; u++) {
+        const uint32_t w = window_bits(s.r);
+        uint32_t e = 0;
+        if (s.k < 64) e = T.skip_at(s.tab + (w >> (32 - kHuffFastBits)));
+        if (e & kSkipEscape) {
+            const uint32_t lut = T.ac_lut(s.tab / kTab);
+            const uint32_t x = sub_entry(L, lut, __ldg(L.sym + lut * kTab + (w >> (32 - kHuffFastBits))), w);
+            if (x & kSymEscape) {
+                e = 0;
+                s.k = 80;
+            } else {
+                const uint32_t one = (kHuffFastBits + (x & 15) + ((x >> 4) & 15)) | ((x >> 8) & 127) << 5;
+                e = one | one << 12;
+            }
+        }
+        if (s.k + (int)((e >> 5) & 127) < 64) e >>= 12;  // the pair: its first symbol leaves the block open
+        window_take(s.r, e & 31);
+        s.k += (int)((e >> 5) & 127);
     }
-    L.scratch_dc[chunk_base + i] = (int16_t)dc_diff;
+}
+
+// The DC symbol at a block boundary: counts the block, adds its difference to
+// dc[component], and leaves the decode at its first AC symbol. False when invalid.
+template <bool kShared>
+__device__ __forceinline__ bool lean_dc(const JpegLaunch &L, const LeanTabs<kShared> &T, Lean &s, int32_t *dc) {
+    const BlockTabs b = T.block(s.si);
+    s.blocks++;
+    uint32_t w = window_bits(s.r);
+    uint32_t e = T.sym_at(b.dc * kTab + (w >> (32 - kHuffFastBits)));
+    if (e & kSymEscape) {
+        e = sub_entry(L, T.dc_lut(b.dc), e, w);
+        if (e & kSymEscape) return false;
+        window_take(s.r, kHuffFastBits);
+        w = window_bits(s.r);
+    }
+    const uint32_t cl = e & 15, size = (e >> 4) & 15;
+    dc[b.comp] += extend(w << cl, size);
+    window_take(s.r, cl + size);
+    s.tab = b.ac * kTab;
+    s.k = 1;
     return true;
 }
 
-// Besides the exit state, checkpoints and counts, the speculative decode stores
-// the levels of the blocks it owns along its own path (SliceOwn): blocks whose DC
-// symbol starts at or past the slice start and before the slice end, the last
-// one decoded to completion past the end.
-// Table indices of MCU block si (fewer live registers than pointers).
-struct TabIdx {
-    uint32_t dc, ac, comp;
-};
+__device__ __forceinline__ bool lean_invalid(const Lean &s) { return s.k > 64 && s.k < 96; }
 
-__device__ __forceinline__ TabIdx tab_idx(const JpegLaunch &L, const JFrame &F, uint32_t si) {
-    const JBlockRec &R = L.brec[F.sched_off + si];
-    return TabIdx{R.dc_lut, R.ac_lut, R.comp};
-}
-
-// 8 CTAs per SM (64 registers): the pass is latency-bound, so resident warps are
-// what it runs on (at 9 it spills and runs slower)
-__global__ void __launch_bounds__(kSliceThreads, MMR_SPEC_CTAS_PER_SM) slice_spec_kernel(JpegLaunch L) {
-    __shared__ __align__(16) int16_t s_stage[kSliceThreads * kStride];
-    __shared__ uint8_t s_zz[64];
-    // per thread: DC sums per component, the scratch chunk and the end of the last
-    // stored block, touched once per block (kept out of registers for occupancy)
-    __shared__ int32_t s_dc[kSliceThreads][4];
-    __shared__ uint32_t s_chunk[kSliceThreads], s_end[kSliceThreads];
-    int16_t *stage = s_stage + threadIdx.x * kStride;
-    int4 *stage4 = reinterpret_cast<int4 *>(stage);
-#pragma unroll
-    for (int q = 0; q < 8; q++) stage4[q] = make_int4(0, 0, 0, 0);
-    if (threadIdx.x < 64) s_zz[threadIdx.x] = c_slice_zz[threadIdx.x];
-    __syncthreads();
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    SliceRef s;
-    if (!slice_ref(L, slot, s)) return;
+// Speculative decode of one slice (not its interval's last).
+template <bool kShared>
+__device__ __forceinline__ void spec_slice(const JpegLaunch &L, const LeanTabs<kShared> &T, const JFrame &F, uint32_t slot,
+                           const SliceRef &s, int32_t *dc) {
     const bool guess = s.j != 0;
-    SliceSync out;
-    out.start = guess ? kStGuess : pack_state(0, 0, 0);
-    out.exit = kStErr;
-    out.blocks = 0;
-    out.pad = 0;
-#pragma unroll
-    for (int c = 0; c < 4; c++) out.dc[c] = 0;
-    {
-        SliceMatch m;  // a first slice starts true; the sync pass finds the others' point
-        m.q = guess ? kMatchNone : kMatchStart;
-        m.blocks = 0;
-#pragma unroll
-        for (int c = 0; c < 4; c++) m.dc[c] = 0;
-        L.match[slot] = m;
-    }
-    if (s.last) {  // nothing reads the last slice's exit or counts; the decode pass redoes it
-        L.sync[slot] = out;
-        L.own[slot].n = 0;
-        L.own[slot].ok = 0;
-        return;
-    }
-    const JFrame &F = *s.F;
-    unsigned long long nominal;
-    uint32_t S;  // this slice's length
-    slice_span(s, F.slice_bits, nominal, S);
-    // a guessed decode starts up to spec_lead(S) bits early; positions below are from p0
-    const uint32_t lead = guess ? (uint32_t)min((unsigned long long)spec_lead(F.slice_bits), nominal) : 0;
-    const unsigned long long p0 = nominal - lead;
+    const uint32_t S = F.slice_bits;
+    const unsigned long long nominal = (unsigned long long)s.j * S;
+    const uint32_t lead = guess ? (uint32_t)min((unsigned long long)spec_lead(S), nominal) : 0;
+    const unsigned long long p0 = nominal - lead;  // positions below are from p0
     const uint32_t end = S + lead;
-    auto mark_at = [&](uint32_t qq) {
-        const uint32_t m = mark_of(qq, S);
-        return m == 0xffffffffu ? m : m + lead;
-    };
-    const unsigned long long lbits = (unsigned long long)(s.v.barrier - s.v.start) * 8;
-    const uint32_t lim = clamp_u32(lbits - p0);  // bits before the barrier, from p0
-    Bits r;
-    bits_init(r, F.tok, (uint64_t)s.v.start * 8 + p0, 0);
-    int k = guess ? 1 : 0;
-    uint32_t si = 0;
-    TabIdx tb = tab_idx(L, F, si);
-    uint32_t blocks = 0;
-    int32_t *dc = s_dc[threadIdx.x];
+    const uint32_t lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - p0);
+    const unsigned long long base = (unsigned long long)s.v.start * 8 + p0;
+    const uint32_t bit0 = (uint32_t)base;
+    Lean d;
+    window_init(d.r, F.tok, base);
+    d.blocks = 0;
+    if (guess) {
+        d.k = 1;
+        d.si = 0;
+        d.tab = T.block(0).ac * kTab;
+    } else {
+        d.k = 64;
+        d.si = F.sched_len - 1;
+        d.tab = 0;
+    }
 #pragma unroll
     for (int c = 0; c < 4; c++) dc[c] = 0;
-    int32_t dcv = 0;  // DC difference of the block in progress (0 before its DC symbol)
-    uint32_t q = 0, recorded = 0;
-    uint32_t next_mark = guess ? mark_at(0) : 0xffffffffu;
+    SliceSpec *sp = L.spec + slot;
+    uint32_t q = 0, valid = 0, next_mark = lead;
     unsigned long long exit_state = kStErr;
-    bool entered = false;  // at or past the slice start
-    bool own_blk = false;  // the block in progress is owned
-    bool own_ok = true;    // the owned blocks so far are stored
-    uint32_t own_n = 0;
-    uint32_t &chunk_base = s_chunk[threadIdx.x];
-    uint32_t &own_end = s_end[threadIdx.x];  // position (from p0) after the last stored one
-    chunk_base = 0;
-    own_end = 0;
     for (;;) {
-        const uint32_t pr = r.used;
-        if (pr >= end) {
-            exit_state = pack_state(p0 + pr, si, k);
-            break;
-        }
-        entered |= pr >= lead;
-        if (pr >= next_mark) {
-            while (pr >= mark_at(q)) {
-                SlicePoint cp;
-                cp.state = pack_state(p0 + pr, si, k);
-                cp.blocks = blocks;
-                cp.own_next = own_n + (own_blk && k != 0 ? 1u : 0u);
+        if (d.k >= 64) {
+            const uint32_t pos = window_pos(d.r, F.tok, bit0);
+            bool ok = !lean_invalid(d);
+            if (ok) {
+                d.si = d.si + 1 == F.sched_len ? 0 : d.si + 1;
+                if (pos > lim) break;  // past the interval's end: exit_state stays kStErr
+                if (pos >= next_mark) {
+                    if (pos >= end) {
+                        exit_state = pack_state(p0 + pos, d.si);
+                        break;
+                    }
+                    SlicePoint cp;
+                    cp.state = pack_state(p0 + pos, d.si);
+                    cp.blocks = d.blocks;
+                    cp.pad = 0;
 #pragma unroll
-                for (int c = 0; c < 4; c++) cp.dc[c] = dc[c] + (tb.comp == (uint32_t)c ? dcv : 0);
-                L.spec[slot].cp[q] = cp;
-                recorded |= 1u << q;
-                q++;
+                    for (int c = 0; c < 4; c++) cp.dc[c] = dc[c];
+                    do {
+                        if (guess) {
+                            sp->cp[q] = cp;
+                            valid |= 1u << q;
+                        }
+                        q++;
+                        const uint32_t m = mark_of(q, S);
+                        next_mark = m == 0xffffffffu ? end : m + lead;
+                    } while (pos >= next_mark && next_mark < end);
+                }
+                ok = lean_dc(L, T, d, dc);
             }
-            next_mark = mark_at(q);
-        }
-        const int k0 = k;
-        blocks += k0 == 0;
-        own_blk = k0 == 0 ? entered : own_blk;
-        int32_t val;
-        uint16_t err;
-        uint32_t eb;
-        if (!decode_symbol(r, lim - pr, L.luts + (k0 == 0 ? tb.dc : tb.ac), L.symbols, k, val, err, eb)) {
-            if (!guess || err == kBarrierErr) break;  // exit_state stays kStErr
-            // A decode from a guessed state met an invalid symbol: start again one bit
-            // later; what came before cannot lead to the exit, so its checkpoints go,
-            // and the owned blocks start again too (this path was not the true one).
-            for (uint32_t x = 0; x < (uint32_t)kSliceCheckpoints; x++)
-                if (recorded & (1u << x)) L.spec[slot].cp[x].state = kStErr;
-            recorded = 0;
-            blocks = 0;
+            if (!ok) {
+                if (!guess || pos >= min(lim, end)) break;
+                // A decode from a guessed state met an invalid symbol: start again one bit
+                // later; what came before cannot lead to the exit, so its checkpoints go.
+                valid = 0;
+                d.blocks = 0;
 #pragma unroll
-            for (int c = 0; c < 4; c++) dc[c] = 0;
-            dcv = 0;
-            k = 1;
-            si = 0;
-            tb = tab_idx(L, F, si);
-            // (the stage may hold a partial block, or one whose store failed)
-#pragma unroll
-            for (int x = 0; x < 8; x++) stage4[x] = make_int4(0, 0, 0, 0);
-            own_blk = false;
-            own_ok = true;
-            own_n = 0;
-            bits_init(r, F.tok, (uint64_t)L.ivs[s.item].start * 8 + p0 + pr + 1, pr + 1);
-            continue;
-        }
-        if (own_blk && own_ok) stage[s_zz[k - 1]] = (int16_t)val;
-        dcv = k0 == 0 ? val : dcv;
-        if (k < 64) continue;
-        if (own_blk && own_ok) {  // block complete
-            own_ok = store_owned(L, slot, own_n, chunk_base, stage4, dcv);
-            own_n++;
-            own_end = r.used;
-        }
-        own_blk = false;
-        add_dc_at(dc, tb.comp, dcv);
-        dcv = 0;
-        k = 0;
-        si = si + 1 == F.sched_len ? 0 : si + 1;
-        tb = tab_idx(L, F, si);
-    }
-    // the owned block straddling the slice end is decoded to completion
-    if (exit_state != kStErr && own_blk && own_ok) {
-        while (k < 64) {
-            int32_t val;
-            uint16_t err;
-            uint32_t eb;
-            if (!decode_symbol(r, lim - r.used, L.luts + tb.ac, L.symbols, k, val, err, eb)) {
-                own_ok = false;
-                break;
+                for (int c = 0; c < 4; c++) dc[c] = 0;
+                window_init(d.r, F.tok, base + pos + 1);
+                d.k = 1;
+                d.si = 0;
+                d.tab = T.block(0).ac * kTab;
             }
-            stage[s_zz[k - 1]] = (int16_t)val;
         }
-        if (own_ok) {
-            own_ok = store_owned(L, slot, own_n, chunk_base, stage4, dcv);
-            own_n++;
-            own_end = r.used;
-        }
+        lean_steps(L, T, d);
     }
-    SliceOwn *own = L.own + slot;
-    own->last_end = p0 + own_end;
-    own->n = own_n;
-    own->ok = own_ok && exit_state != kStErr;
-    add_dc_at(dc, tb.comp, dcv);  // the block in progress is counted, with its DC if decoded
-    if (guess) {
-        for (uint32_t x = 0; x < (uint32_t)kSliceCheckpoints; x++)
-            if (!(recorded & (1u << x))) L.spec[slot].cp[x].state = kStErr;
-        SlicePoint e;
-        e.state = exit_state;
-        e.blocks = blocks;
-        e.own_next = own_n;
-#pragma unroll
-        for (int c = 0; c < 4; c++) e.dc[c] = dc[c];
-        L.spec[slot].exit = e;
-    }
+    SliceSync out;
+    out.start = guess ? kStGuess : pack_state(0, 0);
     out.exit = exit_state;
-    out.blocks = blocks;
+    out.blocks = d.blocks;
+    out.q = kMatchStart;
 #pragma unroll
     for (int c = 0; c < 4; c++) out.dc[c] = dc[c];
     L.sync[slot] = out;
+    if (guess) {
+        SlicePoint e;
+        e.state = exit_state;
+        e.blocks = d.blocks;
+        e.pad = valid;
+#pragma unroll
+        for (int c = 0; c < 4; c++) e.dc[c] = dc[c];
+        sp->exit = e;
+    }
+}
+
+// Shared copies of the lean decode's tables: [kMostShared] DC (16-bit entries), then
+// [kMostShared] AC pair tables, of the CTA's frame.
+struct LeanSmem {
+    uint32_t skip[kMostShared * kTab];
+    uint16_t sym[kMostShared * kTab];
+    uint32_t local[kMaxSched];
+    uint32_t ids[2 * kMostShared];
+    int32_t dc[kSliceThreads][4];
+};
+
+__device__ __forceinline__ void copy16(void *dst, const void *src, uint32_t bytes) {
+    for (uint32_t i = threadIdx.x; i < bytes / 16; i += kSliceThreads)
+        reinterpret_cast<uint4 *>(dst)[i] = __ldg(reinterpret_cast<const uint4 *>(src) + i);
+}
+
+__global__ void __launch_bounds__(kSliceThreads) slice_spec_kernel(JpegLaunch L) {
+    __shared__ __align__(16) LeanSmem S;
+    const uint32_t slot = blockIdx.x * kSliceThreads + threadIdx.x;
+    SliceRef s;
+    const bool used = slice_ref(L, slot, s);
+    // the first slot of a CTA is used if any is, and all are of one frame
+    const bool work = used && !s.last;
+    if (used && s.last && s.j == 0) {  // (the decode pass takes a last slice's start from its predecessor)
+        SliceSync y;
+        y.start = y.exit = pack_state(0, 0);
+        y.blocks = 0;
+        y.q = kMatchStart;
+#pragma unroll
+        for (int c = 0; c < 4; c++) y.dc[c] = 0;
+        L.sync[slot] = y;
+    }
+    if (!__syncthreads_or(work)) return;
+    const JFrame &F = L.frames[L.ivs[L.slot_item[blockIdx.x * kSliceThreads]].frame];
+    const bool small = F.n_dc <= kMostShared && F.n_ac <= kMostShared;
+    if (small) {
+        for (uint32_t i = threadIdx.x; i < F.sched_len; i += kSliceThreads) S.local[i] = L.brec[F.sched_off + i].local;
+        for (uint32_t t = 0; t < F.n_dc; t++) copy16(S.sym + t * kTab, L.sym + F.dc_id[t] * kTab, 2 * kTab);
+        for (uint32_t t = 0; t < F.n_ac; t++) copy16(S.skip + t * kTab, L.skip + F.ac_id[t] * kTab, 4 * kTab);
+        if (threadIdx.x < kMostShared) {
+            S.ids[threadIdx.x] = F.dc_id[threadIdx.x];
+            S.ids[kMostShared + threadIdx.x] = F.ac_id[threadIdx.x];
+        }
+    }
+    __syncthreads();
+    if (!work) return;
+    int32_t *dc = S.dc[threadIdx.x];
+    if (small) {
+        const LeanTabs<true> T{S.skip, S.sym, S.local, S.ids, nullptr};
+        spec_slice(L, T, F, slot, s, dc);
+    } else {
+        const LeanTabs<false> T{L.skip, L.sym, nullptr, nullptr, L.brec + F.sched_off};
+        spec_slice(L, T, F, slot, s, dc);
+    }
+}
+
+// ----------------------------------------------------------------- match ---
+
+// Settles a slice whose true start is its speculative decode's boundary at
+// checkpoint q, given what lies before it: blocks and DC differences.
+__device__ __forceinline__ void settle(const JpegLaunch &L, uint32_t slot, unsigned long long from, uint32_t q,
+                                       uint32_t blocks, const int32_t *dc) {
+    const SliceSpec *sp = L.spec + slot;
+    const SlicePoint cp = sp->cp[q], e = sp->exit;
+    SliceSync y;
+    y.start = from;
+    y.exit = e.state;
+    y.blocks = blocks + e.blocks - cp.blocks;
+    y.q = q;
+#pragma unroll
+    for (int c = 0; c < 4; c++) y.dc[c] = dc[c] + e.dc[c] - cp.dc[c];
+    L.sync[slot] = y;
+}
+
+// Thread per slice: the predecessor's exit is the slice's own first boundary for
+// most; the others go to the first list of the sync passes.
+__global__ void __launch_bounds__(kSliceThreads) slice_match_kernel(JpegLaunch L) {
+    const uint32_t slot = blockIdx.x * kSliceThreads + threadIdx.x, lane = threadIdx.x & 31;
+    SliceRef s;
+    bool list = false;
+    if (slice_ref(L, slot, s) && s.j != 0 && !s.last) {
+        const unsigned long long from = L.sync[slot - 1].exit;
+        const int32_t none[4] = {0, 0, 0, 0};
+        const bool same = (L.spec[slot].exit.pad & 1) && L.spec[slot].cp[0].state == from;
+        if (same) settle(L, slot, from, 0, 0, none);
+        list = !same;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, list);
+    uint32_t base = 0;
+    if (lane == 0 && m) base = atomicAdd(L.sync_count, (uint32_t)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (list) L.sync_list[base + __popc(m & ((1u << lane) - 1u))] = slot;
 }
 
 // ------------------------------------------------------------ sync pass ---
@@ -422,164 +527,132 @@ __global__ void __launch_bounds__(kSliceThreads, MMR_SPEC_CTAS_PER_SM) slice_spe
 // Re-decodes slice `slot` (not the first, not the last) from state `from`, the
 // exit of its predecessor, until it meets one of the slice's speculative
 // checkpoints or passes the slice end. Returns whether the exit state changed.
-__device__ bool resync_slice(const JpegLaunch &L, uint32_t slot, const SliceRef &s, unsigned long long from) {
-    SliceSync out;
-    out.start = from;
-    out.pad = 0;
-    out.blocks = 0;
-#pragma unroll
-    for (int c = 0; c < 4; c++) out.dc[c] = 0;
+__device__ bool resync_slice(const JpegLaunch &L, uint32_t slot, const SliceRef &s, unsigned long long from,
+                             int32_t *dc) {
+    const JFrame &F = L.frames[s.v.frame];
     const unsigned long long old_exit = L.sync[slot].exit;
-    SliceMatch m;
-    m.q = kMatchNone;
-    m.blocks = 0;
+    SliceSync y;
+    y.start = from;
+    y.exit = kStErr;
+    y.blocks = 0;
+    y.q = kMatchNone;
 #pragma unroll
-    for (int c = 0; c < 4; c++) m.dc[c] = 0;
-    if (from == kStErr) {
-        out.exit = kStErr;
-        L.sync[slot] = out;
-        L.match[slot] = m;
-        return old_exit != kStErr;
+    for (int c = 0; c < 4; c++) {
+        dc[c] = 0;
+        y.dc[c] = 0;
     }
-    const JFrame &F = *s.F;
-    unsigned long long nominal;
-    uint32_t S;  // this slice's length
-    slice_span(s, F.slice_bits, nominal, S);
-    const unsigned long long p0 = from >> 16;
-    const uint32_t rel = (uint32_t)(p0 - nominal);  // < one symbol: from is the first boundary past nominal
-    const unsigned long long lbits = (unsigned long long)(s.v.barrier - s.v.start) * 8;
-    const uint32_t lim = clamp_u32(lbits - p0);
-    Bits r;
-    bits_init(r, F.tok, (uint64_t)s.v.start * 8 + p0, 0);
-    int k = (int)(from & 0xff);
-    uint32_t si = (uint32_t)(from >> 8) & 0xff;
-    BlockTabs tb = block_tabs(L, F, si);
-    uint32_t blocks = 0;
-    int32_t dc[4] = {0, 0, 0, 0};
-    int32_t dcv = 0;
-    const SliceSpec *sp = L.spec + slot;
-    uint32_t q = 0;
-    while (mark_of(q, S) <= rel) q++;  // marks already behind
-    uint32_t next_mark = mark_of(q, S);
-    unsigned long long exit_state = kStErr;
-    for (;;) {
-        const uint32_t pr = r.used;
-        const uint32_t pn = pr + rel;  // position from the nominal slice start
-        if (pn >= S) {
-            exit_state = pack_state(p0 + pr, si, k);
-            break;
-        }
-        if (pn >= next_mark) {
-            bool matched = false;
-            while (pn >= mark_of(q, S)) {
-                const unsigned long long cs = sp->cp[q].state;
-                if (cs != kStErr && cs == pack_state(p0 + pr, si, k)) {
-                    // the rest of the slice is the speculative decode's: take its tail
-                    const SlicePoint cp = sp->cp[q], e = sp->exit;
-                    exit_state = e.state;
-                    add_dc(dc, tb.comp, dcv);
-                    dcv = 0;
-                    m.q = q;  // the true decode so far, where it meets the speculative one
-                    m.blocks = blocks;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) m.dc[c] = dc[c];
-                    blocks += e.blocks - cp.blocks;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) dc[c] += e.dc[c] - cp.dc[c];
-                    matched = true;
+    if (from != kStErr) {
+        const uint32_t S = F.slice_bits;
+        const unsigned long long nominal = (unsigned long long)s.j * S, p0 = from >> 8;
+        const uint32_t rel = clamp_u32(p0 - nominal);  // (a block may reach past the slice)
+        const uint32_t lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - p0);
+        const unsigned long long base = (unsigned long long)s.v.start * 8 + p0;
+        const LeanTabs<false> T{L.skip, L.sym, nullptr, nullptr, L.brec + F.sched_off};
+        const SliceSpec *sp = L.spec + slot;
+        const uint32_t valid = sp->exit.pad;
+        Lean d;
+        window_init(d.r, F.tok, base);
+        d.blocks = 0;
+        d.k = 64;
+        d.si = (uint32_t)(from & 0xff);
+        d.tab = 0;
+        uint32_t q = 0, next_mark = 0;
+        bool first = true;
+        for (;;) {
+            if (d.k >= 64) {
+                if (lean_invalid(d)) break;
+                if (!first) d.si = d.si + 1 == F.sched_len ? 0 : d.si + 1;
+                first = false;
+                const uint32_t pos = window_pos(d.r, F.tok, (uint32_t)base);
+                if (pos > lim) break;
+                const uint32_t pn = pos + rel;
+                if (pn >= S) {
+                    y.exit = pack_state(p0 + pos, d.si);
                     break;
                 }
-                q++;
+                if (pn >= next_mark) {
+                    const unsigned long long here = pack_state(p0 + pos, d.si);
+                    bool met = false;
+                    do {
+                        met = (valid >> q & 1) && sp->cp[q].state == here;
+                        if (!met) next_mark = mark_of(++q, S);
+                    } while (!met && pn >= next_mark);
+                    if (met) {  // the rest of the slice is the speculative decode's
+                        settle(L, slot, from, q, d.blocks, dc);
+                        return sp->exit.state != old_exit;
+                    }
+                }
+                if (!lean_dc(L, T, d, dc)) break;
             }
-            if (matched) break;
-            next_mark = mark_of(q, S);
+            lean_steps(L, T, d);
         }
-        const int k0 = k;
-        blocks += k0 == 0;
-        int32_t val, val2;
-        int km;
-        uint16_t err;
-        uint32_t eb;
-        // two symbols per lookup where both end before the next checkpoint or the
-        // slice end (the speculative decode's boundaries there are one-symbol ones)
-        const uint32_t stop = min(next_mark, S) - pn;
-        if (!decode_step(r, lim - pr, stop, k0 == 0 ? tb.dc : tb.ac, L.symbols, k, val, val2, km, err, eb)) break;
-        dcv = k0 == 0 ? val : dcv;
-        if (k < 64) continue;
-        add_dc(dc, tb.comp, dcv);
-        dcv = 0;
-        k = 0;
-        si = si + 1 == F.sched_len ? 0 : si + 1;
-        tb = block_tabs(L, F, si);
-    }
-    add_dc(dc, tb.comp, dcv);
-    out.exit = exit_state;
-    out.blocks = blocks;
+        y.blocks = d.blocks;
 #pragma unroll
-    for (int c = 0; c < 4; c++) out.dc[c] = dc[c];
-    L.sync[slot] = out;
-    L.match[slot] = m;
-    return exit_state != old_exit;
+        for (int c = 0; c < 4; c++) y.dc[c] = dc[c];
+    }
+    L.sync[slot] = y;
+    return y.exit != old_exit;
 }
 
-// Persistent threads take slots from a counter: re-decode lengths vary a lot
-// (most slices meet their first checkpoint, a few run to their end), so a lane
-// that is done takes the next slot instead of idling beside the slow ones. The
-// lanes that reach the counter together take consecutive slots with one atomic
-// (one per slot serialised on the counter's address).
+// Persistent threads take listed slots from a counter (re-decode lengths vary a lot;
+// the lanes that reach the counter together take consecutive entries with one
+// atomic). A changed exit lists the next slice for the pass after; after the last
+// pass it is left to slice_fix_kernel, from the interval's first such slice on.
 __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L, uint32_t pass) {
-    // a pass after one that changed no exit state has nothing to do: every start
-    // then equals its predecessor's exit
-    if (pass > 0 && *(volatile const uint32_t *)&L.sync_dirty[pass - 1] == 0) return;
-    uint32_t *next = L.sync_dirty + kSyncPasses + pass;
+    __shared__ int32_t s_dc[kSliceThreads][4];
+    const uint32_t n = L.sync_count[pass];
+    const uint32_t *list = L.sync_list + (uint64_t)(pass & 1) * L.n_slots;
+    uint32_t *next_list = L.sync_list + (uint64_t)(~pass & 1) * L.n_slots;
+    uint32_t *taken = L.sync_count + kSyncPasses + 1 + pass;
     const uint32_t lane = threadIdx.x & 31;
     for (;;) {
         const unsigned act = __activemask();
         const int leader = __ffs(act) - 1;
         uint32_t base = 0;
-        if ((int)lane == leader) base = atomicAdd(next, (uint32_t)__popc(act));
+        if ((int)lane == leader) base = atomicAdd(taken, (uint32_t)__popc(act));
         base = __shfl_sync(act, base, leader);
-        const uint32_t slot = base + __popc(act & ((1u << lane) - 1u));
-        if (slot >= L.n_slots) return;
+        const uint32_t at = base + __popc(act & ((1u << lane) - 1u));
+        if (at >= n) return;
+        const uint32_t slot = list[at];
         SliceRef s;
-        if (!slice_ref(L, slot, s) || s.j == 0) continue;
+        slice_ref(L, slot, s);
         const unsigned long long prev = *(volatile const unsigned long long *)&L.sync[slot - 1].exit;
-        const unsigned long long cur = L.sync[slot].start;
-        if (prev == cur) continue;
-        if (s.last) {
-            L.sync[slot].start = prev;
-            continue;
+        if (prev == L.sync[slot].start) continue;
+        if (!resync_slice(L, slot, s, prev, s_dc[threadIdx.x]) || s.j + 2 >= s.v.n_slices) continue;
+        if (pass + 1 < (uint32_t)kSyncPasses) next_list[atomicAdd(L.sync_count + pass + 1, 1u)] = slot + 1;
+        else {
+            atomicAdd(L.sync_count + kSyncPasses, 1u);
+            atomicMin(L.iv_pend + s.item, slot + 1 - s.v.slot_first);
         }
-        if (resync_slice(L, slot, s, prev)) atomicAdd(&L.sync_dirty[pass], 1u);
     }
 }
 
-// One warp per interval; runs only when the last sync pass still changed an exit state.
-__global__ void slice_fix_kernel(JpegLaunch L) {
-    if (*(volatile uint32_t *)&L.sync_dirty[kSyncPasses - 1] == 0) return;
-    const uint32_t item = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+// One warp per interval that still has a listed slice.
+__global__ void __launch_bounds__(kSliceThreads) slice_fix_kernel(JpegLaunch L) {
+    __shared__ int32_t s_dc[kSliceThreads][4];
+    if (L.sync_count[kSyncPasses] == 0) return;
+    const uint32_t item = blockIdx.x * (kSliceThreads / 32) + threadIdx.x / 32;
     const uint32_t lane = threadIdx.x & 31;
     if (item >= L.n_items_small) return;
+    const uint32_t pend = L.iv_pend[item];
+    if (pend == 0xffffffffu) return;
     const IvInfo v = L.ivs[item];
-    for (uint32_t c = 1; c < v.n_slices; c += 32) {
+    for (uint32_t c = pend; c + 1 < v.n_slices; c += 32) {  // (the last slice has no exit)
         for (;;) {
             const uint32_t j = c + lane;
             bool bad = false;
-            if (j < v.n_slices) {
+            if (j + 1 < v.n_slices) {
                 const uint32_t slot = v.slot_first + j;
                 bad = *(volatile unsigned long long *)&L.sync[slot].start !=
                       *(volatile unsigned long long *)&L.sync[slot - 1].exit;
             }
             const uint32_t m = __ballot_sync(0xffffffffu, bad);
             if (!m) break;
-            const uint32_t first = __ffs(m) - 1;
-            if (lane == first) {
+            if (lane == (uint32_t)__ffs(m) - 1) {
                 const uint32_t slot = v.slot_first + j;
                 SliceRef s;
                 slice_ref(L, slot, s);
-                const unsigned long long prev = *(volatile unsigned long long *)&L.sync[slot - 1].exit;
-                if (s.last) L.sync[slot].start = prev;
-                else resync_slice(L, slot, s, prev);
+                resync_slice(L, slot, s, *(volatile unsigned long long *)&L.sync[slot - 1].exit, s_dc[threadIdx.x]);
                 __threadfence_block();
             }
             __syncwarp();
@@ -589,52 +662,103 @@ __global__ void slice_fix_kernel(JpegLaunch L) {
 
 // ---------------------------------------------------------------- prefix ---
 
-__global__ void slice_prefix_kernel(JpegLaunch L) {
-    const uint32_t item = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+constexpr int kPrefixThreads = 256;
+constexpr uint32_t kPrefixLong = 512;  // slices an interval is worth the whole CTA from
+
+struct SliceSums {
+    uint32_t blocks;
+    long long dc[4];
+};
+
+__device__ __forceinline__ void add_slice(const JpegLaunch &L, const IvInfo &v, uint32_t j, SliceSums &a) {
+    if (j + 1 >= v.n_slices) return;  // the last slice's counts are never needed
+    const SliceSync &y = L.sync[v.slot_first + j];
+    a.blocks += y.blocks;
+#pragma unroll
+    for (int c = 0; c < 4; c++) a.dc[c] += y.dc[c];
+}
+
+// Inclusive prefix over the warp.
+__device__ __forceinline__ void warp_prefix(SliceSums &a) {
     const uint32_t lane = threadIdx.x & 31;
-    if (item >= L.n_items_small) return;
-    const IvInfo v = L.ivs[item];
-    uint32_t carry_b = 0;
-    long long carry_d[4] = {0, 0, 0, 0};
-    for (uint32_t c = 0; c < v.n_slices; c += 32) {
-        const uint32_t j = c + lane;
-        uint32_t b = 0;
-        long long d[4] = {0, 0, 0, 0};
-        if (j + 1 < v.n_slices) {  // the last slice's counts are never needed
-            const SliceSync &y = L.sync[v.slot_first + j];
-            b = y.blocks;
 #pragma unroll
-            for (int q = 0; q < 4; q++) d[q] = y.dc[q];
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t b = __shfl_up_sync(0xffffffffu, a.blocks, o);
+        long long d[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) d[c] = __shfl_up_sync(0xffffffffu, a.dc[c], o);
+        if (lane >= (uint32_t)o) {
+            a.blocks += b;
+#pragma unroll
+            for (int c = 0; c < 4; c++) a.dc[c] += d[c];
         }
-        uint32_t ib = b;
-        long long id[4] = {d[0], d[1], d[2], d[3]};
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t tb = __shfl_up_sync(0xffffffffu, ib, o);
-            long long td[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) td[q] = __shfl_up_sync(0xffffffffu, id[q], o);
-            if (lane >= (uint32_t)o) {
-                ib += tb;
-#pragma unroll
-                for (int q = 0; q < 4; q++) id[q] += td[q];
-            }
-        }
-        if (j < v.n_slices) {
-            SlicePrefix P;
-            P.base = carry_b + ib - b;
-            P.pad = 0;
-#pragma unroll
-            for (int q = 0; q < 4; q++) P.dc[q] = carry_d[q] + id[q] - d[q];
-            L.prefix[v.slot_first + j] = P;
-        }
-        carry_b += __shfl_sync(0xffffffffu, ib, 31);
-#pragma unroll
-        for (int q = 0; q < 4; q++) carry_d[q] += __shfl_sync(0xffffffffu, id[q], 31);
     }
 }
 
-// ----------------------------------------------------------------- place ---
+__device__ __forceinline__ void write_prefix(const JpegLaunch &L, const IvInfo &v, uint32_t j, const SliceSums &a) {
+    SlicePrefix P;
+    P.base = a.blocks;
+    P.pad = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) P.dc[c] = a.dc[c];
+    L.prefix[v.slot_first + j] = P;
+}
+
+// Warp per interval; intervals of many slices (scans without restart markers) are
+// taken by the whole CTA, a run of slices per thread (a warp per interval took
+// 1.5 ms for the 10k slices of 4K scans). One-slice intervals need no prefix.
+__global__ void __launch_bounds__(kPrefixThreads) slice_prefix_kernel(JpegLaunch L) {
+    __shared__ SliceSums s_warp[kPrefixThreads / 32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t item0 = blockIdx.x * (kPrefixThreads / 32), item = item0 + warp;
+    if (item < L.n_items_small) {
+        const IvInfo v = L.ivs[item];
+        if (v.n_slices > 1 && v.n_slices < kPrefixLong) {
+            SliceSums carry{};
+            for (uint32_t c = 0; c < v.n_slices; c += 32) {
+                SliceSums a{}, own{};
+                add_slice(L, v, c + lane, own);
+                a = own;
+                warp_prefix(a);
+                const SliceSums incl = a;
+                a.blocks += carry.blocks - own.blocks;
+#pragma unroll
+                for (int q = 0; q < 4; q++) a.dc[q] += carry.dc[q] - own.dc[q];
+                if (c + lane < v.n_slices) write_prefix(L, v, c + lane, a);
+                carry.blocks += __shfl_sync(0xffffffffu, incl.blocks, 31);
+#pragma unroll
+                for (int q = 0; q < 4; q++) carry.dc[q] += __shfl_sync(0xffffffffu, incl.dc[q], 31);
+            }
+        }
+    }
+    for (uint32_t i = 0; i < kPrefixThreads / 32 && item0 + i < L.n_items_small; i++) {
+        const IvInfo v = L.ivs[item0 + i];
+        if (v.n_slices < kPrefixLong) continue;  // uniform over the CTA
+        const uint32_t per = (v.n_slices + kPrefixThreads - 1) / kPrefixThreads;
+        const uint32_t j0 = min(threadIdx.x * per, v.n_slices), j1 = min(j0 + per, v.n_slices);
+        SliceSums own{};
+        for (uint32_t j = j0; j < j1; j++) add_slice(L, v, j, own);
+        SliceSums a = own;
+        warp_prefix(a);
+        __syncthreads();
+        if (lane == 31) s_warp[warp] = a;
+        __syncthreads();
+        a.blocks -= own.blocks;
+#pragma unroll
+        for (int q = 0; q < 4; q++) a.dc[q] -= own.dc[q];
+        for (uint32_t w = 0; w < warp; w++) {
+            a.blocks += s_warp[w].blocks;
+#pragma unroll
+            for (int q = 0; q < 4; q++) a.dc[q] += s_warp[w].dc[q];
+        }
+        for (uint32_t j = j0; j < j1; j++) {
+            write_prefix(L, v, j, a);
+            add_slice(L, v, j, a);
+        }
+    }
+}
+
+// ---------------------------------------------------------------- decode ---
 
 // Records a slice's first event: an error, or the interval's completion.
 __device__ __forceinline__ void report(const JpegLaunch &L, const SliceRef &s, uint32_t slot, unsigned long long pos,
@@ -646,268 +770,254 @@ __device__ __forceinline__ void report(const JpegLaunch &L, const SliceRef &s, u
     atomicMin(&L.iv_key[s.item], (pos << kKeyBits) | s.j);
 }
 
-
-// A thread per slice. The owned blocks that start after the point where the
-// slice's true decode met its speculative decode (SliceMatch) are final: their
-// DC predictors are settled as the final decode would (decoder.rs:507-515) and
-// the block map points at their levels. The final decode pass writes the blocks
-// before that point, and the whole slice when there is no such point, anything
-// failed, or it is the interval's last slice
-// (its decode reports the interval's completion; a placed last block reports it
-// here). A DC overflow among the placed blocks also sends the whole slice there
-// (reported with its position). Returns the final decode pass's work in the
-// slice: the leading blocks it writes (0: none, UINT32_MAX: all).
-__device__ uint32_t place_slice(const JpegLaunch &L, uint32_t slot, const SliceRef &s) {
-    const SliceSync y = L.sync[slot];
-    if (y.start == kStErr || y.start == kStGuess) return 0;  // not reached: nothing to decode
-    const SlicePrefix P = L.prefix[slot];
-    const uint32_t B = s.v.blocks;
-    if (P.base >= B) return 0;
-    const uint32_t nown = s.last ? B - P.base : min(y.blocks, B - P.base);
-    if (nown == 0) return 0;
-    const SliceOwn *O = L.own + slot;
-    const SliceMatch M = L.match[slot];
-    uint32_t spec_first = 0;
-    bool usable = !s.last && O->ok && M.q != kMatchNone && M.blocks <= nown;
-    if (usable && M.q != kMatchStart) spec_first = L.spec[slot].cp[M.q].own_next;
-    usable = usable && spec_first <= O->n && O->n - spec_first == nown - M.blocks;
-    if (usable && M.blocks < nown) {
-        const JFrame &F = *s.F;
-        const uint32_t sched_len = F.sched_len, mcu_cols = F.mcu_cols;
-        const uint32_t b0 = P.base + M.blocks;  // interval-relative block of the first placed one
-        const uint32_t mcu = L.items[s.item].y * F.ri + b0 / sched_len;
-        uint32_t mx = mcu % mcu_cols, my = mcu / mcu_cols, si = b0 % sched_len;
-        const JBlockRec *recs = L.brec + F.sched_off;
-        long long pred[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) pred[c] = P.dc[c] + M.dc[c];
-        for (uint32_t i = 0; i < nown - M.blocks; i++) {
-            const JBlockRec R = recs[si];
-            const uint64_t blk = F.blk_off + R.base_off + mx * R.mul_x + (uint64_t)my * R.mul_y;
-            const uint32_t own_i = spec_first + i;
-            const uint32_t sb = O->chunk[own_i / kOwnChunkBlocks] + own_i % kOwnChunkBlocks;
-            long long pc = 0;
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (R.comp == (uint32_t)c) pc = pred[c];
-            const long long pn = pc + L.scratch_dc[sb];
-            const long long d = pn * (long long)R.q0;
-            if (pn > INT32_MAX || pn < INT32_MIN || d > INT32_MAX || d < INT32_MIN) {
-                usable = false;
-                break;
-            }
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (R.comp == (uint32_t)c) pred[c] = pn;
-            L.dc[blk] = (int32_t)d;
-            L.blk_map[blk] = sb;
-            if (++si == sched_len) {
-                si = 0;
-                if (++mx == mcu_cols) {
-                    mx = 0;
-                    my++;
-                }
-            }
-        }
-    }
-    if (usable && M.blocks < nown && P.base + nown == B) {  // the interval's last block, placed
-        const unsigned long long endbit = O->last_end;
-        report(L, s, slot, endbit, make_diag(kDiagNone, s.v.start + (uint32_t)((endbit + 7) / 8)), 1);
-    }
-    const uint32_t redo = usable ? M.blocks : 0xffffffffu;
-    L.redo[slot] = redo;
-    return redo;
-}
-
-// Adds the lanes' flags to a counter, one atomic per warp.
-__device__ __forceinline__ void count_lanes(uint32_t *counter, bool flag) {
-    const uint32_t m = __ballot_sync(0xffffffffu, flag);
-    if ((threadIdx.x & 31) == 0 && m) atomicAdd(counter, (uint32_t)__popc(m));
-}
-
-// Also lists the slots with short work for the final decode (leading blocks, or an
-// interval's last slice, at most kSliceTail bits), so that its warps take those
-// tasks packed and lanes without work do not ride along. Whole slices redone from
-// their start stay in slot order: few and long, they run best spread over the
-// warps (a packed warp of them waits on 32 lanes' loads per step).
-__global__ void __launch_bounds__(kSliceThreads) slice_place_kernel(JpegLaunch L) {
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    SliceRef s;
-    const bool valid = slice_ref(L, slot, s);
-    count_lanes(L.fix_count + 3, valid);
-    uint32_t redo = 0;
-    if (valid) redo = place_slice(L, slot, s);
-    count_lanes(L.fix_count + 2, redo != 0);
-    count_lanes(L.fix_count + 5, redo == 0xffffffffu);
-    const uint32_t lane = threadIdx.x & 31;
-    const unsigned shrt = __ballot_sync(0xffffffffu, redo != 0 && (redo != 0xffffffffu || s.last));
-    uint32_t base = 0;
-    if (lane == 0 && shrt) base = atomicAdd(L.fix_count + 4, (uint32_t)__popc(shrt));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (shrt & (1u << lane)) L.work[base + __popc(shrt & ((1u << lane) - 1u))] = slot;
-}
-
-
-// ---------------------------------------------------------------- decode ---
-
-
-__global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch L) {
-    __shared__ __align__(16) int16_t s_stage[kSliceThreads * kStride];
-    __shared__ uint8_t s_zz[64];  // lanes index it freely: a shared table serves them in one pass
-    int16_t *stage = s_stage + threadIdx.x * kStride;
-    int4 *stage4 = reinterpret_cast<int4 *>(stage);
-#pragma unroll
-    for (int q = 0; q < 8; q++) stage4[q] = make_int4(0, 0, 0, 0);
-    if (threadIdx.x < 64) s_zz[threadIdx.x] = c_slice_zz[threadIdx.x];
-    __syncthreads();
-    // The first half of the grid takes the short tasks, packed from the work list
-    // (slice_place_kernel); the second half the whole slices redone from their
-    // start, in slot order.
-    const uint32_t half = gridDim.x >> 1;
-    uint32_t slot;
-    if (blockIdx.x < half) {
-        const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-        if (t >= L.fix_count[4]) return;
-        slot = L.work[t];
-    } else {
-        slot = (blockIdx.x - half) * blockDim.x + threadIdx.x;
-    }
-    SliceRef s;
-    if (!slice_ref(L, slot, s)) return;
-    const uint32_t redo = L.redo[slot];  // leading blocks to write; the rest are placed
-    if (!redo || (blockIdx.x >= half && (redo != 0xffffffffu || s.last))) return;
-    const unsigned long long from = L.sync[slot].start;
-    if (from == kStErr || from == kStGuess) return;
-    const SlicePrefix P = L.prefix[slot];
-    const uint32_t B = s.v.blocks;
-    if (P.base >= B) return;
-    const uint32_t nown = min(s.last ? B - P.base : min(L.sync[slot].blocks, B - P.base), redo);
-    if (nown == 0) return;
-    const JFrame &F = *s.F;
-    const uint32_t iv = L.items[s.item].y;
-    const unsigned long long p0 = from >> 16;
-    const unsigned long long lbits = (unsigned long long)(s.v.barrier - s.v.start) * 8;
-    const uint32_t lim = clamp_u32(lbits - p0);
-    const uint32_t sched_len = F.sched_len;
+// The block whose DC symbol starts at bit `at` of the interval failed: decodes it
+// again with the reference's checks in its order (decoder.rs:501-546; the DC checks of
+// :507-515 right after the DC symbol) and reports what the serial decoder stops at.
+__device__ __noinline__ void report_bad_block(const JpegLaunch &L, const SliceRef &s, uint32_t slot,
+                                              unsigned long long at, uint32_t si, long long pred) {
+    const JFrame &F = L.frames[s.v.frame];
+    const JBlockRec R = L.brec[F.sched_off + si];
+    const uint32_t lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - at);
     Bits r;
-    bits_init(r, F.tok, (uint64_t)s.v.start * 8 + p0, 0);
-    int k = (int)(from & 0xff);
-    uint32_t si = (uint32_t)(from >> 8) & 0xff;
-    int32_t val;
-    uint16_t err;
-    uint32_t eb;
-    if (k != 0) {  // the block straddling the start belongs to an earlier slice
-        const HuffLut *acl = block_tabs(L, F, si).ac;
-        while (k < 64)
-            if (!decode_symbol(r, lim - r.used, acl, L.symbols, k, val, err, eb)) return;
-        si = si + 1 == sched_len ? 0 : si + 1;
-        k = 0;
-    }
-    long long pred[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) pred[c] = P.dc[c];
-    // MCU of the first owned block, then advanced block by block
-    const uint32_t mcu = iv * F.ri + P.base / sched_len;
-    const uint32_t mcu_cols = F.mcu_cols;
-    uint32_t mx = mcu % mcu_cols, my = mcu / mcu_cols;
-    uint32_t b = P.base;
-    const uint32_t bend = P.base + nown;
-    const HuffLut *dcl, *acl;
-    uint64_t blk;
-    int32_t q0;
-    uint32_t comp;
-    const JBlockRec *recs = L.brec + F.sched_off;
-    auto setup = [&]() {
-        const JBlockRec R = recs[si];
-        comp = R.comp;
-        dcl = L.luts + R.dc_lut;
-        acl = L.luts + R.ac_lut;
-        blk = F.blk_off + R.base_off + mx * R.mul_x + (uint64_t)my * R.mul_y;
-        q0 = R.q0;
-    };
-    setup();
-    // The DC difference is staged at zigzag index 0 like a level and turned into the
-    // dequantised DC when the block completes; an error inside the block first
-    // settles the DC checks the reference makes right after the DC symbol.
-    uint32_t blk_at = r.used;  // start of the block's DC symbol
-    uint32_t dc_end = 0;       // reader position after the DC difference
-    for (;;) {
+    bits_init(r, F.tok, (uint64_t)s.v.start * 8 + at, 0);
+    int k = 0;
+    uint16_t kind = kDeviceError;  // (never kept: the fast decode only refuses what this one does)
+    uint32_t errpos = 0, ev_at = 0;
+    while (k < 64) {
         const uint32_t sym_at = r.used;
         const int k0 = k;
-        const bool ok = decode_symbol(r, lim - sym_at, k0 == 0 ? dcl : acl, L.symbols, k, val, err, eb);
-        if (ok) {
-            stage[s_zz[k - 1]] = (int16_t)val;
-            dc_end = k0 == 0 ? r.used : dc_end;
-            if (k < 64) continue;
-        }
-        // block complete, or an error: the block's DC checks (decoder.rs:507-515) first
-        uint16_t kind = kDiagNone;
-        uint32_t errpos = 0, ev_at = sym_at;
-        int32_t dq = 0;
-        if (ok || k0 > 0) {
-            long long pc = 0;
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (comp == (uint32_t)c) pc = pred[c];
-            const long long pn = pc + stage[0];
-            if (pn > INT32_MAX || pn < INT32_MIN) {
-                kind = kJDcPredOverflow;
-                errpos = dc_end;
-                ev_at = blk_at;
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (comp == (uint32_t)c) pred[c] = pn;
-                const long long d = pn * (long long)q0;
-                if (d > INT32_MAX || d < INT32_MIN) {
-                    kind = kJDcDeqOverflow;
-                    errpos = dc_end;
-                    ev_at = blk_at;
-                }
-                dq = (int32_t)d;
-            }
-        }
-        if (kind == kDiagNone && !ok) {
+        int32_t val;
+        uint16_t err;
+        uint32_t eb;
+        if (!decode_symbol(r, lim > sym_at ? lim - sym_at : 0, L.luts + (k0 == 0 ? R.dc_lut : R.ac_lut), L.symbols, k, val, err, eb)) {
             kind = err;
             errpos = eb;
+            ev_at = sym_at;
+            break;
         }
-        if (kind != kDiagNone) {
-            Diag d;
-            if (kind == kBarrierErr) {
-                d = (s.v.flags & 1)
-                        ? make_diag(kJMarkerInData, s.v.barrier, 0xd0 + L.rsts[F.rst_off + iv].number)
-                        : make_diag(kJEndOfData, L.states[L.items[s.item].x].n_tokens);
-            } else {
-                d = make_diag(kind, s.v.start + (uint32_t)((p0 + errpos + 7) / 8));
-            }
-            report(L, s, slot, p0 + ev_at, d, 0);
-            return;
+        if (k0 != 0) continue;
+        const long long pn = pred + val, d = pn * (long long)R.q0;
+        const bool pred_bad = pn > INT32_MAX || pn < INT32_MIN;
+        if (pred_bad || d > INT32_MAX || d < INT32_MIN) {
+            kind = pred_bad ? kJDcPredOverflow : kJDcDeqOverflow;
+            errpos = r.used;
+            break;
         }
-        int4 *dst = reinterpret_cast<int4 *>(L.coef + blk * 64);
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            dst[q] = stage4[q];
-            stage4[q] = make_int4(0, 0, 0, 0);
-        }
-        L.dc[blk] = dq;
-        L.blk_map[blk] = kLevelsInPlace;  // (place may have mapped the first blocks before an overflow)
-        if (b + 1 == B) {
-            const unsigned long long endbit = p0 + r.used;
-            report(L, s, slot, endbit, make_diag(kDiagNone, s.v.start + (uint32_t)((endbit + 7) / 8)), 1);
-            return;
-        }
-        if (++b == bend) return;
-        if (++si == sched_len) {
-            si = 0;
-            if (++mx == mcu_cols) {
-                mx = 0;
-                my++;
-            }
-        }
-        setup();
-        k = 0;
-        blk_at = r.used;
     }
+    Diag d;
+    if (kind == kBarrierErr) {
+        d = (s.v.flags & 1) ? make_diag(kJMarkerInData, s.v.barrier, 0xd0 + L.rsts[F.rst_off + L.items[s.item].y].number)
+                            : make_diag(kJEndOfData, L.states[s.v.frame].n_tokens);
+    } else {
+        d = make_diag(kind, s.v.start + (uint32_t)((at + errpos + 7) / 8));
+    }
+    report(L, s, slot, at + ev_at, d, 0);
+}
+
+struct DecodeSmem {
+    __align__(16) int16_t stage[kSliceThreads * kStride];
+    __align__(16) uint16_t sym[2 * kMostShared * kTab];  // DC tables, then AC tables
+    JBlockRec recs[kMaxSched];
+    long long pred[4][kSliceThreads];
+    uint32_t ids[2 * kMostShared];
+    uint8_t zz[160];  // stage slot of k - 1: natural index, or past the block for EOB (k + 95 at most 158)
+};
+
+// What the final decode needs while it is in a slice.
+struct Walk {
+    Window r;
+    int k;
+    uint32_t tab;      // table of the next symbol: the block's DC table, then its AC table
+    uint32_t ac;       // its AC table
+};
+
+// kDecodeSteps symbols (none for a lane whose block has ended): each level into the
+// lane's stage; the DC difference at zigzag index 0.
+template <bool kShared>
+__device__ __forceinline__ void decode_steps(const JpegLaunch &L, const DecodeSmem &S, int16_t *stage, Walk &d) {
+#pragma unroll
+    for (int u = 0; u < kDecodeSteps; u++) {
+        uint32_t w = window_bits(d.r);
+        uint32_t e = 0;
+        const uint32_t at = d.tab + (w >> (32 - kHuffFastBits));
+        if (d.k < 64) e = kShared ? S.sym[at] : __ldg(L.sym + at);
+        if (e & kSymEscape) {
+            const uint32_t t = d.tab / kTab;
+            e = sub_entry(L, kShared ? S.ids[t] : t, e, w);
+            if (e & kSymEscape) {
+                e = 0;
+                d.k = 80;
+            } else {
+                window_take(d.r, kHuffFastBits);
+                w = window_bits(d.r);
+            }
+        }
+        const uint32_t cl = e & 15, size = (e >> 4) & 15;
+        const int32_t val = extend(w << cl, size);
+        const int k = d.k + (int)(e >> 8);
+        if (e) stage[S.zz[k - 1]] = (int16_t)val;
+        d.k = k;
+        window_take(d.r, cl + size);
+        d.tab = d.ac;
+    }
+}
+
+// Warps stay together: lanes decode kDecodeSteps symbols, then those whose block is
+// complete settle it (DC, address, the next block), and the warp writes the completed
+// blocks together, eight lanes per block, as whole 128-byte lines.
+template <bool kShared>
+__device__ __forceinline__ void decode_slices(const JpegLaunch &L, DecodeSmem &S, const JFrame &F, uint32_t slot,
+                                              const SliceRef &s, uint32_t n, unsigned long long from, uint32_t base) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    int16_t *stage = S.stage + tid * kStride;
+    bool live = n != 0;
+    Walk d;
+    d.k = 128;
+    d.tab = d.ac = 0;
+    d.r.w0 = d.r.w1 = d.r.pf = d.r.off = 0;
+    d.r.next = reinterpret_cast<const uint32_t *>(F.tok);
+    const unsigned long long p0 = from >> 8;
+    uint32_t si = (uint32_t)(from & 0xff), lim = 0, bit0 = 0, blk_at = 0;
+    uint32_t mx = 0, my = 0, left = n;
+    uint64_t blk = 0;
+    int32_t q0 = 0;
+    uint32_t comp = 0;
+    auto setup = [&]() {
+        const JBlockRec &R = S.recs[si];
+        comp = R.comp;
+        q0 = R.q0;
+        blk = F.blk_off + R.base_off + mx * R.mul_x + (uint64_t)my * R.mul_y;
+        if (kShared) {
+            d.tab = ((R.local >> 8) & 0xff) * kTab;
+            d.ac = (kMostShared + (R.local >> 16)) * kTab;
+        } else {
+            d.tab = R.dc_lut * kTab;
+            d.ac = R.ac_lut * kTab;
+        }
+        d.k = 0;
+    };
+    if (live) {
+        const unsigned long long b0 = (unsigned long long)s.v.start * 8 + p0;
+        bit0 = (uint32_t)b0;
+        lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - p0);
+        window_init(d.r, F.tok, b0);
+        const uint32_t mcu = L.items[s.item].y * F.ri + base / F.sched_len;
+        my = mcu / F.mcu_cols;
+        mx = mcu - my * F.mcu_cols;
+        setup();
+    }
+    while (__any_sync(0xffffffffu, live)) {
+        decode_steps<kShared>(L, S, stage, d);
+        bool put = false;
+        uint32_t to = 0;  // the completed block (the arena holds less than 2^32)
+        if (live && d.k >= 64) {
+            const uint32_t pos = window_pos(d.r, F.tok, bit0);
+            const long long pn = S.pred[comp][tid] + stage[0], dq = pn * (long long)q0;
+            const bool ok = (d.k == 64 || d.k >= 96) && pos <= lim && pn <= INT32_MAX && pn >= INT32_MIN &&
+                            dq <= INT32_MAX && dq >= INT32_MIN;
+            if (!ok) {
+                report_bad_block(L, s, slot, p0 + blk_at, si, S.pred[comp][tid]);
+                live = false;
+            } else {
+                S.pred[comp][tid] = pn;
+                L.dc[blk] = (int32_t)dq;
+                to = (uint32_t)blk;
+                put = true;
+                blk_at = pos;
+                if (++base == s.v.blocks) {  // the interval's last block
+                    const unsigned long long endbit = p0 + pos;
+                    report(L, s, slot, endbit, make_diag(kDiagNone, s.v.start + (uint32_t)((endbit + 7) / 8)), 1);
+                }
+                live = --left != 0;
+                if (++si == F.sched_len) {
+                    si = 0;
+                    if (++mx == F.mcu_cols) {
+                        mx = 0;
+                        my++;
+                    }
+                }
+                if (live) setup();
+            }
+        }
+        unsigned m = __ballot_sync(0xffffffffu, put);
+        while (m) {
+            // lanes 8i .. 8i + 7 write the i-th block left
+            unsigned mine = m;
+            for (uint32_t i = 0; i < lane >> 3; i++) mine &= mine - 1;
+            const int src = __ffs(mine) - 1;
+            const uint32_t g = __shfl_sync(0xffffffffu, to, src & 31);
+            if (src >= 0) {
+                int4 *st = reinterpret_cast<int4 *>(S.stage + ((tid & ~31u) + src) * kStride) + (lane & 7);
+                reinterpret_cast<int4 *>(L.coef + (uint64_t)g * 64)[lane & 7] = *st;
+                *st = make_int4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) m &= m - 1;
+        }
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch L) {
+    extern __shared__ __align__(16) uint8_t s_raw[];
+    DecodeSmem &S = *reinterpret_cast<DecodeSmem *>(s_raw);
+    const uint32_t tid = threadIdx.x, slot = blockIdx.x * kSliceThreads + tid;
+    SliceRef s;
+    s.item = 0;
+    const bool used = slice_ref(L, slot, s);
+    // the blocks this slice decodes
+    uint32_t n = 0, base = 0;
+    unsigned long long from = 0;
+    bool redone = false, whole = false;
+    if (used) {
+        if (s.v.n_slices > 1) {
+            const SlicePrefix P = L.prefix[slot];
+            base = P.base;
+#pragma unroll
+            for (int c = 0; c < 4; c++) S.pred[c][tid] = P.dc[c];
+            from = s.j == 0 ? pack_state(0, 0) : L.sync[slot - 1].exit;
+            if (!s.last) {
+                const SliceSync &y = L.sync[slot];
+                n = y.blocks;
+                redone = s.j != 0 && y.q != 0;
+                whole = y.q == kMatchNone;
+            } else {
+                n = 0xffffffffu;
+            }
+            n = from == kStErr || base >= s.v.blocks ? 0 : min(n, s.v.blocks - base);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; c++) S.pred[c][tid] = 0;
+            from = pack_state(0, 0);
+            n = s.v.blocks;
+        }
+    }
+    const int n_used = __syncthreads_count(used), n_redone = __syncthreads_count(redone),
+              n_whole = __syncthreads_count(whole);
+    if (!n_used) return;
+    if (tid == 0) {
+        atomicAdd(L.fix_count + 3, (uint32_t)n_used);
+        if (n_redone) atomicAdd(L.fix_count + 2, (uint32_t)n_redone);
+        if (n_whole) atomicAdd(L.fix_count + 5, (uint32_t)n_whole);
+    }
+    const JFrame &F = L.frames[L.ivs[L.slot_item[blockIdx.x * kSliceThreads]].frame];
+    const bool small = F.n_dc <= kMostShared && F.n_ac <= kMostShared;
+    for (uint32_t i = tid; i < kSliceThreads * kStride / 8; i += kSliceThreads)
+        reinterpret_cast<int4 *>(S.stage)[i] = make_int4(0, 0, 0, 0);
+    for (uint32_t i = tid; i < 160; i += kSliceThreads) S.zz[i] = i < 64 ? c_slice_zz[i] : 64;
+    copy16(S.recs, L.brec + F.sched_off, F.sched_len * (uint32_t)sizeof(JBlockRec));
+    if (small) {
+        for (uint32_t t = 0; t < F.n_dc; t++) copy16(S.sym + t * kTab, L.sym + F.dc_id[t] * kTab, 2 * kTab);
+        for (uint32_t t = 0; t < F.n_ac; t++)
+            copy16(S.sym + (kMostShared + t) * kTab, L.sym + F.ac_id[t] * kTab, 2 * kTab);
+        if (tid < kMostShared) {
+            S.ids[tid] = F.dc_id[tid];
+            S.ids[kMostShared + tid] = F.ac_id[tid];
+        }
+    }
+    __syncthreads();
+    if (small) decode_slices<true>(L, S, F, slot, s, n, from, base);
+    else decode_slices<false>(L, S, F, slot, s, n, from, base);
 }
 
 // --------------------------------------------------------------- resolve ---
@@ -955,25 +1065,22 @@ void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks,
         if (marks) capturing ? cudaEventRecordWithFlags(marks[k], s, cudaEventRecordExternal) : cudaEventRecord(marks[k], s);
     };
     const bool run = L.n_items_small && L.n_slots;
-    const uint32_t warps_per_cta = 4;
-    const uint32_t grid = (L.n_slots + kSliceThreads - 1) / kSliceThreads;
-    const uint32_t ivgrid = (L.n_items_small + warps_per_cta - 1) / warps_per_cta;
+    const uint32_t grid = L.n_slots / kSliceThreads;  // (frames reserve whole CTAs of slots)
+    const uint32_t warps = kSliceThreads / 32, pwarps = kPrefixThreads / 32;
     if (run) {
-        slice_plan_kernel<<<(L.n_frames + warps_per_cta - 1) / warps_per_cta, 32 * warps_per_cta, 0, s>>>(L);
+        slice_plan_kernel<<<L.n_frames, kPlanThreads, 0, s>>>(L);
         slice_spec_kernel<<<grid, kSliceThreads, 0, s>>>(L);
     }
     mark(0);
     if (run) {
+        slice_match_kernel<<<grid, kSliceThreads, 0, s>>>(L);
         const uint32_t sync_grid = std::min<uint32_t>(grid, 152 * 8);
         for (uint32_t p = 0; p < (uint32_t)kSyncPasses; p++) slice_sync_kernel<<<sync_grid, kSliceThreads, 0, s>>>(L, p);
-        slice_fix_kernel<<<ivgrid, 32 * warps_per_cta, 0, s>>>(L);
-        slice_prefix_kernel<<<ivgrid, 32 * warps_per_cta, 0, s>>>(L);
+        slice_fix_kernel<<<(L.n_items_small + warps - 1) / warps, kSliceThreads, 0, s>>>(L);
+        slice_prefix_kernel<<<(L.n_items_small + pwarps - 1) / pwarps, kPrefixThreads, 0, s>>>(L);
     }
     mark(1);
-    if (run) {
-        slice_place_kernel<<<grid, kSliceThreads, 0, s>>>(L);
-        slice_decode_kernel<<<2 * grid, kSliceThreads, 0, s>>>(L);
-    }
+    if (run) slice_decode_kernel<<<grid, kSliceThreads, sizeof(DecodeSmem), s>>>(L);
     mark(2);
     if (run) slice_resolve_kernel<<<(L.n_items_small + 127) / 128, 128, 0, s>>>(L);
 }

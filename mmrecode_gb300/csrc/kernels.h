@@ -38,8 +38,8 @@ struct JpegLaunch {
     uint64_t n_blocks;
     uint32_t *item_ok;           // per batch item: 1 while decoding has not failed
     ulonglong2 *fix;             // blocks the fp32 IDCT could not fully decide: (block, sample mask)
-    uint32_t *fix_count;         // entries, samples, slices redone, slices, short redos listed, slices
-                                 // redone whole (8 counters, zeroed per batch)
+    uint32_t *fix_count;         // entries, samples, slices decoded again by the sync passes, slices, unused,
+                                 // those decoded again whole (8 counters, zeroed per batch)
     uint32_t fixup_grid;         // CTAs of the grid-stride fixup pass
     // chunked entropy decoder (frames with <= 4 components; items [0, n_items_small))
     uint32_t n_slots;
@@ -50,29 +50,21 @@ struct JpegLaunch {
     SlicePrefix *prefix;         // per slot
     SliceEvent *events;          // per slot
     unsigned long long *iv_key;  // per item: (position << 26 | slice) of its first event
-    uint32_t *sync_dirty;        // per sync pass: slices whose exit state changed, then per pass the
-                                 // next slot to take (2 x kSyncPasses, zeroed per batch)
-    // levels written by the speculative decode (SliceOwn): per slot what it owns,
-    // the scratch arena, its allocation counter (zeroed per batch), and per block
-    // where its levels are (scratch block, or kLevelsInPlace: the coefficient arena)
-    SliceOwn *own;
-    SliceMatch *match;           // per slot (written by the speculative and sync passes)
-    uint32_t *redo;              // per slot: leading owned blocks the final decode pass writes
-                                 // (0: none, UINT32_MAX: all; zeroed per batch)
-    uint32_t *work;              // n_slots: slots with short work for the final decode (count in fix_count[4])
-    int16_t *scratch;            // 64 levels per scratch block
-    int16_t *scratch_dc;         // DC difference per scratch block
-    uint32_t scratch_blocks;
-    unsigned long long *scratch_next;
-    uint32_t *blk_map;           // per block (all 0xff per batch); nullptr: levels in place
+    uint32_t *iv_pend;           // per item: first slice still to settle after the sync passes
+    uint32_t *sync_list;         // 2 x n_slots: slots listed for the current and the next sync pass
+    uint32_t *sync_count;        // per sync pass the slots listed, then those left after the last, then per
+                                 // pass the entries taken (kSyncCounters, zeroed per batch)
+    const uint16_t *sym;         // per LUT: 2^kHuffFastBits symbol entries (plan.h)
+    const uint32_t *skip;        // per LUT: as many skip entries
+    const uint16_t *sub;         // blocks of kSubEntries entries for longer codes
+    const uint32_t *sub_first;   // per LUT: its first entry in sub
     const long long *fixw;       // fixed-point IDCT weights (exact_fixed.h)
 };
 
-// Parallel sync passes before the serial fix-up walk; a pass after one that changed
-// nothing returns at once (measured: 4 passes take VGA 4:2:0 restart-less frames
-// from 0.49 to 0.42 ms of sync per 30 frames and cost 1080p batches nothing; 6 are
-// slower again)
+// Parallel sync passes before the serial fix-up walk; a pass whose list is empty
+// returns at once.
 constexpr int kSyncPasses = 4;
+constexpr int kSyncCounters = 2 * kSyncPasses + 1;
 
 void launch_jpeg_scan(const JpegLaunch &L, cudaStream_t s);
 void launch_jpeg_entropy(const JpegLaunch &L, cudaStream_t s);   // frames with > 4 components

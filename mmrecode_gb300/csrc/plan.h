@@ -38,6 +38,24 @@ struct HuffLut {
     uint32_t pad[2];       // size multiple of 16
 };
 
+// Lookups of the chunked decoder (jpeg_slices.cu), per table, made from a HuffLut:
+//   sym[next 11 bits]   code bits | size << 4 | advance << 8 for codes of at most 11
+//       bits (size: magnitude bits after the code; advance of the coefficient index: 1
+//       for a DC difference, run + 1 for an AC level, 16 for ZRL, 96 for EOB, so that
+//       a block ends with an index of 64 or from 97 to 159 and an overrun lies
+//       between); kSymEscape | block for longer ones: entry (next 5 bits) of that
+//       block of `sub`, its code bits counting from the 12th; kSymInvalid for bits no
+//       code matches and symbols the reference rejects.
+//   skip[next 11 bits]  AC tables, for decodes that only follow positions: bits |
+//       advance << 5 of the first symbol (magnitude included), and the same at << 12
+//       of the first two where the second's code lies within the 11 bits too (else of
+//       the first); kSkipEscape where sym escapes.
+constexpr uint32_t kSymEscape = 0x8000u;
+constexpr uint32_t kSymInvalid = 0xffffu;
+constexpr uint32_t kSkipEscape = 0x80000000u;
+constexpr uint32_t kSymEob = 96;
+constexpr uint32_t kSubEntries = 1u << (16 - kHuffFastBits);
+
 // One frame component (SOF0 order).
 struct JComp {
     uint32_t plane_w, plane_h;  // visible samples (decoder.rs:440-445)
@@ -66,8 +84,9 @@ struct JBlockRec {
     uint32_t mul_x;
     uint32_t comp;      // frame component (scan components = frame components)
     int32_t q0;         // DC quantiser
-    uint32_t pad;
+    uint32_t local;     // comp | DC table << 8 | AC table << 16, numbered within the frame
 };
+constexpr uint32_t kMaxSched = 64;  // blocks per MCU of a frame with at most four components
 
 struct JFrame {
     const uint8_t *in;      // packet (device)
@@ -92,16 +111,20 @@ struct JFrame {
     uint32_t n_blocks;
     uint32_t item;          // caller's batch item
     uint32_t slot_first;    // first slice slot of the chunked entropy decoder
-    uint32_t slot_count;    // slots reserved: ceil(8 * in_len / slice_bits) + 2 * n_intervals
+    uint32_t slot_count;    // slots reserved: ceil(8 * in_len / slice_bits) + n_intervals, in whole CTAs
     uint32_t slice_bits;    // bits per slice (multiple of 32, >= 128)
+    uint32_t n_dc, n_ac;    // distinct DC and AC tables of the scan, and the first four of each
+    uint32_t dc_id[4], ac_id[4];
     uint32_t pad;
 };
 
 // --------------------------------------------- chunked entropy decoding ----
 //
-// A decoder state is packed as (bit position << 16) | (MCU block index << 8) | k,
-// the bit position counted from the interval's first entropy-coded token and k
-// the zigzag index of the next coefficient (0: the DC symbol comes next).
+// Decoder states are block boundaries, packed as (bit position << 8) | block of the
+// MCU that starts there, the position counted from the interval's first entropy-coded
+// token.
+
+constexpr int kSliceThreads = 128;  // slots per CTA; frames reserve whole CTAs
 
 // One restart interval (the whole scan without DRI) of a frame with <= 4 components.
 struct IvInfo {
@@ -111,81 +134,42 @@ struct IvInfo {
     uint32_t n_slices;    // 0: not decoded (header failure, or no RST precedes it)
     uint32_t blocks;      // coefficient blocks in the interval
     uint32_t flags;       // bit 0: the barrier is an RST marker
-    uint32_t tail;        // bits of the last slice when the interval's end was split off (else 0)
+    uint32_t frame;
     uint32_t pad;
-};
-
-// Slices are slice_bits long from the interval's start, except that the last one
-// is at most kSliceTail bits: when the remainder is longer, its end is split off
-// as an extra slice (the final decode pass redoes every last slice in full).
-constexpr uint32_t kSliceTail = 256;
-
-// Per slice: the state its decode starts from and what that decode produced.
-struct SliceSync {
-    unsigned long long start;  // start state (guess marker before the first sync pass)
-    unsigned long long exit;   // state at the first symbol boundary at or past the slice end
-    uint32_t blocks;           // blocks whose DC symbol starts in [start, exit)
-    int32_t dc[4];             // sum of their DC differences, per scan component
-    uint32_t pad;
-};
-
-// A point of the speculative decode: its state and the counts accumulated before
-// it, and the index among its owned blocks (SliceOwn) of the first block that
-// starts at or after it.
-struct SlicePoint {
-    unsigned long long state;
-    uint32_t blocks;
-    int32_t dc[4];
-    uint32_t own_next;
-};
-
-// Checkpoints 64, 128, 256, 512, 768, 1024, 1536 and 2048 bits into a slice
-// (those inside it). The speculative decode of a slice starts spec_lead(S) bits
-// before the slice: the synchronisation distance of Huffman-coded JPEG data is a
-// few hundred bits (longer where the MCU's block phase must also fall into
-// place), so it has usually met the true decode by the first checkpoint, and a
-// re-decode from the predecessor's exit matches there after a few symbols; the
-// later ones bound how far the final decode pass must redo a slice whose
-// speculative decode met the true one late. Short slices take a longer lead
-// relative to their length: their sync passes and serial fix-up cost more than
-// the extra decoding (measured: 1024-bit slices of 4:2:0 VGA frames 512 -> 1024
-// -> 1536 bits, 1.29 -> 1.14 -> 1.13 ms per 30 frames, 2048 bits no better;
-// 4096-bit slices of 4:2:2 1080p frames 512 -> 768 bits, 5.71 -> 5.68 ms of
-// entropy decode per 300 frames).
-constexpr int kSliceCheckpoints = 8;
-MMR_HD constexpr uint32_t spec_lead(uint32_t slice_bits) { return slice_bits <= 1024 ? 1536u : slice_bits <= 2048 ? 1024u : 768u; }
-
-struct SliceSpec {
-    SlicePoint exit;                      // end of the speculative decode
-    SlicePoint cp[kSliceCheckpoints];     // state at the first symbol boundary past each mark
-};
-
-// The levels of the blocks a speculative decode owns along its own path (the
-// blocks whose DC symbol starts in [slice start, slice end), counted from its
-// last restart), written to a scratch arena in chunks of kOwnChunkBlocks while
-// the decode runs. Where the true decode of the slice meets the speculative one
-// (at the slice start for a slice's first slice, else at the checkpoint the sync
-// pass matched), every owned block that starts after that point is final; the
-// final decode pass writes only the blocks before it (all of them when there is
-// no such point, or anything went wrong).
-constexpr uint32_t kOwnChunkBlocks = 16;
-constexpr int kOwnChunks = 16;
-constexpr uint32_t kLevelsInPlace = 0xffffffffu;  // block map: levels in the coefficient arena
-
-struct SliceOwn {
-    unsigned long long last_end; // bit position (from the interval's start) after the last one
-    uint32_t n;                  // owned blocks written
-    uint32_t ok;                 // 1: all n are complete, error-free and stored
-    uint32_t chunk[kOwnChunks];  // first scratch block of each chunk
 };
 
 // Where the true decode of a slice met its speculative decode.
 constexpr uint32_t kMatchNone = 0xffffffffu;
 constexpr uint32_t kMatchStart = 0xfffffffeu;  // a first slice: the speculative decode is the true one
-struct SliceMatch {
-    uint32_t q;        // checkpoint index, kMatchStart, or kMatchNone
-    uint32_t blocks;   // true blocks started before the point (counting the one in progress)
-    int32_t dc[4];     // their DC differences, per scan component
+
+// Per slice: the state its decode starts from and what that decode produced.
+struct SliceSync {
+    unsigned long long start;  // start state (guess marker until it is settled)
+    unsigned long long exit;   // first block boundary at or past the slice end
+    uint32_t blocks;           // blocks that start in [start, exit)
+    int32_t dc[4];             // sum of their DC differences, per scan component
+    uint32_t q;                // checkpoint where it met the speculative decode (kMatch*)
+};
+
+// A block boundary of the speculative decode and the counts accumulated before it.
+struct SlicePoint {
+    unsigned long long state;
+    uint32_t blocks;
+    int32_t dc[4];
+    uint32_t pad;  // SliceSpec::exit: bit q set when cp[q] is on the way to it
+};
+
+// Checkpoints: the first block boundary 0, 64, 128, 256, 512, 768, 1024 and 1536 bits
+// into a slice (those inside it). The speculative decode of a slice starts
+// spec_lead(S) bits before the slice: the synchronisation distance of Huffman-coded
+// JPEG data is a few hundred bits (longer where the MCU's block phase must also fall
+// into place), so it has usually met the true decode by the slice's first boundary.
+constexpr int kSliceCheckpoints = 8;
+MMR_HD constexpr uint32_t spec_lead(uint32_t slice_bits) { return slice_bits <= 1024 ? 1536u : slice_bits <= 2048 ? 1024u : 768u; }
+
+struct SliceSpec {
+    SlicePoint exit;                      // end of the speculative decode
+    SlicePoint cp[kSliceCheckpoints];
 };
 
 // Block index and DC predictors at a slice's start (interval-relative).
