@@ -134,6 +134,29 @@ uint32_t tune_class_of(const JPlan &p, size_t len) {
     return layout << 8 | lg;
 }
 
+// Slice size, and lead and number of the speculative decodes per slice of a batch.
+struct SlicePlan {
+    uint32_t bits, lead, paths;
+};
+
+// Small batches leave the GPU idle, so their time is that of one thread's slice: short
+// slices, and every block of the MCU guessed, which finds the true state after 250 to
+// 500 bits (99 % of starts) where one guess takes 1,000 to 5,000. Large batches are
+// bound by the instructions of all threads: long slices and one guess. Measured, us,
+// by slice bits / lead / paths:
+//   one 320x240 4:2:0 frame (0.13 Mbit)   256/384/6 307   512/384/6 317   1024/384/6 352
+//   one 1080p 4:2:2 frame (9 Mbit)        256/384/6 350   512/384/6 327   1024/384/6 359
+//   30 VGA 4:2:0 frames (14 Mbit)         512/384/6 471   1024/384/6 421  1024/1024/1 492   2048/768/1 544
+//   64 mixed frames (four of 106 Mbit)    1024/1024/1 3271   2048/768/1 3079   4096/768/1 3128
+//   300 1080p frames (eight of 341 Mbit)  2048/768/1 7930   4096/768/1 7469   2048/384/4 11003
+SlicePlan auto_slices(uint64_t total_bits) {
+    if (total_bits <= 2u << 20) return SlicePlan{256, 384, 6};
+    if (total_bits <= 12u << 20) return SlicePlan{512, 384, 6};
+    if (total_bits <= 32u << 20) return SlicePlan{1024, 384, 6};
+    if (total_bits <= 160u << 20) return SlicePlan{2048, 768, 1};
+    return SlicePlan{4096, 768, 1};
+}
+
 // Huffman LUT source: counts + symbols bytes (as in the DHT payload).
 struct LutSource {
     std::vector<uint8_t> key;  // 16 counts then symbols
@@ -617,7 +640,7 @@ Probe probe_packet(uint32_t codec, const uint8_t *data, size_t len) {
 struct Engine::Impl {
     DevBuf d_in, d_tok, d_blob, d_tile_tok, d_tile_rst, d_rsts, d_results, d_coef, d_dc, d_planes, d_out, d_dvcoef,
         d_modes, d_flags, d_segerr, d_vlc, d_fix, d_slot_item, d_ivs, d_sync, d_spec, d_prefix, d_events, d_ivkey,
-        d_ivpend, d_synclist,
+        d_ivpend,
         d_fixtab;  // fixed-point transform weights: MJPEG, DV 8-8, DV 2-4-8 (exact_fixed.h)
     PinBuf h_blob, h_back;
     std::vector<uint32_t> vlc;
@@ -749,8 +772,9 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         std::vector<JBlockRec> brecs;
         std::vector<JComp> comps;
         std::vector<HuffLut> luts;
-        std::vector<uint16_t> lut_sym, lut_sub;  // the chunked decoder's lookups of the same tables
-        std::vector<uint32_t> lut_skip, lut_sub_first;
+        std::vector<uint16_t> lut_sym;  // the chunked decoder's lookups of the same tables
+        std::vector<uint32_t> lut_skip;
+        std::vector<LutMeta> lut_meta;
         std::vector<uint8_t> symbols;
         std::vector<uint16_t> quant;
         std::vector<uint2> items_small, items_big;
@@ -768,16 +792,11 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         uint32_t rst_total = 0;
         uint64_t blocks = 0;
         uint64_t n_slots = 0;
-        // Automatic slice size: about 64k slices over the batch's compressed MJPEG
-        // bits, 1024..4096 bits each (small batches want parallelism, large ones
-        // fewer slice boundaries).
-        uint32_t auto_bits = 1024;
-        {
-            uint64_t total_bits = 0;
-            for (size_t i = 0; i < n; i++)
-                if (items[i].codec == kCodecMjpeg) total_bits += 8 * (uint64_t)items[i].len;
-            while (auto_bits < 4096 && (uint64_t)auto_bits * 2 * 65536 <= total_bits) auto_bits *= 2;
-        }
+        uint64_t total_bits = 0;  // compressed MJPEG bits of the batch
+        for (size_t i = 0; i < n; i++)
+            if (items[i].codec == kCodecMjpeg) total_bits += 8 * (uint64_t)items[i].len;
+        const SlicePlan auto_plan = auto_slices(total_bits);
+        uint32_t most_paths = 1;
         std::vector<size_t> in_off(n, 0), out_off(n, 0), planes_off(n, SIZE_MAX);
         std::vector<std::array<size_t, 6>> plane_geom(n);  // (offset, bytes) of up to 3 planes
         // per JPEG plan: JFrame index (or -1)
@@ -864,11 +883,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                         symbols.insert(symbols.end(), key.begin() + 16, key.end() - 1);
                         f = lut_index.emplace(key, (uint32_t)luts.size()).first;
                         luts.push_back(L);
-                        lut_sub_first.push_back((uint32_t)lut_sub.size());
-                        lut_sym.resize(luts.size() << kHuffFastBits);
-                        lut_skip.resize(luts.size() << kHuffFastBits);
-                        build_sym(key.data(), key.size() - 1, s >= 4, lut_sym.data() + ((luts.size() - 1) << kHuffFastBits),
-                                  lut_skip.data() + ((luts.size() - 1) << kHuffFastBits), &lut_sub);
+                        lut_meta.push_back(build_sym(key.data(), key.size() - 1, s >= 4, &lut_sym, &lut_skip));
                     }
                     F.lut[s] = f->second;
                 }
@@ -901,15 +916,29 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                     }
                     brecs.push_back(R);
                 }
+                F.shared_tabs = F.n_dc <= kSharedTabs && F.n_ac <= kSharedTabs;
+                for (uint32_t t = 0; t < 4; t++) {
+                    if (t < F.n_dc) F.shared_tabs &= lut_meta[F.dc_id[t]].len <= kSharedTab;
+                    if (t < F.n_ac) F.shared_tabs &= lut_meta[F.ac_id[t]].len <= kSharedTab;
+                }
                 F.rst_off = rst_total;
                 rst_total += p.n_intervals;
                 if (p.ncomp <= 4) {
-                    uint32_t slice_bits = slice_bits_ ? slice_bits_ : auto_bits;
+                    uint32_t slice_bits = slice_bits_ ? slice_bits_ : auto_plan.bits;
                     if (!slice_bits_) {
                         auto t = tuned.find(tune_class_of(p, it.len));
                         if (t != tuned.end()) slice_bits = t->second;
+                        // Intervals shorter than a slice are one slice each. An interval's slots start at
+                        // its bits / S plus its number (slice_plan_kernel), so a larger S leaves fewer slots
+                        // unused between them.
+                        const uint64_t four = 4 * 8 * (uint64_t)it.len / p.n_intervals;
+                        if (four < 4 * (uint64_t)slice_bits && four > slice_bits) slice_bits = (uint32_t)align_up(four, 32);
                     }
                     F.slice_bits = slice_bits;
+                    F.lead = auto_plan.lead;
+                    // (with one block per MCU, or one interval per slice, all guesses are alike)
+                    F.paths = p.ri * F.sched_len > 1 ? std::min<uint32_t>(auto_plan.paths, F.sched_len) : 1;
+                    most_paths = std::max(most_paths, F.paths);
                     F.slot_first = (uint32_t)n_slots;
                     F.slot_count = (uint32_t)align_up((8 * (uint64_t)it.len + slice_bits - 1) / slice_bits + p.n_intervals, kSliceThreads);
                     n_slots += F.slot_count;
@@ -1090,14 +1119,13 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         if (n_slots > 0xffffffffull) throw std::runtime_error("batch too large for the chunked entropy decoder");
         I.d_slot_item.ensure(std::max<size_t>(n_slots * 4, 256));
         I.d_sync.ensure(std::max<size_t>(n_slots * sizeof(SliceSync), 256));
-        I.d_spec.ensure(std::max<size_t>(n_slots * sizeof(SliceSpec), 256));
+        I.d_spec.ensure(std::max<size_t>(most_paths * n_slots * sizeof(SliceSpec), 256));
         I.d_prefix.ensure(std::max<size_t>(n_slots * sizeof(SlicePrefix), 256));
         I.d_events.ensure(std::max<size_t>(n_slots * sizeof(SliceEvent), 256));
         I.d_ivs.ensure(std::max<size_t>(items_small.size() * sizeof(IvInfo), 256));
         I.d_ivkey.ensure(std::max<size_t>(items_small.size() * 8, 256));
         if (blocks > 0xffffffffull) throw std::runtime_error("batch too large for the chunked entropy decoder");
         I.d_ivpend.ensure(std::max<size_t>(items_small.size() * 4, 256));
-        I.d_synclist.ensure(std::max<size_t>(2 * n_slots * 4, 256));
 
         uint8_t *d_in = I.d_in.as<uint8_t>();
         auto in_ptr = [&](size_t i) -> const uint8_t * { return items[i].dev_data ? items[i].dev_data : d_in + in_off[i]; };
@@ -1128,8 +1156,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         size_t o_jframes = blob.add_vec(jframes), o_jstates = blob.add_vec(jstates),
                o_tile_first = blob.add_vec(tile_first), o_sched = blob.add_vec(sched), o_brec = blob.add_vec(brecs), o_comps = blob.add_vec(comps),
                o_luts = blob.add_vec(luts), o_symbols = blob.add_vec(symbols), o_quant = blob.add_vec(quant);
-        size_t o_sym = blob.add_vec(lut_sym), o_skip = blob.add_vec(lut_skip), o_sub = blob.add_vec(lut_sub),
-               o_subfirst = blob.add_vec(lut_sub_first);
+        size_t o_sym = blob.add_vec(lut_sym), o_skip = blob.add_vec(lut_skip), o_meta = blob.add_vec(lut_meta);
         std::vector<uint2> all_items(items_small);
         all_items.insert(all_items.end(), items_big.begin(), items_big.end());
         size_t o_items = blob.add_vec(all_items), o_ranges = blob.add_vec(ranges), o_idctcta = blob.add_vec(idct_cta), o_itemok = blob.add_vec(item_ok),
@@ -1146,8 +1173,8 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         // again whole
         uint32_t zero_counters[8] = {};
         size_t o_fixcount = blob.add(zero_counters, sizeof(zero_counters));
-        uint32_t zero_sync[kSyncCounters] = {};
-        size_t o_sync = blob.add(zero_sync, sizeof(zero_sync));
+        uint32_t zero_left[4] = {};  // unsettled intervals
+        size_t o_left = blob.add(zero_left, sizeof(zero_left));
         size_t blob_size = std::max<size_t>(blob.bytes.size(), 256);
         I.d_blob.ensure(blob_size);
         I.h_blob.ensure(blob_size);
@@ -1212,16 +1239,15 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         JL.ivs = I.d_ivs.as<IvInfo>();
         JL.sync = I.d_sync.as<SliceSync>();
         JL.spec = I.d_spec.as<SliceSpec>();
+        JL.paths = most_paths;
         JL.prefix = I.d_prefix.as<SlicePrefix>();
         JL.events = I.d_events.as<SliceEvent>();
         JL.iv_key = I.d_ivkey.as<unsigned long long>();
         JL.iv_pend = I.d_ivpend.as<uint32_t>();
-        JL.sync_list = I.d_synclist.as<uint32_t>();
-        JL.sync_count = reinterpret_cast<uint32_t *>(db + o_sync);
+        JL.sync_left = reinterpret_cast<uint32_t *>(db + o_left);
+        JL.lut_meta = reinterpret_cast<const LutMeta *>(db + o_meta);
         JL.sym = reinterpret_cast<const uint16_t *>(db + o_sym);
         JL.skip = reinterpret_cast<const uint32_t *>(db + o_skip);
-        JL.sub = reinterpret_cast<const uint16_t *>(db + o_sub);
-        JL.sub_first = reinterpret_cast<const uint32_t *>(db + o_subfirst);
         JL.fixw = I.d_fixtab.as<long long>();
         if (!jframes.empty()) {
             launch_jpeg_scan(JL, s);
@@ -1321,7 +1347,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             // states them so that no change of shape can replay a stale graph
             for (uintptr_t v : {(uintptr_t)jframes.size(), (uintptr_t)tile_first.back(), (uintptr_t)luts.size(),
                                 (uintptr_t)items_small.size(), (uintptr_t)n_items, (uintptr_t)ranges.size(),
-                                (uintptr_t)idct_cta.back(), (uintptr_t)n_slots,
+                                (uintptr_t)idct_cta.back(), (uintptr_t)n_slots, (uintptr_t)most_paths,
                                 (uintptr_t)blocks, (uintptr_t)dframes.size(), (uintptr_t)seg_first.back(),
                                 (uintptr_t)dif_first.back(), (uintptr_t)dv_blocks, (uintptr_t)rgbjobs.size(),
                                 (uintptr_t)rgbcta.back()})
@@ -1333,7 +1359,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             for (const DevBuf *b : {&I.d_in, &I.d_tok, &I.d_blob, &I.d_tile_tok, &I.d_tile_rst, &I.d_rsts,
                                     &I.d_results, &I.d_coef, &I.d_dc, &I.d_planes, &I.d_out, &I.d_dvcoef, &I.d_modes,
                                     &I.d_flags, &I.d_segerr, &I.d_vlc, &I.d_fix, &I.d_slot_item, &I.d_ivs, &I.d_sync,
-                                    &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_ivpend, &I.d_synclist})
+                                    &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_ivpend})
                 key.push_back((uintptr_t)b->ptr);
             for (size_t i = 0; i < n; i++) {
                 const Item &it = items[i];

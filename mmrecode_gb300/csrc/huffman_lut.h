@@ -94,59 +94,68 @@ inline void build_lut(const uint8_t *key, size_t key_len, uint32_t sym_off, bool
     lut->nsym = (uint32_t)(key_len - 16);
 }
 
-// The chunked decoder's lookups of the same table (plan.h: sym, skip and its blocks of
-// `sub`, appended to *sub; skip only for AC tables). The table is not oversubscribed.
-inline void build_sym(const uint8_t *key, size_t key_len, bool ac, uint16_t *sym, uint32_t *skip,
-                      std::vector<uint16_t> *sub) {
+// The chunked decoder's lookups of the same table (plan.h), appended to *sym and
+// *skip (which stay parallel; skip is filled for AC tables). The table is not
+// oversubscribed.
+inline LutMeta build_sym(const uint8_t *key, size_t key_len, bool ac, std::vector<uint16_t> *sym,
+                         std::vector<uint32_t> *skip) {
     constexpr uint32_t FB = kHuffFastBits;
-    for (uint32_t x = 0; x < (1u << FB); x++) sym[x] = (uint16_t)kSymInvalid;
     const uint8_t *symbols = key + 16;
-    const size_t first_sub = sub->size();
+    LutMeta m;
+    m.off = (uint32_t)sym->size();
+    m.first_long = m.last = 0xffffffffu;
+    uint64_t end = 0;  // of the used code space, left-aligned
+    {
+        uint64_t code = 0;
+        for (uint32_t l = 1; l <= 16; l++, code <<= 1) {
+            if (l == FB + 1) m.first_long = (uint32_t)(code << (32 - l) > 0xffffffffull ? 0xffffffffu : code << (32 - l));
+            code += key[l - 1];
+            if (key[l - 1]) end = code << (32 - l);
+        }
+    }
+    if (end <= m.first_long) m.first_long = 0xffffffffu;  // no long codes
+    if (m.first_long != 0xffffffffu && (0x100000000ull - m.first_long) >> 16 > kSharedLong && end <= 0xffffffffull)
+        m.last = (uint32_t)end;
+    m.len = (lut_entry_index(m.last, m.first_long) + 1 + 7) & ~7u;
+    sym->resize(m.off + m.len, 0);
+    skip->resize(m.off + m.len, 0);
+    uint16_t *e = sym->data() + m.off;
     uint32_t code = 0, k = 0;
     for (uint32_t l = 1; l <= 16; l++, code <<= 1) {
         for (uint32_t i = 0; i < key[l - 1] && k < key_len - 16; i++, code++, k++) {
             const uint32_t s = symbols[k], size = ac ? s & 15 : s, run = s >> 4;
             uint32_t adv = ac ? run + 1 : 1;
-            bool ok = size <= (ac ? 10u : 11u);
+            if (size > (ac ? 10u : 11u)) continue;
             if (ac && size == 0) {
-                ok = run == 0 || run == 15;
+                if (run != 0 && run != 15) continue;
                 if (run == 0) adv = kSymEob;
             }
-            const uint32_t rest = (size << 4) | (adv << 8);
-            if (l <= FB) {
-                const uint16_t e = (uint16_t)(ok ? rest | l : kSymInvalid);
-                const uint32_t at = code << (FB - l), n = 1u << (FB - l);
-                for (uint32_t j = 0; j < n && at + j < (1u << FB); j++) sym[at + j] = e;
-                continue;
+            const uint32_t first = lut_entry_index(code << (32 - l), m.first_long);
+            const uint32_t n = l <= FB ? 1u << (FB - l) : 1u << (16 - l);
+            // (a long code's patterns may straddle an 11-bit prefix: one entry further each)
+            for (uint32_t j = 0; j < n; j++) {
+                const uint32_t at = l <= FB ? first + j : lut_entry_index((code << (32 - l)) + (j << 16), m.first_long);
+                if (at < m.len) e[at] = (uint16_t)(l | size << 5 | adv << 9);
             }
-            const uint32_t prefix = code >> (l - FB);
-            if (prefix >= (1u << FB)) continue;
-            if (sym[prefix] == kSymInvalid) {
-                sym[prefix] = (uint16_t)(kSymEscape | (uint32_t)((sub->size() - first_sub) / kSubEntries));
-                sub->insert(sub->end(), kSubEntries, (uint16_t)kSymInvalid);
-            }
-            uint16_t *block = sub->data() + first_sub + (size_t)(sym[prefix] & 0x7fffu) * kSubEntries;
-            const uint32_t low = (code << (16 - l)) & (kSubEntries - 1), n = 1u << (16 - l);
-            for (uint32_t j = 0; j < n && low + j < kSubEntries; j++)
-                block[low + j] = (uint16_t)(ok ? rest | (l - FB) : kSymInvalid);
         }
     }
-    if (!ac) return;
-    for (uint32_t x = 0; x < (1u << FB); x++) {
-        const uint32_t e = sym[x];
-        if (e & kSymEscape) {
-            skip[x] = kSkipEscape;
-            continue;
+    if (!ac) return m;
+    uint32_t *p = skip->data() + m.off;
+    for (uint32_t x = 0; x < m.len; x++) {
+        if (!e[x]) continue;
+        const uint32_t cl = e[x] & 31, len = cl + ((e[x] >> 5) & 15), adv = e[x] >> 9;
+        uint32_t len2 = len, adv2 = adv;
+        // (windows below first_long have no long entries before theirs: x is the prefix)
+        if (cl <= FB && adv < kSymEob && len < FB) {
+            const uint32_t y = (x << len) & ((1u << FB) - 1);  // what is left of the 11 bits, then zeros
+            if ((uint64_t)y << (32 - FB) < m.first_long && e[y] && (e[y] & 31u) <= FB - len) {
+                len2 += (e[y] & 31) + ((e[y] >> 5) & 15);
+                adv2 += e[y] >> 9;
+            }
         }
-        const uint32_t cl = e & 15, len = cl + ((e >> 4) & 15), adv = e >> 8;
-        uint32_t one = len | adv << 5, two = one;
-        if (adv < kSymEob && len < FB) {
-            const uint32_t e2 = sym[(x << len) & ((1u << FB) - 1)];
-            if (!(e2 & kSymEscape) && (e2 & 15) <= FB - len)  // (it depends on its code bits only)
-                two = (len + (e2 & 15) + ((e2 >> 4) & 15)) | (adv + (e2 >> 8)) << 5;
-        }
-        skip[x] = one | two << 12;
+        p[x] = adv << 24 | len << 16 | adv2 << 8 | len2;
     }
+    return m;
 }
 
 }  // namespace mmr

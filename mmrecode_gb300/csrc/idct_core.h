@@ -75,10 +75,10 @@ __device__ __forceinline__ uint8_t exact_sample(const int32_t *c, int stride, in
 // are in c (shared memory; all 32 lanes of the warp call this together). First
 // the warp forms each sample's exact fixed-point value (exact_fixed.h, offset
 // +128); the samples still too close to a half-integer take the reference
-// order: once for the whole block when it has no nonzero AC coefficient (every
-// M[x][0] is the same literal, so all 64 reference samples are equal: DC-only
-// blocks whose value is a half-integer leave all 64 undecided), else one sample
-// per lane in parallel. put(y, x, sample) may run on any lane.
+// order, one sample per lane in parallel. A block with no nonzero AC coefficient
+// is evaluated once (DC-only blocks whose value is a half-integer leave all 64
+// samples undecided: sample by sample they were half the time of the 4:4:4
+// transform of pictures with flat areas). put(y, x, sample) may run on any lane.
 template <class Put>
 __device__ __forceinline__ void settle_samples(const long long *fixw, const int32_t *c, unsigned long long mask,
                                                Put put) {
@@ -87,6 +87,17 @@ __device__ __forceinline__ void settle_samples(const long long *fixw, const int3
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c1 += __shfl_xor_sync(0xffffffffu, c1, o);
     const bool flat = __ballot_sync(0xffffffffu, (lane != 0 && c[lane] != 0) || c[lane + 32] != 0) == 0;
+    if (flat) {  // every M[x][0] is the same literal: all 64 samples are equal, one evaluation settles them
+        int v = -1;
+        if (c1 < kFixMaxC1) v = fixed_round(fixw[0] * (long long)c[0], (int32_t)c1, 128);
+        if (v < 0) {
+            if (lane == 0) v = exact_sample(c, 8, 0, 0);
+            v = __shfl_sync(0xffffffffu, v, 0);
+        }
+        for (int b = lane; b < 64; b += 32)
+            if (mask >> b & 1) put(b >> 3, b & 7, (uint8_t)v);
+        return;
+    }
     unsigned long long left = 0;  // samples for the reference order
     for (unsigned long long m = mask; m; m &= m - 1) {
         const int b = __ffsll((long long)m) - 1, y = b >> 3, x = b & 7;
@@ -97,17 +108,6 @@ __device__ __forceinline__ void settle_samples(const long long *fixw, const int3
         } else {
             left |= 1ull << b;
         }
-    }
-    if (!left) return;
-    if (flat) {
-        uint8_t v = 0;
-        if (lane == 0) v = exact_sample(c, 8, 0, 0);
-        v = (uint8_t)__shfl_sync(0xffffffffu, (uint32_t)v, 0);
-        for (unsigned long long m = left; m; m &= m - 1) {
-            const int b = __ffsll((long long)m) - 1;
-            if (((b ^ lane) & 31) == 0) put(b >> 3, b & 7, v);  // lanes b and b - 32 share the stores
-        }
-        return;
     }
     while (left) {  // lane i takes the i-th remaining sample
         unsigned long long m = left;

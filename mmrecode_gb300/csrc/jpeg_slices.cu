@@ -14,19 +14,20 @@
 // finds the states (code lengths and coefficient advances, two symbols per lookup,
 // nothing stored), then one from the true states that writes the levels.
 //
-//   slice_plan     per frame: interval token ranges, slice counts, slot -> interval map
-//   slice_spec     the lean decode of every slice from a guessed state spec_lead(S) bits
+//   slice_plan     per interval: token range, slices, slots
+//   slice_spec     the lean decode of every slice from a guessed state JFrame::lead bits
 //                  before it (the first slice from the true one) to its exit; keeps the
-//                  first block boundary past each of eight marks (checkpoints)
-//   slice_match    slices whose predecessor's exit is their own first boundary are
-//                  settled; the others are listed
-//   slice_sync     (kSyncPasses passes) listed slices decode again from their
-//                  predecessor's exit until they meet one of their checkpoints (then
-//                  the rest is known) or their end; a changed exit lists the next slice
-//   slice_fix      per interval with slices still listed: walks its slices in order
-//                  until every start equals the previous exit. Then slice 0 starts in
-//                  the true state and each exit is the true state at that point, so
-//                  every start is the true one.
+//                  first block boundary past each of eight marks (checkpoints). Small
+//                  batches decode each slice from several guesses (JFrame::paths)
+//   slice_sync     (one to kSyncPasses passes) a slice whose start is not its predecessor's exit
+//                  takes it: where that is the first boundary of a speculative decode the
+//                  rest is known, else it decodes again from there until it meets one of
+//                  the checkpoints or its end; each CTA repeats this over its slices until
+//                  nothing changes
+//   slice_fix      per interval in which the last pass changed the last exit of a CTA:
+//                  walks its slices in order until every start equals the previous exit.
+//                  Then slice 0 starts in the true state and each exit is the true state
+//                  at that point, so every start is the true one.
 //   slice_prefix   per interval: block index and DC predictors at each slice start
 //   slice_decode   from the true states: quantised AC levels, dequantised DC, and each
 //                  slice's first event (an error, or the interval's last block completed)
@@ -38,11 +39,12 @@
 // the serial decoder stops at.
 //
 // Both decodes are bound by the instructions per symbol and by how few lanes of a
-// warp take the same path: a block ends every 10 to 60 symbols, at a different step
+// warp take the same path: a block ends every 5 to 60 symbols, at a different step
 // in each lane, and what happens there (the next tables, the DC difference, 128
-// bytes of levels) costs more than a symbol. So lanes take kSteps symbols (or pairs)
-// at a time without a branch, a lane whose block has ended standing still (its table
-// entry reads as zero), and the block ends are handled once per kSteps.
+// bytes of levels) costs more than a symbol. So lanes take a few symbols (or pairs)
+// at a time without a branch, a lane whose block has ended, or whose next bits are no
+// valid symbol, standing still (its table entry reads as zero), and what ended is
+// handled once per group of steps.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -56,13 +58,22 @@ namespace {
 
 constexpr unsigned long long kStErr = ~0ull;        // no state: the decode failed before this point
 constexpr unsigned long long kStGuess = ~0ull - 1;  // start not yet derived from the predecessor
+
+// Slices only ever take real states from their predecessors. After a true error the
+// slices that follow keep what they guessed: they may decode nonsense, but events count
+// by slice, so theirs come after the one that matters.
+__device__ __forceinline__ bool is_state(unsigned long long x) { return x < kStGuess; }
+
 constexpr int kStride = 72;  // int16 per staged block: 64 levels, and 64.. for what EOB steps store
-constexpr int kKeyBits = 26;
-constexpr int kSpecSteps = 4;    // lookups between block-end checks, lean decode
-constexpr int kDecodeSteps = 4;  // and final decode
-constexpr uint32_t kTab = 1u << kHuffFastBits;
+#ifndef MMR_SPEC_STEPS
+#define MMR_SPEC_STEPS 4
+#endif
+#ifndef MMR_DECODE_STEPS
+#define MMR_DECODE_STEPS 4
+#endif
+constexpr int kSpecSteps = MMR_SPEC_STEPS;      // lookups per group, lean decode
+constexpr int kDecodeSteps = MMR_DECODE_STEPS;  // symbols per group, final decode
 __constant__ uint8_t c_slice_zz[64] = MMR_ZIGZAG_INIT;
-constexpr uint32_t kMostShared = 2;  // DC and AC tables a CTA keeps in shared memory, of each
 
 __device__ __forceinline__ unsigned long long pack_state(unsigned long long p, uint32_t si) { return (p << 8) | si; }
 
@@ -115,21 +126,30 @@ __device__ __forceinline__ void window_init(Window &r, const uint8_t *tok, unsig
 
 __device__ __forceinline__ uint32_t window_bits(const Window &r) { return __funnelshift_l(r.w1, r.w0, r.off); }
 
+// n < 32. Predicated, so that lanes crossing a word at different steps stay together.
 __device__ __forceinline__ void window_take(Window &r, uint32_t n) {
-    r.off += n;
-    if (r.off >= 32) {
-        r.off -= 32;
-        r.w0 = r.w1;
-        r.w1 = bswap32(r.pf);
-        r.pf = __ldg(r.next);
-        r.next++;
-    }
+    asm("{\n\t"
+        ".reg .pred p;\n\t"
+        "add.u32 %0, %0, %5;\n\t"
+        "setp.ge.u32 p, %0, 32;\n\t"
+        "@p mov.b32 %1, %2;\n\t"
+        "@p prmt.b32 %2, %3, 0, 0x0123;\n\t"
+        "@p ld.global.nc.u32 %3, [%4];\n\t"
+        "@p add.u64 %4, %4, 4;\n\t"
+        "and.b32 %0, %0, 31;\n\t"
+        "}"
+        : "+r"(r.off), "+r"(r.w0), "+r"(r.w1), "+r"(r.pf), "+l"(r.next)
+        : "r"(n));
 }
 
-// Bits taken since the reader stood at bit `bit0` of the token stream at `tok`
-// (modulo 2^32: a slice and its lead stay far below).
-__device__ __forceinline__ uint32_t window_pos(const Window &r, const uint8_t *tok, uint32_t bit0) {
-    return (uint32_t)(r.next - 3 - reinterpret_cast<const uint32_t *>(tok)) * 32 + r.off - bit0;
+// What window_pos subtracts for positions counted from bit `bit0` of the tokens.
+__device__ __forceinline__ uint32_t window_zero(const uint8_t *tok, unsigned long long bit0) {
+    return (uint32_t)reinterpret_cast<uintptr_t>(tok) * 8 + 96 + (uint32_t)bit0;
+}
+
+// Position of the window (modulo 2^32: a slice and its lead stay far below).
+__device__ __forceinline__ uint32_t window_pos(const Window &r, uint32_t zero) {
+    return (uint32_t)reinterpret_cast<uintptr_t>(r.next) * 8 + r.off - zero;
 }
 
 // The signed value of `size` magnitude bits at the top of t (receive_extend,
@@ -141,528 +161,560 @@ __device__ __forceinline__ int32_t extend(uint32_t t, uint32_t size) {
     return (int32_t)((w ^ neg) - neg);
 }
 
-// A code of more than kHuffFastBits bits: its entry (code bits past the first 11,
-// magnitude size, advance), or the invalid marker.
-__device__ __noinline__ uint32_t sub_entry(const JpegLaunch &L, uint32_t lut, uint32_t e, uint32_t window) {
-    if (e == kSymInvalid) return e;
-    return __ldg(L.sub + __ldg(L.sub_first + lut) + (e & 0x7fffu) * kSubEntries + ((window >> 16) & (kSubEntries - 1)));
-}
-
 // --------------------------------------------------------------- tables ---
 //
-// Lookup tables of the CTA's frame. Frames with at most two DC and two AC tables
-// (all but exotic ones) keep them in shared memory, where 32 lanes' lookups cost a
-// few bank conflicts instead of as many L1 lines; offsets count table entries from
-// s_tab. Others read the batch's tables.
+// Lookup tables as a decode reads them. Where a frame's tables fit (JFrame::
+// shared_tabs: all but exotic ones) each CTA, whose slots are all of one frame, keeps
+// them in shared memory: 32 lanes' lookups there cost a few bank conflicts instead of
+// as many L1 lines, and no table byte is fetched from L2 in the middle of a decode.
 
-// What the lean decode needs of an MCU block: its component and tables (the frame's
-// own numbers where they are in shared memory, else the batch's).
-struct BlockTabs {
-    uint32_t comp, dc, ac;
+// A table: its first entry (shared: byte address in shared memory; else entry in the
+// batch's tables), and the window limits of lut_entry_index.
+struct Tab {
+    uint32_t at, first_long, last;
 };
+
+// Per MCU block: its component and tables.
+struct BlockTabs {
+    Tab dc, ac;
+    uint32_t comp;
+};
+
+__device__ __forceinline__ Tab batch_tab(const JpegLaunch &L, uint32_t lut) {
+    const LutMeta m = L.lut_meta[lut];
+    return Tab{m.off, m.first_long, m.last};
+}
+
+__device__ __forceinline__ BlockTabs batch_tabs(const JpegLaunch &L, const JBlockRec &R) {
+    return BlockTabs{batch_tab(L, R.dc_lut), batch_tab(L, R.ac_lut), R.comp};
+}
+
+// The sym or skip entry of window w; 0 unless `on`.
+template <bool kShared>
+__device__ __forceinline__ uint32_t sym_entry(const JpegLaunch &L, const Tab &t, uint32_t w, bool on) {
+    uint32_t e = 0;
+    if (kShared) {
+        const uint32_t a = t.at + 2 * lut_entry_index(w, t.first_long);
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.u16 %0, [%1];\n\t}"
+            : "+r"(e) : "r"(a), "r"((uint32_t)on));
+    } else if (on) {
+        e = __ldg(L.sym + t.at + lut_entry_index(min(w, t.last), t.first_long));
+    }
+    return e;
+}
+
+template <bool kShared>
+__device__ __forceinline__ uint32_t skip_entry(const JpegLaunch &L, const Tab &t, uint32_t w, int k) {
+    uint32_t e = 0;
+    if (kShared) {
+        const uint32_t a = t.at + 4 * lut_entry_index(w, t.first_long);
+        asm("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, 64;\n\t@p ld.shared.u32 %0, [%1];\n\t}"
+            : "+r"(e) : "r"(a), "r"(k));
+    } else if (k < 64) {
+        e = __ldg(L.skip + t.at + lut_entry_index(min(w, t.last), t.first_long));
+    }
+    return e;
+}
+
+// (a multiple of 16 bytes; four loads in flight per thread)
+__device__ __forceinline__ void copy16(void *dst, const void *src, uint32_t bytes) {
+    const uint32_t n = bytes / 16;
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 4 * kSliceThreads) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (i0 + u * kSliceThreads < n) v[u] = __ldg(reinterpret_cast<const uint4 *>(src) + i0 + u * kSliceThreads);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (i0 + u * kSliceThreads < n) reinterpret_cast<uint4 *>(dst)[i0 + u * kSliceThreads] = v[u];
+    }
+}
+
+__device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // ------------------------------------------------------------------ plan ---
 
-constexpr int kPlanThreads = 512;
-constexpr int kPlanPer = 8;  // consecutive intervals per thread and step
+// Thread per restart interval. An interval's slots start at its first token's bits / S
+// plus its number: such ranges never overlap (floor(a) + ceil(b) <= floor(a + b) + 1)
+// and need no prefix sum over the frame; slots between them stay unused. (A warp per
+// frame, 32 intervals per step, took 6.0 of the 17.1 ms of a mixed batch whose 4:4:4
+// frames have up to 32k intervals; a CTA per frame 0.36 ms.)
+constexpr int kPlanThreads = 128;
 
-// CTA per frame: kPlanThreads * kPlanPer intervals per step, one prefix sum each (a
-// warp per frame with 32 intervals per step took 6.0 ms of the 17.1 ms of a mixed
-// batch whose 4:4:4 frames have up to 32k intervals).
 __global__ void __launch_bounds__(kPlanThreads) slice_plan_kernel(JpegLaunch L) {
-    __shared__ uint32_t s_warp[kPlanThreads / 32];
-    const uint32_t f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const JFrame &F = L.frames[f];
-    if (!F.decode || F.ncomp > 4) return;
-    const JState &st = L.states[f];
-    const unsigned long long termv = st.term;
-    const bool scan_ok = termv != ~0ull && !((termv >> 8) & 1);
-    const uint32_t n_int = F.n_intervals;
-    const uint32_t n_rst = min(st.n_rst, n_int), n_tok = st.n_tokens;
-    const RstEntry *rst = L.rsts + F.rst_off;
-    const uint32_t S = F.slice_bits;
-    uint32_t used = 0;
-    for (uint32_t c = 0; c < n_int; c += kPlanThreads * kPlanPer) {
-        const uint32_t iv0 = c + tid * kPlanPer;
-        uint32_t start[kPlanPer], barrier[kPlanPer], n_s[kPlanPer], sum = 0;
-        uint32_t prev = iv0 == 0 ? 0 : iv0 - 1 < n_rst ? rst[iv0 - 1].tok : 0xffffffffu;
-#pragma unroll
-        for (int i = 0; i < kPlanPer; i++) {
-            const uint32_t iv = iv0 + i;
-            n_s[i] = 0;
-            start[i] = prev;
-            barrier[i] = prev;
-            const uint32_t end = iv < n_rst ? rst[iv].tok : n_tok;
-            // an interval that no RST precedes: an earlier one fails its restart check
-            if (iv < n_int && scan_ok && prev != 0xffffffffu) {
-                barrier[i] = end;
-                n_s[i] = max(1u, (uint32_t)(((unsigned long long)(end - prev) * 8 + S - 1) / S));
-            }
-            prev = iv < n_rst ? end : 0xffffffffu;
-            sum += n_s[i];
+    const uint32_t item = blockIdx.x * kPlanThreads + threadIdx.x, lane = threadIdx.x & 31;
+    uint32_t first = 0, n_s = 0, limit = 0;  // slots [first, first + n_s) used, up to limit unused
+    if (item < L.n_items_small) {
+        const uint32_t f = L.items[item].x, iv = L.items[item].y;
+        const JFrame &F = L.frames[f];
+        const JState &st = L.states[f];
+        const unsigned long long termv = st.term;
+        const bool scan_ok = termv != ~0ull && !((termv >> 8) & 1);
+        const uint32_t n_rst = min(st.n_rst, F.n_intervals), S = F.slice_bits;
+        const RstEntry *rst = L.rsts + F.rst_off;
+        uint32_t start = 0, end = 0;
+        // an interval that no RST precedes: an earlier one fails its restart check
+        const bool dec = scan_ok && iv <= n_rst;
+        if (dec) {
+            start = iv ? rst[iv - 1].tok : 0;
+            end = iv < n_rst ? rst[iv].tok : st.n_tokens;
+            n_s = max(1u, (uint32_t)(((unsigned long long)(end - start) * 8 + S - 1) / S));
+            first = F.slot_first + (uint32_t)((unsigned long long)start * 8 / S) + iv;
+            limit = iv == n_rst || iv + 1 == F.n_intervals
+                        ? F.slot_first + F.slot_count
+                        : F.slot_first + (uint32_t)((unsigned long long)end * 8 / S) + iv + 1;
+        } else if (iv == 0) {
+            first = F.slot_first;
+            limit = first + F.slot_count;
         }
-        uint32_t incl = sum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= (uint32_t)d) incl += o;
-        }
-        __syncthreads();  // (the last step's sums are read)
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        uint32_t first = used + incl - sum, total = 0;
-#pragma unroll
-        for (uint32_t w = 0; w < kPlanThreads / 32; w++) {
-            if (w < warp) first += s_warp[w];
-            total += s_warp[w];
-        }
-        const bool fits = used + total <= F.slot_count;  // always: slot_count bounds the token count
-#pragma unroll
-        for (int i = 0; i < kPlanPer; i++) {
-            const uint32_t iv = iv0 + i;
-            if (!fits) n_s[i] = 0;
-            if (iv < n_int) {
-                const uint32_t mcu0 = iv * F.ri, mcu1 = min(mcu0 + F.ri, F.total_mcus);
-                IvInfo v;
-                v.start = start[i];
-                v.barrier = barrier[i];
-                v.slot_first = F.slot_first + first;
-                v.n_slices = n_s[i];
-                v.blocks = n_s[i] ? (mcu1 - mcu0) * F.sched_len : 0;
-                v.flags = n_s[i] && iv < n_rst ? 1u : 0u;
-                v.frame = f;
-                v.pad = 0;
-                L.ivs[F.item_base + iv] = v;
-                L.iv_key[F.item_base + iv] = ~0ull;
-                L.iv_pend[F.item_base + iv] = 0xffffffffu;
-            }
-            const bool own = n_s[i] <= 8;
-            if (own)
-                for (uint32_t x = 0; x < n_s[i]; x++) L.slot_item[F.slot_first + first + x] = F.item_base + iv;
-            for (uint32_t m = __ballot_sync(0xffffffffu, !own); m; m &= m - 1) {  // the warp fills long ones
-                const int src = __ffs(m) - 1;
-                const uint32_t nt = __shfl_sync(0xffffffffu, n_s[i], src), ft = __shfl_sync(0xffffffffu, first, src);
-                const uint32_t it = __shfl_sync(0xffffffffu, F.item_base + iv, src);
-                for (uint32_t x = lane; x < nt; x += 32) L.slot_item[F.slot_first + ft + x] = it;
-            }
-            first += n_s[i];
-        }
-        if (fits) used += total;
+        const uint32_t mcu0 = iv * F.ri, mcu1 = min(mcu0 + F.ri, F.total_mcus);
+        IvInfo v;
+        v.start = start;
+        v.barrier = end;
+        v.slot_first = first;
+        v.n_slices = n_s;
+        v.blocks = (mcu1 - mcu0) * F.sched_len;
+        v.flags = iv < n_rst ? 1u : 0u;
+        v.frame = f;
+        v.pad = 0;
+        L.ivs[item] = v;
+        L.iv_key[item] = ~0ull;
+        L.iv_pend[item] = 0xffffffffu;
     }
-    for (uint32_t x = used + tid; x < F.slot_count; x += kPlanThreads) L.slot_item[F.slot_first + x] = 0xffffffffu;
+    const bool own = limit - first <= 4;
+    if (own)
+        for (uint32_t x = first; x < limit; x++) L.slot_item[x] = x - first < n_s ? item : 0xffffffffu;
+    for (uint32_t m = __ballot_sync(0xffffffffu, !own); m; m &= m - 1) {  // the warp fills longer ones
+        const int src = __ffs(m) - 1;
+        const uint32_t ft = __shfl_sync(0xffffffffu, first, src), nt = __shfl_sync(0xffffffffu, n_s, src);
+        const uint32_t lt = __shfl_sync(0xffffffffu, limit, src), it = __shfl_sync(0xffffffffu, item, src);
+        for (uint32_t x = ft + lane; x < lt; x += 32) L.slot_item[x] = x - ft < nt ? it : 0xffffffffu;
+    }
 }
 
 // ------------------------------------------------------------ lean decode ---
 
-// Tables as the lean decode reads them: kShared from the CTA's copies, else the batch's.
-template <bool kShared>
-struct LeanTabs {
-    const uint32_t *skip;  // AC: one or two symbols per entry (huffman_lut.h)
-    const uint16_t *sym;   // DC
-    const uint32_t *local;   // kShared: per MCU block JBlockRec::local
-    const uint32_t *ids;     // kShared: batch index of each of the frame's tables, DC then AC
-    const JBlockRec *recs;   // the frame's records
-    __device__ __forceinline__ uint32_t skip_at(uint32_t i) const { return kShared ? skip[i] : __ldg(skip + i); }
-    __device__ __forceinline__ uint32_t sym_at(uint32_t i) const { return kShared ? sym[i] : __ldg(sym + i); }
-    __device__ __forceinline__ uint32_t dc_lut(uint32_t t) const { return kShared ? ids[t] : t; }
-    __device__ __forceinline__ uint32_t ac_lut(uint32_t t) const { return kShared ? ids[kMostShared + t] : t; }
-    __device__ __forceinline__ BlockTabs block(uint32_t si) const {
-        if (kShared) {
-            const uint32_t p = local[si];
-            return BlockTabs{p & 0xff, (p >> 8) & 0xff, p >> 16};
-        }
-        const JBlockRec &R = recs[si];
-        return BlockTabs{R.comp, R.dc_lut, R.ac_lut};
-    }
+// The lean decode's tables in shared memory: DC and AC (pair) tables of the CTA's
+// frame, then per MCU block its BlockTabs.
+struct LeanSmem {
+    __align__(16) uint32_t skip[kSharedTabs][kSharedTab];
+    __align__(16) uint16_t sym[kSharedTabs][kSharedTab];
+    BlockTabs tabs[kMaxSched];
+    int32_t dc[4][kSliceThreads];  // DC sums of the slice, per component
+    uint32_t frame;
 };
 
-// State of a lean decode between block boundaries.
+__device__ __forceinline__ void lean_load(const JpegLaunch &L, const JFrame &F, LeanSmem &S) {
+    if (F.shared_tabs) {
+        for (uint32_t t = 0; t < F.n_dc; t++) {
+            const LutMeta m = L.lut_meta[F.dc_id[t]];
+            copy16(S.sym[t], L.sym + m.off, 2 * m.len);
+        }
+        for (uint32_t t = 0; t < F.n_ac; t++) {
+            const LutMeta m = L.lut_meta[F.ac_id[t]];
+            copy16(S.skip[t], L.skip + m.off, 4 * m.len);
+        }
+    }
+    for (uint32_t i = threadIdx.x; i < F.sched_len; i += kSliceThreads) {
+        const JBlockRec &R = L.brec[F.sched_off + i];
+        BlockTabs b = batch_tabs(L, R);
+        if (F.shared_tabs) {
+            b.dc.at = shared_address(S.sym[(R.local >> 8) & 0xff]);
+            b.ac.at = shared_address(S.skip[R.local >> 16]);
+        }
+        S.tabs[i] = b;
+    }
+}
+
+// State of a lean decode.
 struct Lean {
     Window r;
-    int k;           // next coefficient; 64 or 96 and more: the block is complete, 65..95: invalid
-    uint32_t si;     // block of the MCU
-    uint32_t tab;    // its AC table's first entry
-    uint32_t blocks; // blocks started
+    int k;            // next coefficient; 64 or from 96 on: the block is complete, 65..95: overrun
+    uint32_t si;      // block of the MCU
+    Tab ac;           // its AC table
+    uint32_t blocks;  // blocks started
 };
 
-// kSpecSteps lookups (none for a lane whose block has ended).
+// kSpecSteps lookups (none for a lane whose block has ended). Returns 0 when the last
+// one found no valid symbol (or the block has ended).
 template <bool kShared>
-__device__ __forceinline__ void lean_steps(const JpegLaunch &L, const LeanTabs<kShared> &T, Lean &s) {
+__device__ __forceinline__ uint32_t lean_steps(const JpegLaunch &L, Lean &s) {
+    uint32_t e = 0;
 #pragma unroll
     for (int u = 0; u < kSpecSteps; u++) {
-        const uint32_t w = window_bits(s.r);
-        uint32_t e = 0;
-        if (s.k < 64) e = T.skip_at(s.tab + (w >> (32 - kHuffFastBits)));
-        if (e & kSkipEscape) {
-            const uint32_t lut = T.ac_lut(s.tab / kTab);
-            const uint32_t x = sub_entry(L, lut, __ldg(L.sym + lut * kTab + (w >> (32 - kHuffFastBits))), w);
-            if (x & kSymEscape) {
-                e = 0;
-                s.k = 80;
-            } else {
-                const uint32_t one = (kHuffFastBits + (x & 15) + ((x >> 4) & 15)) | ((x >> 8) & 127) << 5;
-                e = one | one << 12;
-            }
-        }
-        if (s.k + (int)((e >> 5) & 127) < 64) e >>= 12;  // the pair: its first symbol leaves the block open
-        window_take(s.r, e & 31);
-        s.k += (int)((e >> 5) & 127);
+        e = skip_entry<kShared>(L, s.ac, window_bits(s.r), s.k);
+        if (s.k + (int)(e >> 24) >= 64) e >>= 16;  // the first symbol ends the block: it alone
+        window_take(s.r, e & 0xff);
+        s.k += (int)((e >> 8) & 0xff);
     }
+    return e;
 }
 
-// The DC symbol at a block boundary: counts the block, adds its difference to
-// dc[component], and leaves the decode at its first AC symbol. False when invalid.
+__device__ __forceinline__ bool lean_complete(const Lean &s) { return s.k == 64 || s.k >= 96; }
+
+// The DC symbol at a block boundary: counts the block, adds its difference to its
+// component's sum, and leaves the decode at its first AC symbol. False when invalid.
 template <bool kShared>
-__device__ __forceinline__ bool lean_dc(const JpegLaunch &L, const LeanTabs<kShared> &T, Lean &s, int32_t *dc) {
-    const BlockTabs b = T.block(s.si);
+__device__ __forceinline__ bool lean_dc(const JpegLaunch &L, LeanSmem &S, Lean &s) {
+    const BlockTabs &b = S.tabs[s.si];
     s.blocks++;
-    uint32_t w = window_bits(s.r);
-    uint32_t e = T.sym_at(b.dc * kTab + (w >> (32 - kHuffFastBits)));
-    if (e & kSymEscape) {
-        e = sub_entry(L, T.dc_lut(b.dc), e, w);
-        if (e & kSymEscape) return false;
-        window_take(s.r, kHuffFastBits);
-        w = window_bits(s.r);
-    }
-    const uint32_t cl = e & 15, size = (e >> 4) & 15;
-    dc[b.comp] += extend(w << cl, size);
+    const uint32_t w = window_bits(s.r);
+    const uint32_t e = sym_entry<kShared>(L, b.dc, w, true), cl = e & 31, size = (e >> 5) & 15;
+    S.dc[b.comp][threadIdx.x] += extend(w << cl, size);
     window_take(s.r, cl + size);
-    s.tab = b.ac * kTab;
+    s.ac = b.ac;
     s.k = 1;
-    return true;
+    return e != 0;
 }
 
-__device__ __forceinline__ bool lean_invalid(const Lean &s) { return s.k > 64 && s.k < 96; }
+__device__ __forceinline__ void lean_clear(LeanSmem &S, Lean &s) {
+    s.blocks = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++) S.dc[c][threadIdx.x] = 0;
+}
 
-// Speculative decode of one slice (not its interval's last).
+__device__ __forceinline__ void lean_point(const LeanSmem &S, const Lean &s, unsigned long long state, SlicePoint &p) {
+    p.state = state;
+    p.blocks = s.blocks;
+#pragma unroll
+    for (int c = 0; c < 4; c++) p.dc[c] = S.dc[c][threadIdx.x];
+}
+
+// Speculative decode `path` of one slice (not its interval's last).
 template <bool kShared>
-__device__ __forceinline__ void spec_slice(const JpegLaunch &L, const LeanTabs<kShared> &T, const JFrame &F, uint32_t slot,
-                           const SliceRef &s, int32_t *dc) {
+__device__ __forceinline__ void spec_slice(const JpegLaunch &L, LeanSmem &S, const JFrame &F, uint32_t slot,
+                                           const SliceRef &s, uint32_t path) {
     const bool guess = s.j != 0;
-    const uint32_t S = F.slice_bits;
-    const unsigned long long nominal = (unsigned long long)s.j * S;
-    const uint32_t lead = guess ? (uint32_t)min((unsigned long long)spec_lead(S), nominal) : 0;
+    const uint32_t bits = F.slice_bits, sched_len = F.sched_len;
+    const unsigned long long nominal = (unsigned long long)s.j * bits;
+    const uint32_t lead = guess ? (uint32_t)min((unsigned long long)F.lead, nominal) : 0;
     const unsigned long long p0 = nominal - lead;  // positions below are from p0
-    const uint32_t end = S + lead;
+    const uint32_t end = bits + lead;              // (less than lim: the next slice has a bit at least)
     const uint32_t lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - p0);
     const unsigned long long base = (unsigned long long)s.v.start * 8 + p0;
-    const uint32_t bit0 = (uint32_t)base;
+    const uint32_t zero = window_zero(F.tok, base);
     Lean d;
     window_init(d.r, F.tok, base);
-    d.blocks = 0;
-    if (guess) {
-        d.k = 1;
-        d.si = 0;
-        d.tab = T.block(0).ac * kTab;
-    } else {
-        d.k = 64;
-        d.si = F.sched_len - 1;
-        d.tab = 0;
-    }
-#pragma unroll
-    for (int c = 0; c < 4; c++) dc[c] = 0;
-    SliceSpec *sp = L.spec + slot;
-    uint32_t q = 0, valid = 0, next_mark = lead;
+    lean_clear(S, d);
+    const uint32_t si0 = path * sched_len / F.paths;  // paths guess different blocks of the MCU
+    d.ac = S.tabs[si0].ac;
+    d.k = guess ? 1 : 64;
+    d.si = guess ? si0 : sched_len - 1;
+    SliceSpec *sp = L.spec + (uint64_t)path * L.n_slots + slot;
+    uint32_t q = 0, valid = 0, next_mark = lead, e = 1;
     unsigned long long exit_state = kStErr;
     for (;;) {
-        if (d.k >= 64) {
-            const uint32_t pos = window_pos(d.r, F.tok, bit0);
-            bool ok = !lean_invalid(d);
+        if (d.k >= 64 || e == 0) {
+            const uint32_t pos = window_pos(d.r, zero);
+            bool ok = lean_complete(d);
             if (ok) {
-                d.si = d.si + 1 == F.sched_len ? 0 : d.si + 1;
-                if (pos > lim) break;  // past the interval's end: exit_state stays kStErr
+                d.si = d.si + 1 == sched_len ? 0 : d.si + 1;
                 if (pos >= next_mark) {
+                    const unsigned long long here = pack_state(p0 + pos, d.si);
                     if (pos >= end) {
-                        exit_state = pack_state(p0 + pos, d.si);
+                        if (pos <= lim) exit_state = here;  // (else past the interval's end)
                         break;
                     }
-                    SlicePoint cp;
-                    cp.state = pack_state(p0 + pos, d.si);
-                    cp.blocks = d.blocks;
-                    cp.pad = 0;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) cp.dc[c] = dc[c];
                     do {
                         if (guess) {
+                            SlicePoint cp;
+                            lean_point(S, d, here, cp);
+                            cp.pad = 0;
                             sp->cp[q] = cp;
                             valid |= 1u << q;
                         }
-                        q++;
-                        const uint32_t m = mark_of(q, S);
+                        const uint32_t m = mark_of(++q, bits);
                         next_mark = m == 0xffffffffu ? end : m + lead;
                     } while (pos >= next_mark && next_mark < end);
                 }
-                ok = lean_dc(L, T, d, dc);
+                ok = lean_dc<kShared>(L, S, d);
             }
             if (!ok) {
                 if (!guess || pos >= min(lim, end)) break;
                 // A decode from a guessed state met an invalid symbol: start again one bit
                 // later; what came before cannot lead to the exit, so its checkpoints go.
                 valid = 0;
-                d.blocks = 0;
-#pragma unroll
-                for (int c = 0; c < 4; c++) dc[c] = 0;
+                lean_clear(S, d);
                 window_init(d.r, F.tok, base + pos + 1);
                 d.k = 1;
-                d.si = 0;
-                d.tab = T.block(0).ac * kTab;
+                d.si = si0;
+                d.ac = S.tabs[si0].ac;
             }
         }
-        lean_steps(L, T, d);
+        e = lean_steps<kShared>(L, d);
     }
+    SlicePoint x;
+    lean_point(S, d, exit_state, x);
+    x.pad = valid;
+    if (guess) sp->exit = x;
+    if (path != 0) return;
     SliceSync out;
     out.start = guess ? kStGuess : pack_state(0, 0);
     out.exit = exit_state;
-    out.blocks = d.blocks;
+    out.blocks = x.blocks;
     out.q = kMatchStart;
 #pragma unroll
-    for (int c = 0; c < 4; c++) out.dc[c] = dc[c];
+    for (int c = 0; c < 4; c++) out.dc[c] = x.dc[c];
     L.sync[slot] = out;
-    if (guess) {
-        SlicePoint e;
-        e.state = exit_state;
-        e.blocks = d.blocks;
-        e.pad = valid;
-#pragma unroll
-        for (int c = 0; c < 4; c++) e.dc[c] = dc[c];
-        sp->exit = e;
-    }
-}
-
-// Shared copies of the lean decode's tables: [kMostShared] DC (16-bit entries), then
-// [kMostShared] AC pair tables, of the CTA's frame.
-struct LeanSmem {
-    uint32_t skip[kMostShared * kTab];
-    uint16_t sym[kMostShared * kTab];
-    uint32_t local[kMaxSched];
-    uint32_t ids[2 * kMostShared];
-    int32_t dc[kSliceThreads][4];
-};
-
-__device__ __forceinline__ void copy16(void *dst, const void *src, uint32_t bytes) {
-    for (uint32_t i = threadIdx.x; i < bytes / 16; i += kSliceThreads)
-        reinterpret_cast<uint4 *>(dst)[i] = __ldg(reinterpret_cast<const uint4 *>(src) + i);
 }
 
 __global__ void __launch_bounds__(kSliceThreads) slice_spec_kernel(JpegLaunch L) {
-    __shared__ __align__(16) LeanSmem S;
+    __shared__ LeanSmem S;
     const uint32_t slot = blockIdx.x * kSliceThreads + threadIdx.x;
     SliceRef s;
-    const bool used = slice_ref(L, slot, s);
-    // the first slot of a CTA is used if any is, and all are of one frame
-    const bool work = used && !s.last;
-    if (used && s.last && s.j == 0) {  // (the decode pass takes a last slice's start from its predecessor)
-        SliceSync y;
-        y.start = y.exit = pack_state(0, 0);
-        y.blocks = 0;
-        y.q = kMatchStart;
-#pragma unroll
-        for (int c = 0; c < 4; c++) y.dc[c] = 0;
-        L.sync[slot] = y;
+    // (a last slice has no exit, and the decode pass takes its start from its predecessor)
+    const uint32_t path = blockIdx.y;
+    bool work = slice_ref(L, slot, s) && !s.last;
+    if (work) {
+        S.frame = s.v.frame;  // the same for all
+        work = path == 0 || (s.j != 0 && path < L.frames[s.v.frame].paths);
     }
     if (!__syncthreads_or(work)) return;
-    const JFrame &F = L.frames[L.ivs[L.slot_item[blockIdx.x * kSliceThreads]].frame];
-    const bool small = F.n_dc <= kMostShared && F.n_ac <= kMostShared;
-    if (small) {
-        for (uint32_t i = threadIdx.x; i < F.sched_len; i += kSliceThreads) S.local[i] = L.brec[F.sched_off + i].local;
-        for (uint32_t t = 0; t < F.n_dc; t++) copy16(S.sym + t * kTab, L.sym + F.dc_id[t] * kTab, 2 * kTab);
-        for (uint32_t t = 0; t < F.n_ac; t++) copy16(S.skip + t * kTab, L.skip + F.ac_id[t] * kTab, 4 * kTab);
-        if (threadIdx.x < kMostShared) {
-            S.ids[threadIdx.x] = F.dc_id[threadIdx.x];
-            S.ids[kMostShared + threadIdx.x] = F.ac_id[threadIdx.x];
-        }
-    }
+    const JFrame &F = L.frames[S.frame];
+    lean_load(L, F, S);
     __syncthreads();
     if (!work) return;
-    int32_t *dc = S.dc[threadIdx.x];
-    if (small) {
-        const LeanTabs<true> T{S.skip, S.sym, S.local, S.ids, nullptr};
-        spec_slice(L, T, F, slot, s, dc);
-    } else {
-        const LeanTabs<false> T{L.skip, L.sym, nullptr, nullptr, L.brec + F.sched_off};
-        spec_slice(L, T, F, slot, s, dc);
-    }
+    if (F.shared_tabs) spec_slice<true>(L, S, F, slot, s, path);
+    else spec_slice<false>(L, S, F, slot, s, path);
 }
 
-// ----------------------------------------------------------------- match ---
+// ------------------------------------------------------------------ sync ---
 
-// Settles a slice whose true start is its speculative decode's boundary at
-// checkpoint q, given what lies before it: blocks and DC differences.
-__device__ __forceinline__ void settle(const JpegLaunch &L, uint32_t slot, unsigned long long from, uint32_t q,
-                                       uint32_t blocks, const int32_t *dc) {
-    const SliceSpec *sp = L.spec + slot;
+// Settles a slice whose true decode, from `from`, is its speculative decode from
+// checkpoint q on, given what lies before it; y.blocks and y.dc hold that.
+__device__ __forceinline__ void settle(const SliceSpec *sp, uint32_t q, SliceSync &y) {
     const SlicePoint cp = sp->cp[q], e = sp->exit;
-    SliceSync y;
-    y.start = from;
     y.exit = e.state;
-    y.blocks = blocks + e.blocks - cp.blocks;
     y.q = q;
+    y.blocks += e.blocks - cp.blocks;
 #pragma unroll
-    for (int c = 0; c < 4; c++) y.dc[c] = dc[c] + e.dc[c] - cp.dc[c];
-    L.sync[slot] = y;
+    for (int c = 0; c < 4; c++) y.dc[c] += e.dc[c] - cp.dc[c];
 }
 
-// Thread per slice: the predecessor's exit is the slice's own first boundary for
-// most; the others go to the first list of the sync passes.
-__global__ void __launch_bounds__(kSliceThreads) slice_match_kernel(JpegLaunch L) {
-    const uint32_t slot = blockIdx.x * kSliceThreads + threadIdx.x, lane = threadIdx.x & 31;
-    SliceRef s;
-    bool list = false;
-    if (slice_ref(L, slot, s) && s.j != 0 && !s.last) {
-        const unsigned long long from = L.sync[slot - 1].exit;
-        const int32_t none[4] = {0, 0, 0, 0};
-        const bool same = (L.spec[slot].exit.pad & 1) && L.spec[slot].cp[0].state == from;
-        if (same) settle(L, slot, from, 0, 0, none);
-        list = !same;
+// The speculative decode of the slice that passes checkpoint q in state `here`.
+__device__ __forceinline__ const SliceSpec *meets(const JpegLaunch &L, uint32_t slot, uint32_t paths, uint32_t q,
+                                                  unsigned long long here) {
+    const SliceSpec *found = nullptr;
+    for (uint32_t h = 0; h < paths; h++) {
+        const SliceSpec *sp = L.spec + (uint64_t)h * L.n_slots + slot;
+        if ((sp->exit.pad >> q & 1) && sp->cp[q].state == here) found = sp;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, list);
-    uint32_t base = 0;
-    if (lane == 0 && m) base = atomicAdd(L.sync_count, (uint32_t)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (list) L.sync_list[base + __popc(m & ((1u << lane) - 1u))] = slot;
+    return found;
 }
 
-// ------------------------------------------------------------ sync pass ---
-
-// Re-decodes slice `slot` (not the first, not the last) from state `from`, the
-// exit of its predecessor, until it meets one of the slice's speculative
-// checkpoints or passes the slice end. Returns whether the exit state changed.
-__device__ bool resync_slice(const JpegLaunch &L, uint32_t slot, const SliceRef &s, unsigned long long from,
-                             int32_t *dc) {
-    const JFrame &F = L.frames[s.v.frame];
-    const unsigned long long old_exit = L.sync[slot].exit;
-    SliceSync y;
+// What slice `slot` (not the first, not the last) gives from state `from`, the exit of
+// its predecessor: it decodes until it meets one of its speculative checkpoints or
+// passes its end.
+template <bool kShared>
+__device__ __forceinline__ void resync_slice(const JpegLaunch &L, LeanSmem &S, const JFrame &F, uint32_t slot,
+                                             const SliceRef &s, unsigned long long from, SliceSync &y) {
     y.start = from;
     y.exit = kStErr;
     y.blocks = 0;
     y.q = kMatchNone;
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        dc[c] = 0;
-        y.dc[c] = 0;
-    }
-    if (from != kStErr) {
-        const uint32_t S = F.slice_bits;
-        const unsigned long long nominal = (unsigned long long)s.j * S, p0 = from >> 8;
-        const uint32_t rel = clamp_u32(p0 - nominal);  // (a block may reach past the slice)
-        const uint32_t lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - p0);
-        const unsigned long long base = (unsigned long long)s.v.start * 8 + p0;
-        const LeanTabs<false> T{L.skip, L.sym, nullptr, nullptr, L.brec + F.sched_off};
-        const SliceSpec *sp = L.spec + slot;
-        const uint32_t valid = sp->exit.pad;
-        Lean d;
-        window_init(d.r, F.tok, base);
-        d.blocks = 0;
-        d.k = 64;
-        d.si = (uint32_t)(from & 0xff);
-        d.tab = 0;
-        uint32_t q = 0, next_mark = 0;
-        bool first = true;
-        for (;;) {
-            if (d.k >= 64) {
-                if (lean_invalid(d)) break;
-                if (!first) d.si = d.si + 1 == F.sched_len ? 0 : d.si + 1;
-                first = false;
-                const uint32_t pos = window_pos(d.r, F.tok, (uint32_t)base);
-                if (pos > lim) break;
-                const uint32_t pn = pos + rel;
-                if (pn >= S) {
-                    y.exit = pack_state(p0 + pos, d.si);
+    for (int c = 0; c < 4; c++) y.dc[c] = 0;
+    const uint32_t bits = F.slice_bits, sched_len = F.sched_len;
+    const unsigned long long nominal = (unsigned long long)s.j * bits, p0 = from >> 8;
+    const uint32_t rel = clamp_u32(p0 - nominal);  // (a block may reach past the slice)
+    const uint32_t lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - p0);
+    const unsigned long long base = (unsigned long long)s.v.start * 8 + p0;
+    const uint32_t zero = window_zero(F.tok, base);
+    const uint32_t paths = F.paths;
+    Lean d;
+    window_init(d.r, F.tok, base);
+    lean_clear(S, d);
+    d.ac = S.tabs[0].ac;
+    d.k = 64;
+    const uint32_t si0 = (uint32_t)(from & 0xff);
+    d.si = si0 == 0 ? sched_len - 1 : si0 - 1;
+    uint32_t q = 0, next_mark = 0, e = 1;
+    const SliceSpec *met = nullptr;
+    for (;;) {
+        if (d.k >= 64 || e == 0) {
+            if (!lean_complete(d)) break;
+            d.si = d.si + 1 == sched_len ? 0 : d.si + 1;
+            const uint32_t pos = window_pos(d.r, zero), pn = pos + rel;
+            if (pn >= min(next_mark, bits)) {
+                const unsigned long long here = pack_state(p0 + pos, d.si);
+                if (pn >= bits) {
+                    if (pos <= lim) y.exit = here;
                     break;
                 }
-                if (pn >= next_mark) {
-                    const unsigned long long here = pack_state(p0 + pos, d.si);
-                    bool met = false;
-                    do {
-                        met = (valid >> q & 1) && sp->cp[q].state == here;
-                        if (!met) next_mark = mark_of(++q, S);
-                    } while (!met && pn >= next_mark);
-                    if (met) {  // the rest of the slice is the speculative decode's
-                        settle(L, slot, from, q, d.blocks, dc);
-                        return sp->exit.state != old_exit;
-                    }
-                }
-                if (!lean_dc(L, T, d, dc)) break;
+                do {
+                    met = meets(L, slot, paths, q, here);
+                    if (!met) next_mark = mark_of(++q, bits);
+                } while (!met && pn >= next_mark);
+                if (met) break;
             }
-            lean_steps(L, T, d);
+            if (!lean_dc<kShared>(L, S, d)) break;
         }
-        y.blocks = d.blocks;
+        e = lean_steps<kShared>(L, d);
+    }
+    y.blocks = d.blocks;
 #pragma unroll
-        for (int c = 0; c < 4; c++) y.dc[c] = dc[c];
-    }
-    L.sync[slot] = y;
-    return y.exit != old_exit;
+    for (int c = 0; c < 4; c++) y.dc[c] = S.dc[c][threadIdx.x];
+    if (met) settle(met, q, y);
 }
 
-// Persistent threads take listed slots from a counter (re-decode lengths vary a lot;
-// the lanes that reach the counter together take consecutive entries with one
-// atomic). A changed exit lists the next slice for the pass after; after the last
-// pass it is left to slice_fix_kernel, from the interval's first such slice on.
-__global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L, uint32_t pass) {
-    __shared__ int32_t s_dc[kSliceThreads][4];
-    const uint32_t n = L.sync_count[pass];
-    const uint32_t *list = L.sync_list + (uint64_t)(pass & 1) * L.n_slots;
-    uint32_t *next_list = L.sync_list + (uint64_t)(~pass & 1) * L.n_slots;
-    uint32_t *taken = L.sync_count + kSyncPasses + 1 + pass;
-    const uint32_t lane = threadIdx.x & 31;
-    for (;;) {
-        const unsigned act = __activemask();
-        const int leader = __ffs(act) - 1;
-        uint32_t base = 0;
-        if ((int)lane == leader) base = atomicAdd(taken, (uint32_t)__popc(act));
-        base = __shfl_sync(act, base, leader);
-        const uint32_t at = base + __popc(act & ((1u << lane) - 1u));
-        if (at >= n) return;
-        const uint32_t slot = list[at];
-        SliceRef s;
-        slice_ref(L, slot, s);
-        const unsigned long long prev = *(volatile const unsigned long long *)&L.sync[slot - 1].exit;
-        if (prev == L.sync[slot].start) continue;
-        if (!resync_slice(L, slot, s, prev, s_dc[threadIdx.x]) || s.j + 2 >= s.v.n_slices) continue;
-        if (pass + 1 < (uint32_t)kSyncPasses) next_list[atomicAdd(L.sync_count + pass + 1, 1u)] = slot + 1;
-        else {
-            atomicAdd(L.sync_count + kSyncPasses, 1u);
-            atomicMin(L.iv_pend + s.item, slot + 1 - s.v.slot_first);
+// A CTA's slices take their predecessors' exits until nothing changes. A slice whose
+// predecessor's exit is the first boundary of one of its speculative decodes takes that
+// one's exit, from registers: these steps are repeated until none changes anything
+// (wrong exits die out within a few slices), and only then do the slices that no
+// speculative decode fits decode again, from tables loaded for them. (Decoding again
+// at once, half of it from exits that were still wrong, took 1.3 ms of the 1.9 ms of
+// 30 restart-less 4:2:0 VGA frames.) The slice before the CTA's first is read once:
+// what another CTA still changes there is the next pass's, and after the last pass
+// slice_fix_kernel's, from the interval's first such slice on.
+__global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L, bool first_pass, bool last_pass) {
+    __shared__ LeanSmem S;
+    __shared__ unsigned long long s_exit[kSliceThreads + 1];  // of the slice before the CTA's first, then of each
+    const uint32_t tid = threadIdx.x, slot = blockIdx.x * kSliceThreads + tid;
+    SliceRef s;
+    bool work = slice_ref(L, slot, s) && !s.last;
+    unsigned long long start = 0, exit = 0, entry[kMostPaths], leave[kMostPaths];
+    if (work) {
+        S.frame = s.v.frame;
+        const uint32_t paths = L.frames[s.v.frame].paths;
+        start = L.sync[slot].start;
+        exit = L.sync[slot].exit;
+#pragma unroll
+        for (uint32_t h = 0; h < kMostPaths; h++) {
+            entry[h] = leave[h] = kStGuess;  // (never an exit)
+            if (s.j == 0 || h >= paths) continue;
+            const SliceSpec *sp = L.spec + (uint64_t)h * L.n_slots + slot;
+            leave[h] = sp->exit.state;
+            if (sp->exit.pad & 1) entry[h] = sp->cp[0].state;
         }
+        if (start == kStGuess) {  // to begin with, the exit most decodes agree on
+            uint32_t most = 0;
+#pragma unroll
+            for (uint32_t h = 0; h < kMostPaths; h++) {
+                uint32_t n = 0;
+#pragma unroll
+                for (uint32_t i = 0; i < kMostPaths; i++) n += leave[i] == leave[h];
+                if (is_state(leave[h]) && n > most) {
+                    most = n;
+                    exit = leave[h];
+                }
+            }
+        }
+        if (tid == 0 && s.j != 0) s_exit[0] = *(volatile const unsigned long long *)&L.sync[slot - 1].exit;
+    }
+    work = work && s.j != 0;
+    s_exit[tid + 1] = exit;
+    const unsigned long long exit_before = exit;
+    __syncthreads();
+    if (!first_pass && !__syncthreads_or(work && is_state(s_exit[tid]) && s_exit[tid] != start)) return;
+    bool loaded = false;
+    uint32_t met = kMostPaths;                 // the speculative decode the slice takes, if it changes
+    unsigned long long refused = kStGuess;     // an exit no speculative decode fits
+    for (;;) {
+        for (;;) {
+            const unsigned long long from = work ? s_exit[tid] : 0;
+            bool take = false;
+            if (work && is_state(from) && from != start && from != refused) {
+                uint32_t m = kMostPaths;
+#pragma unroll
+                for (uint32_t h = 0; h < kMostPaths; h++)
+                    if (entry[h] == from) m = h;
+                if (m < kMostPaths) {
+                    take = true;
+                    met = m;
+                    start = from;
+#pragma unroll
+                    for (uint32_t h = 0; h < kMostPaths; h++)
+                        if (m == h) exit = leave[h];
+                } else {
+                    refused = from;
+                }
+            }
+            if (!__syncthreads_or(take)) break;  // (everyone has read the exits)
+            if (take) s_exit[tid + 1] = exit;
+            __syncthreads();
+        }
+        const unsigned long long from = work ? s_exit[tid] : 0;
+        const bool go = work && is_state(from) && from != start;
+        if (!__syncthreads_or(go)) break;
+        const JFrame &F = L.frames[S.frame];
+        if (!loaded) {
+            lean_load(L, F, S);
+            loaded = true;
+            __syncthreads();
+        }
+        if (go) {
+            SliceSync y;
+            if (F.shared_tabs) resync_slice<true>(L, S, F, slot, s, from, y);
+            else resync_slice<false>(L, S, F, slot, s, from, y);
+            L.sync[slot] = y;
+            met = kMostPaths;
+            start = from;
+            exit = y.exit;
+            s_exit[tid + 1] = exit;
+        }
+        __syncthreads();
+    }
+    if (met < kMostPaths) {
+        const SliceSpec *sp = L.spec + (uint64_t)met * L.n_slots + slot;
+        SliceSync y;
+        y.start = start;
+        y.blocks = 0;
+#pragma unroll
+        for (int c = 0; c < 4; c++) y.dc[c] = 0;
+        settle(sp, 0, y);
+        L.sync[slot] = y;
+    }
+    if (last_pass && tid == kSliceThreads - 1 && work && exit != exit_before && s.j + 2 < s.v.n_slices) {
+        atomicAdd(L.sync_left, 1u);
+        atomicMin(L.iv_pend + s.item, s.j + 1);
     }
 }
 
-// One warp per interval that still has a listed slice.
+// One warp per interval that the sync passes left unsettled.
 __global__ void __launch_bounds__(kSliceThreads) slice_fix_kernel(JpegLaunch L) {
-    __shared__ int32_t s_dc[kSliceThreads][4];
-    if (L.sync_count[kSyncPasses] == 0) return;
-    const uint32_t item = blockIdx.x * (kSliceThreads / 32) + threadIdx.x / 32;
+    __shared__ LeanSmem S;
+    if (*L.sync_left == 0) return;
     const uint32_t lane = threadIdx.x & 31;
-    if (item >= L.n_items_small) return;
-    const uint32_t pend = L.iv_pend[item];
-    if (pend == 0xffffffffu) return;
-    const IvInfo v = L.ivs[item];
-    for (uint32_t c = pend; c + 1 < v.n_slices; c += 32) {  // (the last slice has no exit)
-        for (;;) {
-            const uint32_t j = c + lane;
-            bool bad = false;
-            if (j + 1 < v.n_slices) {
-                const uint32_t slot = v.slot_first + j;
-                bad = *(volatile unsigned long long *)&L.sync[slot].start !=
-                      *(volatile unsigned long long *)&L.sync[slot - 1].exit;
+    for (uint32_t i = 0; i < kSliceThreads / 32; i++) {  // (one interval of the CTA's four at a time: they share the tables)
+        const uint32_t item = blockIdx.x * (kSliceThreads / 32) + i;
+        if (item >= L.n_items_small) return;
+        const uint32_t pend = L.iv_pend[item];
+        if (pend == 0xffffffffu) continue;
+        const IvInfo v = L.ivs[item];
+        const JFrame &F = L.frames[v.frame];
+        __syncthreads();
+        lean_load(L, F, S);
+        __syncthreads();
+        if (threadIdx.x >= 32) continue;
+        for (uint32_t c = pend; c + 1 < v.n_slices; c += 32) {  // (the last slice has no exit)
+            for (;;) {
+                const uint32_t j = c + lane, slot = v.slot_first + j;
+                unsigned long long from = 0;
+                bool bad = false;
+                if (j + 1 < v.n_slices) {
+                    from = *(volatile unsigned long long *)&L.sync[slot - 1].exit;
+                    bad = is_state(from) && *(volatile unsigned long long *)&L.sync[slot].start != from;
+                }
+                const uint32_t m = __ballot_sync(0xffffffffu, bad);
+                if (!m) break;
+                if (lane == (uint32_t)__ffs(m) - 1) {
+                    SliceRef s;
+                    slice_ref(L, slot, s);
+                    SliceSync y;
+                    if (F.shared_tabs) resync_slice<true>(L, S, F, slot, s, from, y);
+                    else resync_slice<false>(L, S, F, slot, s, from, y);
+                    L.sync[slot] = y;
+                    __threadfence_block();
+                }
+                __syncwarp();
             }
-            const uint32_t m = __ballot_sync(0xffffffffu, bad);
-            if (!m) break;
-            if (lane == (uint32_t)__ffs(m) - 1) {
-                const uint32_t slot = v.slot_first + j;
-                SliceRef s;
-                slice_ref(L, slot, s);
-                resync_slice(L, slot, s, *(volatile unsigned long long *)&L.sync[slot - 1].exit, s_dc[threadIdx.x]);
-                __threadfence_block();
-            }
-            __syncwarp();
         }
     }
 }
 
 // ---------------------------------------------------------------- prefix ---
 
-constexpr int kPrefixThreads = 256;
+constexpr int kPrefixThreads = 512;
 constexpr uint32_t kPrefixLong = 512;  // slices an interval is worth the whole CTA from
 
 struct SliceSums {
@@ -761,20 +813,20 @@ __global__ void __launch_bounds__(kPrefixThreads) slice_prefix_kernel(JpegLaunch
 // ---------------------------------------------------------------- decode ---
 
 // Records a slice's first event: an error, or the interval's completion.
-__device__ __forceinline__ void report(const JpegLaunch &L, const SliceRef &s, uint32_t slot, unsigned long long pos,
-                                       const Diag &d, uint32_t complete) {
+__device__ __forceinline__ void report(const JpegLaunch &L, const SliceRef &s, uint32_t slot, const Diag &d,
+                                       uint32_t complete) {
     SliceEvent e;
     e.diag = d;
     e.complete = complete;
     L.events[slot] = e;
-    atomicMin(&L.iv_key[s.item], (pos << kKeyBits) | s.j);
+    atomicMin(&L.iv_key[s.item], (unsigned long long)s.j);
 }
 
 // The block whose DC symbol starts at bit `at` of the interval failed: decodes it
 // again with the reference's checks in its order (decoder.rs:501-546; the DC checks of
 // :507-515 right after the DC symbol) and reports what the serial decoder stops at.
 __device__ __noinline__ void report_bad_block(const JpegLaunch &L, const SliceRef &s, uint32_t slot,
-                                              unsigned long long at, uint32_t si, long long pred) {
+                                              unsigned long long at, uint32_t si, int32_t pred) {
     const JFrame &F = L.frames[s.v.frame];
     const JBlockRec R = L.brec[F.sched_off + si];
     const uint32_t lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - at);
@@ -782,7 +834,7 @@ __device__ __noinline__ void report_bad_block(const JpegLaunch &L, const SliceRe
     bits_init(r, F.tok, (uint64_t)s.v.start * 8 + at, 0);
     int k = 0;
     uint16_t kind = kDeviceError;  // (never kept: the fast decode only refuses what this one does)
-    uint32_t errpos = 0, ev_at = 0;
+    uint32_t errpos = 0;
     while (k < 64) {
         const uint32_t sym_at = r.used;
         const int k0 = k;
@@ -792,11 +844,10 @@ __device__ __noinline__ void report_bad_block(const JpegLaunch &L, const SliceRe
         if (!decode_symbol(r, lim > sym_at ? lim - sym_at : 0, L.luts + (k0 == 0 ? R.dc_lut : R.ac_lut), L.symbols, k, val, err, eb)) {
             kind = err;
             errpos = eb;
-            ev_at = sym_at;
             break;
         }
         if (k0 != 0) continue;
-        const long long pn = pred + val, d = pn * (long long)R.q0;
+        const long long pn = (long long)pred + val, d = pn * (long long)R.q0;
         const bool pred_bad = pn > INT32_MAX || pn < INT32_MIN;
         if (pred_bad || d > INT32_MAX || d < INT32_MIN) {
             kind = pred_bad ? kJDcPredOverflow : kJDcDeqOverflow;
@@ -811,139 +862,117 @@ __device__ __noinline__ void report_bad_block(const JpegLaunch &L, const SliceRe
     } else {
         d = make_diag(kind, s.v.start + (uint32_t)((at + errpos + 7) / 8));
     }
-    report(L, s, slot, at + ev_at, d, 0);
+    report(L, s, slot, d, 0);
 }
 
 struct DecodeSmem {
     __align__(16) int16_t stage[kSliceThreads * kStride];
-    __align__(16) uint16_t sym[2 * kMostShared * kTab];  // DC tables, then AC tables
-    JBlockRec recs[kMaxSched];
-    long long pred[4][kSliceThreads];
-    uint32_t ids[2 * kMostShared];
+    __align__(16) uint16_t sym[2 * kSharedTabs][kSharedTab];  // DC tables, then AC tables
+    BlockTabs tabs[kMaxSched];
+    uint32_t base_off[kMaxSched], mul_x[kMaxSched], mul_y[kMaxSched];
+    int32_t q0[kMaxSched];
+    int32_t pred[4][kSliceThreads];
+    uint32_t frame;
     uint8_t zz[160];  // stage slot of k - 1: natural index, or past the block for EOB (k + 95 at most 158)
 };
 
-// What the final decode needs while it is in a slice.
-struct Walk {
-    Window r;
-    int k;
-    uint32_t tab;      // table of the next symbol: the block's DC table, then its AC table
-    uint32_t ac;       // its AC table
-};
-
-// kDecodeSteps symbols (none for a lane whose block has ended): each level into the
-// lane's stage; the DC difference at zigzag index 0.
-template <bool kShared>
-__device__ __forceinline__ void decode_steps(const JpegLaunch &L, const DecodeSmem &S, int16_t *stage, Walk &d) {
-#pragma unroll
-    for (int u = 0; u < kDecodeSteps; u++) {
-        uint32_t w = window_bits(d.r);
-        uint32_t e = 0;
-        const uint32_t at = d.tab + (w >> (32 - kHuffFastBits));
-        if (d.k < 64) e = kShared ? S.sym[at] : __ldg(L.sym + at);
-        if (e & kSymEscape) {
-            const uint32_t t = d.tab / kTab;
-            e = sub_entry(L, kShared ? S.ids[t] : t, e, w);
-            if (e & kSymEscape) {
-                e = 0;
-                d.k = 80;
-            } else {
-                window_take(d.r, kHuffFastBits);
-                w = window_bits(d.r);
-            }
-        }
-        const uint32_t cl = e & 15, size = (e >> 4) & 15;
-        const int32_t val = extend(w << cl, size);
-        const int k = d.k + (int)(e >> 8);
-        if (e) stage[S.zz[k - 1]] = (int16_t)val;
-        d.k = k;
-        window_take(d.r, cl + size);
-        d.tab = d.ac;
-    }
-}
-
-// Warps stay together: lanes decode kDecodeSteps symbols, then those whose block is
-// complete settle it (DC, address, the next block), and the warp writes the completed
-// blocks together, eight lanes per block, as whole 128-byte lines.
+// Warps stay together: lanes decode kDecodeSteps AC symbols, then those whose block is
+// complete settle it and decode the next block's DC symbol, and the warp writes the
+// completed blocks together, eight lanes per block, as whole 128-byte lines.
 template <bool kShared>
 __device__ __forceinline__ void decode_slices(const JpegLaunch &L, DecodeSmem &S, const JFrame &F, uint32_t slot,
                                               const SliceRef &s, uint32_t n, unsigned long long from, uint32_t base) {
     const uint32_t tid = threadIdx.x, lane = tid & 31;
-    int16_t *stage = S.stage + tid * kStride;
+    const uint32_t stage = shared_address(S.stage + tid * kStride), zz = shared_address(S.zz);
+    const uint32_t sched_len = F.sched_len, mcu_cols = F.mcu_cols, blk_off = (uint32_t)F.blk_off;
     bool live = n != 0;
-    Walk d;
-    d.k = 128;
-    d.tab = d.ac = 0;
-    d.r.w0 = d.r.w1 = d.r.pf = d.r.off = 0;
-    d.r.next = reinterpret_cast<const uint32_t *>(F.tok);
+    Window r;
+    r.w0 = r.w1 = r.pf = r.off = 0;
+    r.next = reinterpret_cast<const uint32_t *>(F.tok);
+    Tab ac{0, 0xffffffffu, 0};
+    int k = 128;  // (no block yet, nothing to step)
     const unsigned long long p0 = from >> 8;
-    uint32_t si = (uint32_t)(from & 0xff), lim = 0, bit0 = 0, blk_at = 0;
-    uint32_t mx = 0, my = 0, left = n;
-    uint64_t blk = 0;
-    int32_t q0 = 0;
-    uint32_t comp = 0;
-    auto setup = [&]() {
-        const JBlockRec &R = S.recs[si];
-        comp = R.comp;
-        q0 = R.q0;
-        blk = F.blk_off + R.base_off + mx * R.mul_x + (uint64_t)my * R.mul_y;
-        if (kShared) {
-            d.tab = ((R.local >> 8) & 0xff) * kTab;
-            d.ac = (kMostShared + (R.local >> 16)) * kTab;
-        } else {
-            d.tab = R.dc_lut * kTab;
-            d.ac = R.ac_lut * kTab;
-        }
-        d.k = 0;
+    uint32_t si = (uint32_t)(from & 0xff), lim = 0, zero = 0, blk_at = 0, left = n;
+    uint32_t mx = 0, my = 0, blk = 0, e = 1;
+    int32_t diff = 0;
+    bool bad_dc = false;
+    // the DC symbol of block si of MCU (mx, my), at bit blk_at
+    auto begin = [&]() {
+        const BlockTabs &b = S.tabs[si];
+        blk = blk_off + S.base_off[si] + mx * S.mul_x[si] + my * S.mul_y[si];
+        const uint32_t w = window_bits(r);
+        const uint32_t x = sym_entry<kShared>(L, b.dc, w, true), cl = x & 31, size = (x >> 5) & 15;
+        diff = extend(w << cl, size);
+        window_take(r, cl + size);
+        ac = b.ac;
+        bad_dc = x == 0;
+        k = 1;
     };
     if (live) {
         const unsigned long long b0 = (unsigned long long)s.v.start * 8 + p0;
-        bit0 = (uint32_t)b0;
+        zero = window_zero(F.tok, b0);
         lim = clamp_u32((unsigned long long)(s.v.barrier - s.v.start) * 8 - p0);
-        window_init(d.r, F.tok, b0);
-        const uint32_t mcu = L.items[s.item].y * F.ri + base / F.sched_len;
-        my = mcu / F.mcu_cols;
-        mx = mcu - my * F.mcu_cols;
-        setup();
+        window_init(r, F.tok, b0);
+        const uint32_t mcu = L.items[s.item].y * F.ri + base / sched_len;
+        my = mcu / mcu_cols;
+        mx = mcu - my * mcu_cols;
+        begin();
     }
     while (__any_sync(0xffffffffu, live)) {
-        decode_steps<kShared>(L, S, stage, d);
+#pragma unroll
+        for (int u = 0; u < kDecodeSteps; u++) {
+            const uint32_t w = window_bits(r);
+            e = sym_entry<kShared>(L, ac, w, k < 64);
+            const uint32_t cl = e & 31, size = (e >> 5) & 15;
+            const int32_t val = extend(w << cl, size);
+            k += (int)(e >> 9);
+            asm volatile("{\n\t"
+                         ".reg .pred p;\n\t"
+                         ".reg .u32 z, a;\n\t"
+                         "setp.ne.u32 p, %0, 0;\n\t"
+                         "@p ld.shared.u8 z, [%1];\n\t"
+                         "@p mad.lo.u32 a, z, 2, %2;\n\t"
+                         "@p st.shared.u16 [a], %3;\n\t"
+                         "}" ::"r"(e), "r"(zz + (uint32_t)k - 1), "r"(stage), "h"((short)val)
+                         : "memory");
+            window_take(r, cl + size);
+        }
         bool put = false;
-        uint32_t to = 0;  // the completed block (the arena holds less than 2^32)
-        if (live && d.k >= 64) {
-            const uint32_t pos = window_pos(d.r, F.tok, bit0);
-            const long long pn = S.pred[comp][tid] + stage[0], dq = pn * (long long)q0;
-            const bool ok = (d.k == 64 || d.k >= 96) && pos <= lim && pn <= INT32_MAX && pn >= INT32_MIN &&
-                            dq <= INT32_MAX && dq >= INT32_MIN;
-            if (!ok) {
-                report_bad_block(L, s, slot, p0 + blk_at, si, S.pred[comp][tid]);
+        uint32_t to = 0;
+        if (live && (k >= 64 || e == 0 || bad_dc)) {
+            const uint32_t pos = window_pos(r, zero), comp = S.tabs[si].comp;
+            const int32_t q0 = S.q0[si], pred = S.pred[comp][tid], pn = (int32_t)((uint32_t)pred + (uint32_t)diff);
+            const int32_t dq = (int32_t)((uint32_t)pn * (uint32_t)q0);
+            const bool over = ((pn ^ pred) & (pn ^ diff)) < 0 || __mulhi(pn, q0) != dq >> 31;
+            if ((k != 64 && k < 96) || bad_dc || pos > lim || over) {
+                report_bad_block(L, s, slot, p0 + blk_at, si, pred);
                 live = false;
+                k = 128;
             } else {
                 S.pred[comp][tid] = pn;
-                L.dc[blk] = (int32_t)dq;
-                to = (uint32_t)blk;
+                L.dc[blk] = dq;
+                to = blk;
                 put = true;
                 blk_at = pos;
                 if (++base == s.v.blocks) {  // the interval's last block
                     const unsigned long long endbit = p0 + pos;
-                    report(L, s, slot, endbit, make_diag(kDiagNone, s.v.start + (uint32_t)((endbit + 7) / 8)), 1);
+                    report(L, s, slot, make_diag(kDiagNone, s.v.start + (uint32_t)((endbit + 7) / 8)), 1);
                 }
                 live = --left != 0;
-                if (++si == F.sched_len) {
+                if (++si == sched_len) {
                     si = 0;
-                    if (++mx == F.mcu_cols) {
+                    if (++mx == mcu_cols) {
                         mx = 0;
                         my++;
                     }
                 }
-                if (live) setup();
+                if (live) begin();
             }
         }
         unsigned m = __ballot_sync(0xffffffffu, put);
-        while (m) {
-            // lanes 8i .. 8i + 7 write the i-th block left
-            unsigned mine = m;
-            for (uint32_t i = 0; i < lane >> 3; i++) mine &= mine - 1;
+        while (m) {  // lanes 8i .. 8i + 7 write the i-th block left
+            const unsigned m1 = m & (m - 1), m2 = m1 & (m1 - 1), m3 = m2 & (m2 - 1);
+            const unsigned mine = lane < 16 ? lane < 8 ? m : m1 : lane < 24 ? m2 : m3;
             const int src = __ffs(mine) - 1;
             const uint32_t g = __shfl_sync(0xffffffffu, to, src & 31);
             if (src >= 0) {
@@ -951,45 +980,44 @@ __device__ __forceinline__ void decode_slices(const JpegLaunch &L, DecodeSmem &S
                 reinterpret_cast<int4 *>(L.coef + (uint64_t)g * 64)[lane & 7] = *st;
                 *st = make_int4(0, 0, 0, 0);
             }
-#pragma unroll
-            for (int i = 0; i < 4; i++) m &= m - 1;
+            m = m3 & (m3 - 1);
         }
         __syncwarp();
     }
 }
 
 __global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch L) {
-    extern __shared__ __align__(16) uint8_t s_raw[];
-    DecodeSmem &S = *reinterpret_cast<DecodeSmem *>(s_raw);
+    __shared__ DecodeSmem S;
     const uint32_t tid = threadIdx.x, slot = blockIdx.x * kSliceThreads + tid;
     SliceRef s;
     s.item = 0;
     const bool used = slice_ref(L, slot, s);
     // the blocks this slice decodes
     uint32_t n = 0, base = 0;
-    unsigned long long from = 0;
+    unsigned long long from = pack_state(0, 0);
     bool redone = false, whole = false;
+#pragma unroll
+    for (int c = 0; c < 4; c++) S.pred[c][tid] = 0;
     if (used) {
+        S.frame = s.v.frame;  // the same for all
+        n = s.v.blocks;
         if (s.v.n_slices > 1) {
             const SlicePrefix P = L.prefix[slot];
             base = P.base;
+            bool over = false;  // (then a DC check fails in an earlier slice, which reports it)
 #pragma unroll
-            for (int c = 0; c < 4; c++) S.pred[c][tid] = P.dc[c];
-            from = s.j == 0 ? pack_state(0, 0) : L.sync[slot - 1].exit;
+            for (int c = 0; c < 4; c++) {
+                S.pred[c][tid] = (int32_t)P.dc[c];
+                over |= P.dc[c] != (int32_t)P.dc[c];
+            }
+            if (s.j != 0) from = L.sync[slot - 1].exit;
             if (!s.last) {
                 const SliceSync &y = L.sync[slot];
                 n = y.blocks;
                 redone = s.j != 0 && y.q != 0;
                 whole = y.q == kMatchNone;
-            } else {
-                n = 0xffffffffu;
             }
-            n = from == kStErr || base >= s.v.blocks ? 0 : min(n, s.v.blocks - base);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 4; c++) S.pred[c][tid] = 0;
-            from = pack_state(0, 0);
-            n = s.v.blocks;
+            n = !is_state(from) || over || base >= s.v.blocks ? 0 : min(n, s.v.blocks - base);
         }
     }
     const int n_used = __syncthreads_count(used), n_redone = __syncthreads_count(redone),
@@ -1000,23 +1028,35 @@ __global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch 
         if (n_redone) atomicAdd(L.fix_count + 2, (uint32_t)n_redone);
         if (n_whole) atomicAdd(L.fix_count + 5, (uint32_t)n_whole);
     }
-    const JFrame &F = L.frames[L.ivs[L.slot_item[blockIdx.x * kSliceThreads]].frame];
-    const bool small = F.n_dc <= kMostShared && F.n_ac <= kMostShared;
+    const JFrame &F = L.frames[S.frame];
     for (uint32_t i = tid; i < kSliceThreads * kStride / 8; i += kSliceThreads)
         reinterpret_cast<int4 *>(S.stage)[i] = make_int4(0, 0, 0, 0);
     for (uint32_t i = tid; i < 160; i += kSliceThreads) S.zz[i] = i < 64 ? c_slice_zz[i] : 64;
-    copy16(S.recs, L.brec + F.sched_off, F.sched_len * (uint32_t)sizeof(JBlockRec));
-    if (small) {
-        for (uint32_t t = 0; t < F.n_dc; t++) copy16(S.sym + t * kTab, L.sym + F.dc_id[t] * kTab, 2 * kTab);
-        for (uint32_t t = 0; t < F.n_ac; t++)
-            copy16(S.sym + (kMostShared + t) * kTab, L.sym + F.ac_id[t] * kTab, 2 * kTab);
-        if (tid < kMostShared) {
-            S.ids[tid] = F.dc_id[tid];
-            S.ids[kMostShared + tid] = F.ac_id[tid];
+    if (F.shared_tabs) {
+        for (uint32_t t = 0; t < F.n_dc; t++) {
+            const LutMeta m = L.lut_meta[F.dc_id[t]];
+            copy16(S.sym[t], L.sym + m.off, 2 * m.len);
+        }
+        for (uint32_t t = 0; t < F.n_ac; t++) {
+            const LutMeta m = L.lut_meta[F.ac_id[t]];
+            copy16(S.sym[kSharedTabs + t], L.sym + m.off, 2 * m.len);
         }
     }
+    for (uint32_t i = tid; i < F.sched_len; i += kSliceThreads) {
+        const JBlockRec &R = L.brec[F.sched_off + i];
+        BlockTabs b = batch_tabs(L, R);
+        if (F.shared_tabs) {
+            b.dc.at = shared_address(S.sym[(R.local >> 8) & 0xff]);
+            b.ac.at = shared_address(S.sym[kSharedTabs + (R.local >> 16)]);
+        }
+        S.tabs[i] = b;
+        S.base_off[i] = R.base_off;
+        S.mul_x[i] = R.mul_x;
+        S.mul_y[i] = R.mul_y;
+        S.q0[i] = R.q0;
+    }
     __syncthreads();
-    if (small) decode_slices<true>(L, S, F, slot, s, n, from, base);
+    if (F.shared_tabs) decode_slices<true>(L, S, F, slot, s, n, from, base);
     else decode_slices<false>(L, S, F, slot, s, n, from, base);
 }
 
@@ -1036,7 +1076,7 @@ __global__ void slice_resolve_kernel(JpegLaunch L) {
     if (key == ~0ull) {
         out = make_diag(kDeviceError);  // every decoded interval ends in an event
     } else {
-        const SliceEvent e = L.events[v.slot_first + (uint32_t)(key & ((1u << kKeyBits) - 1))];
+        const SliceEvent e = L.events[v.slot_first + (uint32_t)key];
         if (!e.complete) {
             out = e.diag;
         } else if (iv + 1 < F.n_intervals) {
@@ -1058,7 +1098,14 @@ __global__ void slice_resolve_kernel(JpegLaunch L) {
 
 }  // namespace
 
-int jpeg_slice_launches(const JpegLaunch &L) { return L.n_items_small ? 7 + kSyncPasses : 0; }
+// One CTA of slots has no neighbours to settle with.
+static uint32_t jpeg_sync_passes(const JpegLaunch &L) { return L.n_slots > (uint32_t)kSliceThreads ? kSyncPasses : 1; }
+
+int jpeg_slice_launches(const JpegLaunch &L) {
+    if (!L.n_items_small) return 0;
+    const uint32_t passes = jpeg_sync_passes(L);
+    return 5 + (int)passes + (passes > 1 ? 1 : 0);
+}
 
 void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks, bool capturing) {
     auto mark = [&](int k) {
@@ -1066,23 +1113,22 @@ void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks,
     };
     const bool run = L.n_items_small && L.n_slots;
     const uint32_t grid = L.n_slots / kSliceThreads;  // (frames reserve whole CTAs of slots)
-    const uint32_t warps = kSliceThreads / 32, pwarps = kPrefixThreads / 32;
+    auto per_item = [&](uint32_t items) { return (L.n_items_small + items - 1) / items; };
     if (run) {
-        slice_plan_kernel<<<L.n_frames, kPlanThreads, 0, s>>>(L);
-        slice_spec_kernel<<<grid, kSliceThreads, 0, s>>>(L);
+        slice_plan_kernel<<<per_item(kPlanThreads), kPlanThreads, 0, s>>>(L);
+        slice_spec_kernel<<<dim3(grid, L.paths), kSliceThreads, 0, s>>>(L);
     }
     mark(0);
     if (run) {
-        slice_match_kernel<<<grid, kSliceThreads, 0, s>>>(L);
-        const uint32_t sync_grid = std::min<uint32_t>(grid, 152 * 8);
-        for (uint32_t p = 0; p < (uint32_t)kSyncPasses; p++) slice_sync_kernel<<<sync_grid, kSliceThreads, 0, s>>>(L, p);
-        slice_fix_kernel<<<(L.n_items_small + warps - 1) / warps, kSliceThreads, 0, s>>>(L);
-        slice_prefix_kernel<<<(L.n_items_small + pwarps - 1) / pwarps, kPrefixThreads, 0, s>>>(L);
+        const uint32_t passes = jpeg_sync_passes(L);
+        for (uint32_t p = 0; p < passes; p++) slice_sync_kernel<<<grid, kSliceThreads, 0, s>>>(L, p == 0, p + 1 == passes);
+        if (passes > 1) slice_fix_kernel<<<per_item(kSliceThreads / 32), kSliceThreads, 0, s>>>(L);
+        slice_prefix_kernel<<<per_item(kPrefixThreads / 32), kPrefixThreads, 0, s>>>(L);
     }
     mark(1);
-    if (run) slice_decode_kernel<<<grid, kSliceThreads, sizeof(DecodeSmem), s>>>(L);
+    if (run) slice_decode_kernel<<<grid, kSliceThreads, 0, s>>>(L);
     mark(2);
-    if (run) slice_resolve_kernel<<<(L.n_items_small + 127) / 128, 128, 0, s>>>(L);
+    if (run) slice_resolve_kernel<<<per_item(128), 128, 0, s>>>(L);
 }
 
 }  // namespace mmr

@@ -46,25 +46,22 @@ struct JpegLaunch {
     uint32_t *slot_item;         // per slot: item, UINT32_MAX when unused
     IvInfo *ivs;                 // per item
     SliceSync *sync;             // per slot
-    SliceSpec *spec;             // per slot
+    SliceSpec *spec;             // paths x n_slots
+    uint32_t paths;              // most speculative decodes per slice of any frame
     SlicePrefix *prefix;         // per slot
     SliceEvent *events;          // per slot
-    unsigned long long *iv_key;  // per item: (position << 26 | slice) of its first event
+    unsigned long long *iv_key;  // per item: first slice that reports an event
     uint32_t *iv_pend;           // per item: first slice still to settle after the sync passes
-    uint32_t *sync_list;         // 2 x n_slots: slots listed for the current and the next sync pass
-    uint32_t *sync_count;        // per sync pass the slots listed, then those left after the last, then per
-                                 // pass the entries taken (kSyncCounters, zeroed per batch)
-    const uint16_t *sym;         // per LUT: 2^kHuffFastBits symbol entries (plan.h)
-    const uint32_t *skip;        // per LUT: as many skip entries
-    const uint16_t *sub;         // blocks of kSubEntries entries for longer codes
-    const uint32_t *sub_first;   // per LUT: its first entry in sub
+    uint32_t *sync_left;         // intervals the sync passes left unsettled (zeroed per batch)
+    const LutMeta *lut_meta;     // per LUT, its entries in:
+    const uint16_t *sym;
+    const uint32_t *skip;
     const long long *fixw;       // fixed-point IDCT weights (exact_fixed.h)
 };
 
-// Parallel sync passes before the serial fix-up walk; a pass whose list is empty
-// returns at once.
-constexpr int kSyncPasses = 4;
-constexpr int kSyncCounters = 2 * kSyncPasses + 1;
+// Sync passes before the serial fix-up walk: the first settles the slices inside each
+// CTA, the others what changed across CTA boundaries.
+constexpr int kSyncPasses = 2;
 
 void launch_jpeg_scan(const JpegLaunch &L, cudaStream_t s);
 void launch_jpeg_entropy(const JpegLaunch &L, cudaStream_t s);   // frames with > 4 components

@@ -38,23 +38,39 @@ struct HuffLut {
     uint32_t pad[2];       // size multiple of 16
 };
 
-// Lookups of the chunked decoder (jpeg_slices.cu), per table, made from a HuffLut:
-//   sym[next 11 bits]   code bits | size << 4 | advance << 8 for codes of at most 11
-//       bits (size: magnitude bits after the code; advance of the coefficient index: 1
-//       for a DC difference, run + 1 for an AC level, 16 for ZRL, 96 for EOB, so that
-//       a block ends with an index of 64 or from 97 to 159 and an overrun lies
-//       between); kSymEscape | block for longer ones: entry (next 5 bits) of that
-//       block of `sub`, its code bits counting from the 12th; kSymInvalid for bits no
-//       code matches and symbols the reference rejects.
-//   skip[next 11 bits]  AC tables, for decodes that only follow positions: bits |
-//       advance << 5 of the first symbol (magnitude included), and the same at << 12
-//       of the first two where the second's code lies within the 11 bits too (else of
-//       the first); kSkipEscape where sym escapes.
-constexpr uint32_t kSymEscape = 0x8000u;
-constexpr uint32_t kSymInvalid = 0xffffu;
-constexpr uint32_t kSkipEscape = 0x80000000u;
+// Lookups of the chunked decoder (jpeg_slices.cu), per table. Canonical codes of more
+// than 11 bits are the last of the code space, from the 32-bit left-aligned code
+// `first_long` on, so one table serves both: the entry of a window w (the next 32 bits)
+// is lut_entry_index(w): its 11-bit prefix, plus one entry per 16-bit pattern from
+// first_long on (192 of them for Annex K's AC tables), without a second lookup.
+//   sym   code bits | size << 5 | advance << 9 (size: magnitude bits after the code;
+//         advance of the coefficient index: 1 for a DC difference, run + 1 for an AC
+//         level, 16 for ZRL, kSymEob for EOB, so that a block ends with an index of 64
+//         or from 97 to 159 and an overrun lies between); 0 for bits no code matches
+//         and for symbols the reference rejects.
+//   skip  AC tables, for decodes that only follow positions. Byte 3: advance of the
+//         first symbol, byte 2: its bits, magnitude included; bytes 1 and 0: the same
+//         of the first two where the second's code lies within the 11 bits too (else of
+//         the first); 0 where sym is 0.
 constexpr uint32_t kSymEob = 96;
-constexpr uint32_t kSubEntries = 1u << (16 - kHuffFastBits);
+
+struct LutMeta {
+    uint32_t off;         // first entry in sym and skip (a multiple of 8)
+    uint32_t len;         // entries
+    uint32_t first_long;  // 0xffffffff: no codes of more than 11 bits
+    uint32_t last;        // windows are clamped to it (the first pattern past the last code, an
+                          // invalid one); 0xffffffff where the table covers every pattern
+};
+
+// Long-code patterns a table may have to be kept in shared memory (such tables cover
+// every pattern and need no clamp).
+constexpr uint32_t kSharedLong = 512;
+constexpr uint32_t kSharedTab = (1u << kHuffFastBits) + kSharedLong;
+constexpr uint32_t kSharedTabs = 2;  // DC and AC tables a CTA keeps in shared memory, of each
+
+MMR_HD uint32_t lut_entry_index(uint32_t w, uint32_t first_long) {
+    return (w >> (32 - kHuffFastBits)) + (((w > first_long ? w : first_long) - first_long) >> 16);
+}
 
 // One frame component (SOF0 order).
 struct JComp {
@@ -86,6 +102,7 @@ struct JBlockRec {
     int32_t q0;         // DC quantiser
     uint32_t local;     // comp | DC table << 8 | AC table << 16, numbered within the frame
 };
+constexpr uint32_t kMostPaths = 6;
 constexpr uint32_t kMaxSched = 64;  // blocks per MCU of a frame with at most four components
 
 struct JFrame {
@@ -115,7 +132,8 @@ struct JFrame {
     uint32_t slice_bits;    // bits per slice (multiple of 32, >= 128)
     uint32_t n_dc, n_ac;    // distinct DC and AC tables of the scan, and the first four of each
     uint32_t dc_id[4], ac_id[4];
-    uint32_t pad;
+    uint32_t lead, paths;   // of the speculative decodes: bits before a slice, and how many (1..kMostPaths)
+    uint32_t shared_tabs;   // 1: they fit a CTA's shared memory (kSharedTabs of each, kSharedLong)
 };
 
 // --------------------------------------------- chunked entropy decoding ----
@@ -160,12 +178,8 @@ struct SlicePoint {
 };
 
 // Checkpoints: the first block boundary 0, 64, 128, 256, 512, 768, 1024 and 1536 bits
-// into a slice (those inside it). The speculative decode of a slice starts
-// spec_lead(S) bits before the slice: the synchronisation distance of Huffman-coded
-// JPEG data is a few hundred bits (longer where the MCU's block phase must also fall
-// into place), so it has usually met the true decode by the slice's first boundary.
+// into a slice (those inside it).
 constexpr int kSliceCheckpoints = 8;
-MMR_HD constexpr uint32_t spec_lead(uint32_t slice_bits) { return slice_bits <= 1024 ? 1536u : slice_bits <= 2048 ? 1024u : 768u; }
 
 struct SliceSpec {
     SlicePoint exit;                      // end of the speculative decode
