@@ -918,8 +918,8 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                 }
                 F.shared_tabs = F.n_dc <= kSharedTabs && F.n_ac <= kSharedTabs;
                 for (uint32_t t = 0; t < 4; t++) {
-                    if (t < F.n_dc) F.shared_tabs &= lut_meta[F.dc_id[t]].len <= kSharedTab;
-                    if (t < F.n_ac) F.shared_tabs &= lut_meta[F.ac_id[t]].len <= kSharedTab;
+                    if (t < F.n_dc) F.shared_tabs &= lut_fits_shared(lut_meta[F.dc_id[t]]);
+                    if (t < F.n_ac) F.shared_tabs &= lut_fits_shared(lut_meta[F.ac_id[t]]);
                 }
                 F.rst_off = rst_total;
                 rst_total += p.n_intervals;

@@ -68,6 +68,9 @@ constexpr uint32_t kSharedLong = 512;
 constexpr uint32_t kSharedTab = (1u << kHuffFastBits) + kSharedLong;
 constexpr uint32_t kSharedTabs = 2;  // DC and AC tables a CTA keeps in shared memory, of each
 
+// Whether a table can be read from shared memory, where windows are not clamped.
+MMR_HD bool lut_fits_shared(const LutMeta &m) { return m.last == 0xffffffffu && m.len <= kSharedTab; }
+
 MMR_HD uint32_t lut_entry_index(uint32_t w, uint32_t first_long) {
     return (w >> (32 - kHuffFastBits)) + (((w > first_long ? w : first_long) - first_long) >> 16);
 }

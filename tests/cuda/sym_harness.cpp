@@ -9,7 +9,8 @@
 #include "huffman_lut.h"
 
 // key: 16 counts then the symbols (a DHT table body). sym and skip: 65536 entries each,
-// of the windows p << 16; meta: entries, first_long, last. `before` entries precede the
+// of the windows p << 16; meta: entries, first_long, last, whether the table may be read
+// without clamping the window, and the largest entry any window then indexes. `before` entries precede the
 // table, as in a batch of several.
 extern "C" void mmr_test_sym(const uint8_t *key, size_t key_len, int ac, size_t before, uint16_t *sym, uint32_t *skip,
                              uint32_t *meta) {
@@ -24,4 +25,7 @@ extern "C" void mmr_test_sym(const uint8_t *key, size_t key_len, int ac, size_t 
     meta[0] = m.len;
     meta[1] = m.first_long;
     meta[2] = m.last;
+    meta[3] = mmr::lut_fits_shared(m);
+    meta[4] = 0;
+    for (uint32_t p = 0; p < 65536; p++) meta[4] = std::max(meta[4], mmr::lut_entry_index(p << 16 | 0xffffu, m.first_long));
 }
