@@ -3,11 +3,13 @@
 //
 // Both transforms are first evaluated in fp32 as separable sums (8 + 8 terms for
 // 8-8; butterfly, 8 + 4 terms for 2-4-8), each factor cu * cos the fp32 product
-// of the fp32 roundings (3u, u = 2^-24) and each pass an FMA chain. Against the
-// exact real value of the reference's terms (its doubles: FRAC_1_SQRT_2, the cos
-// table, the integer c) the fp32 sum is off by at most (3u + 8u) + (3u + 8u) = 22u B
-// for 8-8 and 11u + 3u + 4u = 18u B for 2-4-8; the binary64 sequence by < 70 *
-// 2^-53 B. B = sum |terms| <= C1 = sum |c| for 8-8 (|cos| <= 1, cu cv <= 1) and
+// of the fp32 roundings (3u, u = 2^-24); the horizontal pass takes its even and odd
+// terms as two four-term FMA chains, added and subtracted for the outputs x and 7 - x
+// (the fp32 factors are exactly symmetric), the vertical pass is one FMA chain.
+// Against the exact real value of the reference's terms (its doubles: FRAC_1_SQRT_2,
+// the cos table, the integer c) the fp32 sum is off by at most (3u + 5u) + (3u + 8u) =
+// 19u B for 8-8 and 8u + 3u + 4u = 15u B for 2-4-8 (the bounds below take 22u); the
+// binary64 sequence by < 70 * 2^-53 B. B = sum |terms| <= C1 = sum |c| for 8-8 (|cos| <= 1, cu cv <= 1) and
 // <= C1 / 2 per 2-4-8 field (a butterfly output is at most |c1| + |c2|); after the
 // final / 4.0 or / 2.0, |value32 - value64| <= 5.5u C1 < delta = 2^-21 C1 + 2^-30
 // (= 8u C1 + 2^-30, margin 1.45). If no half-integer lies within delta of value32
@@ -23,6 +25,7 @@
 #include <stdint.h>
 
 #include "exact_fixed.h"
+#include "packed.h"
 #include "rounding.h"
 
 namespace mmr {
@@ -41,16 +44,19 @@ constexpr double kFrac = 0.7071067811865476;  // FRAC_1_SQRT_2
 // The reference's binary64 8-8 direct sum for sample (y, x) (decoder.rs:520-548):
 // terms ((((cu*cv)*c)*cos_u)*cos_v) accumulated in (v, u) order, then / 4.0. Zero
 // coefficients are skipped: their term is +-0.0, which leaves any sum that is not
-// -0.0 unchanged, and these sums are never -0.0.
+// -0.0 unchanged, and these sums are never -0.0. (c: 16-byte aligned rows.)
 __device__ __noinline__ double exact_88(const int32_t *c, int y, int x) {
     const double kk00 = __dmul_rn(kFrac, kFrac);
     double sum = 0.0;
     for (int v = 0; v < 8; v++) {
+        const int4 lo = reinterpret_cast<const int4 *>(c + v * 8)[0], hi = reinterpret_cast<const int4 *>(c + v * 8)[1];
+        const int32_t row[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        if (!(lo.x | lo.y | lo.z | lo.w | hi.x | hi.y | hi.z | hi.w)) continue;
+#pragma unroll
         for (int u = 0; u < 8; u++) {
-            const int32_t cv = c[v * 8 + u];
-            if (cv == 0) continue;
+            if (row[u] == 0) continue;
             const double k = (u == 0 && v == 0) ? kk00 : (u == 0 || v == 0) ? kFrac : 1.0;
-            double t = __dmul_rn(k, (double)cv);
+            double t = __dmul_rn(k, (double)row[u]);
             t = __dmul_rn(t, c_cos16[(2 * x + 1) * u]);
             t = __dmul_rn(t, c_cos16[(2 * y + 1) * v]);
             sum = __dadd_rn(sum, t);
@@ -65,11 +71,16 @@ __device__ __noinline__ double exact_248(const int32_t *c, int y, int x) {
     const int field = y & 1, yy = y >> 1;
     double sum = 0.0;
     for (int v = 0; v < 4; v++) {
-        const int row = v * 2 + field, pair = row >> 1;
+        const int4 *p = reinterpret_cast<const int4 *>(c + v * 16);
+        const int4 a0 = p[0], a1 = p[1], b0 = p[2], b1 = p[3];
+        const int32_t first[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        const int32_t second[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
         double hs = 0.0;
+#pragma unroll
         for (int u = 0; u < 8; u++) {
-            const double first = (double)c[pair * 16 + u], second = (double)c[pair * 16 + 8 + u];
-            const double b = (row & 1) ? __dsub_rn(first, second) : __dadd_rn(first, second);
+            if ((first[u] | second[u]) == 0) continue;
+            const double b = field ? __dsub_rn((double)first[u], (double)second[u])
+                                   : __dadd_rn((double)first[u], (double)second[u]);
             if (b != 0.0) hs = __dadd_rn(hs, __dmul_rn(__dmul_rn(u == 0 ? kFrac : 1.0, b), c_cos16[(2 * x + 1) * u]));
         }
         const double h = hs / 2.0;
@@ -78,34 +89,29 @@ __device__ __noinline__ double exact_248(const int32_t *c, int y, int x) {
     return sum / 2.0;
 }
 
-// The fp32 value's sample when it is certain: no half-integer within delta of
-// the value (c1 = sum |c| of the block), or the value so far beyond 255.5 or
-// below -0.5 that the reference clamps it whatever its rounding (the comparison
-// constants leave room for the fp32 rounding of 256 + delta). -1: undecided.
-__device__ __forceinline__ int dv_decide32(float value, float c1) {
-    const float delta = c1 * 0x1p-21f + 0x1p-30f;
-    float r;
-    const int32_t v = round_nearest(value, r);
-    if (fabsf(value - r) < 0.5f - delta && fabsf(value) < 0x1p22f) return min(max(v, 0), 255);
-    if (value > 256.0f + delta) return 255;
-    if (value < -1.0f - delta) return 0;
-    return -1;
+// Rounds half away from zero and clamps to 0..255.
+__device__ __forceinline__ int dv_round_clamp(double e) {
+    if (!(e > 0.0)) return 0;
+    if (e >= 255.0) return 255;
+    const int n = __double2int_rd(e);
+    return n + (__dsub_rn(e, (double)n) >= 0.5 ? 1 : 0);
 }
 
 // The reference order for sample (y, x), rounded and clamped.
 __device__ __forceinline__ uint8_t dv_exact_sample(const int32_t *c, bool mode248, int y, int x) {
-    const double e = mode248 ? exact_248(c, y, x) : exact_88(c, y, x);
-    return (uint8_t)fmin(fmax(round(e), 0.0), 255.0);
+    return (uint8_t)dv_round_clamp(mode248 ? exact_248(c, y, x) : exact_88(c, y, x));
 }
 
 // The sample of every position of a block whose only nonzero coefficient is the
 // DC: all 64 are equal (cos16[0] = cos8[0] = 1.0, and only the u = v = 0 terms
-// are nonzero), so the reference-order value of position (0, 0) is computed once
-// per block. These blocks are common in smooth content, and with an odd DC level
-// their exact value is a half-integer: every sample would go to the binary64
-// pass one by one.
+// are nonzero: their factors of 1.0 and the sums with 0.0 change nothing). These
+// blocks are common in smooth content, and with an odd DC level their exact value is
+// a half-integer.
 __device__ __forceinline__ uint8_t dv_flat_sample(const int32_t *c, bool mode248) {
-    return dv_exact_sample(c, mode248, 0, 0);
+    const double dc = (double)c[0];
+    const double h = mode248 ? __dmul_rn(kFrac, __dmul_rn(kFrac, dc) * 0.5) * 0.5
+                             : __dmul_rn(__dmul_rn(kFrac, kFrac), dc) * 0.25;
+    return (uint8_t)dv_round_clamp(h);
 }
 
 // ---------------------------------------------------------------------------
@@ -144,57 +150,59 @@ __device__ __forceinline__ void dv_row_pass8(const int32_t *c, const float *wt, 
 #pragma unroll
         for (int u = 0; u < 8; u++) b[u] = (float)c[r * 8 + u];
     }
-    float h[8];
-#pragma unroll
-    for (int x = 0; x < 8; x++) h[x] = 0.0f;
+    // outputs x and 7 - x share their even and odd sums, x pairs in packed FMAs
+    F2 e[2] = {}, o[2] = {};
 #pragma unroll
     for (int u = 0; u < 8; u++) {
-        const float4 w0 = reinterpret_cast<const float4 *>(wt + u * 8)[0];
-        const float4 w1 = reinterpret_cast<const float4 *>(wt + u * 8)[1];
-        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-        for (int x = 0; x < 8; x++) h[x] = fmaf(w[x], b[u], h[x]);
+        const float4 w = reinterpret_cast<const float4 *>(wt + u * 8)[0];
+        F2(&t)[2] = u & 1 ? o : e;
+        t[0] = fma2(f2(w.x, w.y), f2(b[u], b[u]), t[0]);
+        t[1] = fma2(f2(w.z, w.w), f2(b[u], b[u]), t[1]);
     }
-    if (mode248) {
+    const float half = mode248 ? 0.5f : 1.0f;  // (exact)
+    float h[8];
 #pragma unroll
-        for (int x = 0; x < 8; x++) h[x] *= 0.5f;
+    for (int i = 0; i < 2; i++) {
+        float ea, eb, oa, ob;
+        split2(e[i], ea, eb);
+        split2(o[i], oa, ob);
+        h[2 * i] = (ea + oa) * half;
+        h[2 * i + 1] = (eb + ob) * half;
+        h[7 - 2 * i] = (ea - oa) * half;
+        h[6 - 2 * i] = (eb - ob) * half;
     }
     reinterpret_cast<float4 *>(hrow)[0] = make_float4(h[0], h[1], h[2], h[3]);
     reinterpret_cast<float4 *>(hrow)[1] = make_float4(h[4], h[5], h[6], h[7]);
+}
+
+__device__ __forceinline__ void dv_add_row(F2 (&s)[4], const float *h, float w) {
+    const float4 h0 = reinterpret_cast<const float4 *>(h)[0], h1 = reinterpret_cast<const float4 *>(h)[1];
+    s[0] = fma2(f2(w, w), f2(h0.x, h0.y), s[0]);
+    s[1] = fma2(f2(w, w), f2(h0.z, h0.w), s[1]);
+    s[2] = fma2(f2(w, w), f2(h1.x, h1.y), s[2]);
+    s[3] = fma2(f2(w, w), f2(h1.z, h1.w), s[3]);
 }
 
 // Pass 2 for output row y: value[0..7] from the block's 64 pass-1 outputs h
 // (row-major, 16-byte aligned rows).
 __device__ __forceinline__ void dv_column_pass8(const float *h, const float *wt, const float *v4, bool mode248, int y,
                                                 float *value) {
-    float s[8];
-#pragma unroll
-    for (int x = 0; x < 8; x++) s[x] = 0.0f;
+    F2 s[4] = {};
     if (mode248) {
         const int field = y & 1, yy = y >> 1;
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const float wv = v4[yy * 4 + v];
-            const float4 h0 = reinterpret_cast<const float4 *>(h + (v * 2 + field) * 8)[0];
-            const float4 h1 = reinterpret_cast<const float4 *>(h + (v * 2 + field) * 8)[1];
-            const float hv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-#pragma unroll
-            for (int x = 0; x < 8; x++) s[x] = fmaf(wv, hv[x], s[x]);
-        }
-#pragma unroll
-        for (int x = 0; x < 8; x++) value[x] = s[x] * 0.5f;
+        for (int v = 0; v < 4; v++) dv_add_row(s, h + (v * 2 + field) * 8, v4[yy * 4 + v]);
     } else {
 #pragma unroll
-        for (int v = 0; v < 8; v++) {
-            const float wv = wt[v * 8 + y];  // V[y][v] = W[v][y]
-            const float4 h0 = reinterpret_cast<const float4 *>(h + v * 8)[0];
-            const float4 h1 = reinterpret_cast<const float4 *>(h + v * 8)[1];
-            const float hv[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+        for (int v = 0; v < 8; v++) dv_add_row(s, h + v * 8, wt[v * 8 + y]);  // V[y][v] = W[v][y]
+    }
+    const float scale = mode248 ? 0.5f : 0.25f;
 #pragma unroll
-            for (int x = 0; x < 8; x++) s[x] = fmaf(wv, hv[x], s[x]);
-        }
-#pragma unroll
-        for (int x = 0; x < 8; x++) value[x] = s[x] * 0.25f;
+    for (int i = 0; i < 4; i++) {
+        float a, b;
+        split2(s[i], a, b);
+        value[2 * i] = a * scale;
+        value[2 * i + 1] = b * scale;
     }
 }
 
@@ -215,28 +223,44 @@ __device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h
     }
     float value[8];
     dv_column_pass8(h, wt, v4, mode248, y, value);
-    unsigned long long out = 0;
+    // A value is certain when no half-integer lies within delta = 2^-21 C1 + 2^-30 of
+    // it. (round_nearest holds below 2^22; |value| <= C1 / 4 + delta beyond that makes
+    // delta more than a half.) Values past 256 + delta or below -1 - delta are clamped
+    // whatever their rounding.
+    const float delta = c1 * 0x1p-21f + 0x1p-30f, near = 0.5f - delta;
+    int32_t n[8];
     uint32_t und = 0;
 #pragma unroll
     for (int x = 0; x < 8; x++) {
-        const int d = dv_decide32(value[x], c1);
-        if (d < 0) und |= 1u << x;
-        else out |= (unsigned long long)d << (8 * x);
+        float r;
+        n[x] = round_nearest(value[x], r);
+        und |= (fabsf(value[x] - r) < near ? 0u : 1u) << x;
     }
-    *row = out;
+    if (und) {
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+            if (!(und >> x & 1)) continue;
+            const bool over = value[x] > 256.0f + delta, under = value[x] < -1.0f - delta;
+            if (over || under) und &= ~(1u << x);
+            n[x] = over ? 255 : 0;  // (an undecided one is filled in later)
+        }
+    }
+    *row = (unsigned long long)sat_quad_u8(n[4], n[5], n[6], n[7]) << 32 | sat_quad_u8(n[0], n[1], n[2], n[3]);
     return und;
 }
 
 // Settles the undecided samples of every lane of the warp (all 32 lanes call
-// this; und = 0 for lanes with none): one sample at a time the whole warp forms
-// its exact fixed-point value (exact_fixed.h), and the owner lane takes it, or
-// the reference order when that value is too close to a half-integer.
+// this; und = 0 for lanes with none, whose bytes of row are 0). One sample at a time
+// the whole warp forms its exact fixed-point value (exact_fixed.h); those too close to
+// a half-integer for that take the reference order, each lane its own. (A block whose
+// few coefficients have rational factors ties in all its samples: one after another
+// they made one frame's transform wait 0.1 ms for one warp.)
 // c: the lane's block coefficients (shared), c1i = sum |c| exactly, fix: the
 // 8-8 table followed by the 2-4-8 table.
 __device__ __forceinline__ void dv_resolve_row(uint32_t und, unsigned long long &row, const int32_t *c,
                                                bool mode248, int y, int32_t c1i, const long long *fix) {
     const int lane = threadIdx.x & 31;
-    uint32_t m;
+    uint32_t m, left = 0;
     while ((m = __ballot_sync(0xffffffffu, und != 0)) != 0) {
         const int src = __ffs(m) - 1;
         const uint32_t sund = __shfl_sync(0xffffffffu, und, src);
@@ -249,10 +273,14 @@ __device__ __forceinline__ void dv_resolve_row(uint32_t und, unsigned long long 
         int smp = -1;
         if (sc1 < kFixMaxC1) smp = fixed_round(fixed_sum(fix + smode * kFixEntries + (sy * 8 + x) * 64, sc), sc1, 0);
         if (lane == src) {
-            if (smp < 0) smp = dv_exact_sample(c, mode248, y, x);
-            row |= (unsigned long long)smp << (8 * x);
+            if (smp < 0) left |= 1u << x;
+            else row |= (unsigned long long)smp << (8 * x);
             und &= und - 1;
         }
+    }
+    for (; left; left &= left - 1) {
+        const int x = __ffs(left) - 1;
+        row |= (unsigned long long)dv_exact_sample(c, mode248, y, x) << (8 * x);
     }
 }
 

@@ -17,20 +17,12 @@
 
 #include "idct_core.h"
 #include "kernels.h"
+#include "packed.h"
 
 namespace mmr {
 namespace {
 
 constexpr int kFStride = 68;  // floats per staged block (16-byte rows, conflict-free over 8 blocks)
-
-// Four channel values saturated to 0..255 and packed, b0 in the low byte
-// (cvt.pack.sat: d = c << 16 | sat(a) << 8 | sat(b)).
-__device__ __forceinline__ uint32_t pack4_sat_u8(int32_t b0, int32_t b1, int32_t b2, int32_t b3) {
-    uint32_t hi, d;
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(b3), "r"(b2), "r"(0));
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(b1), "r"(b0), "r"(hi));
-    return d;
-}
 
 template <int HM, int VM, int NM>
 struct FusedShape {
@@ -183,7 +175,7 @@ __device__ __forceinline__ void fused_tile(const JpegLaunch &L, const FusedLaunc
                 }
 #pragma unroll
                 for (int j = 0; j < 3; j++)
-                    word[3 * g + j] = pack4_sat_u8(ch[4 * j], ch[4 * j + 1], ch[4 * j + 2], ch[4 * j + 3]);
+                    word[3 * g + j] = sat_quad_u8(ch[4 * j], ch[4 * j + 1], ch[4 * j + 2], ch[4 * j + 3]);
             }
             uint4 *o = reinterpret_cast<uint4 *>(J.out + ((uint64_t)(y0 + ly) * J.width + x0 + lx) * 3);
             o[0] = make_uint4(word[0], word[1], word[2], word[3]);
@@ -210,7 +202,7 @@ __device__ __forceinline__ void fused_tile(const JpegLaunch &L, const FusedLaunc
         }
         uint32_t word[3];
 #pragma unroll
-        for (int j = 0; j < 3; j++) word[j] = pack4_sat_u8(ch[4 * j], ch[4 * j + 1], ch[4 * j + 2], ch[4 * j + 3]);
+        for (int j = 0; j < 3; j++) word[j] = sat_quad_u8(ch[4 * j], ch[4 * j + 1], ch[4 * j + 2], ch[4 * j + 3]);
         uint32_t *o = direct ? reinterpret_cast<uint32_t *>(J.out + ((uint64_t)(y0 + ly) * J.width + x0 + lx) * 3)
                              : reinterpret_cast<uint32_t *>(S.rgb + ly * Sh::RW + lx * 3);
         o[0] = word[0];
