@@ -1,8 +1,7 @@
 // DV25 decode kernels for sm_103a.
 //
-//   dif_check  one thread per 80-byte DIF block: identifier vs canonical layout
-//              (crates/codecs/dv/src/dif.rs:181-253).
-//   segment    a CTA per four video segments (5 macroblocks, 30 blocks each):
+//   segment    four video segments (5 macroblocks, 30 blocks each) per CTA step: DIF
+//              identifiers vs the canonical layout (crates/codecs/dv/src/dif.rs:181-253),
 //              DC/mode/class fields, VLC decode and the three-level spill of
 //              unused bits -- block region (a thread per block), macroblock pool
 //              (a thread per macroblock), segment pool (a thread per segment)
@@ -15,6 +14,8 @@
 //              near-ties (decoder.rs:520-602, dv_idct_core.h); then placement
 //              (decoder.rs:395-505).
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "dv_idct_core.h"
 #include "kernels.h"
@@ -65,18 +66,6 @@ __device__ __forceinline__ void expected_id(uint32_t pos, uint32_t *section, uin
     }
 }
 
-__global__ void dif_check_kernel(DvLaunch L) {
-    uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= L.n_dif) return;
-    uint32_t f = upper_index32(L.dif_first, L.n_frames, g);
-    uint32_t local = g - L.dif_first[f];
-    const uint8_t *b = L.frames[f].in + (size_t)local * 80;
-    uint32_t es, en;
-    expected_id(local % 150, &es, &en);
-    bool bad = (uint32_t)(b[0] >> 5) != es || (uint32_t)(b[1] >> 4) != local / 150 || (uint32_t)b[2] != en;
-    L.flags[g] = bad ? 1 : 0;
-}
-
 // ---- bit buffers (MSB-first, 32-bit words) ----
 
 __device__ __forceinline__ uint32_t get32(const uint32_t *w, uint32_t bit) {
@@ -112,83 +101,10 @@ struct DvBlock {
     uint8_t pad;
 };
 
-// consume_ac (decoder.rs:245-284) on the virtual stream (partial bits ++ buf[pos, end)).
-// On completion *pos is left after the EOB; otherwise the remaining bits become the
-// block's partial and *pos == end.
-__device__ void consume_ac(DvBlock &b, const uint32_t *buf, uint32_t &pos, uint32_t end, int16_t *coef,
-                           uint32_t qno, const uint32_t *__restrict__ vlc, bool &bad_vlc) {
-    if (b.complete) return;
-    uint32_t pval = b.pval;
-    int plen = b.plen;
-    b.plen = 0;
-    b.pval = 0;
-    for (;;) {
-        uint32_t avail = (uint32_t)plen + (end - pos);
-        // next 16 bits of (partial ++ input), zero-padded
-        uint32_t w16;
-        if (plen) {
-            uint32_t rest = get32(buf, pos) >> 16;  // 16 bits from pos (beyond end: don't care, masked below)
-            w16 = ((pval << (16 - plen)) | (rest >> plen)) & 0xffffu;
-        } else {
-            w16 = get32(buf, pos) >> 16;
-        }
-        if (avail < 16) w16 &= 0xffffu << (16 - avail);
-        uint32_t e = vlc[w16 >> (16 - kDvVlcL1Bits)];
-        if (e & 0x80000000u) e = vlc[(e & 0xffffu) + (w16 & ((1u << (16 - kDvVlcL1Bits)) - 1))];
-        uint32_t len = e & 31;
-        if (len != 0 && len <= avail) {
-            // consume len bits: all partial bits first (a partial never holds a whole code)
-            if ((int)len <= plen) {
-                plen -= (int)len;
-                pval &= (1u << plen) - 1;
-            } else {
-                pos += len - (uint32_t)plen;
-                plen = 0;
-                pval = 0;
-            }
-            uint32_t run = (e >> 5) & 127;
-            int32_t level = (int32_t)((e >> 12) & 511) - 256;
-            uint32_t p = b.position + run + 1;
-            if (p >= 64) {
-                b.position = 64;
-                b.complete = 1;
-                return;
-            }
-            b.position = (uint8_t)p;
-            if (level != 0) {
-                // inverse_factor_for_encoding (decoder.rs:290-310)
-                uint32_t q = qno + (uint32_t)c_dv_qoff[b.cls];
-                uint32_t area = p <= 5 ? 0 : p <= 20 ? 1 : p <= 42 ? 2 : 3;
-                int32_t weight = b.mode ? c_dv_w248[p] : c_dv_w88[p];
-                int32_t factor = weight << (c_dv_shifts[q * 4 + area] + 1 + (b.cls == 3));
-                int32_t lv = (level * factor + 8192) >> 14;
-                coef[b.mode ? c_dv_zz248[p] : c_dv_zz88[p]] = (int16_t)lv;
-            }
-        } else if (avail < 16) {
-            // save as partial: remaining partial bits then the rest of the input
-            uint32_t v = pval;
-            int n = plen;
-            uint32_t in_n = end - pos;
-            if (in_n) {
-                v = (v << in_n) | (get32(buf, pos) >> (32 - in_n));
-                n += (int)in_n;
-            }
-            b.pval = (uint16_t)v;
-            b.plen = (uint8_t)n;
-            pos = end;
-            return;
-        } else {
-            bad_vlc = true;  // unreachable: the DV VLC code is complete (Kraft sum 1)
-            pos = end;
-            return;
-        }
-    }
-}
-
-// A CTA per four video segments (dv/src/decoder.rs:152-317), in the reference's
-// three levels, each level's independent parts in parallel:
+// A CTA takes four video segments per step (dv/src/decoder.rs:152-317), in the
+// reference's three levels, each level's independent parts in parallel:
 //   1. a thread per block (120): DC/mode/class and the AC codes inside the
-//      block's own region of its macroblock's payload;
+//      block's own region of its macroblock's payload, the region's bits in registers;
 //   2. a thread per macroblock (20): the leftover bits of its complete blocks, in
 //      block order, make the macroblock pool, which its incomplete blocks
 //      consume in order (decode_macroblock, decoder.rs:193-243);
@@ -196,162 +112,270 @@ __device__ void consume_ac(DvBlock &b, const uint32_t *buf, uint32_t &pos, uint3
 //      order, make the segment pool, which the segment's incomplete blocks
 //      consume in order (consume_pool_for_macroblocks, decoder.rs:225-233).
 // Payload, pools and dequantised coefficients stay in shared memory; every
-// block's 64 coefficients (zeros included) then leave as 16-byte stores.
+// block's 64 coefficients (zeros included) then leave as 16-byte stores. CTAs are
+// persistent: the VLC table and the dequantisation tables, which the lanes index
+// freely, are copied to shared memory once (constant memory and L1 served such
+// lookups a lane at a time).
 constexpr int kSegPerCta = 4;
 constexpr int kSegBlocks = kSegPerCta * 30;
+constexpr int kSegMbs = kSegPerCta * 5;
 constexpr int kSegThreads = 128;
+constexpr int kSegCtasPerSm = 6;
 
 struct SegSmem {
     __align__(16) int16_t coef[kSegBlocks][64];
-    uint32_t pay[kSegPerCta][5 * 19 + 1];  // payload words of the five macroblocks (+1: reads past the end)
-    uint32_t mbpool[kSegPerCta * 5][20];
+    __align__(16) uint32_t vlc[kDvVlcEntries];
+    uint32_t dequant[2][64];            // per mode and zigzag index: weight | natural index << 16 | 8 * area << 24
+    uint32_t shifts[22];                // per quantiser row: the four areas' shifts, a byte each
+    uint32_t pay[kSegPerCta][5 * 19 + 5];  // payload words of the five macroblocks (+5: reads past the end)
+    uint32_t mbpool[kSegMbs][20];
     uint32_t segpool[kSegPerCta][5 * 19 + 2];
     DvBlock blk[kSegBlocks];
     uint16_t left_start[kSegBlocks], left_len[kSegBlocks];  // unused bits of a complete block's region
-    uint16_t mb_pos[kSegPerCta * 5], mb_len[kSegPerCta * 5];
-    uint32_t dif_off[kSegPerCta * 5];  // byte offset of each macroblock's DIF block in the frame
+    uint16_t mb_pos[kSegMbs], mb_len[kSegMbs];
+    uint32_t dif_off[kSegMbs];  // byte offset of each macroblock's DIF block in the frame
     uint32_t frame[kSegPerCta], local[kSegPerCta];
-    uint8_t qno[kSegPerCta * 5];
+    uint8_t qno[kSegMbs], damaged[kSegMbs];
     uint8_t bad[kSegBlocks];
     uint16_t kind[kSegPerCta];
 };
 
-__global__ void __launch_bounds__(kSegThreads) segment_kernel(DvLaunch L) {
+// Entry of the next 16 bits. The codes of more than kDvVlcL1Bits bits are the last of
+// the code space, so the level-2 blocks follow one another in code order and one index
+// reaches both levels (dv_vlc_one_index checks the table).
+__device__ __forceinline__ uint32_t vlc_entry(const SegSmem &S, uint32_t w16) {
+    return S.vlc[w16 < kDvVlcLong ? w16 >> (16 - kDvVlcL1Bits) : (1u << kDvVlcL1Bits) + w16 - kDvVlcLong];
+}
+
+// A block's dequantisation: its table, and its quantiser row's shifts
+// (inverse_factor_for_encoding, decoder.rs:290-310).
+struct Dequant {
+    const uint32_t *table;
+    uint32_t shifts;
+    int16_t *coef;
+};
+
+__device__ __forceinline__ Dequant dequant_of(SegSmem &S, const DvBlock &b, uint32_t block, uint32_t qno) {
+    Dequant d;
+    d.table = S.dequant[b.mode];
+    d.shifts = S.shifts[qno + (uint32_t)c_dv_qoff[b.cls]] + (b.cls == 3 ? 0x02020202u : 0x01010101u);
+    d.coef = S.coef[block];
+    return d;
+}
+
+// Moves the position past the entry's run; true when that completes the block, else its
+// level is stored (a zero level changes nothing).
+__device__ __forceinline__ bool take_level(const Dequant &d, uint32_t e, uint32_t &p) {
+    p += ((e >> 5) & 127) + 1;
+    if (p >= 64) return true;
+    const uint32_t t = d.table[p];
+    const int32_t level = (int32_t)((e >> 12) & 511) - 256;
+    const int32_t factor = (int32_t)((t & 0xffff) << ((d.shifts >> (t >> 24)) & 0xff));
+    d.coef[(t >> 16) & 63] = (int16_t)((level * factor + 8192) >> 14);
+    return false;
+}
+
+// consume_ac (decoder.rs:245-284) on a pool, the virtual stream (partial bits ++
+// buf[pos, end)). On completion pos is left after the EOB; otherwise the remaining
+// bits become the block's partial and pos == end.
+__device__ void consume_pool(SegSmem &S, uint32_t block, uint32_t qno, const uint32_t *buf, uint32_t &pos, uint32_t end,
+                             bool &bad_vlc) {
+    DvBlock &b = S.blk[block];
+    const Dequant d = dequant_of(S, b, block, qno);
+    uint32_t p = b.position, plen = b.plen, avail = plen + (end - pos);
+    uint32_t w16 = get32(buf, pos) >> 16;
+    if (plen) w16 = (((uint32_t)b.pval << (16 - plen)) | (w16 >> plen)) & 0xffffu;
+    b.plen = 0;
+    b.pval = 0;
+    for (;;) {
+        const uint32_t e = vlc_entry(S, w16), len = e & 31;
+        if (len == 0) {  // unreachable: the DV VLC code is complete (Kraft sum 1)
+            bad_vlc = true;
+            pos = end;
+            break;
+        }
+        if (len > avail) {  // fewer than 16 bits: the next partial
+            b.pval = (uint16_t)(w16 >> (16 - avail));
+            b.plen = (uint8_t)avail;
+            pos = end;
+            break;
+        }
+        avail -= len;
+        pos += len - plen;  // (a partial never holds a whole code)
+        plen = 0;
+        if (take_level(d, e, p)) {
+            b.complete = 1;
+            p = 64;
+            break;
+        }
+        w16 = get32(buf, pos) >> 16;
+    }
+    b.position = (uint8_t)p;
+}
+
+__global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvLaunch L) {
     __shared__ SegSmem S;
     const uint32_t t = threadIdx.x;
-    const uint32_t g0 = blockIdx.x * kSegPerCta;
-    // segment records: frame, segment in frame, DIF blocks, damaged identifiers
-    if (t < (uint32_t)kSegPerCta) {
-        const uint32_t g = g0 + t;
-        uint16_t kind = 0xffff;  // no segment
-        if (g < L.n_segments) {
-            const uint32_t f = upper_index32(L.seg_first, L.n_frames, g);
-            const DvFrame &F = L.frames[f];
-            const uint32_t local = g - L.seg_first[f];
-            const uint32_t sequence = local / 27, slot = local % 27;
-            kind = kDiagNone;
-            for (int m = 0; m < 5; m++) {
-                const uint32_t vn = slot * 5 + m;
-                const uint32_t dif = sequence * 150 + 7 + (vn / 15) * 16 + vn % 15;
-                if (kind == kDiagNone && L.flags[F.dif_first + dif]) kind = kDvDamagedId;
-                S.dif_off[t * 5 + m] = dif * 80;
-                S.qno[t * 5 + m] = F.in[(size_t)dif * 80 + 3] & 0x0f;
-            }
-            S.frame[t] = f;
-            S.local[t] = local;
-        }
-        S.kind[t] = kind;
+    for (uint32_t i = t; i < (uint32_t)kDvVlcEntries; i += kSegThreads) S.vlc[i] = __ldg(L.vlc + i);
+    {
+        const uint32_t p = t & 63, m = t >> 6;  // kSegThreads = 2 x 64
+        const uint32_t area = p <= 5 ? 0 : p <= 20 ? 1 : p <= 42 ? 2 : 3;
+        S.dequant[m][p] = (uint32_t)(m ? c_dv_w248[p] : c_dv_w88[p]) |
+                          (uint32_t)(m ? c_dv_zz248[p] : c_dv_zz88[p]) << 16 | area << 27;
+        if (t < 22)
+            S.shifts[t] = c_dv_shifts[t * 4] | c_dv_shifts[t * 4 + 1] << 8 | c_dv_shifts[t * 4 + 2] << 16 |
+                          (uint32_t)c_dv_shifts[t * 4 + 3] << 24;
     }
-    __syncthreads();
-    // payload words (bytes 4..80 of each DIF block), big-endian
-    for (uint32_t i = t; i < (uint32_t)kSegPerCta * 96; i += kSegThreads) {
-        const uint32_t sg = i / 96, wi = i % 96;
-        uint32_t v = 0;
-        if (wi < 95 && S.kind[sg] == kDiagNone) {
-            const uint32_t m = wi / 19;
-            const uint8_t *src = L.frames[S.frame[sg]].in + S.dif_off[sg * 5 + m] + 4 + (wi % 19) * 4;
-            v = ((uint32_t)src[0] << 24) | ((uint32_t)src[1] << 16) | ((uint32_t)src[2] << 8) | (uint32_t)src[3];
-        }
-        S.pay[sg][wi] = v;
-    }
-    for (uint32_t i = t; i < (uint32_t)kSegBlocks * 8; i += kSegThreads)
-        reinterpret_cast<int4 *>(&S.coef[0][0])[i] = make_int4(0, 0, 0, 0);
-    for (uint32_t i = t; i < (uint32_t)kSegPerCta * 5 * 20; i += kSegThreads) (&S.mbpool[0][0])[i] = 0;
-    for (uint32_t i = t; i < (uint32_t)kSegPerCta * 97; i += kSegThreads) (&S.segpool[0][0])[i] = 0;
-    __syncthreads();
-    // 1. a thread per block: its own region
-    if (t < (uint32_t)kSegBlocks) {
-        const uint32_t sg = t / 30, b = t % 30, m = b / 6, bi = b % 6;
-        DvBlock &B = S.blk[t];
-        B.position = 0;
-        B.complete = 0;
-        B.mode = 0;
-        B.cls = 0;
-        B.pval = 0;
-        B.plen = 0;
-        B.pad = 0;
-        uint16_t ls = 0, ll = 0;
-        bool bad = false;
-        if (S.kind[sg] == kDiagNone) {
-            const uint32_t *w = S.pay[sg] + m * 19;
-            const uint32_t r0 = bi < 4 ? bi * 112 : 448 + (bi - 4) * 80, bits = bi < 4 ? 112 : 80;
-            const uint32_t head = get32(w, r0) >> 20;  // 12 bits: dc(9) mode(1) class(2)
-            int32_t dc = (int32_t)(head >> 3);
-            if (dc & 0x100) dc -= 512;
-            B.mode = (head >> 2) & 1;
-            B.cls = head & 3;
-            S.coef[t][0] = (int16_t)(dc * 4 + 1024);
-            uint32_t pos = r0 + 12;
-            const uint32_t end = r0 + bits;
-            consume_ac(B, w, pos, end, S.coef[t], S.qno[sg * 5 + m], L.vlc, bad);
-            if (B.complete) {
-                ls = (uint16_t)pos;
-                ll = (uint16_t)(end - pos);
-            }
-        }
-        S.left_start[t] = ls;
-        S.left_len[t] = ll;
-        S.bad[t] = bad ? 1 : 0;
-    }
-    __syncthreads();
-    // 2. a thread per macroblock: its pool
-    if (t < (uint32_t)kSegPerCta * 5) {
-        const uint32_t sg = t / 5, m = t % 5;
-        uint32_t pos = 0, mbn = 0;
-        if (S.kind[sg] == kDiagNone) {
-            const uint32_t *w = S.pay[sg] + m * 19;
-            const uint32_t j0 = sg * 30 + m * 6;
-            for (uint32_t j = j0; j < j0 + 6; j++)
-                if (S.blk[j].complete) append_bits(S.mbpool[t], mbn, w, S.left_start[j], S.left_len[j]);
-            bool bad = false;
-            for (uint32_t j = j0; j < j0 + 6; j++)
-                if (!S.blk[j].complete && pos < mbn)
-                    consume_ac(S.blk[j], S.mbpool[t], pos, mbn, S.coef[j], S.qno[t], L.vlc, bad);
-            if (bad) S.bad[j0] = 1;
-        }
-        S.mb_pos[t] = (uint16_t)pos;
-        S.mb_len[t] = (uint16_t)mbn;
-    }
-    __syncthreads();
-    // 3. a thread per segment: its pool, then its result
-    if (t < (uint32_t)kSegPerCta && S.kind[t] == kDiagNone) {
-        uint32_t segn = 0;
-        for (uint32_t m = 0; m < 5; m++) {
-            const uint32_t k = t * 5 + m;
-            if (S.mb_pos[k] < S.mb_len[k])
-                append_bits(S.segpool[t], segn, S.mbpool[k], S.mb_pos[k], S.mb_len[k] - S.mb_pos[k]);
-        }
-        uint32_t pos = 0;
-        bool bad = false;
-        for (uint32_t j = 0; j < 30; j++) {
-            const uint32_t jj = t * 30 + j;
-            if (!S.blk[jj].complete && pos < segn)
-                consume_ac(S.blk[jj], S.segpool[t], pos, segn, S.coef[jj], S.qno[t * 5 + j / 6], L.vlc, bad);
-        }
-        for (uint32_t j = 0; j < 30; j++) bad |= S.bad[t * 30 + j] != 0;
-        uint16_t kind = kDiagNone;
-        if (bad) kind = kDvBadVlc;
-        else
-            for (uint32_t j = 0; j < 30; j++)
-                if (!S.blk[t * 30 + j].complete) {
-                    kind = kDvIncomplete;
-                    break;
+    for (uint32_t g0 = blockIdx.x * kSegPerCta; g0 < L.n_segments; g0 += gridDim.x * kSegPerCta) {
+        __syncthreads();  // the tables; the last step's results
+        // macroblock records: DIF block, its identifier against the canonical layout
+        // (dif.rs:181-253), quantiser
+        if (t < (uint32_t)kSegMbs) {
+            const uint32_t sg = t / 5, m = t % 5, g = g0 + sg;
+            if (g < L.n_segments) {
+                const uint32_t f = upper_index32(L.seg_first, L.n_frames, g);
+                const uint32_t local = g - L.seg_first[f], sequence = local / 27, slot = local % 27;
+                const uint32_t vn = slot * 5 + m, pos = 7 + (vn / 15) * 16 + vn % 15;  // DIF block of the sequence
+                const uint32_t off = (sequence * 150 + pos) * 80;
+                const uint8_t *b = L.frames[f].in + off;
+                uint32_t es, en;
+                expected_id(pos, &es, &en);
+                S.damaged[t] = (uint32_t)(b[0] >> 5) != es || (uint32_t)(b[1] >> 4) != sequence || (uint32_t)b[2] != en;
+                S.qno[t] = b[3] & 0x0f;
+                S.dif_off[t] = off;
+                if (m == 0) {
+                    S.frame[sg] = f;
+                    S.local[sg] = local;
                 }
-        S.kind[t] = kind;
-    }
-    __syncthreads();
-    // coefficients out (the CTA's segments are consecutive: blocks g0 * 30 ..), modes, results
-    const uint32_t n_seg = min((uint32_t)kSegPerCta, L.n_segments - g0);
-    int4 *dst = reinterpret_cast<int4 *>(L.coef + (uint64_t)g0 * 30 * 64);
-    const int4 *src = reinterpret_cast<const int4 *>(&S.coef[0][0]);
-    for (uint32_t i = t; i < n_seg * 30 * 8; i += kSegThreads) dst[i] = src[i];
-    if (t < n_seg * 30) L.modes[(uint64_t)g0 * 30 + t] = S.blk[t].mode;
-    if (t < n_seg) {
-        const uint16_t kind = S.kind[t];
-        L.seg_err[g0 + t] = (uint8_t)kind;
-        if (kind != kDiagNone) {
-            atomicMin(&L.states[S.frame[t]].bad_segment, S.local[t]);
-            atomicAdd(&L.states[S.frame[t]].failed, 1u);
+            }
+        }
+        for (uint32_t i = t; i < (uint32_t)kSegBlocks * 8; i += kSegThreads)
+            reinterpret_cast<int4 *>(&S.coef[0][0])[i] = make_int4(0, 0, 0, 0);
+        for (uint32_t i = t; i < (uint32_t)kSegMbs * 20; i += kSegThreads) (&S.mbpool[0][0])[i] = 0;
+        for (uint32_t i = t; i < (uint32_t)kSegPerCta * 97; i += kSegThreads) (&S.segpool[0][0])[i] = 0;
+        __syncthreads();
+        if (t < (uint32_t)kSegPerCta) {
+            uint16_t kind = g0 + t < L.n_segments ? kDiagNone : 0xffff;  // 0xffff: no segment
+            for (int m = 0; m < 5; m++)
+                if (kind == kDiagNone && S.damaged[t * 5 + m]) kind = kDvDamagedId;
+            S.kind[t] = kind;
+        }
+        // payload words (bytes 4..80 of each DIF block), big-endian
+        for (uint32_t i = t; i < (uint32_t)kSegPerCta * 100; i += kSegThreads) {
+            const uint32_t sg = i / 100, wi = i - sg * 100;
+            uint32_t v = 0;
+            if (wi < 95 && g0 + sg < L.n_segments) {
+                const uint32_t m = wi / 19;
+                const uint8_t *src = L.frames[S.frame[sg]].in + S.dif_off[sg * 5 + m] + 4 + (wi - m * 19) * 4;
+                if ((reinterpret_cast<uintptr_t>(src) & 3) == 0)
+                    v = __byte_perm(__ldg(reinterpret_cast<const uint32_t *>(src)), 0, 0x0123);
+                else
+                    v = ((uint32_t)src[0] << 24) | ((uint32_t)src[1] << 16) | ((uint32_t)src[2] << 8) | (uint32_t)src[3];
+            }
+            S.pay[sg][wi] = v;
+        }
+        __syncthreads();
+        // 1. a thread per block: its own region
+        if (t < (uint32_t)kSegBlocks) {
+            const uint32_t sg = t / 30, b = t % 30, m = b / 6, bi = b % 6;
+            DvBlock B{};
+            uint16_t ls = 0, ll = 0;
+            bool bad = false;
+            if (S.kind[sg] == kDiagNone) {
+                const uint32_t *w = S.pay[sg] + m * 19;
+                const uint32_t r0 = bi < 4 ? bi * 112 : 448 + (bi - 4) * 80, bits = bi < 4 ? 112 : 80;
+                const uint32_t head = get32(w, r0) >> 20;  // 12 bits: dc(9) mode(1) class(2)
+                int32_t dc = (int32_t)(head >> 3);
+                if (dc & 0x100) dc -= 512;
+                B.mode = (head >> 2) & 1;
+                B.cls = head & 3;
+                const Dequant d = dequant_of(S, B, t, S.qno[sg * 5 + m]);
+                d.coef[0] = (int16_t)(dc * 4 + 1024);
+                // the region's bits after the header (at most 100), left-aligned
+                const uint32_t at = r0 + 12, i = at >> 5, o = at & 31;
+                uint32_t a0 = __funnelshift_l(w[i + 1], w[i], o), a1 = __funnelshift_l(w[i + 2], w[i + 1], o);
+                uint32_t a2 = __funnelshift_l(w[i + 3], w[i + 2], o), a3 = __funnelshift_l(w[i + 4], w[i + 3], o);
+                uint32_t left = bits - 12, p = 0;
+                for (;;) {
+                    const uint32_t e = vlc_entry(S, a0 >> 16), len = e & 31;
+                    if (len == 0) bad = true;  // unreachable: the code is complete
+                    if (len == 0 || len > left) {
+                        B.pval = (uint16_t)(left < 16 ? a0 >> 16 >> (16 - left) : 0);  // the partial
+                        B.plen = (uint8_t)(left < 16 ? left : 0);
+                        break;
+                    }
+                    a0 = __funnelshift_l(a1, a0, len);
+                    a1 = __funnelshift_l(a2, a1, len);
+                    a2 = __funnelshift_l(a3, a2, len);
+                    a3 <<= len;
+                    left -= len;
+                    if (take_level(d, e, p)) {
+                        p = 64;
+                        B.complete = 1;
+                        ls = (uint16_t)(r0 + bits - left);
+                        ll = (uint16_t)left;
+                        break;
+                    }
+                }
+                B.position = (uint8_t)p;
+            }
+            S.blk[t] = B;
+            S.left_start[t] = ls;
+            S.left_len[t] = ll;
+            S.bad[t] = bad ? 1 : 0;
+        }
+        __syncthreads();
+        // 2. a thread per macroblock: its pool
+        if (t < (uint32_t)kSegMbs) {
+            const uint32_t sg = t / 5, m = t % 5;
+            uint32_t pos = 0, mbn = 0;
+            if (S.kind[sg] == kDiagNone) {
+                const uint32_t *w = S.pay[sg] + m * 19;
+                const uint32_t j0 = sg * 30 + m * 6;
+                for (uint32_t j = j0; j < j0 + 6; j++)
+                    if (S.blk[j].complete) append_bits(S.mbpool[t], mbn, w, S.left_start[j], S.left_len[j]);
+                bool bad = false;
+                for (uint32_t j = j0; j < j0 + 6 && pos < mbn; j++)
+                    if (!S.blk[j].complete) consume_pool(S, j, S.qno[t], S.mbpool[t], pos, mbn, bad);
+                if (bad) S.bad[j0] = 1;
+            }
+            S.mb_pos[t] = (uint16_t)pos;
+            S.mb_len[t] = (uint16_t)mbn;
+        }
+        __syncthreads();
+        // 3. a thread per segment: its pool, then its result
+        if (t < (uint32_t)kSegPerCta && S.kind[t] == kDiagNone) {
+            uint32_t segn = 0;
+            for (uint32_t m = 0; m < 5; m++) {
+                const uint32_t k = t * 5 + m;
+                if (S.mb_pos[k] < S.mb_len[k])
+                    append_bits(S.segpool[t], segn, S.mbpool[k], S.mb_pos[k], S.mb_len[k] - S.mb_pos[k]);
+            }
+            uint32_t pos = 0;
+            bool bad = false, incomplete = false;
+            for (uint32_t j = 0; j < 30; j++) {
+                const uint32_t jj = t * 30 + j;
+                if (!S.blk[jj].complete && pos < segn)
+                    consume_pool(S, jj, S.qno[t * 5 + j / 6], S.segpool[t], pos, segn, bad);
+                bad |= S.bad[jj] != 0;
+                incomplete |= !S.blk[jj].complete;
+            }
+            S.kind[t] = bad ? kDvBadVlc : incomplete ? kDvIncomplete : kDiagNone;
+        }
+        __syncthreads();
+        // coefficients out (the CTA's segments are consecutive: blocks g0 * 30 ..), modes, results
+        const uint32_t n_seg = min((uint32_t)kSegPerCta, L.n_segments - g0);
+        int4 *dst = reinterpret_cast<int4 *>(L.coef + (uint64_t)g0 * 30 * 64);
+        const int4 *src = reinterpret_cast<const int4 *>(&S.coef[0][0]);
+        for (uint32_t i = t; i < n_seg * 30 * 8; i += kSegThreads) dst[i] = src[i];
+        if (t < n_seg * 30) L.modes[(uint64_t)g0 * 30 + t] = S.blk[t].mode;
+        if (t < n_seg) {
+            const uint16_t kind = S.kind[t];
+            L.seg_err[g0 + t] = (uint8_t)kind;
+            if (kind != kDiagNone) {
+                atomicMin(&L.states[S.frame[t]].bad_segment, S.local[t]);
+                atomicAdd(&L.states[S.frame[t]].failed, 1u);
+            }
         }
     }
 }
@@ -534,8 +558,8 @@ __global__ void __launch_bounds__(kIdctThreads) dv_idct_kernel(DvLaunch L) {
 }  // namespace
 
 void launch_dv_decode(const DvLaunch &L, cudaStream_t s) {
-    if (L.n_dif) dif_check_kernel<<<(L.n_dif + 255) / 256, 256, 0, s>>>(L);
-    if (L.n_segments) segment_kernel<<<(L.n_segments + kSegPerCta - 1) / kSegPerCta, kSegThreads, 0, s>>>(L);
+    const uint32_t steps = (L.n_segments + kSegPerCta - 1) / kSegPerCta;
+    if (steps) segment_kernel<<<std::min<uint32_t>(steps, 152 * kSegCtasPerSm), kSegThreads, 0, s>>>(L);
     if (L.n_frames) dv_resolve_kernel<<<(L.n_frames + 127) / 128, 128, 0, s>>>(L);
 }
 

@@ -38,7 +38,6 @@ constexpr size_t kDvStaticScratchBytes = 2304u * 1024u;  // 2.25 MiB
 constexpr size_t kDvMaxInput = 144000;                   // one 625/50 frame
 constexpr size_t kDvMaxPlanar = 720 * 576 + 2 * 360 * 288;
 constexpr uint32_t kDvMaxSegments = 12 * 27;
-constexpr uint32_t kDvMaxDif = 12 * 150;
 constexpr size_t kVlcMaxEntries = kDvVlcMaxEntries;
 
 static __device__ __align__(256) uint8_t g_dv_scratch[kDvStaticScratchBytes];
@@ -47,8 +46,7 @@ constexpr size_t a256(size_t v) { return (v + 255) / 256 * 256; }
 // Layout of g_dv_scratch (byte offsets).
 constexpr size_t kOffIn = 0;
 constexpr size_t kOffOut = kOffIn + a256(kDvMaxInput);
-constexpr size_t kOffFlags = kOffOut + a256(kDvMaxPlanar);
-constexpr size_t kOffSegErr = kOffFlags + a256(kDvMaxDif);
+constexpr size_t kOffSegErr = kOffOut + a256(kDvMaxPlanar);
 constexpr size_t kOffModes = kOffSegErr + a256(kDvMaxSegments);
 constexpr size_t kOffCoef = kOffModes + a256(kDvMaxSegments * 30);
 constexpr size_t kOffVlc = kOffCoef + a256((size_t)kDvMaxSegments * 30 * 128);
@@ -62,7 +60,6 @@ struct Meta {  // per-call plan and state (lives at kOffMeta)
     DvState state;
     uint32_t item_ok;
     uint32_t seg_first[2];
-    uint32_t dif_first[2];
 };
 static_assert(sizeof(Meta) <= kMetaBytes, "DV static metadata exceeds its region");
 
@@ -90,7 +87,7 @@ cudaError_t setup(int device, uint8_t **ptr, bool redo = false) {
         return cudaSuccess;
     }
     size_t entries = fill_dv_vlc(g_vlc_host, kVlcMaxEntries);
-    if (entries == 0) return cudaErrorInvalidValue;
+    if (entries == 0 || !dv_vlc_one_index(g_vlc_host, entries)) return cudaErrorInvalidValue;
     e = cudaMemcpy((uint8_t *)p + kOffVlc, g_vlc_host, entries * 4, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return e;
     build_dv_fixed(g_fix_host, g_fix_host + kFixEntries);
@@ -195,7 +192,6 @@ mmr_status run_static(const uint8_t *data, size_t len, uint8_t *out, const Probe
     meta.state.bad_segment = 0xffffffffu;
     meta.item_ok = 1;
     meta.seg_first[1] = seqs * 27;
-    meta.dif_first[1] = seqs * 150;
     Meta *dm = reinterpret_cast<Meta *>(s + kOffMeta);
     DvLaunch L;
     memset(&L, 0, sizeof(L));
@@ -204,9 +200,6 @@ mmr_status run_static(const uint8_t *data, size_t len, uint8_t *out, const Probe
     L.n_frames = 1;
     L.seg_first = dm->seg_first;
     L.n_segments = seqs * 27;
-    L.dif_first = dm->dif_first;
-    L.n_dif = seqs * 150;
-    L.flags = s + kOffFlags;
     L.seg_err = s + kOffSegErr;
     L.coef = reinterpret_cast<int16_t *>(s + kOffCoef);
     L.modes = s + kOffModes;

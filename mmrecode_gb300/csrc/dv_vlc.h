@@ -58,4 +58,16 @@ inline size_t fill_dv_vlc(uint32_t *table, size_t capacity) {
     return size;
 }
 
+// Whether one index serves both levels of the table (segment_kernel's lookup): its
+// level-2 blocks are those of the windows from kDvVlcLong on, in order.
+inline bool dv_vlc_one_index(const uint32_t *table, size_t size) {
+    if (size != kDvVlcEntries) return false;
+    for (uint32_t i = 0; i < (1u << kDvVlcL1Bits); i++) {
+        const uint32_t first = kDvVlcLong >> (16 - kDvVlcL1Bits);
+        const uint32_t block = 0x80000000u | ((1u << kDvVlcL1Bits) + ((i - first) << (16 - kDvVlcL1Bits)));
+        if (i < first ? (table[i] & 0x80000000u) != 0 : table[i] != block) return false;
+    }
+    return true;
+}
+
 }  // namespace mmr

@@ -406,6 +406,7 @@ std::vector<uint32_t> build_dv_vlc() {
     std::vector<uint32_t> t(kDvVlcMaxEntries);
     const size_t n = fill_dv_vlc(t.data(), t.size());
     if (n == 0) throw std::runtime_error("DV VLC table exceeds its two-level layout");
+    if (!dv_vlc_one_index(t.data(), n)) throw std::runtime_error("DV VLC table has another layout");
     t.resize(n);
     return t;
 }
@@ -639,7 +640,7 @@ Probe probe_packet(uint32_t codec, const uint8_t *data, size_t len) {
 
 struct Engine::Impl {
     DevBuf d_in, d_tok, d_blob, d_tile_tok, d_tile_rst, d_rsts, d_results, d_coef, d_dc, d_planes, d_out, d_dvcoef,
-        d_modes, d_flags, d_segerr, d_vlc, d_fix, d_slot_item, d_ivs, d_sync, d_spec, d_prefix, d_events, d_ivkey,
+        d_modes, d_segerr, d_vlc, d_fix, d_slot_item, d_ivs, d_sync, d_spec, d_prefix, d_events, d_ivkey,
         d_ivpend,
         d_fixtab;  // fixed-point transform weights: MJPEG, DV 8-8, DV 2-4-8 (exact_fixed.h)
     PinBuf h_blob, h_back;
@@ -1032,7 +1033,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         // ------------------------------------------------------- DV layout
         std::vector<DvFrame> dframes;
         std::vector<DvState> dstates;
-        std::vector<uint32_t> seg_first(1, 0), dif_first(1, 0);
+        std::vector<uint32_t> seg_first(1, 0);
         uint64_t dv_blocks = 0;
         for (size_t k = 0; k < dplans.size(); k++) {
             DvPlan &p = dplans[k];
@@ -1063,9 +1064,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             F.item = (uint32_t)i;
             F.blk_off = dv_blocks;
             F.seg_first = seg_first.back();
-            F.dif_first = dif_first.back();
             seg_first.push_back(seg_first.back() + p.sequences * 27);
-            dif_first.push_back(dif_first.back() + p.sequences * 150);
             dv_blocks += (uint64_t)p.sequences * 27 * 30;
             bool direct = it.output == kOutPlanar;
             if (!direct) {
@@ -1110,7 +1109,6 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         I.d_out.ensure(std::max<size_t>(out_bytes, 256));
         I.d_dvcoef.ensure(std::max<size_t>(dv_blocks * 128, 256));
         I.d_modes.ensure(std::max<size_t>(dv_blocks, 256));
-        I.d_flags.ensure(std::max<size_t>(dif_first.back(), 256));
         I.d_segerr.ensure(std::max<size_t>(seg_first.back(), 256));
         // samples the fp32 IDCT leaves to the exact pass: expected ~0.1 per block; when the
         // queue fills, the kernel recomputes in place instead
@@ -1161,7 +1159,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         all_items.insert(all_items.end(), items_big.begin(), items_big.end());
         size_t o_items = blob.add_vec(all_items), o_ranges = blob.add_vec(ranges), o_idctcta = blob.add_vec(idct_cta), o_itemok = blob.add_vec(item_ok),
                o_dframes = blob.add_vec(dframes), o_dstates = blob.add_vec(dstates), o_segfirst = blob.add_vec(seg_first),
-               o_diffirst = blob.add_vec(dif_first), o_rgbjobs = blob.add_vec(rgbjobs),
+               o_rgbjobs = blob.add_vec(rgbjobs),
                o_rgbcta = blob.add_vec(rgbcta);
         size_t o_fjobs[kFusedSlots], o_fcta[kFusedSlots];
         for (int v = 0; v < kFusedSlots; v++) {
@@ -1279,9 +1277,6 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         DL.n_frames = (uint32_t)dframes.size();
         DL.seg_first = reinterpret_cast<const uint32_t *>(db + o_segfirst);
         DL.n_segments = seg_first.back();
-        DL.dif_first = reinterpret_cast<const uint32_t *>(db + o_diffirst);
-        DL.n_dif = dif_first.back();
-        DL.flags = I.d_flags.as<uint8_t>();
         DL.seg_err = I.d_segerr.as<uint8_t>();
         DL.coef = I.d_dvcoef.as<int16_t>();
         DL.modes = I.d_modes.as<uint8_t>();
@@ -1293,7 +1288,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             launch_dv_decode(DL, s);
             MMR_CUDA(record_event(I.dv_mark, s, capturing));
             launch_dv_idct(DL, s);
-            launches_ += 4;
+            launches_ += 3;
         }
         MMR_CUDA(record_event(I.ev[5], s, capturing));
         RgbLaunch RL;
@@ -1349,7 +1344,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                                 (uintptr_t)items_small.size(), (uintptr_t)n_items, (uintptr_t)ranges.size(),
                                 (uintptr_t)idct_cta.back(), (uintptr_t)n_slots, (uintptr_t)most_paths,
                                 (uintptr_t)blocks, (uintptr_t)dframes.size(), (uintptr_t)seg_first.back(),
-                                (uintptr_t)dif_first.back(), (uintptr_t)dv_blocks, (uintptr_t)rgbjobs.size(),
+                                (uintptr_t)dv_blocks, (uintptr_t)rgbjobs.size(),
                                 (uintptr_t)rgbcta.back()})
                 key.push_back(v);
             for (int v = 0; v < kFusedSlots; v++) {
@@ -1358,7 +1353,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             }
             for (const DevBuf *b : {&I.d_in, &I.d_tok, &I.d_blob, &I.d_tile_tok, &I.d_tile_rst, &I.d_rsts,
                                     &I.d_results, &I.d_coef, &I.d_dc, &I.d_planes, &I.d_out, &I.d_dvcoef, &I.d_modes,
-                                    &I.d_flags, &I.d_segerr, &I.d_vlc, &I.d_fix, &I.d_slot_item, &I.d_ivs, &I.d_sync,
+                                    &I.d_segerr, &I.d_vlc, &I.d_fix, &I.d_slot_item, &I.d_ivs, &I.d_sync,
                                     &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_ivpend})
                 key.push_back((uintptr_t)b->ptr);
             for (size_t i = 0; i < n; i++) {

@@ -105,9 +105,6 @@ struct DvLaunch {
     uint32_t n_frames;
     const uint32_t *seg_first;   // n_frames + 1 prefix of segments
     uint32_t n_segments;
-    const uint32_t *dif_first;   // n_frames + 1 prefix of DIF blocks
-    uint32_t n_dif;
-    uint8_t *flags;              // per DIF block: 1 if its identifier is damaged
     uint8_t *seg_err;            // per segment: DiagKind (0 = ok)
     int16_t *coef;               // 64 per block, natural order
     uint8_t *modes;              // per block: 1 = 2-4-8
@@ -136,5 +133,9 @@ void launch_rgb(const RgbLaunch &L, cudaStream_t s);
 //   bit 31 set: level-2 block at bits 0..15 (entry index)
 //   otherwise: len (bits 0..4), run (bits 5..11), level + 256 (bits 12..20); len 0 = no code
 constexpr int kDvVlcL1Bits = 10;
+// The DV code's table: 32 level-1 entries, those of the 16-bit windows from kDvVlcLong
+// on, have level-2 blocks, in window order.
+constexpr uint32_t kDvVlcLong = 0xf800;
+constexpr size_t kDvVlcEntries = (1u << kDvVlcL1Bits) + (0x10000u - kDvVlcLong);
 
 }  // namespace mmr

@@ -236,7 +236,6 @@ struct DvFrame {
     uint32_t item;
     uint64_t blk_off;    // first block in the DV coefficient arena (sequences*27*30 blocks)
     uint32_t seg_first;  // first segment in the segment arrays
-    uint32_t dif_first;  // first DIF block in the issue-flag array
 };
 
 struct DvState {
