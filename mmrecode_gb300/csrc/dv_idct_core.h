@@ -3,12 +3,12 @@
 //
 // Both transforms are first evaluated in fp32 as separable sums (8 + 8 terms for
 // 8-8; butterfly, 8 + 4 terms for 2-4-8), each factor cu * cos the fp32 product
-// of the fp32 roundings (3u, u = 2^-24); the horizontal pass takes its even and odd
-// terms as two four-term FMA chains, added and subtracted for the outputs x and 7 - x
-// (the fp32 factors are exactly symmetric), the vertical pass is one FMA chain.
-// Against the exact real value of the reference's terms (its doubles: FRAC_1_SQRT_2,
-// the cos table, the integer c) the fp32 sum is off by at most (3u + 5u) + (3u + 8u) =
-// 19u B for 8-8 and 8u + 3u + 4u = 15u B for 2-4-8 (the bounds below take 22u); the
+// of the fp32 roundings (3u, u = 2^-24), every eight-term sum as two four-term FMA
+// chains (even and odd terms) added and subtracted for two outputs (the fp32 factors
+// are exactly symmetric). Against the exact real value of the reference's terms (its
+// doubles: FRAC_1_SQRT_2, the cos table, the integer c) the fp32 sum is off by at most
+// (3u + 5u) + (3u + 5u) = 16u B for 8-8 and (u + 3u + 4u) + (3u + 5u) = 16u B for 2-4-8
+// (the bounds below take 22u); the
 // binary64 sequence by < 70 * 2^-53 B. B = sum |terms| <= C1 = sum |c| for 8-8 (|cos| <= 1, cu cv <= 1) and
 // <= C1 / 2 per 2-4-8 field (a butterfly output is at most |c1| + |c2|); after the
 // final / 4.0 or / 2.0, |value32 - value64| <= 5.5u C1 < delta = 2^-21 C1 + 2^-30
@@ -115,103 +115,82 @@ __device__ __forceinline__ uint8_t dv_flat_sample(const int32_t *c, bool mode248
 }
 
 // ---------------------------------------------------------------------------
-// Row-parallel form: eight threads per block, thread r producing output row r.
-// The factors are fp32 products of the fp32 roundings, W[u][x] = (u ? 1 : FRAC)
-// * cos16f[(2x+1)u] (transposed: a thread reads the eight x of one u as two
-// 16-byte loads) and V4[yy][v] = (v ? 1 : FRAC) * cos16f[2(2yy+1)v]. Pass 1 is an
-// FMA chain over u per output, pass 2 one over v, the 2-4-8 butterfly and the
-// halvings exact: the evaluation the bound above describes.
+// Eight threads per block: thread r takes column r in the vertical pass (with the
+// 2-4-8 butterfly, exact), then row r in the horizontal pass. The factors are fp32
+// products of the fp32 roundings, W[u][x] = (u ? 1 : FRAC) * cos16f[(2x+1)u] and
+// V4[yy][v] = (v ? 1 : FRAC) * cos16f[2(2yy+1)v]. Where the outputs x and 7 - x share
+// an eight-term sum (W[u][7-x] = (-1)^u W[u][x]), one packed FMA per pair of terms
+// keeps the even and the odd sum side by side; a 2-4-8 column keeps its two fields
+// side by side. All in all 32 packed FMAs a thread in either mode.
 
-// Fills the tables (64 + 16 floats) cooperatively; callers synchronise before use.
-__device__ __forceinline__ void dv_fill_tables(float *wt, float *v4) {
-    for (int i = threadIdx.x; i < 80; i += blockDim.x) {
-        if (i < 64) {
-            const int u = i >> 3, x = i & 7;
+// Fills the tables (48 floats) cooperatively; callers synchronise before use. Row x < 4
+// of wt holds W[0..7][x], then row yy < 4 (of four) V4[yy][0..3]. (No second table any
+// more: the argument is for callers that have one.)
+constexpr int kDvTable = 48;
+constexpr int kDvV4 = 32;  // offset of V4 in it
+
+__device__ __forceinline__ void dv_fill_tables(float *wt, float * = nullptr) {
+    for (int i = threadIdx.x; i < kDvTable; i += blockDim.x) {
+        if (i < kDvV4) {
+            const int x = i >> 3, u = i & 7;
             wt[i] = (u == 0 ? (float)kFrac : 1.0f) * c_cos16f[(2 * x + 1) * u];
         } else {
-            const int yy = (i - 64) >> 2, v = (i - 64) & 3;
-            v4[i - 64] = (v == 0 ? (float)kFrac : 1.0f) * c_cos16f[2 * (2 * yy + 1) * v];
+            const int yy = (i - kDvV4) >> 2, v = (i - kDvV4) & 3;
+            wt[i] = (v == 0 ? (float)kFrac : 1.0f) * c_cos16f[2 * (2 * yy + 1) * v];
         }
     }
 }
 
-// Pass 1 for row r: h[r][0..7] into hrow (16-byte aligned). c: the block's 64
-// coefficients (natural order).
-__device__ __forceinline__ void dv_row_pass8(const int32_t *c, const float *wt, bool mode248, int r, float *hrow) {
-    float b[8];
-    if (mode248) {
-        const int pair = r >> 1;
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const float first = (float)c[pair * 16 + u], second = (float)c[pair * 16 + 8 + u];
-            b[u] = (r & 1) ? first - second : first + second;  // exact: |c| < 2^23
-        }
-    } else {
-#pragma unroll
-        for (int u = 0; u < 8; u++) b[u] = (float)c[r * 8 + u];
-    }
-    // outputs x and 7 - x share their even and odd sums, x pairs in packed FMAs
-    F2 e[2] = {}, o[2] = {};
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        const float4 w = reinterpret_cast<const float4 *>(wt + u * 8)[0];
-        F2(&t)[2] = u & 1 ? o : e;
-        t[0] = fma2(f2(w.x, w.y), f2(b[u], b[u]), t[0]);
-        t[1] = fma2(f2(w.z, w.w), f2(b[u], b[u]), t[1]);
-    }
-    const float half = mode248 ? 0.5f : 1.0f;  // (exact)
-    float h[8];
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        float ea, eb, oa, ob;
-        split2(e[i], ea, eb);
-        split2(o[i], oa, ob);
-        h[2 * i] = (ea + oa) * half;
-        h[2 * i + 1] = (eb + ob) * half;
-        h[7 - 2 * i] = (ea - oa) * half;
-        h[6 - 2 * i] = (eb - ob) * half;
-    }
-    reinterpret_cast<float4 *>(hrow)[0] = make_float4(h[0], h[1], h[2], h[3]);
-    reinterpret_cast<float4 *>(hrow)[1] = make_float4(h[4], h[5], h[6], h[7]);
-}
-
-__device__ __forceinline__ void dv_add_row(F2 (&s)[4], const float *h, float w) {
-    const float4 h0 = reinterpret_cast<const float4 *>(h)[0], h1 = reinterpret_cast<const float4 *>(h)[1];
-    s[0] = fma2(f2(w, w), f2(h0.x, h0.y), s[0]);
-    s[1] = fma2(f2(w, w), f2(h0.z, h0.w), s[1]);
-    s[2] = fma2(f2(w, w), f2(h1.x, h1.y), s[2]);
-    s[3] = fma2(f2(w, w), f2(h1.z, h1.w), s[3]);
-}
-
-// Pass 2 for output row y: value[0..7] from the block's 64 pass-1 outputs h
-// (row-major, 16-byte aligned rows).
-__device__ __forceinline__ void dv_column_pass8(const float *h, const float *wt, const float *v4, bool mode248, int y,
-                                                float *value) {
-    F2 s[4] = {};
-    if (mode248) {
-        const int field = y & 1, yy = y >> 1;
-#pragma unroll
-        for (int v = 0; v < 4; v++) dv_add_row(s, h + (v * 2 + field) * 8, v4[yy * 4 + v]);
-    } else {
-#pragma unroll
-        for (int v = 0; v < 8; v++) dv_add_row(s, h + v * 8, wt[v * 8 + y]);  // V[y][v] = W[v][y]
-    }
-    const float scale = mode248 ? 0.5f : 0.25f;
+// The eight-point sums out[i] = sum_u W[u][i] b[u], b as the pairs (b[0], b[1]), ...
+__device__ __forceinline__ void dv_eight_point(const F2 (&b)[4], const float *wt, float (&out)[8]) {
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        float a, b;
-        split2(s[i], a, b);
-        value[2 * i] = a * scale;
-        value[2 * i + 1] = b * scale;
+        const float4 w0 = reinterpret_cast<const float4 *>(wt + i * 8)[0];
+        const float4 w1 = reinterpret_cast<const float4 *>(wt + i * 8)[1];
+        F2 s;  // (even, odd) terms
+        s = fma2(f2(w0.x, w0.y), b[0], s);
+        s = fma2(f2(w0.z, w0.w), b[1], s);
+        s = fma2(f2(w1.x, w1.y), b[2], s);
+        s = fma2(f2(w1.z, w1.w), b[3], s);
+        float e, o;
+        split2(s, e, o);
+        out[i] = e + o;
+        out[7 - i] = e - o;
     }
 }
 
-// The samples of row y that the fp32 evaluation decides, packed little-endian
-// (x = 0 in the low byte) into *row; returns the undecided ones as bits (x).
-// For a flat block (no nonzero AC coefficient) lane `flat_src` of the warp
-// computes the one reference-order value and broadcasts it (all eight lanes of
-// the block's group call this together).
-__device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h, const float *wt, const float *v4,
+// First pass, thread r: the vertical sums of column r, outputs y = 0..7 into hcol
+// (16-byte aligned). c: the block's 64 coefficients (natural order).
+__device__ __forceinline__ void dv_row_pass8(const int32_t *c, const float *wt, bool mode248, int r, float *hcol) {
+    float b[8], out[8];
+#pragma unroll
+    for (int v = 0; v < 8; v++) b[v] = (float)c[v * 8 + r];
+    if (mode248) {
+        F2 s[4];  // (field 0, field 1) of row yy
+#pragma unroll
+        for (int yy = 0; yy < 4; yy++) {
+            const float4 w = reinterpret_cast<const float4 *>(wt + kDvV4 + yy * 4)[0];
+            // the butterfly of each row pair is exact: |c| < 2^23
+            s[yy] = fma2(f2(w.x, w.x), f2(b[0] + b[1], b[0] - b[1]), s[yy]);
+            s[yy] = fma2(f2(w.y, w.y), f2(b[2] + b[3], b[2] - b[3]), s[yy]);
+            s[yy] = fma2(f2(w.z, w.z), f2(b[4] + b[5], b[4] - b[5]), s[yy]);
+            s[yy] = fma2(f2(w.w, w.w), f2(b[6] + b[7], b[6] - b[7]), s[yy]);
+            split2(s[yy], out[2 * yy], out[2 * yy + 1]);
+        }
+    } else {
+        const F2 p[4] = {f2(b[0], b[1]), f2(b[2], b[3]), f2(b[4], b[5]), f2(b[6], b[7])};
+        dv_eight_point(p, wt, out);
+    }
+    reinterpret_cast<float4 *>(hcol)[0] = make_float4(out[0], out[1], out[2], out[3]);
+    reinterpret_cast<float4 *>(hcol)[1] = make_float4(out[4], out[5], out[6], out[7]);
+}
+
+// Second pass, thread y: the samples of row y that the fp32 evaluation decides, packed
+// little-endian (x = 0 in the low byte) into *row; returns the undecided ones as bits
+// (x). h: the first pass's outputs, column u's at h + 8 * u. For a flat block (no nonzero
+// AC coefficient) lane `flat_src` of the warp computes the one reference-order value and
+// broadcasts it (all eight lanes of the block's group call this together).
+__device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h, const float *wt, const float *,
                                                 bool mode248, int y, float c1, bool flat, int flat_src,
                                                 unsigned group_mask, unsigned long long *row) {
     if (flat) {
@@ -221,8 +200,11 @@ __device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h
         *row = 0x0101010101010101ull * v;
         return 0;
     }
+    const F2 p[4] = {f2(h[y], h[8 + y]), f2(h[16 + y], h[24 + y]), f2(h[32 + y], h[40 + y]), f2(h[48 + y], h[56 + y])};
     float value[8];
-    dv_column_pass8(h, wt, v4, mode248, y, value);
+    dv_eight_point(p, wt, value);
+#pragma unroll
+    for (int x = 0; x < 8; x++) value[x] *= 0.25f;  // (exact; 8-8's / 4.0, 2-4-8's two / 2.0)
     // A value is certain when no half-integer lies within delta = 2^-21 C1 + 2^-30 of
     // it. (round_nearest holds below 2^22; |value| <= C1 / 4 + delta beyond that makes
     // delta more than a half.) Values past 256 + delta or below -1 - delta are clamped

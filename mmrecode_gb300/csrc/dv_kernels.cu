@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "dv_idct_core.h"
+#include "dv_layout.h"
 #include "kernels.h"
 #include "rounding.h"
 #include "tables.h"
@@ -392,36 +393,6 @@ __global__ void dv_resolve_kernel(DvLaunch L) {
     }
 }
 
-// decoder.rs:395-422 macroblock_coordinates (in 8-sample units); the per-macroblock
-// offsets in constant memory (indexed per lane, as local arrays they went to the stack)
-__constant__ uint32_t c_mb_off[5] = {2, 6, 8, 0, 4};
-__constant__ uint32_t c_mb_shuf3[5] = {18, 9, 27, 0, 36};
-__constant__ uint32_t c_mb_lstart[5] = {9, 4, 13, 0, 18};
-
-__device__ __forceinline__ void mb_coords(bool pal, uint32_t seqs, uint32_t sequence, uint32_t slot, uint32_t m,
-                                          uint32_t *mbx, uint32_t *mby) {
-    if (pal) {
-        // SERPENT1[slot] = 0,1,2,2,1,0 repeating
-        uint32_t s6 = slot % 6;
-        uint32_t serp1 = s6 < 3 ? s6 : 5 - s6;
-        uint32_t x = c_mb_shuf3[m] + slot / 3;
-        uint32_t y = serp1 + ((sequence + c_mb_off[m]) % seqs) * 3;
-        *mbx = x * 2;
-        *mby = y * 2;
-    } else {
-        uint32_t row = (sequence + c_mb_off[m]) % seqs;
-        uint32_t k = slot + ((m == 1 || m == 2) ? 3 : 0);
-        uint32_t x = c_mb_lstart[m] + k / 6;
-        // SERPENT2[k] = 0..5,5..0 repeating
-        uint32_t k12 = k % 12;
-        uint32_t serp2 = k12 < 6 ? k12 : 11 - k12;
-        uint32_t y = serp2 + row * 6;
-        if (x > 21) y = y * 2 - row * 6;
-        *mbx = x * 4;
-        *mby = y;
-    }
-}
-
 constexpr int kIdctBlocks = 16;                  // blocks per CTA
 constexpr int kIdctThreads = kIdctBlocks * 8;    // eight threads (rows) per block
 
@@ -448,25 +419,27 @@ __device__ __forceinline__ void store_row4(uint8_t *dst, uint32_t row) {
     }
 }
 
-// Eight threads per block, thread r producing row r: the fp32 row and column
-// passes with the exact fallback (dv_idct_core.h), then placement
-// (decoder.rs:432-505) with 8-byte row stores. A warp holds four blocks of one
-// frame (frames start at multiples of 4 blocks: 8100 and 9720 blocks per frame),
-// so one search per warp finds it; the eight threads of a block synchronise
-// through their warp only.
+// Eight threads per block: the fp32 passes with the exact fallback (dv_idct_core.h),
+// then placement (decoder.rs:432-505) with 8-byte row stores. A warp holds four blocks
+// of one frame (frames start at multiples of 4 blocks: 8100 and 9720 blocks per frame),
+// found by one division where all frames are of one system; the eight threads of a
+// block synchronise through their warp only.
+constexpr int kBlockStride = 72;  // ints or floats per block: four blocks' column accesses on distinct banks
+
 __global__ void __launch_bounds__(kIdctThreads) dv_idct_kernel(DvLaunch L) {
-    __shared__ __align__(16) int32_t s_c[kIdctBlocks][64];
-    __shared__ __align__(16) float s_h[kIdctBlocks][64];
-    __shared__ __align__(16) float s_wt[64];
-    __shared__ __align__(16) float s_v4[16];
-    dv_fill_tables(s_wt, s_v4);
+    __shared__ __align__(16) int32_t s_c[kIdctBlocks][kBlockStride];
+    __shared__ __align__(16) float s_h[kIdctBlocks][kBlockStride];
+    __shared__ __align__(16) float s_wt[kDvTable];
+    dv_fill_tables(s_wt);
     __syncthreads();
     const int lane = threadIdx.x & 31, lb = threadIdx.x >> 3, r = threadIdx.x & 7;
     const unsigned group_mask = 0xffu << (lane & 24);
-    const uint64_t gb = (uint64_t)blockIdx.x * kIdctBlocks + lb;
+    const uint32_t gb = blockIdx.x * kIdctBlocks + lb;
     bool valid = gb < L.n_blocks;
-    uint32_t f = 0;
-    if (lane == 0 && valid) {
+    uint32_t f;
+    if (L.frame_blocks) {
+        f = min(gb / L.frame_blocks, L.n_frames - 1);
+    } else {
         uint32_t lo = 0, hi = L.n_frames;
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -475,48 +448,37 @@ __global__ void __launch_bounds__(kIdctThreads) dv_idct_kernel(DvLaunch L) {
         }
         f = lo;
     }
-    f = __shfl_sync(0xffffffffu, f, 0);
     const DvFrame *F = &L.frames[f];
     bool failed = false, mode = false;
     uint32_t local_blk = 0;
     int4 lv = make_int4(0, 0, 0, 0);
     if (valid) {
-        local_blk = (uint32_t)(gb - F->blk_off);
+        local_blk = gb - (uint32_t)F->blk_off;
         valid = L.item_ok[F->item] != 0;
         if (valid) {
             failed = L.seg_err[F->seg_first + local_blk / 30] != 0;
             mode = L.modes[gb] != 0;
-            if (!failed) lv = reinterpret_cast<const int4 *>(L.coef + gb * 64)[r];  // row r: 8 int16
+            if (!failed) lv = reinterpret_cast<const int4 *>(L.coef + (uint64_t)gb * 64)[r];  // row r: 8 int16
         }
     }
     int32_t *c = s_c[lb];
+    // C1 of the block (at most 2^21, exact as a float too) and whether any AC
+    // coefficient is nonzero, over its eight threads
+    int32_t c1 = 0;
     {
-        const int16_t *q = reinterpret_cast<const int16_t *>(&lv);
+        const uint32_t w[4] = {(uint32_t)lv.x, (uint32_t)lv.y, (uint32_t)lv.z, (uint32_t)lv.w};
         int32_t row[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) row[u] = q[u];
+        for (int u = 0; u < 8; u++) {
+            row[u] = u & 1 ? (int32_t)w[u >> 1] >> 16 : (int32_t)(int16_t)w[u >> 1];
+            c1 += abs(row[u]);
+        }
         reinterpret_cast<int4 *>(c + r * 8)[0] = make_int4(row[0], row[1], row[2], row[3]);
         reinterpret_cast<int4 *>(c + r * 8)[1] = make_int4(row[4], row[5], row[6], row[7]);
     }
-    // C1 of the block (fp32 for the first decision, exact for the second) and
-    // whether any AC coefficient is nonzero, over its eight threads
-    float a = 0.0f;
-    int32_t ai = 0;
-    bool ac = false;
-    {
-        const int16_t *q = reinterpret_cast<const int16_t *>(&lv);
+    const bool ac = ((r ? lv.x : lv.x & (int)0xffff0000) | lv.y | lv.z | lv.w) != 0;
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            a += fabsf((float)q[u]);
-            ai += abs((int32_t)q[u]);
-            ac |= (r | u) != 0 && q[u] != 0;
-        }
-    }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        ai += __shfl_xor_sync(0xffffffffu, ai, o);
-    }
+    for (int o = 1; o < 8; o <<= 1) c1 += __shfl_xor_sync(0xffffffffu, c1, o);
     const bool flat = (__ballot_sync(0xffffffffu, ac) & group_mask) == 0;
     const bool active = valid && !failed;
     __syncwarp();
@@ -524,34 +486,20 @@ __global__ void __launch_bounds__(kIdctThreads) dv_idct_kernel(DvLaunch L) {
     __syncwarp();
     unsigned long long row = 0;
     uint32_t und = 0;
-    if (active) und = dv_row_fp32(c, s_h[lb], s_wt, s_v4, mode, r, a, flat, lane & 24, group_mask, &row);
-    dv_resolve_row(und, row, c, mode, r, ai, L.fixw);  // every lane of the warp takes part
+    if (active)
+        und = dv_row_fp32(c, s_h[lb], s_wt, nullptr, mode, r, (float)c1, flat, lane & 24, group_mask, &row);
+    dv_resolve_row(und, row, c, mode, r, c1, L.fixw);  // every lane of the warp takes part
     if (!valid) return;
-    // placement (decoder.rs:432-505)
-    const uint32_t seg = local_blk / 30, j = local_blk % 30;
-    const uint32_t sequence = seg / 27, slot = seg % 27, m = j / 6, bi = j % 6;
-    uint32_t mbx, mby;
-    mb_coords(F->pal != 0, F->sequences, sequence, slot, m, &mbx, &mby);
-    const uint32_t X = mbx * 8, Y = mby * 8;
-    const uint32_t W = F->width, H = F->height, cw = F->cw, ch = F->ch;
-    uint8_t *yp = F->planes, *cbp = F->planes + (size_t)W * H, *crp = cbp + (size_t)cw * ch;
-    const bool chroma = bi >= 4;
+    const uint32_t e = __ldg(L.place + (F->pal ? kDvBlocks525 : 0) + local_blk);
+    const bool chroma = (e & kDvPlaceChroma) != 0;
     if (failed) row = 0x0101010101010101ull * (chroma ? 128u : 16u);
-    if (F->pal || mbx >= 88) {
-        if (!chroma) {
-            store_row8(yp + (size_t)(Y + (bi >> 1) * 8 + r) * W + X + (bi & 1) * 8, row);
-        } else {
-            uint8_t *plane = bi == 4 ? crp : cbp;
-            if (F->pal) {
-                store_row8(plane + (size_t)(Y / 2 + r) * cw + X / 2, row);
-            } else {  // put_split_chroma: columns 0-3 to rows y.., 4-7 to rows y+8..
-                store_row4(plane + (size_t)(Y + r) * cw + X / 4, (uint32_t)row);
-                store_row4(plane + (size_t)(Y + 8 + r) * cw + X / 4, (uint32_t)(row >> 32));
-            }
-        }
+    const uint32_t stride = chroma ? F->cw : F->width;
+    uint8_t *dst = F->planes + (e & kDvPlaceOffset) + r * stride;
+    if (e & kDvPlaceSplit) {
+        store_row4(dst, (uint32_t)row);
+        store_row4(dst + 8 * stride, (uint32_t)(row >> 32));
     } else {
-        if (!chroma) store_row8(yp + (size_t)(Y + r) * W + X + bi * 8, row);
-        else store_row8((bi == 4 ? crp : cbp) + (size_t)(Y + r) * cw + X / 4, row);
+        store_row8(dst, row);
     }
 }
 
@@ -565,8 +513,7 @@ void launch_dv_decode(const DvLaunch &L, cudaStream_t s) {
 
 void launch_dv_idct(const DvLaunch &L, cudaStream_t s) {
     if (L.n_blocks == 0) return;
-    const uint64_t grid = (L.n_blocks + kIdctBlocks - 1) / kIdctBlocks;
-    dv_idct_kernel<<<(unsigned)grid, kIdctThreads, 0, s>>>(L);
+    dv_idct_kernel<<<(unsigned)((L.n_blocks + kIdctBlocks - 1) / kIdctBlocks), kIdctThreads, 0, s>>>(L);
 }
 
 }  // namespace mmr

@@ -23,6 +23,7 @@
 #include <string>
 
 #include "../../include/mmrecode_gpu.h"
+#include "dv_layout.h"
 #include "dv_vlc.h"
 #include "exact_fixed.h"
 #include "engine.h"
@@ -38,7 +39,7 @@ constexpr size_t kDvStaticScratchBytes = 2304u * 1024u;  // 2.25 MiB
 constexpr size_t kDvMaxInput = 144000;                   // one 625/50 frame
 constexpr size_t kDvMaxPlanar = 720 * 576 + 2 * 360 * 288;
 constexpr uint32_t kDvMaxSegments = 12 * 27;
-constexpr size_t kVlcMaxEntries = kDvVlcMaxEntries;
+constexpr size_t kVlcMaxEntries = kDvVlcEntries;
 
 static __device__ __align__(256) uint8_t g_dv_scratch[kDvStaticScratchBytes];
 
@@ -51,7 +52,8 @@ constexpr size_t kOffModes = kOffSegErr + a256(kDvMaxSegments);
 constexpr size_t kOffCoef = kOffModes + a256(kDvMaxSegments * 30);
 constexpr size_t kOffVlc = kOffCoef + a256((size_t)kDvMaxSegments * 30 * 128);
 constexpr size_t kOffFix = kOffVlc + a256(kVlcMaxEntries * 4);  // DV fixed-point weights (exact_fixed.h)
-constexpr size_t kOffMeta = kOffFix + a256(2 * kFixEntries * sizeof(long long));
+constexpr size_t kOffPlace = kOffFix + a256(2 * kFixEntries * sizeof(long long));  // block placement (dv_layout.h)
+constexpr size_t kOffMeta = kOffPlace + a256(kDvPlaceEntries * 4);
 constexpr size_t kMetaBytes = 1024;
 static_assert(kOffMeta + kMetaBytes <= kDvStaticScratchBytes, "DV static scratch layout exceeds the array");
 
@@ -68,6 +70,7 @@ static_assert(sizeof(Meta) <= kMetaBytes, "DV static metadata exceeds its region
 // the scratch at set-up.
 uint32_t g_vlc_host[kVlcMaxEntries];
 long long g_fix_host[2 * kFixEntries];
+uint32_t g_place_host[kDvPlaceEntries];
 
 std::mutex g_setup_mutex;
 uint8_t *g_scratch_ptr[64] = {};  // device address of g_dv_scratch, per device
@@ -92,6 +95,9 @@ cudaError_t setup(int device, uint8_t **ptr, bool redo = false) {
     if (e != cudaSuccess) return e;
     build_dv_fixed(g_fix_host, g_fix_host + kFixEntries);
     e = cudaMemcpy((uint8_t *)p + kOffFix, g_fix_host, sizeof(g_fix_host), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    fill_dv_place(g_place_host);
+    e = cudaMemcpy((uint8_t *)p + kOffPlace, g_place_host, sizeof(g_place_host), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return e;
     g_scratch_ptr[device] = (uint8_t *)p;
     *ptr = (uint8_t *)p;
@@ -205,7 +211,9 @@ mmr_status run_static(const uint8_t *data, size_t len, uint8_t *out, const Probe
     L.modes = s + kOffModes;
     L.vlc = reinterpret_cast<const uint32_t *>(s + kOffVlc);
     L.fixw = reinterpret_cast<const long long *>(s + kOffFix);
+    L.place = reinterpret_cast<const uint32_t *>(s + kOffPlace);
     L.n_blocks = (uint64_t)seqs * 27 * 30;
+    L.frame_blocks = seqs * 27 * 30;
     L.item_ok = &dm->item_ok;
     // the calling thread's default stream: no creation, no allocation, and no
     // implicit synchronisation with the application's other (blocking) streams

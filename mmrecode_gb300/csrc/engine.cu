@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "dv_layout.h"
 #include "dv_vlc.h"
 #include "exact_fixed.h"
 #include "huffman_lut.h"
@@ -642,6 +643,7 @@ struct Engine::Impl {
     DevBuf d_in, d_tok, d_blob, d_tile_tok, d_tile_rst, d_rsts, d_results, d_coef, d_dc, d_planes, d_out, d_dvcoef,
         d_modes, d_segerr, d_vlc, d_fix, d_slot_item, d_ivs, d_sync, d_spec, d_prefix, d_events, d_ivkey,
         d_ivpend,
+        d_place,   // DV block placement (dv_layout.h)
         d_fixtab;  // fixed-point transform weights: MJPEG, DV 8-8, DV 2-4-8 (exact_fixed.h)
     PinBuf h_blob, h_back;
     std::vector<uint32_t> vlc;
@@ -679,6 +681,12 @@ Engine::Engine(int device, int levels) : device_(device), slice_bits_(0), impl_(
     impl_->vlc = build_dv_vlc();
     impl_->d_vlc.ensure(impl_->vlc.size() * 4);
     MMR_CUDA(cudaMemcpy(impl_->d_vlc.ptr, impl_->vlc.data(), impl_->vlc.size() * 4, cudaMemcpyHostToDevice));
+    {
+        std::vector<uint32_t> place(kDvPlaceEntries);
+        fill_dv_place(place.data());
+        impl_->d_place.ensure(place.size() * 4);
+        MMR_CUDA(cudaMemcpy(impl_->d_place.ptr, place.data(), place.size() * 4, cudaMemcpyHostToDevice));
+    }
     {
         std::vector<long long> fix(3 * (size_t)kFixEntries);
         build_jpeg_fixed(fix.data());
@@ -1093,6 +1101,10 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             dstates.push_back(S);
         }
 
+        if (dv_blocks > 0xffffffffull) throw std::runtime_error("DV batch too large");
+        bool dv_uniform = !dframes.empty();
+        for (const DvFrame &F : dframes) dv_uniform &= F.sequences == dframes[0].sequences;
+
         // ------------------------------------------------- device arenas
         I.d_in.ensure(std::max<size_t>(in_bytes, 256));
         // +512: the entropy decoders' 32-bit word readers may read a few bytes, and the lean
@@ -1282,7 +1294,9 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         DL.modes = I.d_modes.as<uint8_t>();
         DL.vlc = I.d_vlc.as<uint32_t>();
         DL.fixw = I.d_fixtab.as<long long>() + kFixEntries;
+        DL.place = I.d_place.as<uint32_t>();
         DL.n_blocks = dv_blocks;
+        DL.frame_blocks = dv_uniform ? dframes[0].sequences * 27 * 30 : 0;
         DL.item_ok = JL.item_ok;
         if (!dframes.empty()) {
             launch_dv_decode(DL, s);

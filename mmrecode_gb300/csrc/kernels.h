@@ -110,7 +110,9 @@ struct DvLaunch {
     uint8_t *modes;              // per block: 1 = 2-4-8
     const uint32_t *vlc;         // two-level VLC table
     const long long *fixw;       // fixed-point transform weights: 8-8 then 2-4-8 (exact_fixed.h)
-    uint64_t n_blocks;
+    const uint32_t *place;       // where blocks land (dv_layout.h)
+    uint64_t n_blocks;           // less than 2^32
+    uint32_t frame_blocks;       // of every frame, 0 when they differ
     uint32_t *item_ok;
 };
 
