@@ -231,6 +231,8 @@ __device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h
     return und;
 }
 
+constexpr int kDvManyTies = 12;
+
 // Settles the undecided samples of every lane of the warp (all 32 lanes call
 // this; und = 0 for lanes with none, whose bytes of row are 0). One sample at a time
 // the whole warp forms its exact fixed-point value (exact_fixed.h); those too close to
@@ -243,6 +245,15 @@ __device__ __forceinline__ void dv_resolve_row(uint32_t und, unsigned long long 
                                                bool mode248, int y, int32_t c1i, const long long *fix) {
     const int lane = threadIdx.x & 31;
     uint32_t m, left = 0;
+    if (__ballot_sync(0xffffffffu, und != 0) == 0) return;
+    // a block with many undecided samples ties in them: straight to the reference order
+    int open = __popc(und);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) open += __shfl_xor_sync(0xffffffffu, open, o);
+    if (open >= kDvManyTies) {
+        left = und;
+        und = 0;
+    }
     while ((m = __ballot_sync(0xffffffffu, und != 0)) != 0) {
         const int src = __ffs(m) - 1;
         const uint32_t sund = __shfl_sync(0xffffffffu, und, src);

@@ -61,9 +61,14 @@ struct JpegEncodePlan {
     uint8_t qt[2][64];                  // natural order
     HuffCode dc[2][256], ac[2][256];
     std::vector<uint8_t> header;        // SOI .. SOS
+    size_t size_at = 0;                 // where the header holds the frame's height and width (two bytes each)
 };
 
-bool plan_jpeg_encode(const FrameIn &frame, const JpegEncodeOptions &opt, JpegEncodePlan *plan);
+// The part of the plan that depends on the frame alone (validation, geometry) and the
+// rest, which frames of one format and one set of options share but for their size.
+bool plan_jpeg_frame(const FrameIn &frame, const JpegEncodeOptions &opt, JpegEncodePlan *plan);
+bool plan_jpeg_tables(const FrameIn &frame, const JpegEncodeOptions &opt, JpegEncodePlan *plan);
+bool plan_jpeg_encode(const FrameIn &frame, const JpegEncodeOptions &opt, JpegEncodePlan *plan);  // both
 
 enum DvModePolicy : uint32_t {
     kDvMode88 = 0,        // reference behaviour: every block in 8-8 mode

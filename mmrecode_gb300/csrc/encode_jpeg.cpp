@@ -176,7 +176,7 @@ struct Comp {
 
 }  // namespace
 
-bool plan_jpeg_encode(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncodePlan *plan) {
+bool plan_jpeg_frame(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncodePlan *plan) {
     JpegEncodePlan &P = *plan;
     auto fail = [&](int32_t st, const char *m) {
         P.status = st;
@@ -231,6 +231,13 @@ bool plan_jpeg_encode(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncode
     P.mcu_cols = (f.width + (size_t)hmax * 8 - 1) / ((size_t)hmax * 8);
     P.mcu_rows = (f.height + (size_t)vmax * 8 - 1) / ((size_t)vmax * 8);
     P.restart_interval = opt.restart_interval;
+    return true;
+}
+
+bool plan_jpeg_tables(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncodePlan *plan) {
+    JpegEncodePlan &P = *plan;
+    static const uint8_t kIds[3] = {1, 2, 3};
+    const size_t nc = P.ncomp;
     scale_quant(kLumaQ, opt.quality, P.qt[0]);
     scale_quant(kChromaQ, opt.quality, P.qt[1]);
     const bool multi = nc > 1;
@@ -249,8 +256,11 @@ bool plan_jpeg_encode(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncode
     for (int k = 0; k < 2; k++)
         for (int i = 0; i < 256; i++) P.dc[k][i] = P.ac[k][i] = {0, 0, false};
     for (auto &t : tables)
-        if (!huffman_encoder(t, t.cls ? P.ac[t.id] : P.dc[t.id]))
-            return fail(kInvalidData, "JPEG Huffman table is oversubscribed");
+        if (!huffman_encoder(t, t.cls ? P.ac[t.id] : P.dc[t.id])) {
+            P.status = kInvalidData;
+            P.message = "JPEG Huffman table is oversubscribed";
+            return false;
+        }
 
     std::vector<uint8_t> &out = P.header;
     out = {0xff, 0xd8};
@@ -269,10 +279,11 @@ bool plan_jpeg_encode(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncode
         std::vector<uint8_t> p = {8, (uint8_t)(f.height >> 8), (uint8_t)f.height, (uint8_t)(f.width >> 8),
                                   (uint8_t)f.width, (uint8_t)nc};
         for (size_t i = 0; i < nc; i++) {
-            p.push_back(comps[i].id);
-            p.push_back((uint8_t)((comps[i].h << 4) | comps[i].v));
-            p.push_back(comps[i].tq);
+            p.push_back(kIds[i]);
+            p.push_back((uint8_t)((P.comp_h[i] << 4) | P.comp_v[i]));
+            p.push_back(P.comp_tq[i]);
         }
+        P.size_at = out.size() + 5;  // marker, length, precision
         segment(out, 0xc0, p);
     }
     {  // DHT (encoder.rs:312-325)
@@ -288,7 +299,7 @@ bool plan_jpeg_encode(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncode
     {  // SOS (encoder.rs:327-335)
         std::vector<uint8_t> p = {(uint8_t)nc};
         for (size_t i = 0; i < nc; i++) {
-            p.push_back(comps[i].id);
+            p.push_back(kIds[i]);
             p.push_back((uint8_t)((P.comp_table[i] << 4) | P.comp_table[i]));
         }
         p.push_back(0);
@@ -297,6 +308,10 @@ bool plan_jpeg_encode(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncode
         segment(out, 0xda, p);
     }
     return true;
+}
+
+bool plan_jpeg_encode(const FrameIn &f, const JpegEncodeOptions &opt, JpegEncodePlan *plan) {
+    return plan_jpeg_frame(f, opt, plan) && plan_jpeg_tables(f, opt, plan);
 }
 
 EncodeResult encode_jpeg(const FrameIn &f, const JpegEncodeOptions &opt) {

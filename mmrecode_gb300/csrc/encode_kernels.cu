@@ -9,16 +9,18 @@
 //                      reference's operation order
 //   bits_kernel        thread per block: Huffman bit count (DC difference against the
 //                      previous block of the component in its restart interval)
-//   scan (3 kernels)   exclusive prefix of the bit counts, of the segment words and
-//                      chunks, of the 0xFF counts and of the frame sizes
-//   segment_kernel     thread per restart interval ("segment"): its bits, bytes,
-//                      words and 16-byte chunks
+//   scans              exclusive prefix of the bit counts, of the segment chunks and of
+//                      the 0xFF counts (two launches each)
+//   segment_kernel     thread per restart interval ("segment"): its bits and 16-byte
+//                      chunks
 //   write_bits_kernel  thread per block: its codes into the segment's bit buffer
 //                      (interior words stored, the two shared edge words OR-ed)
 //   ff_count_kernel    thread per 16-byte chunk: 0xFF bytes (each gets a stuffed 0x00)
-//   layout_kernel      thread per frame: where each segment lands after stuffing
+//   layout_kernel      CTA per frame: where each segment lands after stuffing, the
+//                      frame's size, its header; the last CTA places the frames that are
+//                      staged for host buffers
 //   emit_kernel        thread per chunk: stuffed bytes, then RSTn or EOI after the
-//                      segment's last chunk
+//                      segment's last chunk, straight into device buffers
 // The header bytes (SOI .. SOS) are the host plan's (plan_jpeg_encode).
 #include <cuda_runtime.h>
 
@@ -46,6 +48,9 @@ struct EncFrame {
     uint32_t mcu_cols, mcus, bpm, ri;  // MCUs per row, MCUs, blocks per MCU, restart interval (0: none)
     uint64_t block_base;               // first block of the frame (scan order, batch-wide)
     uint32_t seg_base, nseg;           // first segment, segments (restart intervals)
+    uint8_t *out;                      // device buffer of `cap` bytes, nullptr: staged for a host one
+    uint64_t cap;
+    uint32_t hdr_off, hdr_len;         // header bytes
     uint8_t sched_comp[10], sched_bx[10], sched_by[10];
     uint8_t comp_first[3], comp_count[3], comp_h[3], comp_v[3], comp_tq[3], comp_tab[3];
 };
@@ -60,20 +65,20 @@ struct EncLaunch {
     const float *rq;          // [2][64] fp32 reciprocals of qt
     const uint8_t *nat2zz;    // [64] zigzag position of each natural index
     int16_t *coef;            // 64 per block, zigzag order
+    const uint8_t *headers;
     uint32_t *block_bits;     // per block
     uint64_t *bit_off;        // n_blocks + 1
-    uint32_t *seg_words;      // per segment, 4 per chunk (scanned into seg_word_off)
     uint32_t *seg_chunks;     // per segment (scanned into seg_chunk_off)
     uint64_t *seg_bits;       // per segment
-    uint64_t *seg_word_off;   // n_segs + 1
     uint64_t *seg_chunk_off;  // n_segs + 1
-    uint32_t *raw;            // segment bit buffers, big-endian words
+    uint32_t *raw;            // segment bit buffers, big-endian words, four per chunk
     uint32_t *chunk_ff;       // per chunk
     uint64_t *ff_off;         // n_chunks + 1
     uint32_t *seg_out;        // per segment: its offset in the frame's entropy bytes
     uint32_t *frame_len;      // per frame: entropy bytes, markers and EOI
-    uint64_t *frame_off;      // n_frames + 1
-    uint8_t *out;             // entropy bytes of all frames
+    uint64_t *frame_off;      // per frame staged for a host buffer: its entropy bytes in `out`
+    uint8_t *out;
+    uint32_t *done;           // CTAs of layout_kernel that are through (zeroed)
     unsigned long long *exact;  // coefficients recomputed in binary64
 };
 
@@ -98,8 +103,8 @@ __device__ __forceinline__ uint32_t frame_of_segment(const EncLaunch &L, uint32_
     return lo;
 }
 
-__device__ __forceinline__ uint32_t segment_of_chunk(const EncLaunch &L, uint64_t c) {
-    uint32_t lo = 0, hi = L.n_segs - 1;
+// lo, hi: segments it lies between
+__device__ __forceinline__ uint32_t segment_of_chunk(const EncLaunch &L, uint64_t c, uint32_t lo, uint32_t hi) {
     while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;
         if (L.seg_chunk_off[mid] <= c) lo = mid;
@@ -143,8 +148,16 @@ __device__ __forceinline__ BlockSource block_source(const EncFrame &F, uint64_t 
 // rows and columns past the plane repeat its last).
 __device__ __forceinline__ uint2 source_row(const BlockSource &B, uint32_t r) {
     const uint8_t *row = B.plane + (size_t)min(B.y0 + r, B.ph - 1) * B.stride;
-    if (B.x0 + 8 <= B.pw && (reinterpret_cast<uintptr_t>(row + B.x0) & 7) == 0)  // one 8-byte load
-        return *reinterpret_cast<const uint2 *>(row + B.x0);
+    if (B.x0 + 8 <= B.pw) {  // one aligned 8-byte load, or the two that hold the eight samples
+        const uintptr_t a = reinterpret_cast<uintptr_t>(row + B.x0);
+        const uint2 *q = reinterpret_cast<const uint2 *>(a & ~(uintptr_t)7);
+        const uint32_t sh = (uint32_t)(a & 7) * 8;
+        const uint2 v = q[0];
+        if (sh == 0) return v;
+        const uint2 n = q[1];
+        const unsigned long long x = ((unsigned long long)v.y << 32 | v.x) >> sh | ((unsigned long long)n.y << 32 | n.x) << (64 - sh);
+        return make_uint2((uint32_t)x, (uint32_t)(x >> 32));
+    }
     uint2 w = make_uint2(0, 0);
 #pragma unroll
     for (int x = 0; x < 4; x++) {
@@ -257,63 +270,114 @@ __global__ void __launch_bounds__(kEncThreads) fdct_kernel(EncLaunch L, uint64_t
 
 // ------------------------------------------------------------- Huffman ---
 
-__device__ __forceinline__ uint32_t category(int v) { return v ? 32u - __clz(v < 0 ? -v : v) : 0u; }
+__device__ __forceinline__ uint32_t category(int v) { return 32u - __clz(v < 0 ? -v : v); }
 
-// Walks the symbols of block blk (encode_block, encoder.rs:404-425) and hands each
-// code and amplitude to emit(value, bits).
+// A CTA's blocks and the code tables in shared memory: the blocks come in as whole
+// lines, and a thread then visits its block's nonzero coefficients only, at any index.
+// (A thread reading its own 128 bytes from global memory and testing all 64
+// coefficients took 0.28 ms to count and 0.57 ms to write 3.9 M blocks of 18 nonzeros.)
+constexpr int kSymThreads = 128;
+
+struct SymSmem {
+    __align__(16) uint4 blk[kSymThreads * 9];  // eight per block, the ninth spreads the banks
+    uint32_t codes[4 * 256];
+    uint32_t frame;
+};
+
+__device__ __forceinline__ void load_symbols(const EncLaunch &L, SymSmem &S) {
+    const uint64_t b0 = (uint64_t)blockIdx.x * kSymThreads;
+    if (threadIdx.x == 0) S.frame = frame_of_block(L, b0);
+    const uint4 *src = reinterpret_cast<const uint4 *>(L.coef + b0 * 64);
+    const uint64_t n = min((uint64_t)kSymThreads, L.n_blocks - b0) * 8;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        const uint32_t i = threadIdx.x + u * kSymThreads;
+        if (i < n) S.blk[(i >> 3) * 9 + (i & 7)] = src[i];
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+        reinterpret_cast<uint4 *>(S.codes)[threadIdx.x + u * kSymThreads] =
+            __ldg(reinterpret_cast<const uint4 *>(L.codes) + threadIdx.x + u * kSymThreads);
+    __syncthreads();
+}
+
+// Bits 2i and 2i + 1: whether the halves of word i of 16 are nonzero, given as the
+// low-half flags in bits 0..15 and the high-half flags in bits 16..31.
+__device__ __forceinline__ uint32_t interleave16(uint32_t x) {
+    uint32_t t = (x ^ (x >> 8)) & 0x0000ff00u;
+    x ^= t ^ (t << 8);
+    t = (x ^ (x >> 4)) & 0x00f000f0u;
+    x ^= t ^ (t << 4);
+    t = (x ^ (x >> 2)) & 0x0c0c0c0cu;
+    x ^= t ^ (t << 2);
+    t = (x ^ (x >> 1)) & 0x22222222u;
+    return x ^ t ^ (t << 1);
+}
+
+// Walks the symbols of block blk of frame F (encode_block, encoder.rs:404-425) and
+// hands each code, its amplitude appended, to emit(value, bits): at most 27 bits.
 template <class Emit>
-__device__ __forceinline__ void block_symbols(const EncLaunch &L, const EncFrame &F, uint64_t blk, Emit emit) {
-    const uint64_t i = blk - F.block_base;
-    const uint32_t mcu = (uint32_t)(i / F.bpm), k = (uint32_t)(i % F.bpm);
+__device__ __forceinline__ void block_symbols(const EncLaunch &L, const SymSmem &S, const EncFrame &F, uint64_t blk,
+                                              uint32_t mcu, uint32_t k, Emit emit) {
+    const uint4 *row = S.blk + threadIdx.x * 9;
+    const int16_t *coef = reinterpret_cast<const int16_t *>(row);
     const uint32_t c = F.sched_comp[k];
     // the DC prediction: the previous block of the component in this restart interval
     const bool interval_start = F.ri ? mcu % F.ri == 0 : mcu == 0;
     int pred = 0;
     if (k != F.comp_first[c]) pred = L.coef[(blk - 1) * 64];
     else if (!interval_start) pred = L.coef[(blk - F.bpm + F.comp_count[c] - 1) * 64];
-    // the block's coefficients in zigzag order, eight 16-byte loads
-    const uint4 *cz = reinterpret_cast<const uint4 *>(L.coef + blk * 64);
-    const uint32_t *dc = L.codes + F.comp_tab[c] * 256, *ac = L.codes + (2 + F.comp_tab[c]) * 256;
-    uint4 q = cz[0];
-    const int diff = (int)(int16_t)(q.x & 0xffffu) - pred;
-    const uint32_t dsz = category(diff);
-    const uint32_t dcode = __ldg(dc + dsz);
-    emit(dcode & 0xffffu, dcode >> 16);
-    if (dsz) emit((uint32_t)(diff < 0 ? diff + (1 << dsz) - 1 : diff) & ((1u << dsz) - 1), dsz);
-    uint32_t run = 0;
-#pragma unroll 1
-    for (int ch = 0; ch < 8; ch++) {
-        if (ch) q = cz[ch];
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    const uint32_t *dc = S.codes + F.comp_tab[c] * 256, *ac = S.codes + (2 + F.comp_tab[c]) * 256;
+    // nonzero coefficients, in zigzag order
+    uint32_t mask[2];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (ch == 0 && j == 0) continue;  // the DC
-            const int v = (int)(int16_t)(w[j >> 1] >> (16 * (j & 1)));
-            if (v == 0) {
-                run++;
-                continue;
-            }
-            const uint32_t zrl = __ldg(ac + 0xf0);
-            for (; run >= 16; run -= 16) emit(zrl & 0xffffu, zrl >> 16);
-            const uint32_t sz = category(v);
-            const uint32_t code = __ldg(ac + ((run << 4) | sz));
-            emit(code & 0xffffu, code >> 16);
-            emit((uint32_t)(v < 0 ? v + (1 << sz) - 1 : v) & ((1u << sz) - 1), sz);
-            run = 0;
+    for (int h = 0; h < 2; h++) {
+        uint32_t flags = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint4 v = row[4 * h + q];
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                flags = flags >> 1 | ((((w[j] & 0x7fff7fffu) + 0x7fff7fffu) | w[j]) & 0x80008000u);
         }
+        mask[h] = interleave16(flags);
     }
-    if (run) {
-        const uint32_t eob = __ldg(ac);
-        emit(eob & 0xffffu, eob >> 16);
-    }
+    const int diff = (int)coef[0] - pred;
+    const uint32_t dsz = category(diff), dcode = dc[dsz];
+    emit((dcode & 0xffffu) << dsz | ((uint32_t)(diff < 0 ? diff + (1 << dsz) - 1 : diff) & ((1u << dsz) - 1)),
+         (dcode >> 16) + dsz);
+    mask[0] &= ~1u;
+    uint32_t next = 1;  // the coefficient after the last coded one
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        for (uint32_t m = mask[h]; m; m &= m - 1) {
+            const uint32_t i = (uint32_t)(__ffs(m) - 1) + 32 * h;
+            const int v = coef[i];
+            uint32_t run = i - next;
+            next = i + 1;
+            for (; run >= 16; run -= 16) emit(ac[0xf0] & 0xffffu, ac[0xf0] >> 16);
+            const uint32_t sz = category(v), code = ac[run << 4 | sz];
+            emit((code & 0xffffu) << sz | ((uint32_t)(v < 0 ? v + (1 << sz) - 1 : v) & ((1u << sz) - 1)), (code >> 16) + sz);
+        }
+    if (next < 64) emit(ac[0] & 0xffffu, ac[0] >> 16);
 }
 
-__global__ void __launch_bounds__(256) bits_kernel(EncLaunch L) {
-    const uint64_t blk = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Frame of block blk, from the CTA's first block's on.
+__device__ __forceinline__ const EncFrame &frame_from(const EncLaunch &L, uint32_t f, uint64_t blk) {
+    while (f + 1 < L.n_frames && L.frames[f + 1].block_base <= blk) f++;
+    return L.frames[f];
+}
+
+__global__ void __launch_bounds__(kSymThreads) bits_kernel(EncLaunch L) {
+    __shared__ SymSmem S;
+    load_symbols(L, S);
+    const uint64_t blk = (uint64_t)blockIdx.x * kSymThreads + threadIdx.x;
     if (blk >= L.n_blocks) return;
-    const EncFrame &F = L.frames[frame_of_block(L, blk)];
+    const EncFrame &F = frame_from(L, S.frame, blk);
+    const uint32_t i = (uint32_t)(blk - F.block_base), mcu = i / F.bpm;
     uint32_t bits = 0;
-    block_symbols(L, F, blk, [&](uint32_t, uint32_t n) { bits += n; });
+    block_symbols(L, S, F, blk, mcu, i - mcu * F.bpm, [&](uint32_t, uint32_t n) { bits += n; });
     L.block_bits[blk] = bits;
 }
 
@@ -333,7 +397,6 @@ __global__ void segment_kernel(EncLaunch L) {
     L.seg_bits[s] = bits;
     // whole 16-byte chunks, so that every chunk's 16-byte load is aligned and inside its segment
     L.seg_chunks[s] = (uint32_t)((bytes + 15) / 16);
-    L.seg_words[s] = 4 * L.seg_chunks[s];
 }
 
 // Writes block blk's codes at its bit offset in its segment's big-endian word
@@ -341,15 +404,17 @@ __global__ void segment_kernel(EncLaunch L) {
 // with the previous block unless the block starts on a word) and the last partial
 // one are OR-ed. The segment's last block pads its final byte with 1 bits
 // (EntropyWriter::finish, encoder.rs:530-543).
-__global__ void __launch_bounds__(256) write_bits_kernel(EncLaunch L) {
-    const uint64_t blk = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kSymThreads) write_bits_kernel(EncLaunch L) {
+    __shared__ SymSmem S;
+    load_symbols(L, S);
+    const uint64_t blk = (uint64_t)blockIdx.x * kSymThreads + threadIdx.x;
     if (blk >= L.n_blocks) return;
-    const EncFrame &F = L.frames[frame_of_block(L, blk)];
-    const uint32_t mcu = (uint32_t)((blk - F.block_base) / F.bpm);
+    const EncFrame &F = frame_from(L, S.frame, blk);
+    const uint32_t i = (uint32_t)(blk - F.block_base), mcu = i / F.bpm;
     const uint32_t j = F.ri ? mcu / F.ri : 0u;
     const uint64_t seg0 = segment_block(F, j), seg1 = segment_block(F, j + 1);
     const uint64_t p = L.bit_off[blk] - L.bit_off[seg0];
-    uint32_t *words = L.raw + L.seg_word_off[F.seg_base + j];
+    uint32_t *words = L.raw + 4 * L.seg_chunk_off[F.seg_base + j];
     uint64_t w = p >> 5;
     uint64_t acc = 0;
     uint32_t nacc = (uint32_t)(p & 31);  // pending bits, counting the word's earlier bits as zeros
@@ -367,7 +432,7 @@ __global__ void __launch_bounds__(256) write_bits_kernel(EncLaunch L) {
             acc &= (1ull << nacc) - 1;
         }
     };
-    block_symbols(L, F, blk, emit);
+    block_symbols(L, S, F, blk, mcu, i - mcu * F.bpm, emit);
     if (blk + 1 == seg1) {
         const uint32_t pad = (8u - (uint32_t)((L.bit_off[seg1] - L.bit_off[seg0]) & 7)) & 7u;
         if (pad) emit((1u << pad) - 1, pad);
@@ -381,20 +446,38 @@ __device__ __forceinline__ uint32_t lead_bytes_mask(int nv) {
     return nv >= 4 ? 0x80808080u : nv <= 0 ? 0u : (0x80808080u << (8 * (4 - nv)));
 }
 
-__device__ __forceinline__ void chunk_of(const EncLaunch &L, uint64_t c, uint32_t *s, uint64_t *k, uint32_t *n) {
-    *s = segment_of_chunk(L, c);
+// A CTA's chunks lie between two segments, found once.
+struct ChunkSmem {
+    uint32_t lo, hi;
+};
+
+__device__ __forceinline__ void chunk_range(const EncLaunch &L, uint64_t n_chunks, ChunkSmem &S) {
+    if (threadIdx.x < 2) {
+        const uint64_t first = (uint64_t)blockIdx.x * blockDim.x;
+        const uint64_t c = threadIdx.x ? min(first + blockDim.x, n_chunks) - 1 : first;
+        (threadIdx.x ? S.hi : S.lo) = segment_of_chunk(L, c, 0, L.n_segs - 1);
+    }
+    __syncthreads();
+}
+
+// Segment s of chunk c, its number k in it, and its bytes.
+__device__ __forceinline__ void chunk_of(const EncLaunch &L, const ChunkSmem &S, uint64_t c, uint32_t *s, uint64_t *k,
+                                         uint32_t *n) {
+    *s = segment_of_chunk(L, c, S.lo, S.hi);
     *k = c - L.seg_chunk_off[*s];
     const uint64_t bytes = (L.seg_bits[*s] + 7) / 8;
     *n = (uint32_t)min((uint64_t)16, bytes - 16 * *k);
 }
 
 __global__ void __launch_bounds__(256) ff_count_kernel(EncLaunch L, uint64_t n_chunks) {
+    __shared__ ChunkSmem S;
+    chunk_range(L, n_chunks, S);
     const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n_chunks) return;
     uint32_t s, n;
     uint64_t k;
-    chunk_of(L, c, &s, &k, &n);
-    const uint4 v = *reinterpret_cast<const uint4 *>(L.raw + L.seg_word_off[s] + 4 * k);
+    chunk_of(L, S, c, &s, &k, &n);
+    const uint4 v = *reinterpret_cast<const uint4 *>(L.raw + 4 * c);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     uint32_t count = 0;
 #pragma unroll
@@ -402,56 +485,10 @@ __global__ void __launch_bounds__(256) ff_count_kernel(EncLaunch L, uint64_t n_c
     L.chunk_ff[c] = count;
 }
 
-// thread per frame: each segment's offset in the frame's entropy bytes, each
-// segment followed by its marker (RSTn, or EOI after the last)
-__global__ void layout_kernel(EncLaunch L) {
-    const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= L.n_frames) return;
-    const EncFrame &F = L.frames[f];
-    uint64_t pos = 0;
-    for (uint32_t j = 0; j < F.nseg; j++) {
-        const uint32_t s = F.seg_base + j;
-        L.seg_out[s] = (uint32_t)pos;
-        const uint64_t ff = L.ff_off[L.seg_chunk_off[s + 1]] - L.ff_off[L.seg_chunk_off[s]];
-        pos += (L.seg_bits[s] + 7) / 8 + ff + 2;
-    }
-    L.frame_len[f] = (uint32_t)pos;
-}
-
-// thread per chunk: its bytes with a 0x00 after each 0xFF (EntropyWriter::push,
-// encoder.rs:519-528), then the segment's marker after its last chunk
-__global__ void __launch_bounds__(256) emit_kernel(EncLaunch L, uint64_t n_chunks) {
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_chunks) return;
-    uint32_t s, n;
-    uint64_t k;
-    chunk_of(L, c, &s, &k, &n);
-    const EncFrame &F = L.frames[frame_of_segment(L, s)];
-    const uint32_t j = s - F.seg_base;
-    uint8_t *dst = L.out + L.frame_off[frame_of_segment(L, s)] + L.seg_out[s] + 16 * k +
-                   (L.ff_off[c] - L.ff_off[L.seg_chunk_off[s]]);
-    const uint32_t *w = L.raw + L.seg_word_off[s] + 4 * k;
-    for (uint32_t b = 0; b < n; b++) {
-        const uint8_t v = (uint8_t)(w[b >> 2] >> (24 - 8 * (b & 3)));
-        *dst++ = v;
-        if (v == 0xff) *dst++ = 0x00;
-    }
-    const uint64_t bytes = (L.seg_bits[s] + 7) / 8;
-    if (16 * k + n == bytes) {
-        dst[0] = 0xff;
-        dst[1] = j + 1 < F.nseg ? (uint8_t)(0xd0 + (j & 7)) : (uint8_t)0xd9;
-    }
-}
-
-// ----------------------------------------------------------------- scan ---
-
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;  // consecutive values per thread
-constexpr uint64_t kScanTile = (uint64_t)kScanThreads * kScanItems;
-
-// exclusive prefix of v over the CTA (1024 threads); *total = the CTA's sum
+// Exclusive prefix of v over a CTA of NT threads; *total = the CTA's sum.
+template <int NT>
 __device__ __forceinline__ uint64_t cta_exclusive(uint64_t v, uint64_t *total) {
-    __shared__ uint64_t s_warp[32];
+    __shared__ uint64_t s_warp[NT / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint64_t incl = v;
 #pragma unroll
@@ -462,13 +499,13 @@ __device__ __forceinline__ uint64_t cta_exclusive(uint64_t v, uint64_t *total) {
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        uint64_t w = s_warp[lane], wi = w;
+        uint64_t w = lane < NT / 32 ? s_warp[lane] : 0, wi = w;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const uint64_t o = __shfl_up_sync(0xffffffffu, wi, d);
             if (lane >= d) wi += o;
         }
-        s_warp[lane] = wi - w;
+        if (lane < NT / 32) s_warp[lane] = wi - w;
         if (lane == 31) *total = wi;
     }
     __syncthreads();
@@ -477,28 +514,156 @@ __device__ __forceinline__ uint64_t cta_exclusive(uint64_t v, uint64_t *total) {
     return r;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_t *in, uint64_t n, uint64_t *part) {
+constexpr int kLayoutThreads = 256;
+
+// Where frame f's entropy bytes go; nullptr when its buffer is too small.
+__device__ __forceinline__ uint8_t *frame_dst(const EncLaunch &L, uint32_t f) {
+    const EncFrame &F = L.frames[f];
+    if (!F.out) return L.out + L.frame_off[f];
+    return F.hdr_len + (uint64_t)L.frame_len[f] <= F.cap ? F.out + F.hdr_len : nullptr;
+}
+
+// CTA per frame: each segment's offset in the frame's entropy bytes, each segment
+// followed by its marker (RSTn, or EOI after the last); the frame's header into a
+// device buffer. The last CTA to finish lays out the frames staged for host buffers.
+__global__ void __launch_bounds__(kLayoutThreads) layout_kernel(EncLaunch L) {
     __shared__ uint64_t s_total;
+    __shared__ bool s_last;
+    const uint32_t f = blockIdx.x;
+    const EncFrame &F = L.frames[f];
+    uint64_t pos = 0;
+    for (uint32_t j0 = 0; j0 < F.nseg; j0 += kLayoutThreads) {
+        const uint32_t j = j0 + threadIdx.x, s = F.seg_base + j;
+        uint64_t bytes = 0;
+        if (j < F.nseg)
+            bytes = (L.seg_bits[s] + 7) / 8 + L.ff_off[L.seg_chunk_off[s + 1]] - L.ff_off[L.seg_chunk_off[s]] + 2;
+        const uint64_t ex = cta_exclusive<kLayoutThreads>(bytes, &s_total);
+        if (j < F.nseg) L.seg_out[s] = (uint32_t)(pos + ex);
+        pos += s_total;
+        __syncthreads();
+    }
+    if (F.out && F.hdr_len + pos <= F.cap)
+        for (uint32_t i = threadIdx.x; i < F.hdr_len; i += kLayoutThreads) F.out[i] = L.headers[F.hdr_off + i];
+    if (threadIdx.x == 0) {
+        L.frame_len[f] = (uint32_t)pos;
+        __threadfence();
+        s_last = atomicAdd(L.done, 1u) + 1 == gridDim.x;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    uint64_t carry = 0;
+    for (uint32_t g0 = 0; g0 < L.n_frames; g0 += kLayoutThreads) {
+        const uint32_t g = g0 + threadIdx.x;
+        const uint64_t len = g < L.n_frames && !L.frames[g].out ? *(volatile uint32_t *)&L.frame_len[g] : 0;
+        const uint64_t ex = cta_exclusive<kLayoutThreads>(len, &s_total);
+        if (g < L.n_frames) L.frame_off[g] = carry + ex;
+        carry += s_total;
+        __syncthreads();
+    }
+}
+
+// thread per chunk: its bytes with a 0x00 after each 0xFF (EntropyWriter::push,
+// encoder.rs:519-528), then the segment's marker after its last chunk. A CTA whose
+// chunks are of one frame collects its run of bytes in shared memory and stores it as
+// 16-byte vectors; byte stores took 0.20 ms for the 67 MB of 60 1080p frames.
+constexpr int kEmitThreads = 256;
+
+__global__ void __launch_bounds__(kEmitThreads) emit_kernel(EncLaunch L, uint64_t n_chunks) {
+    __shared__ ChunkSmem S;
+    __shared__ __align__(16) uint8_t s_out[kEmitThreads * 34 + 32];
+    __shared__ uint8_t *s_dst;
+    __shared__ uint32_t s_frame[2], s_len;
+    chunk_range(L, n_chunks, S);
+    if (threadIdx.x < 2) s_frame[threadIdx.x] = frame_of_segment(L, threadIdx.x ? S.hi : S.lo);
+    __syncthreads();
+    const bool one = s_frame[0] == s_frame[1];
+    uint32_t f = s_frame[0];
+    uint8_t *base = frame_dst(L, f);
+    if (one && !base) return;  // (uniform: the frame's buffer is too small)
+    const uint64_t c = (uint64_t)blockIdx.x * kEmitThreads + threadIdx.x;
+    const bool valid = c < n_chunks;
+    uint8_t *dst = base;
+    uint32_t s = 0, n = 0;
+    uint64_t k = 0;
+    if (valid) {
+        chunk_of(L, S, c, &s, &k, &n);
+        if (!one) {
+            f = frame_of_segment(L, s);
+            base = frame_dst(L, f);
+        }
+        dst = base + L.seg_out[s] + 16 * k + (L.ff_off[c] - L.ff_off[L.seg_chunk_off[s]]);
+    }
+    if (threadIdx.x == 0) s_dst = dst;
+    __syncthreads();
+    uint8_t *first = s_dst;  // the CTA's first byte
+    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(first) & 15);
+    uint8_t *p = one ? s_out + mis + (dst - first) : dst;
+    if (valid && base) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(L.raw + 4 * c);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int b = 0; b < 16; b++) {
+            if (b >= (int)n) break;
+            const uint8_t x = (uint8_t)(w[b >> 2] >> (24 - 8 * (b & 3)));
+            *p++ = x;
+            if (x == 0xff) *p++ = 0x00;
+        }
+        const uint64_t bytes = (L.seg_bits[s] + 7) / 8;
+        if (16 * k + n == bytes) {
+            const EncFrame &F = L.frames[f];
+            const uint32_t j = s - F.seg_base;
+            p[0] = 0xff;
+            p[1] = j + 1 < F.nseg ? (uint8_t)(0xd0 + (j & 7)) : (uint8_t)0xd9;
+            p += 2;
+        }
+        if (one && (threadIdx.x == kEmitThreads - 1 || c + 1 == n_chunks)) s_len = (uint32_t)(p - s_out);
+    }
+    if (!one) return;
+    __syncthreads();
+    const uint32_t end = s_len;  // bytes [mis, end) of s_out
+    uint8_t *line = first - mis;
+    for (uint32_t b0 = threadIdx.x * 16; b0 < end; b0 += kEmitThreads * 16) {
+        if (b0 >= mis && b0 + 16 <= end) {
+            *reinterpret_cast<uint4 *>(line + b0) = *reinterpret_cast<const uint4 *>(s_out + b0);
+        } else {
+            for (uint32_t b = max(b0, mis); b < min(b0 + 16, end); b++) line[b] = s_out[b];
+        }
+    }
+}
+
+// ----------------------------------------------------------------- scan ---
+
+constexpr int kScanThreads = 1024;
+constexpr int kScanItems = 4;  // consecutive values per thread
+constexpr uint64_t kScanTile = (uint64_t)kScanThreads * kScanItems;
+
+// Tile sums; the last CTA to finish turns them into their exclusive prefix in place and
+// writes the grand total.
+__global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_t *in, uint64_t n, uint64_t *part,
+                                                                   uint64_t *total, uint32_t *done) {
+    __shared__ uint64_t s_total;
+    __shared__ bool s_last;
     const uint64_t base = blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     uint64_t sum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++)
         if (base + k < n) sum += in[base + k];
-    cta_exclusive(sum, &s_total);
+    cta_exclusive<kScanThreads>(sum, &s_total);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = s_total;
+        __threadfence();
+        s_last = atomicAdd(done, 1u) + 1 == gridDim.x;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) part[blockIdx.x] = s_total;
-}
-
-// one CTA: exclusive prefix of the tile sums in place; the grand total to *total
-__global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(uint64_t *part, uint64_t np, uint64_t *total) {
-    __shared__ uint64_t s_total;
+    if (!s_last) return;
+    __threadfence();
     uint64_t carry = 0;
-    for (uint64_t b = 0; b < np; b += kScanThreads) {
+    for (uint64_t b = 0; b < gridDim.x; b += kScanThreads) {
         const uint64_t i = b + threadIdx.x;
-        const uint64_t v = i < np ? part[i] : 0;
-        const uint64_t ex = cta_exclusive(v, &s_total);
-        __syncthreads();
-        if (i < np) part[i] = carry + ex;
+        const uint64_t v = i < gridDim.x ? *(volatile uint64_t *)&part[i] : 0;
+        const uint64_t ex = cta_exclusive<kScanThreads>(v, &s_total);
+        if (i < gridDim.x) part[i] = carry + ex;
         carry += s_total;
         __syncthreads();
     }
@@ -516,7 +681,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
         v[k] = base + k < n ? in[base + k] : 0u;
         sum += v[k];
     }
-    uint64_t run = part[blockIdx.x] + cta_exclusive(sum, &s_total);
+    uint64_t run = part[blockIdx.x] + cta_exclusive<kScanThreads>(sum, &s_total);
 #pragma unroll
     for (int k = 0; k < kScanItems; k++)
         if (base + k < n) {
@@ -525,16 +690,12 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
         }
 }
 
-// out[0, n) = exclusive prefix of in, out[n] = the sum (part: ceil(n / 4096) scratch)
-void exclusive_scan(const uint32_t *in, uint64_t n, uint64_t *out, uint64_t *part, cudaStream_t s) {
-    const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles == 0) {
-        cudaMemsetAsync(out, 0, sizeof(uint64_t), s);
-        return;
-    }
-    scan_reduce_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, part);
-    scan_partials_kernel<<<1, kScanThreads, 0, s>>>(part, tiles, out + n);
-    scan_apply_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(in, n, part, out);
+// out[0, n) = exclusive prefix of in, out[n] = the sum (part: ceil(n / 4096) scratch,
+// done: a zeroed counter); n > 0
+void exclusive_scan(const uint32_t *in, uint64_t n, uint64_t *out, uint64_t *part, uint32_t *done, cudaStream_t s) {
+    const unsigned tiles = (unsigned)((n + kScanTile - 1) / kScanTile);
+    scan_reduce_kernel<<<tiles, kScanThreads, 0, s>>>(in, n, part, out + n, done);
+    scan_apply_kernel<<<tiles, kScanThreads, 0, s>>>(in, n, part, out);
 }
 
 }  // namespace
@@ -583,6 +744,46 @@ struct DBuf {
     }
 };
 
+struct PBuf {
+    void *p = nullptr;
+    size_t cap = 0;
+    void ensure(size_t bytes) {
+        if (bytes <= cap) return;
+        const size_t want = std::max(bytes, cap + cap / 2);
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        cap = 0;
+        if (cudaHostAlloc(&p, want, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            throw std::runtime_error("GPU encoder: out of pinned memory");
+        }
+        cap = want;
+    }
+    ~PBuf() {
+        if (p) cudaFreeHost(p);
+    }
+};
+
+// Copies host planes up. Planes that follow one another in host memory go up as one
+// copy (a call per plane took a third of the encode of 12 small frames).
+struct PlaneUploads {
+    const uint8_t *src = nullptr;
+    uint8_t *dst = nullptr;
+    size_t bytes = 0;
+
+    void flush(cudaStream_t s) {
+        if (bytes && cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
+            throw std::runtime_error("GPU encoder: upload failed");
+        bytes = 0;
+    }
+    // Whether `more` at p continues the pending copy.
+    bool append(const uint8_t *p, size_t more) {
+        if (!bytes || p != src + bytes) return false;
+        bytes += more;
+        return true;
+    }
+};
+
 }  // namespace
 
 struct GpuJpegEncoder::Impl {
@@ -590,8 +791,9 @@ struct GpuJpegEncoder::Impl {
     cudaStream_t s = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::mutex mu;
-    DBuf frames, tabs, in, coef, block_bits, bit_off, part, seg_bits, seg_words, seg_chunks, seg_word_off,
-        seg_chunk_off, raw, chunk_ff, ff_off, seg_out, frame_len, frame_off, out, exact;
+    DBuf plan, in, coef, block_bits, bit_off, part, seg_bits, seg_chunks, seg_chunk_off, raw, chunk_ff, ff_off, seg_out,
+        frame_len, frame_off, out, counters;
+    PBuf up, back;
 };
 
 GpuJpegEncoder::GpuJpegEncoder(int device) : impl_(new Impl) {
@@ -624,46 +826,32 @@ int32_t GpuJpegEncoder::encode(EncodeItem *items, size_t n, const JpegEncodeOpti
         cudaGetLastError();
         return kInternal;
     }
-    // host plans: validation, tables and header bytes per frame
-    std::vector<JpegEncodePlan> plans(n);
-    std::vector<size_t> live;
+    // host plans: validation and geometry per frame; tables and header bytes per format
+    struct Live {
+        size_t item;
+        uint32_t plan;
+    };
+    JpegEncodePlan plans[5], scratch;  // by pixel format - 1 (validation refuses 4:1:1)
+    bool have[5] = {};
+    std::vector<Live> live;
+    std::vector<EncFrame> fr;
+    std::vector<uint8_t> headers;
+    uint64_t blocks = 0, in_bytes = 0;
+    uint32_t segs = 0;
     for (size_t i = 0; i < n; i++) {
         EncodeItem &it = items[i];
         it.status = kOk;
         it.message.clear();
         it.out_len = 0;
-        if (!plan_jpeg_encode(it.frame, opt, &plans[i])) {
-            it.status = plans[i].status;
-            it.message = plans[i].message;
+        const uint32_t form = it.frame.format - kGray8;
+        JpegEncodePlan &P = form < 5 ? plans[form] : scratch;
+        if (!plan_jpeg_frame(it.frame, opt, &P) || (!have[form] && !plan_jpeg_tables(it.frame, opt, &P))) {
+            it.status = P.status;
+            it.message = P.message;
             continue;
         }
-        live.push_back(i);
-    }
-    if (live.empty()) return kOk;
-    const JpegEncodePlan &P0 = plans[live[0]];  // tables depend on the options only
-    // device tables: qt [2][64] | codes [4][256] | fp32 reciprocals of qt [2][64] | zigzag
-    // position of each natural index [64]
-    std::vector<uint8_t> tab(128 + 4 * 256 * 4 + 2 * 64 * 4 + 64);
-    memcpy(tab.data(), P0.qt, 128);
-    float *rq = reinterpret_cast<float *>(tab.data() + 128 + 4096);
-    for (int t = 0; t < 2; t++)
-        for (int i = 0; i < 64; i++) rq[t * 64 + i] = 1.0f / (float)P0.qt[t][i];
-    static const int kZigzagOrder[64] = MMR_ZIGZAG_INIT;
-    for (int k = 0; k < 64; k++) tab[128 + 4096 + 512 + kZigzagOrder[k]] = (uint8_t)k;
-    uint32_t *codes = reinterpret_cast<uint32_t *>(tab.data() + 128);
-    for (int t = 0; t < 2; t++)
-        for (int sym = 0; sym < 256; sym++) {
-            codes[t * 256 + sym] = P0.dc[t][sym].bits | (uint32_t)P0.dc[t][sym].length << 16;
-            codes[(2 + t) * 256 + sym] = P0.ac[t][sym].bits | (uint32_t)P0.ac[t][sym].length << 16;
-        }
-    // frame records; host planes go up packed (stride = width)
-    std::vector<EncFrame> fr(live.size());
-    uint64_t blocks = 0, in_bytes = 0;
-    uint32_t segs = 0;
-    for (size_t k = 0; k < live.size(); k++) {
-        const EncodeItem &it = items[live[k]];
-        const JpegEncodePlan &P = plans[live[k]];
-        EncFrame &F = fr[k];
+        have[form] = true;
+        EncFrame F;
         memset(&F, 0, sizeof F);
         F.mcu_cols = (uint32_t)P.mcu_cols;
         F.mcus = (uint32_t)(P.mcu_cols * P.mcu_rows);
@@ -692,143 +880,201 @@ int32_t GpuJpegEncoder::encode(EncodeItem *items, size_t n, const JpegEncodeOpti
         F.block_base = blocks;
         F.seg_base = segs;
         F.nseg = F.ri ? (F.mcus + F.ri - 1) / F.ri : 1;
+        F.out = it.out_on_device ? it.out : nullptr;
+        F.cap = it.out && it.out_on_device ? it.out_capacity : 0;
+        F.hdr_off = (uint32_t)headers.size();
+        F.hdr_len = (uint32_t)P.header.size();
+        headers.insert(headers.end(), P.header.begin(), P.header.end());
+        uint8_t *size = headers.data() + F.hdr_off + P.size_at;
+        size[0] = (uint8_t)(it.frame.height >> 8);
+        size[1] = (uint8_t)it.frame.height;
+        size[2] = (uint8_t)(it.frame.width >> 8);
+        size[3] = (uint8_t)it.frame.width;
         blocks += (uint64_t)F.mcus * bpm;
         segs += F.nseg;
+        fr.push_back(F);
+        live.push_back({i, form});
     }
+    if (live.empty()) return kOk;
+    // the tables depend on the options only; a gray frame's plan lacks the second ones
+    const JpegEncodePlan *P0 = &plans[live[0].plan];
+    for (const Live &l : live)
+        if (plans[l.plan].ncomp > P0->ncomp) P0 = &plans[l.plan];
+    // device tables: qt [2][64] | codes [4][256] | fp32 reciprocals of qt [2][64] | zigzag
+    // position of each natural index [64]
+    constexpr size_t kTabBytes = 128 + 4 * 256 * 4 + 2 * 64 * 4 + 64;
+    uint8_t tab[kTabBytes];
+    memcpy(tab, P0->qt, 128);
+    float *rq = reinterpret_cast<float *>(tab + 128 + 4096);
+    for (int t = 0; t < 2; t++)
+        for (int i = 0; i < 64; i++) {
+            const float r = 1.0f / (float)P0->qt[t][i];
+            memcpy(rq + t * 64 + i, &r, 4);
+        }
+    static const int kZigzagOrder[64] = MMR_ZIGZAG_INIT;
+    for (int k = 0; k < 64; k++) tab[128 + 4096 + 512 + kZigzagOrder[k]] = (uint8_t)k;
+    uint32_t *codes = reinterpret_cast<uint32_t *>(tab + 128);
+    for (int t = 0; t < 2; t++)
+        for (int sym = 0; sym < 256; sym++) {
+            const uint32_t d = P0->dc[t][sym].bits | (uint32_t)P0->dc[t][sym].length << 16;
+            const uint32_t a = P0->ac[t][sym].bits | (uint32_t)P0->ac[t][sym].length << 16;
+            memcpy(codes + t * 256 + sym, &d, 4);
+            memcpy(codes + (2 + t) * 256 + sym, &a, 4);
+        }
     stats_.blocks = blocks;
     try {
         cudaEventRecord(I.ev0, I.s);
         I.in.ensure(std::max<uint64_t>(in_bytes, 256));
         uint64_t at = 0;
+        PlaneUploads up;
         for (size_t k = 0; k < live.size(); k++) {
-            const EncodeItem &it = items[live[k]];
-            for (uint32_t c = 0; c < plans[live[k]].ncomp; c++) {
+            const EncodeItem &it = items[live[k].item];
+            for (uint32_t c = 0; c < plans[live[k].plan].ncomp; c++) {
                 const PlaneIn &pl = it.frame.planes[c];
                 if (it.in_on_device) {
                     fr[k].plane[c] = pl.data;
                     fr[k].stride[c] = pl.stride;
                     continue;
                 }
-                uint8_t *dst = I.in.as<uint8_t>() + at;
-                // contiguous planes go up as one linear copy, strided ones row by row
-                const cudaError_t e =
-                    pl.stride == pl.width
-                        ? cudaMemcpyAsync(dst, pl.data, pl.width * pl.height, cudaMemcpyHostToDevice, I.s)
-                        : cudaMemcpy2DAsync(dst, pl.width, pl.data, pl.stride, pl.width, pl.height,
-                                            cudaMemcpyHostToDevice, I.s);
-                if (e != cudaSuccess) throw std::runtime_error("GPU encoder: upload failed");
-                fr[k].plane[c] = dst;
+                const size_t bytes = pl.width * pl.height;
                 fr[k].stride[c] = pl.width;
-                at += (pl.width * pl.height + 255) / 256 * 256;
+                const uint8_t *before = up.src;
+                if (pl.stride == pl.width && up.append(pl.data, bytes)) {  // packed right behind the last one
+                    fr[k].plane[c] = up.dst + (pl.data - before);
+                    at += bytes;
+                    continue;
+                }
+                up.flush(I.s);
+                at = (at + 255) / 256 * 256;
+                uint8_t *dst = I.in.as<uint8_t>() + at;
+                fr[k].plane[c] = dst;
+                at += bytes;
+                if (pl.stride == pl.width) {
+                    up.src = pl.data;
+                    up.dst = dst;
+                    up.bytes = bytes;
+                } else if (cudaMemcpy2DAsync(dst, pl.width, pl.data, pl.stride, pl.width, pl.height,
+                                             cudaMemcpyHostToDevice, I.s) != cudaSuccess) {  // row by row
+                    throw std::runtime_error("GPU encoder: upload failed");
+                }
             }
         }
+        up.flush(I.s);
+        // the plan: frames | tables | headers, one copy
         const uint32_t nf = (uint32_t)live.size();
-        I.frames.ensure(nf * sizeof(EncFrame));
-        I.tabs.ensure(tab.size());
-        cudaMemcpyAsync(I.frames.p, fr.data(), nf * sizeof(EncFrame), cudaMemcpyHostToDevice, I.s);
-        cudaMemcpyAsync(I.tabs.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, I.s);
+        const size_t o_tab = (nf * sizeof(EncFrame) + 255) / 256 * 256, o_hdr = o_tab + (kTabBytes + 255) / 256 * 256;
+        I.plan.ensure(o_hdr + headers.size());
+        I.up.ensure(o_hdr + headers.size());
+        uint8_t *hp = static_cast<uint8_t *>(I.up.p);
+        memcpy(hp, fr.data(), nf * sizeof(EncFrame));
+        memcpy(hp + o_tab, tab, kTabBytes);
+        memcpy(hp + o_hdr, headers.data(), headers.size());
+        cudaMemcpyAsync(I.plan.p, hp, o_hdr + headers.size(), cudaMemcpyHostToDevice, I.s);
+        // read back: two totals, then the frames' sizes and places and the tie count
+        const size_t b_len = 16, b_off = b_len + (nf * 4 + 15) / 16 * 16, b_exact = b_off + nf * 8;
+        I.back.ensure(b_exact + 8);
+        uint8_t *hb = static_cast<uint8_t *>(I.back.p);
         I.coef.ensure(blocks * 128);
         I.block_bits.ensure(blocks * 4);
         I.bit_off.ensure((blocks + 1) * 8);
         I.part.ensure(((std::max<uint64_t>(blocks, segs) + kScanTile - 1) / kScanTile + 1) * 8);
         I.seg_bits.ensure(segs * 8);
-        I.seg_words.ensure(segs * 4);
         I.seg_chunks.ensure(segs * 4);
-        I.seg_word_off.ensure((segs + 1) * 8);
         I.seg_chunk_off.ensure((segs + 1) * 8);
         I.seg_out.ensure(segs * 4);
         I.frame_len.ensure(nf * 4);
-        I.frame_off.ensure((nf + 1) * 8);
-        I.exact.ensure(8);
+        I.frame_off.ensure(nf * 8);
+        I.counters.ensure(32);
         EncLaunch L;
         memset(&L, 0, sizeof L);
-        L.frames = I.frames.as<EncFrame>();
+        L.frames = I.plan.as<EncFrame>();
+        const uint8_t *dt = I.plan.as<uint8_t>() + o_tab;
+        L.headers = I.plan.as<uint8_t>() + o_hdr;
         L.n_frames = nf;
         L.n_blocks = blocks;
         L.n_segs = segs;
-        L.qt = I.tabs.as<uint8_t>();
-        L.codes = reinterpret_cast<const uint32_t *>(I.tabs.as<uint8_t>() + 128);
-        L.rq = reinterpret_cast<const float *>(I.tabs.as<uint8_t>() + 128 + 4096);
-        L.nat2zz = I.tabs.as<uint8_t>() + 128 + 4096 + 512;
+        L.qt = dt;
+        L.codes = reinterpret_cast<const uint32_t *>(dt + 128);
+        L.rq = reinterpret_cast<const float *>(dt + 128 + 4096);
+        L.nat2zz = dt + 128 + 4096 + 512;
         L.coef = I.coef.as<int16_t>();
         L.block_bits = I.block_bits.as<uint32_t>();
         L.bit_off = I.bit_off.as<uint64_t>();
-        L.seg_words = I.seg_words.as<uint32_t>();
         L.seg_chunks = I.seg_chunks.as<uint32_t>();
         L.seg_bits = I.seg_bits.as<uint64_t>();
-        L.seg_word_off = I.seg_word_off.as<uint64_t>();
         L.seg_chunk_off = I.seg_chunk_off.as<uint64_t>();
         L.seg_out = I.seg_out.as<uint32_t>();
         L.frame_len = I.frame_len.as<uint32_t>();
         L.frame_off = I.frame_off.as<uint64_t>();
-        L.exact = I.exact.as<unsigned long long>();
-        cudaMemsetAsync(L.exact, 0, 8, I.s);
-        const unsigned bgrid = (unsigned)((blocks + 255) / 256);
+        L.exact = I.counters.as<unsigned long long>();
+        uint32_t *done = I.counters.as<uint32_t>() + 2;  // of three scans and the layout
+        L.done = done + 3;
+        cudaMemsetAsync(I.counters.p, 0, 32, I.s);
+        const unsigned bgrid = (unsigned)((blocks + kSymThreads - 1) / kSymThreads);
         const uint64_t tiles = (blocks + kEncBlocksPerTile - 1) / kEncBlocksPerTile;
         // one wave of resident CTAs (64 registers: four per SM)
         fdct_kernel<<<(unsigned)std::min<uint64_t>(tiles, 152 * 4), kEncThreads, 0, I.s>>>(L, tiles);
-        bits_kernel<<<bgrid, 256, 0, I.s>>>(L);
-        exclusive_scan(L.block_bits, blocks, L.bit_off, I.part.as<uint64_t>(), I.s);
+        bits_kernel<<<bgrid, kSymThreads, 0, I.s>>>(L);
+        exclusive_scan(L.block_bits, blocks, L.bit_off, I.part.as<uint64_t>(), done, I.s);
         segment_kernel<<<(segs + 255) / 256, 256, 0, I.s>>>(L);
-        exclusive_scan(L.seg_words, segs, L.seg_word_off, I.part.as<uint64_t>(), I.s);
-        exclusive_scan(L.seg_chunks, segs, L.seg_chunk_off, I.part.as<uint64_t>(), I.s);
-        uint64_t totals[2] = {0, 0};
-        cudaMemcpyAsync(&totals[0], L.seg_word_off + segs, 8, cudaMemcpyDeviceToHost, I.s);
-        cudaMemcpyAsync(&totals[1], L.seg_chunk_off + segs, 8, cudaMemcpyDeviceToHost, I.s);
+        exclusive_scan(L.seg_chunks, segs, L.seg_chunk_off, I.part.as<uint64_t>(), done + 1, I.s);
+        cudaMemcpyAsync(hb, L.seg_chunk_off + segs, 8, cudaMemcpyDeviceToHost, I.s);
         if (cudaStreamSynchronize(I.s) != cudaSuccess) throw std::runtime_error("GPU encoder: device failure");
-        const uint64_t words = totals[0], chunks = totals[1];
+        const uint64_t chunks = *reinterpret_cast<const uint64_t *>(hb), words = 4 * chunks;
         I.raw.ensure(std::max<uint64_t>(words, 4) * 4);
         I.chunk_ff.ensure(std::max<uint64_t>(chunks, 1) * 4);
         I.ff_off.ensure((chunks + 1) * 8);
-        I.part.ensure(((std::max<uint64_t>(chunks, nf) + kScanTile - 1) / kScanTile + 1) * 8);
+        I.part.ensure(((chunks + kScanTile - 1) / kScanTile + 1) * 8);
         I.out.ensure(std::max<uint64_t>(chunks * 32 + (uint64_t)segs * 2, 16));
         L.raw = I.raw.as<uint32_t>();
         L.chunk_ff = I.chunk_ff.as<uint32_t>();
         L.ff_off = I.ff_off.as<uint64_t>();
         L.out = I.out.as<uint8_t>();
         cudaMemsetAsync(L.raw, 0, words * 4, I.s);
-        write_bits_kernel<<<bgrid, 256, 0, I.s>>>(L);
-        ff_count_kernel<<<(unsigned)((chunks + 255) / 256), 256, 0, I.s>>>(L, chunks);
-        exclusive_scan(L.chunk_ff, chunks, L.ff_off, I.part.as<uint64_t>(), I.s);
-        layout_kernel<<<(nf + 127) / 128, 128, 0, I.s>>>(L);
-        exclusive_scan(L.frame_len, nf, L.frame_off, I.part.as<uint64_t>(), I.s);
-        emit_kernel<<<(unsigned)((chunks + 255) / 256), 256, 0, I.s>>>(L, chunks);
+        write_bits_kernel<<<bgrid, kSymThreads, 0, I.s>>>(L);
+        const unsigned cgrid = (unsigned)((chunks + kEmitThreads - 1) / kEmitThreads);
+        ff_count_kernel<<<cgrid, kEmitThreads, 0, I.s>>>(L, chunks);
+        exclusive_scan(L.chunk_ff, chunks, L.ff_off, I.part.as<uint64_t>(), done + 2, I.s);
+        layout_kernel<<<nf, kLayoutThreads, 0, I.s>>>(L);
+        emit_kernel<<<cgrid, kEmitThreads, 0, I.s>>>(L, chunks);
         if (cudaGetLastError() != cudaSuccess) throw std::runtime_error("GPU encoder: launch failed");
-        std::vector<uint32_t> len(nf);
-        std::vector<uint64_t> off(nf + 1);
-        uint64_t exact = 0;
-        cudaMemcpyAsync(len.data(), L.frame_len, nf * 4, cudaMemcpyDeviceToHost, I.s);
-        cudaMemcpyAsync(off.data(), L.frame_off, (nf + 1) * 8, cudaMemcpyDeviceToHost, I.s);
-        cudaMemcpyAsync(&exact, L.exact, 8, cudaMemcpyDeviceToHost, I.s);
+        cudaMemcpyAsync(hb + b_len, L.frame_len, nf * 4, cudaMemcpyDeviceToHost, I.s);
+        cudaMemcpyAsync(hb + b_off, L.frame_off, nf * 8, cudaMemcpyDeviceToHost, I.s);
+        cudaMemcpyAsync(hb + b_exact, L.exact, 8, cudaMemcpyDeviceToHost, I.s);
+        cudaEventRecord(I.ev1, I.s);
         if (cudaStreamSynchronize(I.s) != cudaSuccess) throw std::runtime_error("GPU encoder: device failure");
-        stats_.exact_coefficients = exact;
-        // header (host plan) + entropy bytes into each caller's buffer
+        const uint32_t *len = reinterpret_cast<const uint32_t *>(hb + b_len);
+        const uint64_t *off = reinterpret_cast<const uint64_t *>(hb + b_off);
+        stats_.exact_coefficients = *reinterpret_cast<const uint64_t *>(hb + b_exact);
+        // host buffers: header, then the staged entropy bytes
+        bool copied = false;
         for (size_t k = 0; k < live.size(); k++) {
-            EncodeItem &it = items[live[k]];
-            const std::vector<uint8_t> &hdr = plans[live[k]].header;
-            const size_t total = hdr.size() + len[k];
+            EncodeItem &it = items[live[k].item];
+            const size_t total = (size_t)fr[k].hdr_len + len[k];
             if (!it.out || total > it.out_capacity) {
                 it.status = kInvalidArgument;
                 it.message = "output buffer is smaller than the encoded frame";
                 continue;
             }
-            const cudaMemcpyKind up = it.out_on_device ? cudaMemcpyHostToDevice : cudaMemcpyHostToHost;
-            if (it.out_on_device) cudaMemcpyAsync(it.out, hdr.data(), hdr.size(), up, I.s);
-            else memcpy(it.out, hdr.data(), hdr.size());
-            cudaMemcpyAsync(it.out + hdr.size(), L.out + off[k], len[k],
-                            it.out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, I.s);
+            if (!it.out_on_device) {
+                memcpy(it.out, headers.data() + fr[k].hdr_off, fr[k].hdr_len);
+                cudaMemcpyAsync(it.out + fr[k].hdr_len, L.out + off[k], len[k], cudaMemcpyDeviceToHost, I.s);
+                copied = true;
+            }
             it.out_len = total;
             stats_.bytes_out += total;
         }
-        cudaEventRecord(I.ev1, I.s);
-        if (cudaStreamSynchronize(I.s) != cudaSuccess) throw std::runtime_error("GPU encoder: device failure");
+        if (copied) {
+            cudaEventRecord(I.ev1, I.s);
+            if (cudaStreamSynchronize(I.s) != cudaSuccess) throw std::runtime_error("GPU encoder: device failure");
+        }
         cudaEventElapsedTime(&stats_.device_ms, I.ev0, I.ev1);
     } catch (const std::exception &) {
         cudaGetLastError();
-        for (size_t i : live) {
-            items[i].status = kInternal;
-            items[i].message = "CUDA device failure during encode";
-            items[i].out_len = 0;
+        for (const Live &l : live) {
+            items[l.item].status = kInternal;
+            items[l.item].message = "CUDA device failure during encode";
+            items[l.item].out_len = 0;
         }
         return kInternal;
     }
