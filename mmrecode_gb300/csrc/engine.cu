@@ -805,6 +805,14 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         for (size_t i = 0; i < n; i++)
             if (items[i].codec == kCodecMjpeg) total_bits += 8 * (uint64_t)items[i].len;
         const SlicePlan auto_plan = auto_slices(total_bits);
+        // Strips per CTA of the fused transform: several where the batch fills the GPU
+        // many times over anyway, one where every CTA counts. Measured with narrow (wide)
+        // strips, ms: 300 1080p frames (eight parts of 2.5 M blocks) 4 strips 6.69 (6.76), 8
+        // 6.57 (6.66), 1 (7.33); 64 mixed frames (four of 1.6 M) 4 strips 2.85 (2.98),
+        // 8 2.94 (3.05), 1 (3.11).
+        uint64_t batch_blocks = 0;
+        for (const JPlan &p : jplans) batch_blocks += p.n_blocks;
+        const uint32_t fused_strips = batch_blocks >= (2u << 20) ? 8 : batch_blocks >= (1u << 20) ? 4 : 1;
         uint32_t most_paths = 1;
         std::vector<size_t> in_off(n, 0), out_off(n, 0), planes_off(n, SIZE_MAX);
         std::vector<std::array<size_t, 6>> plane_geom(n);  // (offset, bytes) of up to 3 planes
@@ -955,10 +963,10 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                 F.blk_off = blocks;
                 F.n_blocks = p.n_blocks;
                 // RGB straight from coefficients for the standard MCU layouts, in
-                // strips of the width tuned for the frame's class (wide by default)
+                // strips of the width tuned for the frame's class (narrow by default)
                 const int fused_v = can_output && it.output == kOutRgb24 ? fused_layout(p) : -1;
                 if (fused_v >= 0) {
-                    bool wide = true;
+                    bool wide = false;
                     if (fused_wide >= 0) {
                         wide = fused_wide != 0;
                     } else {
@@ -969,11 +977,12 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                     FusedJob fj;
                     memset(&fj, 0, sizeof(fj));
                     fj.frame = (uint32_t)jframes.size();
-                    fj.strips_x = fused_strips_x(slot, p.mcu_cols);
+                    fj.strips = fused_strips;
+                    fj.groups_x = fused_groups_x(slot, p.mcu_cols, fused_strips);
                     fj.width = p.W;
                     fj.height = p.H;
                     fjobs[slot].push_back(fj);
-                    fcta[slot].push_back(fcta[slot].back() + fj.strips_x * p.mcu_rows);
+                    fcta[slot].push_back(fcta[slot].back() + fj.groups_x * p.mcu_rows);
                 }
                 for (uint32_t c = 0; c < p.ncomp && fused_v < 0; c++) {
                     JBlockRange r;

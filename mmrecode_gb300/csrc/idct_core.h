@@ -6,6 +6,7 @@
 
 #include "exact_fixed.h"
 #include "kernels.h"
+#include "packed.h"
 #include "rounding.h"
 #include "tables.h"
 
@@ -120,18 +121,30 @@ __device__ __forceinline__ void settle_samples(const long long *fixw, const int3
     }
 }
 
-// Dequantises block g (its levels at `levels`) into fp32 rows q and q+4 of `blk` (the product of an
+// What thread q of a block reads of it: level rows q and q + 4, and the DC.
+struct BlockRows {
+    int4 row[2];
+    int32_t dc;
+};
+
+__device__ __forceinline__ BlockRows load_rows(const int16_t *levels, const int32_t *dc, uint64_t g, uint32_t q) {
+    BlockRows b;
+    b.row[0] = reinterpret_cast<const int4 *>(levels)[q];
+    b.row[1] = reinterpret_cast<const int4 *>(levels)[q + 4];
+    b.dc = dc[g];
+    return b;
+}
+
+// Dequantises them into fp32 rows q and q+4 of `blk` (the product of an
 // int16 level and an 8-bit quantiser is exact in fp32; the DC is the decoder's
 // dequantised int32, rounded to fp32 like every c in the bound). Returns the
 // sum of |c| over the two rows.
-__device__ __forceinline__ float stage_rows(const int16_t *levels, const int32_t *dc, uint64_t g, uint32_t q,
-                                            const float *Qf, float *blk) {
-    const int4 *src = reinterpret_cast<const int4 *>(levels);
+__device__ __forceinline__ float stage_rows(const BlockRows &b, uint32_t q, const float *Qf, float *blk) {
     float l1 = 0.0f;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const int row = q + 4 * h;
-        const int4 v = src[row];
+        const int4 v = b.row[h];
         const int16_t *lv = reinterpret_cast<const int16_t *>(&v);
         const float4 qa = reinterpret_cast<const float4 *>(Qf + row * 8)[0];
         const float4 qb = reinterpret_cast<const float4 *>(Qf + row * 8)[1];
@@ -139,7 +152,7 @@ __device__ __forceinline__ float stage_rows(const int16_t *levels, const int32_t
         float f[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) f[j] = (float)lv[j] * qv[j];
-        if (row == 0) f[0] = (float)dc[g];
+        if (row == 0) f[0] = (float)b.dc;
 #pragma unroll
         for (int j = 0; j < 8; j++) l1 += fabsf(f[j]);
         reinterpret_cast<float4 *>(blk + row * 8)[0] = make_float4(f[0], f[1], f[2], f[3]);
@@ -148,36 +161,23 @@ __device__ __forceinline__ float stage_rows(const int16_t *levels, const int32_t
     return l1;
 }
 
-// Sample of an fp32 transform value. Rounding it provably equals rounding the
-// binary64 value when no half-integer lies within delta of acc, i.e. when acc
-// is closer than 0.5 - delta to its nearest integer (with delta >= 0.5 nothing
-// is certain); the exact pass settles the rest, ties included, so the rounding
-// mode's ties-to-even never decides a sample. Clamping after an agreed rounding
-// agrees.
+// Rounding an fp32 transform value provably equals rounding the binary64 value when no
+// half-integer lies within delta of acc, i.e. when acc is closer than near = 0.5 -
+// delta to its nearest integer (with delta >= 0.5 nothing is certain); the exact pass
+// settles the rest, ties included, so the rounding mode's ties-to-even never decides a
+// sample. Clamping after an agreed rounding agrees.
 //
 // round_nearest (rounding.h) avoids conversion instructions and is exact for
 // |acc| < 2^22. Larger values need no check of their own: |s| <= C1/4 and
 // |acc - s| <= delta give C1 > 2^24 for |acc| >= 2^22, so near < 0 and the
-// rounding is unsure already. A value that far beyond the clamp limits
-// (s + 128 > 255.5 or < -0.5 whatever the rounding; 129 and -130 leave room for
-// the fp32 rounding of the bounds) is decided by the clamp. Returns the
-// unclamped integer sample (+128), or one far outside 0..255 for a clamped one.
-__device__ __forceinline__ int32_t round_sample(float acc, float near, bool &unsure) {
-    float r;
-    const int32_t v = round_nearest(acc, r) + 128;
-    unsure = !(fabsf(acc - r) < near);
-    if (unsure) {
-        const float delta = 0.5f - near;
-        if (acc > 129.0f + delta) {
-            unsure = false;
-            return 1 << 20;
-        }
-        if (acc < -130.0f - delta) {
-            unsure = false;
-            return -(1 << 20);
-        }
-    }
-    return v;
+// rounding is unsure already.
+
+// A value so far beyond the clamp limits (s + 128 > 255.5 or < -0.5 whatever the
+// rounding; 129 and -130 leave room for the fp32 rounding of the bounds) is decided by
+// the clamp.
+__device__ __forceinline__ bool clamped(float acc, float near) {
+    const float delta = 0.5f - near;
+    return acc > 129.0f + delta || acc < -130.0f - delta;
 }
 
 // Two samples saturated to 0..255 in one instruction: a in byte 0, b in byte 1.
@@ -192,64 +192,69 @@ __device__ __forceinline__ uint32_t sat_pair_u8(int32_t a, int32_t b) {
 // split of the basis: M[7-x][u] = (-1)^u M[x][u] holds for the fp32 roundings of
 // the reference's literals (the literals themselves differ from exact symmetry by
 // < 2e-15, far inside the fp32 rounding), so
-//   s[x] = E + O, s[7-x] = E - O,  E = sum_{u even} M[x][u] c[u], O = sum_{u odd}.
+//   s[x] = E + O, s[7-x] = E - O,  E = sum_{u even} M[x][u] c[u], O = sum_{u odd},
+// E and O side by side in packed FMAs over the pairs (c[0], c[1]), (c[2], c[3]), ...
 // Per output this is 4 FMAs per half and one add: each pass's error is <= 5u of
 // the sum of |terms|, plus u for each rounded M and c, <= 13u B after both
 // passes (the bound above). |s| <= Mmax^2 C1 < C1/4, so the relative term
-// 2^-40 |s| of the bound is folded into 2^-42 C1.
+// 2^-40 |s| of the bound is folded into 2^-42 C1. One comparison of the largest distance
+// to an integer decides the eight outputs of a column, but for one in a hundred.
 // Returns the samples left to the exact pass as bits (row * 8 + column).
 __device__ __forceinline__ unsigned long long idct_block(const float *blk, uint32_t q, float c1, uint8_t *out,
                                                          int stride) {
-    float mq[8];
+    F2 mq[4];
 #pragma unroll
-    for (int u = 0; u < 8; u++) mq[u] = c_idct32[q * 8 + u];
-    float ta[8], tb[8];
+    for (int u = 0; u < 4; u++) mq[u] = f2(c_idct32[q * 8 + 2 * u], c_idct32[q * 8 + 2 * u + 1]);
+    float t[2][8];  // columns q and 7 - q
 #pragma unroll
     for (int v = 0; v < 8; v++) {
         const float4 c0 = reinterpret_cast<const float4 *>(blk + v * 8)[0];
         const float4 c1v = reinterpret_cast<const float4 *>(blk + v * 8)[1];
-        float e = c0.x * mq[0];
-        e = fmaf(mq[2], c0.z, e);
-        e = fmaf(mq[4], c1v.x, e);
-        e = fmaf(mq[6], c1v.z, e);
-        float o = c0.y * mq[1];
-        o = fmaf(mq[3], c0.w, o);
-        o = fmaf(mq[5], c1v.y, o);
-        o = fmaf(mq[7], c1v.w, o);
-        ta[v] = e + o;
-        tb[v] = e - o;
+        F2 s = mul2(f2(c0.x, c0.y), mq[0]);
+        s = fma2(f2(c0.z, c0.w), mq[1], s);
+        s = fma2(f2(c1v.x, c1v.y), mq[2], s);
+        s = fma2(f2(c1v.z, c1v.w), mq[3], s);
+        float e, o;
+        split2(s, e, o);
+        t[0][v] = e + o;
+        t[1][v] = e - o;
     }
     // delta = 2^-22 C1 >= 13u Mmax^2 C1 (margin 1.28), see the bound above
     const float near = 0.5f - (c1 * (0x1p-22f + 0x1p-42f) + 0x1p-30f);
-    uint32_t bits = 0;  // bit 2*row (column q), 2*row+1 (column 7-q)
-#pragma unroll
-    for (int y = 0; y < 4; y++) {
-#pragma unroll
-        for (int side = 0; side < 2; side++) {
-            const float *t = side ? tb : ta;
-            float e = t[0] * c_idct32[y * 8 + 0];
-            e = fmaf(c_idct32[y * 8 + 2], t[2], e);
-            e = fmaf(c_idct32[y * 8 + 4], t[4], e);
-            e = fmaf(c_idct32[y * 8 + 6], t[6], e);
-            float o = t[1] * c_idct32[y * 8 + 1];
-            o = fmaf(c_idct32[y * 8 + 3], t[3], o);
-            o = fmaf(c_idct32[y * 8 + 5], t[5], o);
-            o = fmaf(c_idct32[y * 8 + 7], t[7], o);
-            const uint32_t col = side ? 7 - q : q;
-            bool u0, u1;
-            const uint32_t pair = sat_pair_u8(round_sample(e + o, near, u0), round_sample(e - o, near, u1));
-            out[y * stride + col] = (uint8_t)pair;
-            out[(7 - y) * stride + col] = (uint8_t)(pair >> 8);
-            bits |= (u0 ? 1u : 0u) << (2 * y + side);
-            bits |= (u1 ? 1u : 0u) << (2 * (7 - y) + side);
-        }
-    }
     unsigned long long mask = 0;
-    if (bits) {
 #pragma unroll
-        for (int row = 0; row < 8; row++) {
-            if (bits & (1u << (2 * row))) mask |= 1ull << (row * 8 + q);
-            if (bits & (2u << (2 * row))) mask |= 1ull << (row * 8 + 7 - q);
+    for (int side = 0; side < 2; side++) {
+        float acc[8], far = 0.0f;
+#pragma unroll
+        for (int y = 0; y < 4; y++) {
+            const float *m = c_idct32 + y * 8;
+            F2 s = mul2(f2(t[side][0], t[side][1]), f2(m[0], m[1]));
+            s = fma2(f2(t[side][2], t[side][3]), f2(m[2], m[3]), s);
+            s = fma2(f2(t[side][4], t[side][5]), f2(m[4], m[5]), s);
+            s = fma2(f2(t[side][6], t[side][7]), f2(m[6], m[7]), s);
+            float e, o;
+            split2(s, e, o);
+            acc[y] = e + o;
+            acc[7 - y] = e - o;
+        }
+        const uint32_t col = side ? 7 - q : q;
+#pragma unroll
+        for (int y = 0; y < 8; y += 2) {
+            float r0, r1;
+            const int32_t n0 = round_nearest(acc[y], r0), n1 = round_nearest(acc[y + 1], r1);
+            far = fmaxf(far, fmaxf(fabsf(acc[y] - r0), fabsf(acc[y + 1] - r1)));
+            const uint32_t pair = sat_pair_u8(n0 + 128, n1 + 128);
+            out[y * stride + col] = (uint8_t)pair;
+            out[(y + 1) * stride + col] = (uint8_t)(pair >> 8);
+        }
+        if (far < near) continue;
+#pragma unroll
+        for (int y = 0; y < 8; y++) {
+            float r;
+            round_nearest(acc[y], r);
+            if (fabsf(acc[y] - r) < near) continue;
+            if (clamped(acc[y], near)) out[y * stride + col] = acc[y] > 0.0f ? 255 : 0;
+            else mask |= 1ull << (y * 8 + col);
         }
     }
     return mask;

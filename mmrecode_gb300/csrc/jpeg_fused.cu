@@ -36,9 +36,23 @@ struct FusedShape {
 };
 
 // MCUs per CTA of each launch slot (layout variant * 2 + wide): a narrow and a
-// wide strip per layout, picked per frame class by the autotuner (wide by default)
+// wide strip per layout, picked per frame class by the autotuner (narrow by default)
 __host__ __device__ constexpr int fused_slot_nm(int slot) {
     return slot == 0 ? 8 : slot == 1 ? 16 : slot == 2 || slot == 4 ? 4 : 8;
+}
+
+// Job of CTA `cta` (a warp: 32 entries of cta_first per step).
+__device__ __forceinline__ uint32_t job_of(const FusedLaunch &FL, uint32_t cta) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, n = FL.n_jobs;  // the job lies in [lo, lo + n)
+    while (n > 1) {
+        const uint32_t step = (n + 31) / 32, at = lo + lane * step;
+        const unsigned m = __ballot_sync(0xffffffffu, lane * step < n && FL.cta_first[at] <= cta);
+        const uint32_t k = 31 - __clz(m);  // (lane 0's entry is never past the CTA)
+        lo += k * step;
+        n = min(step, n - k * step);
+    }
+    return lo;
 }
 
 template <int HM, int VM, int NM>
@@ -52,84 +66,24 @@ struct FusedSmem {
     unsigned long long mask[Sh::NB];  // samples left to the exact pass, per block
     unsigned long long blk[Sh::NB];
     int32_t cx[Sh::THREADS / 32][64];  // per warp: exact coefficients of the block it settles
-    uint32_t n;
 };
 
-// Converts MCUs mx0 .. mx0+NM-1 of MCU row my of job J to RGB; undecided samples
-// are settled first, a warp per block (settle_samples).
+// The block thread group lb handles of a strip: MCU m of the strip, block i of the MCU.
 template <int HM, int VM, int NM>
-__device__ __forceinline__ void fused_tile(const JpegLaunch &L, const FusedLaunch &FL, uint32_t job, uint32_t my,
-                                           uint32_t mx0, FusedSmem<HM, VM, NM> &S) {
-    using Sh = FusedShape<HM, VM, NM>;
-    const FusedJob J = FL.jobs[job];
-    const JFrame &F = L.frames[J.frame];
-    const JComp *comps = L.comps + F.comp_off;
-    if (threadIdx.x == 0) S.n = 0;
-    for (uint32_t i = threadIdx.x; i < 3 * 64; i += blockDim.x)
-        S.q[i >> 6][i & 63] = (float)L.quant[F.quant_off + comps[i >> 6].q * 64 + (i & 63)];
-    const uint32_t nm = min((uint32_t)NM, F.mcu_cols - mx0);
-    const uint32_t lb = threadIdx.x >> 2, q = threadIdx.x & 3;
-    const uint32_t m = lb / Sh::BPM, i = lb % Sh::BPM;
-    const bool valid = lb < (uint32_t)Sh::NB && m < nm;
+__device__ __forceinline__ uint64_t strip_block(const JFrame &F, const JComp *comps, uint32_t my, uint32_t mx,
+                                                uint32_t i) {
     const uint32_t comp = i < HM * VM ? 0 : i - HM * VM + 1;
-    uint64_t g = 0;
-    if (valid) {
-        const JComp &C = comps[comp];
-        const uint32_t mx = mx0 + m;
-        if (comp == 0) g = F.blk_off + C.blk_base + (uint64_t)(my * VM + i / HM) * C.bw + mx * HM + i % HM;
-        else g = F.blk_off + C.blk_base + (uint64_t)my * C.bw + mx;
-        if (q == 0) S.blk[lb] = g;
-    }
-    __syncthreads();  // q, n
-    float *blk = S.f + lb * kFStride;
-    float l1 = valid ? stage_rows(L.coef + g * 64, L.dc, g, q, S.q[comp], blk) : 0.0f;
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-    __syncwarp();
-    unsigned long long mask = 0;
-    if (valid) {
-        uint8_t *out;
-        int stride;
-        if (comp == 0) {
-            out = S.y + (i / HM) * 8 * Sh::YW + (m * HM + i % HM) * 8;
-            stride = Sh::YW;
-        } else {
-            out = S.c[comp - 1] + m * 8;
-            stride = Sh::CW;
-        }
-        mask = idct_block(blk, q, l1, out, stride);
-    }
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) mask |= __shfl_xor_sync(0xffffffffu, mask, o);
-    if (q == 0 && lb < (uint32_t)Sh::NB) {
-        S.mask[lb] = mask;
-        if (mask) atomicAdd(&S.n, (uint32_t)__popcll(mask));
-    }
-    __syncthreads();
-    const uint32_t n_exact = S.n;
-    if (threadIdx.x == 0 && n_exact) atomicAdd(L.fix_count + 1, n_exact);
-    if (n_exact) {  // a warp per block with undecided samples (settle_samples)
-        const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
-        int32_t *cx = S.cx[w];
-        for (uint32_t b = w; b < (uint32_t)Sh::NB; b += nw) {
-            const unsigned long long bits = S.mask[b];
-            if (!bits) continue;
-            const uint32_t bm = b / Sh::BPM, bi = b % Sh::BPM;
-            const uint32_t bc = bi < HM * VM ? 0 : bi - HM * VM + 1;
-            const uint64_t bg = S.blk[b];
-            const uint16_t *Q = L.quant + F.quant_off + comps[bc].q * 64;
-            const int16_t *lv = L.coef + bg * 64;
-            cx[lane] = lane == 0 ? L.dc[bg] : (int32_t)lv[lane] * (int32_t)Q[lane];
-            cx[lane + 32] = (int32_t)lv[lane + 32] * (int32_t)Q[lane + 32];
-            __syncwarp();
-            settle_samples(L.fixw, cx, bits, [&](int y, int x, uint8_t smp) {
-                if (bc == 0) S.y[((bi / HM) * 8 + y) * Sh::YW + (bm * HM + bi % HM) * 8 + x] = smp;
-                else S.c[bc - 1][y * Sh::CW + bm * 8 + x] = smp;
-            });
-            __syncwarp();
-        }
-    }
-    __syncthreads();
+    const JComp &C = comps[comp];
+    if (comp == 0) return F.blk_off + C.blk_base + (uint64_t)(my * VM + i / HM) * C.bw + mx * HM + i % HM;
+    return F.blk_off + C.blk_base + (uint64_t)my * C.bw + mx;
+}
+
+// Converts the staged MCUs mx0 .. mx0+NM-1 of MCU row my to RGB.
+template <int HM, int VM, int NM>
+__device__ __forceinline__ void strip_to_rgb(const JFrame &F, const FusedJob &J, uint32_t my, uint32_t mx0,
+                                             FusedSmem<HM, VM, NM> &S) {
+    using Sh = FusedShape<HM, VM, NM>;
+    const uint32_t nm = min((uint32_t)NM, F.mcu_cols - mx0);
     // colour conversion (terminal_preview.rs:7308-7330, full range). When every row
     // starts 16-byte aligned (width a multiple of 16, aligned output; x0 is a
     // multiple of 64 pixels) a thread converts 16 pixels from one 16-byte luma
@@ -228,26 +182,85 @@ __device__ __forceinline__ void fused_tile(const JpegLaunch &L, const FusedLaunc
     }
 }
 
-// Main pass: a CTA per strip of MCUs.
+// A CTA takes J.strips consecutive strips of an MCU row: it reads the job's and the
+// frame's records once for them (one strip per CTA took 7.33 ms for a step of 300 1080p
+// frames, eight 6.57). The time goes to shared memory (two thirds of its wavefronts) and
+// to waits at the barriers, so strips are narrow and the kernel keeps to 64 registers
+// (levels loaded a strip ahead, or 80 registers: 7.46 and 7.11 ms against 6.76 with four
+// wide strips). Undecided samples are settled before the colour conversion, a warp per
+// block (settle_samples).
 template <int HM, int VM, int NM>
-__global__ void __launch_bounds__(FusedShape<HM, VM, NM>::THREADS) idct_rgb_kernel(JpegLaunch L, FusedLaunch FL) {
+__global__ void __launch_bounds__(FusedShape<HM, VM, NM>::THREADS, 1024 / FusedShape<HM, VM, NM>::THREADS) idct_rgb_kernel(JpegLaunch L, FusedLaunch FL) {
+    using Sh = FusedShape<HM, VM, NM>;
     __shared__ __align__(16) FusedSmem<HM, VM, NM> S;
     __shared__ uint32_t s_job;
-    if (threadIdx.x == 0) {
-        uint32_t lo = 0, hi = FL.n_jobs;
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (FL.cta_first[mid] <= blockIdx.x) lo = mid;
-            else hi = mid;
-        }
-        s_job = lo;
-    }
+    if (threadIdx.x < 32) s_job = job_of(FL, blockIdx.x);
     __syncthreads();
-    const uint32_t job = s_job;
-    const FusedJob &J = FL.jobs[job];
-    if (!L.item_ok[L.frames[J.frame].item]) return;
-    const uint32_t strip = blockIdx.x - FL.cta_first[job];
-    fused_tile<HM, VM, NM>(L, FL, job, strip / J.strips_x, (strip % J.strips_x) * NM, S);
+    const FusedJob J = FL.jobs[s_job];
+    const JFrame &F = L.frames[J.frame];
+    if (!L.item_ok[F.item]) return;
+    const JComp *comps = L.comps + F.comp_off;
+    const uint32_t group = blockIdx.x - FL.cta_first[s_job];
+    const uint32_t my = group / J.groups_x;
+    const uint32_t mcu_cols = F.mcu_cols;
+    uint32_t mx0 = (group - my * J.groups_x) * J.strips * NM;
+    const uint32_t mx_end = min(mx0 + J.strips * NM, mcu_cols);
+    for (uint32_t i = threadIdx.x; i < 3 * 64; i += blockDim.x)
+        S.q[i >> 6][i & 63] = (float)L.quant[F.quant_off + comps[i >> 6].q * 64 + (i & 63)];
+    const uint32_t lb = threadIdx.x >> 2, q = threadIdx.x & 3;
+    const uint32_t m = lb / Sh::BPM, i = lb % Sh::BPM;
+    const bool mine = lb < (uint32_t)Sh::NB;
+    const uint32_t comp = i < HM * VM ? 0 : i - HM * VM + 1;
+    // a strip further is as many blocks further in every component
+    const uint64_t step = comp == 0 ? NM * HM : NM;
+    uint64_t g = mine && mx0 + m < mx_end ? strip_block<HM, VM, NM>(F, comps, my, mx0 + m, i) : 0;
+    float *blk = S.f + lb * kFStride;
+    uint8_t *out = comp == 0 ? S.y + (i / HM) * 8 * Sh::YW + (m * HM + i % HM) * 8 : S.c[comp - 1] + m * 8;
+    const int stride = comp == 0 ? Sh::YW : Sh::CW;
+    __syncthreads();  // q
+    for (; mx0 < mx_end; mx0 += NM, g += step) {
+        const bool valid = mine && mx0 + m < mx_end;
+        float l1 = valid ? stage_rows(load_rows(L.coef + g * 64, L.dc, g, q), q, S.q[comp], blk) : 0.0f;
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+        __syncwarp();
+        unsigned long long mask = 0;
+        if (valid) mask = idct_block(blk, q, l1, out, stride);
+        if (__syncthreads_or(mask != 0)) {
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) mask |= __shfl_xor_sync(0xffffffffu, mask, o);
+            if (q == 0 && mine) {
+                S.mask[lb] = mask;
+                S.blk[lb] = g;
+            }
+            __syncthreads();
+            const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+            int32_t *cx = S.cx[w];
+            uint32_t n = 0;
+            for (uint32_t b = w; b < (uint32_t)Sh::NB; b += nw) {
+                const unsigned long long bits = S.mask[b];
+                if (!bits) continue;
+                n += (uint32_t)__popcll(bits);
+                const uint32_t bm = b / Sh::BPM, bi = b % Sh::BPM;
+                const uint32_t bc = bi < HM * VM ? 0 : bi - HM * VM + 1;
+                const uint64_t bg = S.blk[b];
+                const uint16_t *Q = L.quant + F.quant_off + comps[bc].q * 64;
+                const int16_t *lv = L.coef + bg * 64;
+                cx[lane] = lane == 0 ? L.dc[bg] : (int32_t)lv[lane] * (int32_t)Q[lane];
+                cx[lane + 32] = (int32_t)lv[lane + 32] * (int32_t)Q[lane + 32];
+                __syncwarp();
+                settle_samples(L.fixw, cx, bits, [&](int y, int x, uint8_t smp) {
+                    if (bc == 0) S.y[((bi / HM) * 8 + y) * Sh::YW + (bm * HM + bi % HM) * 8 + x] = smp;
+                    else S.c[bc - 1][y * Sh::CW + bm * 8 + x] = smp;
+                });
+                __syncwarp();
+            }
+            if (lane == 0 && n) atomicAdd(L.fix_count + 1, n);
+            __syncthreads();
+        }
+        strip_to_rgb<HM, VM, NM>(F, J, my, mx0, S);
+        if (mx0 + NM < mx_end) __syncthreads();  // (uniform) the tile is read
+    }
 }
 
 }  // namespace
@@ -263,8 +276,8 @@ int fused_slot(int variant, bool wide) { return variant < 0 ? -1 : 2 * variant +
 
 uint32_t fused_slot_mcus(int slot) { return (uint32_t)fused_slot_nm(slot); }
 
-uint32_t fused_strips_x(int slot, uint32_t mcu_cols) {
-    const uint32_t nm = fused_slot_mcus(slot);
+uint32_t fused_groups_x(int slot, uint32_t mcu_cols, uint32_t strips) {
+    const uint32_t nm = fused_slot_mcus(slot) * strips;
     return (mcu_cols + nm - 1) / nm;
 }
 

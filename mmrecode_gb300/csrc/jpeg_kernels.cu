@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kIdctThreads, 4) idct_kernel(JpegLaunch L) {
     const bool valid = local < nblk;
     const uint64_t g = R.first + local;
     float *blk = s_f + lb * kIdctStride;
-    float l1 = valid ? stage_rows(L.coef + g * 64, L.dc, g, q, s_q, blk) : 0.0f;
+    float l1 = valid ? stage_rows(load_rows(L.coef + g * 64, L.dc, g, q), q, s_q, blk) : 0.0f;
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
     __syncwarp();

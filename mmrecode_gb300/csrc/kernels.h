@@ -77,14 +77,15 @@ uint32_t idct_ctas(uint32_t blocks);
 // 1x1, 2x1 or 2x2): one launch per layout, a CTA per strip of MCUs.
 struct FusedJob {
     uint32_t frame;     // JFrame index
-    uint32_t strips_x;  // strips per MCU row
+    uint32_t groups_x;  // CTAs per MCU row
+    uint32_t strips;    // strips per CTA
     uint32_t width, height;
     uint8_t *out;       // width * height * 3 bytes
 };
 
 struct FusedLaunch {
     const FusedJob *jobs;
-    const uint32_t *cta_first;  // n_jobs + 1 prefix of CTAs (strips_x * mcu_rows per job)
+    const uint32_t *cta_first;  // n_jobs + 1 prefix of CTAs (groups_x * mcu_rows per job)
     uint32_t n_jobs;
     uint32_t n_ctas;
 };
@@ -95,7 +96,7 @@ int fused_variant(uint32_t hmax, uint32_t vmax);  // 0: 1x1, 1: 2x1, 2: 2x2, -1:
 constexpr int kFusedSlots = 6;
 int fused_slot(int variant, bool wide);
 uint32_t fused_slot_mcus(int slot);
-uint32_t fused_strips_x(int slot, uint32_t mcu_cols);
+uint32_t fused_groups_x(int slot, uint32_t mcu_cols, uint32_t strips);
 void launch_jpeg_idct_rgb(const JpegLaunch &L, const FusedLaunch *FL, cudaStream_t s);  // FL[kFusedSlots]
 int fused_launches(const FusedLaunch &FL);
 

@@ -28,9 +28,9 @@ __device__ __forceinline__ F2 fma2(const F2 &a, const F2 &b, const F2 &c) {
     return r;
 }
 
-__device__ __forceinline__ F2 add2(const F2 &a, const F2 &b) {
+__device__ __forceinline__ F2 mul2(const F2 &a, const F2 &b) {
     F2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
     return r;
 }
 
