@@ -26,6 +26,8 @@ namespace {
 
 const int kZigzag[64] = MMR_ZIGZAG_INIT;
 
+constexpr size_t kBounceBytes = 8u << 20;
+
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct CudaError : std::runtime_error {
@@ -642,10 +644,10 @@ Probe probe_packet(uint32_t codec, const uint8_t *data, size_t len) {
 struct Engine::Impl {
     DevBuf d_in, d_tok, d_blob, d_tile_tok, d_tile_rst, d_rsts, d_results, d_coef, d_dc, d_planes, d_out, d_dvcoef,
         d_modes, d_segerr, d_vlc, d_fix, d_slot_item, d_ivs, d_sync, d_spec, d_prefix, d_events, d_ivkey,
-        d_ivpend,
+        d_ivpend, d_skip,
         d_place,   // DV block placement (dv_layout.h)
         d_fixtab;  // fixed-point transform weights: MJPEG, DV 8-8, DV 2-4-8 (exact_fixed.h)
-    PinBuf h_blob, h_back;
+    PinBuf h_blob, h_back, h_out;
     std::vector<uint32_t> vlc;
     // stage boundaries: start, uploads, scan, entropy, idct, dv, rgb, end
     cudaEvent_t ev[8] = {};
@@ -782,8 +784,10 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         std::vector<JComp> comps;
         std::vector<HuffLut> luts;
         std::vector<uint16_t> lut_sym;  // the chunked decoder's lookups of the same tables
-        std::vector<uint32_t> lut_skip;
         std::vector<LutMeta> lut_meta;
+        std::vector<HuffCanon> canon;
+        bool many_comps = false;  // a frame of more than four components: the interval decoder's lookups too
+        for (const JPlan &p : jplans) many_comps |= p.decode && p.ncomp > 4;
         std::vector<uint8_t> symbols;
         std::vector<uint16_t> quant;
         std::vector<uint2> items_small, items_big;
@@ -895,12 +899,15 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                     key.push_back(s >= 4);  // DC and AC lookups differ for the same code table
                     auto f = lut_index.find(key);
                     if (f == lut_index.end()) {
-                        HuffLut L;
-                        build_lut(key.data(), key.size() - 1, (uint32_t)symbols.size(), s >= 4, &L);
+                        canon.emplace_back();
+                        build_canon(key.data(), (uint32_t)symbols.size(), &canon.back());
+                        if (many_comps) {
+                            luts.emplace_back();
+                            build_lut(key.data(), key.size() - 1, (uint32_t)symbols.size(), s >= 4, &luts.back());
+                        }
                         symbols.insert(symbols.end(), key.begin() + 16, key.end() - 1);
-                        f = lut_index.emplace(key, (uint32_t)luts.size()).first;
-                        luts.push_back(L);
-                        lut_meta.push_back(build_sym(key.data(), key.size() - 1, s >= 4, &lut_sym, &lut_skip));
+                        f = lut_index.emplace(key, (uint32_t)lut_meta.size()).first;
+                        lut_meta.push_back(build_sym(key.data(), key.size() - 1, s >= 4, &lut_sym));
                     }
                     F.lut[s] = f->second;
                 }
@@ -1144,6 +1151,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         I.d_ivs.ensure(std::max<size_t>(items_small.size() * sizeof(IvInfo), 256));
         I.d_ivkey.ensure(std::max<size_t>(items_small.size() * 8, 256));
         if (blocks > 0xffffffffull) throw std::runtime_error("batch too large for the chunked entropy decoder");
+        I.d_skip.ensure(std::max<size_t>(lut_sym.size() * 4, 256));
         I.d_ivpend.ensure(std::max<size_t>(items_small.size() * 4, 256));
 
         uint8_t *d_in = I.d_in.as<uint8_t>();
@@ -1172,14 +1180,21 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             for (auto &J : list) J.out = out_ptr(jframes[J.frame].item);
 
         // ------------------------------------------------------ plan blob
-        size_t o_jframes = blob.add_vec(jframes), o_jstates = blob.add_vec(jstates),
-               o_tile_first = blob.add_vec(tile_first), o_sched = blob.add_vec(sched), o_brec = blob.add_vec(brecs), o_comps = blob.add_vec(comps),
+        // what the kernels write and the host reads back comes first, in one piece:
+        // frame states, item flags, and counters (fixup entries, exact samples, slices
+        // decoded again, slices, unused, slices decoded again whole)
+        uint32_t zero_counters[8] = {};
+        const size_t o_jstates = blob.add_vec(jstates), o_dstates = blob.add_vec(dstates),
+                     o_itemok = blob.add_vec(item_ok), o_fixcount = blob.add(zero_counters, sizeof(zero_counters)),
+                     back_blob = blob.bytes.size();
+        size_t o_jframes = blob.add_vec(jframes), o_tile_first = blob.add_vec(tile_first),
+               o_sched = blob.add_vec(sched), o_brec = blob.add_vec(brecs), o_comps = blob.add_vec(comps),
                o_luts = blob.add_vec(luts), o_symbols = blob.add_vec(symbols), o_quant = blob.add_vec(quant);
-        size_t o_sym = blob.add_vec(lut_sym), o_skip = blob.add_vec(lut_skip), o_meta = blob.add_vec(lut_meta);
+        size_t o_sym = blob.add_vec(lut_sym), o_meta = blob.add_vec(lut_meta), o_canon = blob.add_vec(canon);
         std::vector<uint2> all_items(items_small);
         all_items.insert(all_items.end(), items_big.begin(), items_big.end());
-        size_t o_items = blob.add_vec(all_items), o_ranges = blob.add_vec(ranges), o_idctcta = blob.add_vec(idct_cta), o_itemok = blob.add_vec(item_ok),
-               o_dframes = blob.add_vec(dframes), o_dstates = blob.add_vec(dstates), o_segfirst = blob.add_vec(seg_first),
+        size_t o_items = blob.add_vec(all_items), o_ranges = blob.add_vec(ranges), o_idctcta = blob.add_vec(idct_cta),
+               o_dframes = blob.add_vec(dframes), o_segfirst = blob.add_vec(seg_first),
                o_rgbjobs = blob.add_vec(rgbjobs),
                o_rgbcta = blob.add_vec(rgbcta);
         size_t o_fjobs[kFusedSlots], o_fcta[kFusedSlots];
@@ -1188,10 +1203,6 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             o_fcta[v] = blob.add_vec(fcta[v]);
         }
 
-        // fixup entries, exact samples, slices decoded again, slices, unused, slices decoded
-        // again whole
-        uint32_t zero_counters[8] = {};
-        size_t o_fixcount = blob.add(zero_counters, sizeof(zero_counters));
         uint32_t zero_left[4] = {};  // unsettled intervals
         size_t o_left = blob.add(zero_left, sizeof(zero_left));
         size_t blob_size = std::max<size_t>(blob.bytes.size(), 256);
@@ -1200,26 +1211,35 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         memcpy(I.h_blob.ptr, blob.bytes.data(), blob.bytes.size());
         uint8_t *db = I.d_blob.as<uint8_t>();
 
-        // read-back layout (states, item flags, DV segment errors, exact-sample count)
-        size_t back_j = jstates.size() * sizeof(JState), back_d = dstates.size() * sizeof(DvState);
-        size_t back_ok = n * 4, back_seg = seg_first.back();
-        size_t o_b1 = 0, o_b2 = align_up(back_j, 16), o_b3 = align_up(o_b2 + back_d, 16),
-               o_b4 = align_up(o_b3 + back_ok, 16), o_b5 = align_up(o_b4 + back_seg, 16);
-        I.h_back.ensure(std::max<size_t>(o_b5 + 20, 256));
+        // read-back layout: the blob's first part, DV segment errors
+        const size_t back_seg = seg_first.back(), o_backseg = align_up(back_blob, 16);
+        I.h_back.ensure(std::max<size_t>(o_backseg + back_seg, 256));
         uint8_t *hb = reinterpret_cast<uint8_t *>(I.h_back.ptr);
+
+        // Small planes for ordinary host memory come down in one piece through pinned
+        // memory (three pageable copies: 209 us for a 320x240 frame against 196).
+        bool bounce = out_bytes > 0 && out_bytes <= kBounceBytes;
+        for (size_t i = 0; i < n; i++)
+            if (items[i].status == kOk && !items[i].out_on_device && items[i].out_bytes)
+                bounce &= items[i].plane_out[0] && items[i].output == kOutPlanar;
+        if (bounce) I.h_out.ensure(out_bytes);
 
         // ------------------------------------------------------- launches
         cudaStream_t s = stream_;
         bool capturing = false;  // timing events become external graph nodes under capture
+        const bool timed = times != nullptr;
+        auto stamp = [&](cudaEvent_t e) {
+            if (timed) MMR_CUDA(record_event(e, s, capturing));
+        };
         auto enqueue = [&]() {
-        MMR_CUDA(record_event(I.ev[0], s, capturing));
+        stamp(I.ev[0]);
         MMR_CUDA(cudaMemcpyAsync(db, I.h_blob.ptr, blob.bytes.size(), cudaMemcpyHostToDevice, s));
         for (size_t i = 0; i < n; i++) {
             bool planned = items[i].status == kOk && (items[i].codec == kCodecMjpeg || items[i].codec == kCodecDv);
             if (planned && !items[i].dev_data && items[i].len)
                 MMR_CUDA(cudaMemcpyAsync(d_in + in_off[i], items[i].data, items[i].len, cudaMemcpyHostToDevice, s));
         }
-        MMR_CUDA(record_event(I.ev[1], s, capturing));
+        stamp(I.ev[1]);
 
         JpegLaunch JL;
         memset(&JL, 0, sizeof(JL));
@@ -1235,7 +1255,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         JL.brec = reinterpret_cast<const JBlockRec *>(db + o_brec);
         JL.comps = reinterpret_cast<const JComp *>(db + o_comps);
         JL.luts = reinterpret_cast<const HuffLut *>(db + o_luts);
-        JL.n_luts = (uint32_t)luts.size();
+        JL.n_luts = (uint32_t)lut_meta.size();
         JL.symbols = db + o_symbols;
         JL.quant = reinterpret_cast<const uint16_t *>(db + o_quant);
         JL.items = reinterpret_cast<const uint2 *>(db + o_items);
@@ -1266,14 +1286,15 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         JL.sync_left = reinterpret_cast<uint32_t *>(db + o_left);
         JL.lut_meta = reinterpret_cast<const LutMeta *>(db + o_meta);
         JL.sym = reinterpret_cast<const uint16_t *>(db + o_sym);
-        JL.skip = reinterpret_cast<const uint32_t *>(db + o_skip);
+        JL.skip = I.d_skip.as<uint32_t>();
+        JL.canon = reinterpret_cast<const HuffCanon *>(db + o_canon);
         JL.fixw = I.d_fixtab.as<long long>();
         if (!jframes.empty()) {
             launch_jpeg_scan(JL, s);
-            MMR_CUDA(record_event(I.ev[2], s, capturing));
-            launch_jpeg_slices(JL, s, I.marks, capturing);
+            stamp(I.ev[2]);
+            launch_jpeg_slices(JL, s, timed ? I.marks : nullptr, capturing);
             launch_jpeg_entropy(JL, s);
-            MMR_CUDA(record_event(I.ev[3], s, capturing));
+            stamp(I.ev[3]);
             launch_jpeg_idct(JL, s);
             FusedLaunch FL[kFusedSlots];
             for (int v = 0; v < kFusedSlots; v++) {
@@ -1287,10 +1308,10 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             launches_ += (JL.n_tiles ? 3 : 0) + (JL.n_slots ? jpeg_slice_launches(JL) : 0) +
                          (n_items > JL.n_items_small ? 1 : 0) + 1 + (JL.n_idct_ctas ? 2 : 0);
         } else {
-            MMR_CUDA(record_event(I.ev[2], s, capturing));
-            MMR_CUDA(record_event(I.ev[3], s, capturing));
+            stamp(I.ev[2]);
+            stamp(I.ev[3]);
         }
-        MMR_CUDA(record_event(I.ev[4], s, capturing));
+        stamp(I.ev[4]);
         DvLaunch DL;
         memset(&DL, 0, sizeof(DL));
         DL.frames = reinterpret_cast<const DvFrame *>(db + o_dframes);
@@ -1309,11 +1330,11 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         DL.item_ok = JL.item_ok;
         if (!dframes.empty()) {
             launch_dv_decode(DL, s);
-            MMR_CUDA(record_event(I.dv_mark, s, capturing));
+            stamp(I.dv_mark);
             launch_dv_idct(DL, s);
             launches_ += 3;
         }
-        MMR_CUDA(record_event(I.ev[5], s, capturing));
+        stamp(I.ev[5]);
         RgbLaunch RL;
         RL.jobs = reinterpret_cast<const RgbJob *>(db + o_rgbjobs);
         RL.cta_first = reinterpret_cast<const uint32_t *>(db + o_rgbcta);
@@ -1324,16 +1345,14 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             launch_rgb(RL, s);
             launches_ += 1;
         }
-        MMR_CUDA(record_event(I.ev[6], s, capturing));
+        stamp(I.ev[6]);
         MMR_CUDA(cudaGetLastError());
 
         // ------------------------------------------------------- read-back
-        if (back_j) MMR_CUDA(cudaMemcpyAsync(hb + o_b1, db + o_jstates, back_j, cudaMemcpyDeviceToHost, s));
-        if (back_d) MMR_CUDA(cudaMemcpyAsync(hb + o_b2, db + o_dstates, back_d, cudaMemcpyDeviceToHost, s));
-        if (back_ok) MMR_CUDA(cudaMemcpyAsync(hb + o_b3, db + o_itemok, back_ok, cudaMemcpyDeviceToHost, s));
-        if (back_seg) MMR_CUDA(cudaMemcpyAsync(hb + o_b4, I.d_segerr.ptr, back_seg, cudaMemcpyDeviceToHost, s));
-        MMR_CUDA(cudaMemcpyAsync(hb + o_b5, db + o_fixcount + 4, 20, cudaMemcpyDeviceToHost, s));
-        for (size_t i = 0; i < n; i++) {
+        MMR_CUDA(cudaMemcpyAsync(hb, db, back_blob, cudaMemcpyDeviceToHost, s));
+        if (back_seg) MMR_CUDA(cudaMemcpyAsync(hb + o_backseg, I.d_segerr.ptr, back_seg, cudaMemcpyDeviceToHost, s));
+        if (bounce) MMR_CUDA(cudaMemcpyAsync(I.h_out.ptr, I.d_out.ptr, out_bytes, cudaMemcpyDeviceToHost, s));
+        for (size_t i = 0; i < n && !bounce; i++) {
             Item &it = items[i];
             if (it.status != kOk || it.out_on_device || !it.out_bytes) continue;
             const uint8_t *src = I.d_out.as<uint8_t>() + out_off[i];
@@ -1346,7 +1365,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                 MMR_CUDA(cudaMemcpyAsync(it.out, src, it.out_bytes, cudaMemcpyDeviceToHost, s));
             }
         }
-        MMR_CUDA(record_event(I.ev[7], s, capturing));
+        stamp(I.ev[7]);
         };
         // A batch identical to the previous one (same plan image, buffers and
         // caller pointers) is captured into a CUDA graph on its second occurrence
@@ -1359,11 +1378,11 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                                                           (items[i].out_on_device || !items[i].out_bytes));
         const bool use_graphs = graphs_ && device_resident;
         if (use_graphs) {
-            key = {n, (uintptr_t)I.h_blob.ptr, (uintptr_t)I.h_back.ptr, blob.bytes.size()};
+            key = {n, (uintptr_t)I.h_blob.ptr, (uintptr_t)I.h_back.ptr, blob.bytes.size(), (uintptr_t)timed};
             // the launch shapes (every grid size and per-kernel count the enqueue
             // derives); the plan image compared below holds them too, but the key
             // states them so that no change of shape can replay a stale graph
-            for (uintptr_t v : {(uintptr_t)jframes.size(), (uintptr_t)tile_first.back(), (uintptr_t)luts.size(),
+            for (uintptr_t v : {(uintptr_t)jframes.size(), (uintptr_t)tile_first.back(), (uintptr_t)luts.size(), (uintptr_t)lut_meta.size(),
                                 (uintptr_t)items_small.size(), (uintptr_t)n_items, (uintptr_t)ranges.size(),
                                 (uintptr_t)idct_cta.back(), (uintptr_t)n_slots, (uintptr_t)most_paths,
                                 (uintptr_t)blocks, (uintptr_t)dframes.size(), (uintptr_t)seg_first.back(),
@@ -1377,7 +1396,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             for (const DevBuf *b : {&I.d_in, &I.d_tok, &I.d_blob, &I.d_tile_tok, &I.d_tile_rst, &I.d_rsts,
                                     &I.d_results, &I.d_coef, &I.d_dc, &I.d_planes, &I.d_out, &I.d_dvcoef, &I.d_modes,
                                     &I.d_segerr, &I.d_vlc, &I.d_fix, &I.d_slot_item, &I.d_ivs, &I.d_sync,
-                                    &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_ivpend})
+                                    &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_ivpend, &I.d_skip})
                 key.push_back((uintptr_t)b->ptr);
             for (size_t i = 0; i < n; i++) {
                 const Item &it = items[i];
@@ -1442,6 +1461,14 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             }
         }
         MMR_CUDA(cudaStreamSynchronize(s));
+        for (size_t i = 0; i < n && bounce; i++) {
+            const Item &it = items[i];
+            if (it.status != kOk || it.out_on_device || !it.out_bytes) continue;
+            const uint8_t *src = static_cast<const uint8_t *>(I.h_out.ptr) + out_off[i];
+            for (int c = 0; c < 3; c++)
+                if (it.plane_out[c] && plane_geom[i][2 * c + 1])
+                    memcpy(it.plane_out[c], src + plane_geom[i][2 * c], plane_geom[i][2 * c + 1]);
+        }
         if (times) {
             float *dst[8] = {nullptr, &times->upload_ms, &times->scan_ms, &times->entropy_ms, &times->idct_ms,
                              &times->dv_ms, &times->rgb_ms, &times->download_ms};
@@ -1462,10 +1489,10 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             }
             times->jpeg_blocks = blocks;
             times->graph_replays = graph_replayed_ ? 1 : 0;
-            times->idct_exact_samples = *reinterpret_cast<const uint32_t *>(hb + o_b5);
-            times->slices_redone = *reinterpret_cast<const uint32_t *>(hb + o_b5 + 4);
-            times->slices = *reinterpret_cast<const uint32_t *>(hb + o_b5 + 8);
-            times->slices_redone_whole = *reinterpret_cast<const uint32_t *>(hb + o_b5 + 16);
+            times->idct_exact_samples = *reinterpret_cast<const uint32_t *>(hb + o_fixcount + 4);
+            times->slices_redone = *reinterpret_cast<const uint32_t *>(hb + o_fixcount + 8);
+            times->slices = *reinterpret_cast<const uint32_t *>(hb + o_fixcount + 12);
+            times->slices_redone_whole = *reinterpret_cast<const uint32_t *>(hb + o_fixcount + 20);
             times->dv_blocks = dv_blocks;
             times->rgb_pixels = rgbfirst.back();
             times->input_bytes = 0;
@@ -1475,9 +1502,9 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                 times->output_bytes += items[i].out_bytes;
             }
         }
-        const JState *hj = reinterpret_cast<const JState *>(hb + o_b1);
-        const DvState *hd = reinterpret_cast<const DvState *>(hb + o_b2);
-        const uint8_t *hseg = hb + o_b4;
+        const JState *hj = reinterpret_cast<const JState *>(hb + o_jstates);
+        const DvState *hd = reinterpret_cast<const DvState *>(hb + o_dstates);
+        const uint8_t *hseg = hb + o_backseg;
 
         // ------------------------------------------------ status resolution
         for (size_t k = 0; k < jplans.size(); k++) {

@@ -57,7 +57,8 @@ __device__ __forceinline__ void take(Bits &r, int n) {
 
 // Code length of the next Huffman code (entropy.rs:57-70), 0 when none of
 // length <= 16 matches; *sym its symbol.
-__device__ __forceinline__ int slow_symbol(const HuffLut *__restrict__ T, const uint8_t *__restrict__ symbols,
+template <class Canon>  // HuffCanon, or HuffLut with the same fields
+__device__ __forceinline__ int slow_symbol(const Canon *__restrict__ T, const uint8_t *__restrict__ symbols,
                                            uint64_t buf, uint32_t *sym) {
     const uint32_t e = __ldg(&T->fast[buf >> 55]);
     if (e) {
@@ -84,29 +85,11 @@ constexpr uint16_t kBarrierErr = 0xffff;  // the symbol runs into the interval's
 // val: the DC difference or the AC level, 0 for EOB and ZRL, to be stored at
 // zigzag index k - 1 (a zero stored past the last level changes nothing). On
 // failure returns false with err (kBarrierErr when the symbol runs into the
-// barrier) and errbit, the reader position the reference reports.
-__device__ __forceinline__ bool decode_symbol(Bits &r, uint32_t avail, const HuffLut *__restrict__ T,
-                                              const uint8_t *__restrict__ symbols, int &k, int32_t &val,
-                                              uint16_t &err, uint32_t &errbit) {
-    refill(r);
-    const uint32_t fv = __ldg(&T->fastv[r.buf >> (64 - kHuffFastBits)]);
-    const uint32_t fl = fv & 31;
-    const int kn = (fv & kFastEob) ? 64 : k + (int)((fv >> 5) & 127);
-    if (fv & kFastCode) {  // code resolved, magnitude after it (receive_extend, entropy.rs:168-182)
-        const uint32_t size = (fv >> 16) & 15, total = fl + size;
-        if (total - 1u < avail && kn <= 64) {
-            const int32_t v = (int32_t)((r.buf << fl) >> (64 - size));
-            val = v < (1 << (size - 1)) ? v + 1 - (1 << size) : v;
-            take(r, (int)total);
-            k = kn;
-            return true;
-        }
-    } else if (fl - 1u < avail && kn <= 64) {
-        val = (int32_t)fv >> 16;
-        take(r, (int)fl);
-        k = kn;
-        return true;
-    }
+// barrier) and errbit, the reader position the reference reports. r is refilled.
+template <class Canon>
+__device__ __forceinline__ bool checked_symbol(Bits &r, uint32_t avail, const Canon *__restrict__ T,
+                                               const uint8_t *__restrict__ symbols, int &k, int32_t &val,
+                                               uint16_t &err, uint32_t &errbit) {
     uint32_t sym;
     const int l = slow_symbol(T, symbols, r.buf, &sym);
     if (l == 0 || (uint32_t)l > avail) {
@@ -174,6 +157,32 @@ __device__ __forceinline__ bool decode_symbol(Bits &r, uint32_t avail, const Huf
     val = v;
     k += run + 1;
     return true;
+}
+
+// The same with HuffLut's whole-symbol lookup first.
+__device__ __forceinline__ bool decode_symbol(Bits &r, uint32_t avail, const HuffLut *__restrict__ T,
+                                              const uint8_t *__restrict__ symbols, int &k, int32_t &val,
+                                              uint16_t &err, uint32_t &errbit) {
+    refill(r);
+    const uint32_t fv = __ldg(&T->fastv[r.buf >> (64 - kHuffFastBits)]);
+    const uint32_t fl = fv & 31;
+    const int kn = (fv & kFastEob) ? 64 : k + (int)((fv >> 5) & 127);
+    if (fv & kFastCode) {  // code resolved, magnitude after it (receive_extend, entropy.rs:168-182)
+        const uint32_t size = (fv >> 16) & 15, total = fl + size;
+        if (total - 1u < avail && kn <= 64) {
+            const int32_t v = (int32_t)((r.buf << fl) >> (64 - size));
+            val = v < (1 << (size - 1)) ? v + 1 - (1 << size) : v;
+            take(r, (int)total);
+            k = kn;
+            return true;
+        }
+    } else if (fl - 1u < avail && kn <= 64) {
+        val = (int32_t)fv >> 16;
+        take(r, (int)fl);
+        k = kn;
+        return true;
+    }
+    return checked_symbol(r, avail, T, symbols, k, val, err, errbit);
 }
 
 }  // namespace mmr

@@ -11,8 +11,29 @@
 
 namespace mmr {
 
-// key: 16 counts then the symbols; sym_off: the table's first symbol in the
-// batch's symbol pool; ac: an AC table (run/size symbols, EOB, ZRL) or a DC one.
+// key: 16 counts then the symbols; sym_off: the table's first symbol in the batch's
+// symbol pool.
+inline void build_canon(const uint8_t *key, uint32_t sym_off, HuffCanon *c) {
+    memset(c, 0, sizeof(*c));
+    for (int l = 0; l < 18; l++) c->maxcode[l] = -1;
+    uint32_t code = 0, k = 0;
+    for (int l = 1; l <= 16; l++, code <<= 1) {
+        const uint32_t n = key[l - 1];
+        if (n) {
+            c->valptr[l] = (int32_t)k - (int32_t)code;
+            c->maxcode[l] = (int32_t)(code + n - 1);
+        }
+        for (uint32_t i = 0; i < n; i++, code++, k++) {
+            if (l > 9) continue;
+            const uint32_t first = code << (9 - l), cnt = 1u << (9 - l);
+            for (uint32_t j = 0; j < cnt; j++)  // the first code of each 9-bit pattern wins
+                if (!c->fast[first + j]) c->fast[first + j] = (uint16_t)((l << 8) | key[16 + k]);
+        }
+    }
+    c->sym_off = sym_off;
+}
+
+// ac: an AC table (run/size symbols, EOB, ZRL) or a DC one.
 inline void build_lut(const uint8_t *key, size_t key_len, uint32_t sym_off, bool ac, HuffLut *lut) {
     memset(lut, 0, sizeof(*lut));
     for (int l = 0; l < 18; l++) lut->maxcode[l] = -1;
@@ -94,11 +115,9 @@ inline void build_lut(const uint8_t *key, size_t key_len, uint32_t sym_off, bool
     lut->nsym = (uint32_t)(key_len - 16);
 }
 
-// The chunked decoder's lookups of the same table (plan.h), appended to *sym and
-// *skip (which stay parallel; skip is filled for AC tables). The table is not
-// oversubscribed.
-inline LutMeta build_sym(const uint8_t *key, size_t key_len, bool ac, std::vector<uint16_t> *sym,
-                         std::vector<uint32_t> *skip) {
+// The chunked decoder's lookups of the same table (plan.h), appended to *sym. The table
+// is not oversubscribed.
+inline LutMeta build_sym(const uint8_t *key, size_t key_len, bool ac, std::vector<uint16_t> *sym) {
     constexpr uint32_t FB = kHuffFastBits;
     const uint8_t *symbols = key + 16;
     LutMeta m;
@@ -118,7 +137,6 @@ inline LutMeta build_sym(const uint8_t *key, size_t key_len, bool ac, std::vecto
         m.last = (uint32_t)end;
     m.len = (lut_entry_index(m.last, m.first_long) + 1 + 7) & ~7u;
     sym->resize(m.off + m.len, 0);
-    skip->resize(m.off + m.len, 0);
     uint16_t *e = sym->data() + m.off;
     uint32_t code = 0, k = 0;
     for (uint32_t l = 1; l <= 16; l++, code <<= 1) {
@@ -130,30 +148,17 @@ inline LutMeta build_sym(const uint8_t *key, size_t key_len, bool ac, std::vecto
                 if (run != 0 && run != 15) continue;
                 if (run == 0) adv = kSymEob;
             }
-            const uint32_t first = lut_entry_index(code << (32 - l), m.first_long);
-            const uint32_t n = l <= FB ? 1u << (FB - l) : 1u << (16 - l);
-            // (a long code's patterns may straddle an 11-bit prefix: one entry further each)
-            for (uint32_t j = 0; j < n; j++) {
-                const uint32_t at = l <= FB ? first + j : lut_entry_index((code << (32 - l)) + (j << 16), m.first_long);
-                if (at < m.len) e[at] = (uint16_t)(l | size << 5 | adv << 9);
+            const uint16_t entry = (uint16_t)(l | size << 5 | adv << 9);
+            if (l <= FB) {
+                const uint32_t first = code << (FB - l);
+                for (uint32_t j = first; j < first + (1u << (FB - l)) && j < m.len; j++) e[j] = entry;
+            } else {  // (its patterns may straddle an 11-bit prefix: one entry further there)
+                for (uint32_t j = 0; j < 1u << (16 - l); j++) {
+                    const uint32_t at = lut_entry_index((code << (32 - l)) + (j << 16), m.first_long);
+                    if (at < m.len) e[at] = entry;
+                }
             }
         }
-    }
-    if (!ac) return m;
-    uint32_t *p = skip->data() + m.off;
-    for (uint32_t x = 0; x < m.len; x++) {
-        if (!e[x]) continue;
-        const uint32_t cl = e[x] & 31, len = cl + ((e[x] >> 5) & 15), adv = e[x] >> 9;
-        uint32_t len2 = len, adv2 = adv;
-        // (windows below first_long have no long entries before theirs: x is the prefix)
-        if (cl <= FB && adv < kSymEob && len < FB) {
-            const uint32_t y = (x << len) & ((1u << FB) - 1);  // what is left of the 11 bits, then zeros
-            if ((uint64_t)y << (32 - FB) < m.first_long && e[y] && (e[y] & 31u) <= FB - len) {
-                len2 += (e[y] & 31) + ((e[y] >> 5) & 15);
-                adv2 += e[y] >> 9;
-            }
-        }
-        p[x] = adv << 24 | len << 16 | adv2 << 8 | len2;
     }
     return m;
 }

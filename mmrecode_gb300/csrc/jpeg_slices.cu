@@ -241,7 +241,14 @@ __device__ __forceinline__ uint32_t shared_address(const void *p) { return (uint
 // frames have up to 32k intervals; a CTA per frame 0.36 ms.)
 constexpr int kPlanThreads = 128;
 
+// The last n_luts CTAs make the skip tables (host code took 13 us for one).
 __global__ void __launch_bounds__(kPlanThreads) slice_plan_kernel(JpegLaunch L) {
+    if (blockIdx.x + L.n_luts >= gridDim.x) {
+        const LutMeta m = L.lut_meta[gridDim.x - 1 - blockIdx.x];
+        for (uint32_t x = threadIdx.x; x < m.len; x += kPlanThreads)
+            L.skip[m.off + x] = skip_entry_of(L.sym + m.off, m.first_long, x);
+        return;
+    }
     const uint32_t item = blockIdx.x * kPlanThreads + threadIdx.x, lane = threadIdx.x & 31;
     uint32_t first = 0, n_s = 0, limit = 0;  // slots [first, first + n_s) used, up to limit unused
     if (item < L.n_items_small) {
@@ -715,7 +722,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_fix_kernel(JpegLaunch L) 
 // ---------------------------------------------------------------- prefix ---
 
 constexpr int kPrefixThreads = 512;
-constexpr uint32_t kPrefixLong = 512;  // slices an interval is worth the whole CTA from
+constexpr uint32_t kPrefixLong = 192;  // slices an interval is worth the whole CTA from
 
 struct SliceSums {
     uint32_t blocks;
@@ -841,7 +848,9 @@ __device__ __noinline__ void report_bad_block(const JpegLaunch &L, const SliceRe
         int32_t val;
         uint16_t err;
         uint32_t eb;
-        if (!decode_symbol(r, lim > sym_at ? lim - sym_at : 0, L.luts + (k0 == 0 ? R.dc_lut : R.ac_lut), L.symbols, k, val, err, eb)) {
+        refill(r);
+        if (!checked_symbol(r, lim > sym_at ? lim - sym_at : 0, L.canon + (k0 == 0 ? R.dc_lut : R.ac_lut), L.symbols, k,
+                            val, err, eb)) {
             kind = err;
             errpos = eb;
             break;
@@ -1115,7 +1124,7 @@ void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks,
     const uint32_t grid = L.n_slots / kSliceThreads;  // (frames reserve whole CTAs of slots)
     auto per_item = [&](uint32_t items) { return (L.n_items_small + items - 1) / items; };
     if (run) {
-        slice_plan_kernel<<<per_item(kPlanThreads), kPlanThreads, 0, s>>>(L);
+        slice_plan_kernel<<<per_item(kPlanThreads) + L.n_luts, kPlanThreads, 0, s>>>(L);
         slice_spec_kernel<<<dim3(grid, L.paths), kSliceThreads, 0, s>>>(L);
     }
     mark(0);

@@ -21,7 +21,7 @@ struct JpegLaunch {
     const JSched *sched;
     const JBlockRec *brec;       // parallel to sched
     const JComp *comps;
-    const HuffLut *luts;
+    const HuffLut *luts;         // only when a frame has more than four components
     uint32_t n_luts;
     const uint8_t *symbols;
     const uint16_t *quant;       // natural order
@@ -55,7 +55,8 @@ struct JpegLaunch {
     uint32_t *sync_left;         // intervals the sync passes left unsettled (zeroed per batch)
     const LutMeta *lut_meta;     // per LUT, its entries in:
     const uint16_t *sym;
-    const uint32_t *skip;
+    uint32_t *skip;              // written by slice_plan_kernel
+    const HuffCanon *canon;
     const long long *fixw;       // fixed-point IDCT weights (exact_fixed.h)
 };
 

@@ -38,6 +38,16 @@ struct HuffLut {
     uint32_t pad[2];       // size multiple of 16
 };
 
+// The canonical code by itself (HuffLut's fields of the same names), for decodes that go
+// symbol by symbol with the reference's checks.
+struct HuffCanon {
+    uint16_t fast[512];
+    int32_t maxcode[18];
+    int32_t valptr[18];
+    uint32_t sym_off;
+    uint32_t pad[3];
+};
+
 // Lookups of the chunked decoder (jpeg_slices.cu), per table. Canonical codes of more
 // than 11 bits are the last of the code space, from the 32-bit left-aligned code
 // `first_long` on, so one table serves both: the entry of a window w (the next 32 bits)
@@ -48,7 +58,7 @@ struct HuffLut {
 //         level, 16 for ZRL, kSymEob for EOB, so that a block ends with an index of 64
 //         or from 97 to 159 and an overrun lies between); 0 for bits no code matches
 //         and for symbols the reference rejects.
-//   skip  AC tables, for decodes that only follow positions. Byte 3: advance of the
+//   skip  for decodes that only follow positions, made on the device (skip_entry_of). Byte 3: advance of the
 //         first symbol, byte 2: its bits, magnitude included; bytes 1 and 0: the same
 //         of the first two where the second's code lies within the 11 bits too (else of
 //         the first); 0 where sym is 0.
@@ -73,6 +83,25 @@ MMR_HD bool lut_fits_shared(const LutMeta &m) { return m.last == 0xffffffffu && 
 
 MMR_HD uint32_t lut_entry_index(uint32_t w, uint32_t first_long) {
     return (w >> (32 - kHuffFastBits)) + (((w > first_long ? w : first_long) - first_long) >> 16);
+}
+
+// The skip entry x of a table, from its sym entries.
+MMR_HD uint32_t skip_entry_of(const uint16_t *sym, uint32_t first_long, uint32_t x) {
+    constexpr uint32_t FB = kHuffFastBits;
+    const uint32_t e = sym[x];
+    if (!e) return 0;
+    const uint32_t cl = e & 31, len = cl + ((e >> 5) & 15), adv = e >> 9;
+    uint32_t len2 = len, adv2 = adv;
+    // (windows below first_long have no long entries before theirs: x is the prefix)
+    if (cl <= FB && adv < kSymEob && len < FB) {
+        const uint32_t y = (x << len) & ((1u << FB) - 1);  // what is left of the 11 bits, then zeros
+        const uint32_t e2 = y << (32 - FB) < first_long ? sym[y] : 0;
+        if (e2 && (e2 & 31) <= FB - len) {
+            len2 += (e2 & 31) + ((e2 >> 5) & 15);
+            adv2 += e2 >> 9;
+        }
+    }
+    return adv << 24 | len << 16 | adv2 << 8 | len2;
 }
 
 // One frame component (SOF0 order).

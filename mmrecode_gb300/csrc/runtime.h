@@ -73,6 +73,7 @@ public:
     int device() const { return device_; }
     Engine &engine(int k) { return *engines_[k]; }
     static constexpr size_t kMinChunk = 16;
+    static constexpr size_t kMinStagedChunk = 4, kStagedPartBytes = 48u << 20;
 
 private:
     struct Chunk {
@@ -91,6 +92,7 @@ private:
     std::vector<cudaStream_t> down_;  // per engine: downloads of staged outputs
     int device_ = 0;
     // staging of the current batch: device copies of its inputs and outputs
+    size_t staged_bytes_ = 0;  // output bytes of the staged items
     void *stage_ptr_ = nullptr;
     size_t stage_cap_ = 0;
     std::vector<Item> staged_;

@@ -15,8 +15,9 @@
 extern "C" void mmr_test_sym(const uint8_t *key, size_t key_len, int ac, size_t before, uint16_t *sym, uint32_t *skip,
                              uint32_t *meta) {
     std::vector<uint16_t> s(before, 0xabcd);
-    std::vector<uint32_t> k(before, 0xabcdu);
-    const mmr::LutMeta m = mmr::build_sym(key, key_len, ac != 0, &s, &k);
+    const mmr::LutMeta m = mmr::build_sym(key, key_len, ac != 0, &s);
+    std::vector<uint32_t> k(m.off + m.len);
+    for (uint32_t x = 0; x < m.len; x++) k[m.off + x] = mmr::skip_entry_of(s.data() + m.off, m.first_long, x);
     for (uint32_t p = 0; p < 65536; p++) {
         const uint32_t at = m.off + mmr::lut_entry_index(std::min(p << 16, m.last), m.first_long);
         sym[p] = at < s.size() ? s[at] : 0xffff;
