@@ -642,7 +642,7 @@ Probe probe_packet(uint32_t codec, const uint8_t *data, size_t len) {
 // --------------------------------------------------------------- engine ---
 
 struct Engine::Impl {
-    DevBuf d_in, d_tok, d_blob, d_tile_tok, d_tile_rst, d_rsts, d_results, d_coef, d_dc, d_planes, d_out, d_dvcoef,
+    DevBuf d_in, d_tok, d_blob, d_tile_cnt, d_rsts, d_results, d_coef, d_dc, d_planes, d_out, d_dvcoef,
         d_modes, d_segerr, d_vlc, d_fix, d_slot_item, d_ivs, d_sync, d_spec, d_prefix, d_events, d_ivkey,
         d_ivpend, d_skip,
         d_place,   // DV block placement (dv_layout.h)
@@ -869,8 +869,9 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             size_t tok_off = tok_bytes;
             tok_bytes = align_up(tok_bytes + it.len, 256);
             F.tok = reinterpret_cast<uint8_t *>(tok_off);  // relocated after allocation
-            uint32_t base16 = F.data_start & ~15u;
-            uint32_t nt = it.len > base16 ? (uint32_t)((it.len - base16 + kScanTile - 1) / kScanTile) : 0;
+            // (a host packet's copy starts on a 256-byte address)
+            const long long scan0 = scan_base(it.dev_data, F.data_start);
+            uint32_t nt = (uint32_t)(((long long)it.len - scan0 + kScanTile - 1) / kScanTile);
             if (F.data_start >= it.len) nt = 0;
             F.tile_first = tile_first.back();
             tile_first.push_back(tile_first.back() + nt);
@@ -1126,8 +1127,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         // +512: the entropy decoders' 32-bit word readers may read a few bytes, and the lean
         // decode a block (at most 1,728 bits), past a frame's tokens
         I.d_tok.ensure(tok_bytes + 512);
-        I.d_tile_tok.ensure(std::max<size_t>(tile_first.back() * 4, 256));
-        I.d_tile_rst.ensure(std::max<size_t>(tile_first.back() * 4, 256));
+        I.d_tile_cnt.ensure(std::max<size_t>((size_t)tile_first.back() * 8, 256));
         I.d_rsts.ensure(std::max<size_t>(rst_total * sizeof(RstEntry), 256));
         size_t n_items = items_small.size() + items_big.size();
         I.d_results.ensure(std::max<size_t>(n_items * sizeof(Diag), 256));
@@ -1205,6 +1205,8 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
 
         uint32_t zero_left[4] = {};  // unsettled intervals
         size_t o_left = blob.add(zero_left, sizeof(zero_left));
+        // (the scan's group sums: frame f's start at its first tile / 64 + f)
+        const size_t o_groups = blob.add_vec(std::vector<uint64_t>((tile_first.back() >> 6) + jframes.size() + 1));
         size_t blob_size = std::max<size_t>(blob.bytes.size(), 256);
         I.d_blob.ensure(blob_size);
         I.h_blob.ensure(blob_size);
@@ -1248,8 +1250,8 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         JL.n_frames = (uint32_t)jframes.size();
         JL.tile_first = reinterpret_cast<const uint32_t *>(db + o_tile_first);
         JL.n_tiles = tile_first.back();
-        JL.tile_tok = I.d_tile_tok.as<uint32_t>();
-        JL.tile_rst = I.d_tile_rst.as<uint32_t>();
+        JL.tile_cnt = I.d_tile_cnt.as<unsigned long long>();
+        JL.tile_group = reinterpret_cast<unsigned long long *>(db + o_groups);
         JL.rsts = I.d_rsts.as<RstEntry>();
         JL.sched = reinterpret_cast<const JSched *>(db + o_sched);
         JL.brec = reinterpret_cast<const JBlockRec *>(db + o_brec);
@@ -1393,7 +1395,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                 key.push_back((uintptr_t)fjobs[v].size());
                 key.push_back((uintptr_t)fcta[v].back());
             }
-            for (const DevBuf *b : {&I.d_in, &I.d_tok, &I.d_blob, &I.d_tile_tok, &I.d_tile_rst, &I.d_rsts,
+            for (const DevBuf *b : {&I.d_in, &I.d_tok, &I.d_blob, &I.d_tile_cnt, &I.d_rsts,
                                     &I.d_results, &I.d_coef, &I.d_dc, &I.d_planes, &I.d_out, &I.d_dvcoef, &I.d_modes,
                                     &I.d_segerr, &I.d_vlc, &I.d_fix, &I.d_slot_item, &I.d_ivs, &I.d_sync,
                                     &I.d_spec, &I.d_prefix, &I.d_events, &I.d_ivkey, &I.d_ivpend, &I.d_skip})

@@ -7,7 +7,13 @@
 
 namespace mmr {
 
-constexpr int kScanTile = 4096;  // bytes of entropy-coded data per marker-scan CTA
+constexpr int kScanTile = 4096;  // bytes of entropy-coded data per marker-scan warp
+
+// Packet-relative first byte of a frame's first tile: its address is the 16-byte line that
+// data_start lies in, so that it may lie before the packet. (The host sizes by it too.)
+MMR_HD long long scan_base(const uint8_t *in, uint32_t data_start) {
+    return (long long)data_start - (long long)((reinterpret_cast<uintptr_t>(in) + data_start) & 15);
+}
 
 struct JpegLaunch {
     const JFrame *frames;        // device
@@ -15,8 +21,8 @@ struct JpegLaunch {
     uint32_t n_frames;
     const uint32_t *tile_first;  // n_frames + 1 prefix of marker-scan tiles
     uint32_t n_tiles;
-    uint32_t *tile_tok;          // per tile: token count, then its exclusive prefix
-    uint32_t *tile_rst;
+    unsigned long long *tile_cnt;    // per tile: tokens, and restart markers << 32
+    unsigned long long *tile_group;  // their sums over a frame's groups of 64 tiles (zeroed per batch)
     RstEntry *rsts;
     const JSched *sched;
     const JBlockRec *brec;       // parallel to sched
