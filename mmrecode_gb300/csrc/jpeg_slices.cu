@@ -722,6 +722,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_fix_kernel(JpegLaunch L) 
 // ---------------------------------------------------------------- prefix ---
 
 constexpr int kPrefixThreads = 512;
+constexpr uint32_t kPrefixCtas = 4 * 152;      // as many as run at a time
 constexpr uint32_t kPrefixLong = 192;  // slices an interval is worth the whole CTA from
 
 struct SliceSums {
@@ -732,21 +733,20 @@ struct SliceSums {
 __device__ __forceinline__ void add_slice(const JpegLaunch &L, const IvInfo &v, uint32_t j, SliceSums &a) {
     if (j + 1 >= v.n_slices) return;  // the last slice's counts are never needed
     const SliceSync &y = L.sync[v.slot_first + j];
-    a.blocks += y.blocks;
+    a.blocks += __ldg(&y.blocks);
 #pragma unroll
-    for (int c = 0; c < 4; c++) a.dc[c] += y.dc[c];
+    for (int c = 0; c < 4; c++) a.dc[c] += __ldg(&y.dc[c]);
 }
 
-// Inclusive prefix over the warp.
-__device__ __forceinline__ void warp_prefix(SliceSums &a) {
+// Inclusive prefix over the warp's first n lanes.
+__device__ __forceinline__ void warp_prefix(SliceSums &a, uint32_t n) {
     const uint32_t lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (uint32_t o = 1; o < n; o <<= 1) {
         const uint32_t b = __shfl_up_sync(0xffffffffu, a.blocks, o);
         long long d[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) d[c] = __shfl_up_sync(0xffffffffu, a.dc[c], o);
-        if (lane >= (uint32_t)o) {
+        if (lane >= o) {
             a.blocks += b;
 #pragma unroll
             for (int c = 0; c < 4; c++) a.dc[c] += d[c];
@@ -763,57 +763,66 @@ __device__ __forceinline__ void write_prefix(const JpegLaunch &L, const IvInfo &
     L.prefix[v.slot_first + j] = P;
 }
 
-// Warp per interval; intervals of many slices (scans without restart markers) are
-// taken by the whole CTA, a run of slices per thread (a warp per interval took
-// 1.5 ms for the 10k slices of 4K scans). One-slice intervals need no prefix.
-__global__ void __launch_bounds__(kPrefixThreads) slice_prefix_kernel(JpegLaunch L) {
-    __shared__ SliceSums s_warp[kPrefixThreads / 32];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t item0 = blockIdx.x * (kPrefixThreads / 32), item = item0 + warp;
-    if (item < L.n_items_small) {
-        const IvInfo v = L.ivs[item];
-        if (v.n_slices > 1 && v.n_slices < kPrefixLong) {
-            SliceSums carry{};
-            for (uint32_t c = 0; c < v.n_slices; c += 32) {
-                SliceSums a{}, own{};
-                add_slice(L, v, c + lane, own);
-                a = own;
-                warp_prefix(a);
-                const SliceSums incl = a;
-                a.blocks += carry.blocks - own.blocks;
+// Prefixes of slices [j0, j1) after the sums `carry`, by one warp.
+__device__ __forceinline__ void prefix_run(const JpegLaunch &L, const IvInfo &v, uint32_t j0, uint32_t j1, SliceSums carry) {
+    for (uint32_t c = j0; c < j1; c += 32) {
+        const uint32_t j = c + (threadIdx.x & 31);
+        SliceSums own{};
+        if (j < j1) add_slice(L, v, j, own);
+        SliceSums a = own;
+        warp_prefix(a, min(j1 - c, 32u));
+        const SliceSums incl = a;
+        a.blocks += carry.blocks - own.blocks;
 #pragma unroll
-                for (int q = 0; q < 4; q++) a.dc[q] += carry.dc[q] - own.dc[q];
-                if (c + lane < v.n_slices) write_prefix(L, v, c + lane, a);
-                carry.blocks += __shfl_sync(0xffffffffu, incl.blocks, 31);
+        for (int q = 0; q < 4; q++) a.dc[q] += carry.dc[q] - own.dc[q];
+        if (j < j1) write_prefix(L, v, j, a);
+        if (c + 32 >= j1) break;
+        carry.blocks += __shfl_sync(0xffffffffu, incl.blocks, 31);
 #pragma unroll
-                for (int q = 0; q < 4; q++) carry.dc[q] += __shfl_sync(0xffffffffu, incl.dc[q], 31);
-            }
-        }
+        for (int q = 0; q < 4; q++) carry.dc[q] += __shfl_sync(0xffffffffu, incl.dc[q], 31);
     }
-    for (uint32_t i = 0; i < kPrefixThreads / 32 && item0 + i < L.n_items_small; i++) {
+}
+
+// Warp per interval; intervals of many slices (scans without restart markers) are
+// taken by the whole CTA, a run of slices per warp: its sum, then its prefixes (a warp per
+// interval took 1.5 ms for the 10k slices of 4K scans). One-slice intervals need no prefix.
+//
+// A chain of loads and shuffles. A CTA takes `per_cta` intervals, up to one a warp: long
+// ones are taken one after another, so a CTA takes one while they fit on the GPU at a time
+// (30 VGA scans without markers in two CTAs: 37 us, in thirty: 7). Consecutive lanes take
+// consecutive slices (a run of slices per thread touched a line per lane and load: 250 us
+// against 147 in a step of 64 mixed frames).
+__global__ void __launch_bounds__(kPrefixThreads) slice_prefix_kernel(JpegLaunch L, uint32_t per_cta) {
+    constexpr uint32_t kWarps = kPrefixThreads / 32;
+    __shared__ SliceSums s_warp[kWarps];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t item0 = blockIdx.x * per_cta, n = min(per_cta, L.n_items_small - item0);
+    bool any_long = false;
+    if (warp < n) {
+        const IvInfo v = L.ivs[item0 + warp];
+        any_long = v.n_slices >= kPrefixLong;
+        if (v.n_slices > 1 && !any_long) prefix_run(L, v, 0, v.n_slices, SliceSums{});
+    }
+    if (!__syncthreads_or(any_long)) return;
+    for (uint32_t i = 0; i < n; i++) {
         const IvInfo v = L.ivs[item0 + i];
         if (v.n_slices < kPrefixLong) continue;  // uniform over the CTA
-        const uint32_t per = (v.n_slices + kPrefixThreads - 1) / kPrefixThreads;
-        const uint32_t j0 = min(threadIdx.x * per, v.n_slices), j1 = min(j0 + per, v.n_slices);
-        SliceSums own{};
-        for (uint32_t j = j0; j < j1; j++) add_slice(L, v, j, own);
-        SliceSums a = own;
-        warp_prefix(a);
-        __syncthreads();
+        const uint32_t run = (v.n_slices + kPrefixThreads - 1) / kPrefixThreads * 32;
+        const uint32_t j0 = min(warp * run, v.n_slices), j1 = min(j0 + run, v.n_slices);
+        SliceSums a{};
+#pragma unroll 4
+        for (uint32_t j = j0 + lane; j < j1; j += 32) add_slice(L, v, j, a);
+        warp_prefix(a, 32);
+        __syncthreads();  // (the last interval's sums are read)
         if (lane == 31) s_warp[warp] = a;
         __syncthreads();
-        a.blocks -= own.blocks;
-#pragma unroll
-        for (int q = 0; q < 4; q++) a.dc[q] -= own.dc[q];
+        SliceSums carry{};
         for (uint32_t w = 0; w < warp; w++) {
-            a.blocks += s_warp[w].blocks;
+            carry.blocks += s_warp[w].blocks;
 #pragma unroll
-            for (int q = 0; q < 4; q++) a.dc[q] += s_warp[w].dc[q];
+            for (int q = 0; q < 4; q++) carry.dc[q] += s_warp[w].dc[q];
         }
-        for (uint32_t j = j0; j < j1; j++) {
-            write_prefix(L, v, j, a);
-            add_slice(L, v, j, a);
-        }
+        prefix_run(L, v, j0, j1, carry);
     }
 }
 
@@ -1132,7 +1141,8 @@ void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks,
         const uint32_t passes = jpeg_sync_passes(L);
         for (uint32_t p = 0; p < passes; p++) slice_sync_kernel<<<grid, kSliceThreads, 0, s>>>(L, p == 0, p + 1 == passes);
         if (passes > 1) slice_fix_kernel<<<per_item(kSliceThreads / 32), kSliceThreads, 0, s>>>(L);
-        slice_prefix_kernel<<<per_item(kPrefixThreads / 32), kPrefixThreads, 0, s>>>(L);
+        const uint32_t per_cta = std::min<uint32_t>((L.n_items_small + kPrefixCtas - 1) / kPrefixCtas, kPrefixThreads / 32);
+        slice_prefix_kernel<<<per_item(per_cta), kPrefixThreads, 0, s>>>(L, per_cta);
     }
     mark(1);
     if (run) slice_decode_kernel<<<grid, kSliceThreads, 0, s>>>(L);
