@@ -55,69 +55,99 @@ __device__ __forceinline__ double exact_row(const int32_t *crow, int x) {
     return acc;
 }
 
-// Pass 2, +128, round half away from zero, clamp.
-__device__ __forceinline__ uint8_t exact_finish(const double *t, int y) {
-    double acc = 0.0;
-#pragma unroll
-    for (int v = 0; v < 8; v++)
-        if (t[v] != 0.0) acc = __dadd_rn(acc, __dmul_rn(c_idct[y * 8 + v], t[v]));
-    const double px = round(__dadd_rn(acc, 128.0));
-    return (uint8_t)fmin(fmax(px, 0.0), 255.0);
+// + 128, round half away from zero, clamp.
+__device__ __forceinline__ uint8_t exact_pixel(double s) {
+    const double px = __dadd_rn(s, 128.0);
+    if (!(px > 0.0)) return 0;
+    if (px >= 255.0) return 255;
+    const int n = __double2int_rd(px);
+    return (uint8_t)(n + (__dsub_rn(px, (double)n) >= 0.5 ? 1 : 0));
 }
 
-__device__ __forceinline__ uint8_t exact_sample(const int32_t *c, int stride, int y, int x) {
-    double t[8];
-#pragma unroll
-    for (int v = 0; v < 8; v++) t[v] = exact_row(c + v * stride, x);
-    return exact_finish(t, y);
-}
+// A block with at least this many undecided samples ties in them: they take the reference
+// order without trying the fixed-point value first.
+constexpr int kManyTies = 12;
 
 // Settles the samples in `mask` of one block whose exact dequantised coefficients
-// are in c (shared memory; all 32 lanes of the warp call this together). First
-// the warp forms each sample's exact fixed-point value (exact_fixed.h, offset
-// +128); the samples still too close to a half-integer take the reference
-// order, one sample per lane in parallel. A block with no nonzero AC coefficient
-// is evaluated once (DC-only blocks whose value is a half-integer leave all 64
-// samples undecided: sample by sample they were half the time of the 4:4:4
-// transform of pictures with flat areas). put(y, x, sample) may run on any lane.
+// are in c (shared memory; all 32 lanes of the warp call this together). First the exact fixed-point value of each (exact_fixed.h, offset +128), four
+// samples at a time, lane v of eight taking row v of the coefficients; what is still too
+// close to a half-integer takes the reference order, four columns at a time: lane v
+// forms t[v][x], then sample (v, x) from the eight of them. A block with no nonzero AC
+// coefficient is evaluated once. put(y, x, sample) may run on any lane.
+//
+// Bound by the binary64 pipe (16 cycles per warp instruction and SM) where samples tie, by
+// the chains' latency elsewhere. By columns, a block's ties cost 8 row terms and 8 column
+// terms per four columns; a lane per sample cost every nonzero coefficient's term and the
+// column's (the fused 4:4:4 transform of 64 mixed frames: 1367 us, 57 % of it waiting for
+// that pipe; now 693). Of a 320x240 frame's call the fixup takes 14 us instead of 24.
 template <class Put>
 __device__ __forceinline__ void settle_samples(const long long *fixw, const int32_t *c, unsigned long long mask,
                                                Put put) {
-    const int lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31, v = lane & 7, g = lane >> 3;
     long long c1 = llabs((long long)c[lane]) + llabs((long long)c[lane + 32]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) c1 += __shfl_xor_sync(0xffffffffu, c1, o);
-    const bool flat = __ballot_sync(0xffffffffu, (lane != 0 && c[lane] != 0) || c[lane + 32] != 0) == 0;
-    if (flat) {  // every M[x][0] is the same literal: all 64 samples are equal, one evaluation settles them
-        int v = -1;
-        if (c1 < kFixMaxC1) v = fixed_round(fixw[0] * (long long)c[0], (int32_t)c1, 128);
-        if (v < 0) {
-            if (lane == 0) v = exact_sample(c, 8, 0, 0);
-            v = __shfl_sync(0xffffffffu, v, 0);
-        }
+    if (c1 == llabs((long long)c[0])) {  // every M[x][0] is the same literal: all 64 samples are equal
+        int s = -1;
+        if (c1 < kFixMaxC1) s = fixed_round(fixw[0] * (long long)c[0], (int32_t)c1, 128);
+        // (the other terms of both passes are zeros, and 0.0 + x = x)
+        if (s < 0) s = exact_pixel(__dmul_rn(c_idct[0], __dmul_rn(c_idct[0], (double)c[0])));
         for (int b = lane; b < 64; b += 32)
-            if (mask >> b & 1) put(b >> 3, b & 7, (uint8_t)v);
+            if (mask >> b & 1) put(b >> 3, b & 7, (uint8_t)s);
         return;
     }
-    unsigned long long left = 0;  // samples for the reference order
-    for (unsigned long long m = mask; m; m &= m - 1) {
-        const int b = __ffsll((long long)m) - 1, y = b >> 3, x = b & 7;
-        int smp = -1;
-        if (c1 < kFixMaxC1) smp = fixed_round(fixed_sum(fixw + (y * 8 + x) * 64, c), (int32_t)c1, 128);
-        if (smp >= 0) {
-            if (lane == 0) put(y, x, (uint8_t)smp);
-        } else {
-            left |= 1ull << b;
+    unsigned long long left = mask;  // samples for the reference order
+    if (c1 < kFixMaxC1 && __popcll(mask) < kManyTies) {
+        left = 0;
+        while (mask) {
+            if (!(mask & (mask - 1))) {  // one sample: over all lanes
+                const int b = __ffsll((long long)mask) - 1;
+                const int s = fixed_round(fixed_sum(fixw + b * 64, c), (int32_t)c1, 128);
+                if (s < 0) left |= mask;
+                else if (lane == 0) put(b >> 3, b & 7, (uint8_t)s);
+                break;
+            }
+            int b = -1;  // of the lane's group of eight
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                if (k == g && mask) b = __ffsll((long long)mask) - 1;
+                mask &= mask - 1;
+            }
+            long long t = 0;
+            if (b >= 0) {
+                const longlong2 *w = reinterpret_cast<const longlong2 *>(fixw + b * 64 + v * 8);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const longlong2 ww = __ldg(w + u);
+                    t += ww.x * c[v * 8 + 2 * u] + ww.y * c[v * 8 + 2 * u + 1];
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            const int s = b >= 0 ? fixed_round(t, (int32_t)c1, 128) : 0;
+            if (s >= 0 && b >= 0 && v == 0) put(b >> 3, b & 7, (uint8_t)s);
+            for (uint32_t m = __ballot_sync(0xffffffffu, s < 0 && v == 0); m; m &= m - 1)
+                left |= 1ull << __shfl_sync(0xffffffffu, b, __ffs(m) - 1);
         }
     }
-    while (left) {  // lane i takes the i-th remaining sample
-        unsigned long long m = left;
-        for (int i = 0; i < lane && m; i++) m &= m - 1;
-        if (m) {
-            const int b = __ffsll((long long)m) - 1;
-            put(b >> 3, b & 7, exact_sample(c, 8, b >> 3, b & 7));
+    uint32_t cols = (uint32_t)(left | left >> 32);
+    cols |= cols >> 16;
+    cols = (cols | cols >> 8) & 0xffu;
+    while (cols) {
+        int x = -1;  // the group's column
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            if (k == g && cols) x = __ffs(cols) - 1;
+            cols &= cols - 1;
         }
-        for (int i = 0; i < 32 && left; i++) left &= left - 1;
+        const double t = x >= 0 ? exact_row(c + v * 8, x) : 0.0;
+        double acc = 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const double ti = __shfl_sync(0xffffffffu, t, (lane & 24) | i);
+            if (__double_as_longlong(ti) << 1 != 0) acc = __dadd_rn(acc, __dmul_rn(c_idct[v * 8 + i], ti));
+        }
+        if (x >= 0 && left >> (v * 8 + x) & 1) put(v, x, exact_pixel(acc));
     }
 }
 

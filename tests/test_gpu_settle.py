@@ -43,4 +43,4 @@ def test_settled_samples_equal_the_oracle(harness, kind):  # noqa: F811
     assert harness.harness_jpeg_idct(c.ctypes.data, len(c), gpu.ctypes.data, ctypes.byref(exact)) == 0
     bad, msg = _first_mismatches(gpu, oracle.jpeg_idct_many(c), kind, c)
     assert len(bad) == 0, msg
-    assert exact.value > 0
+    assert exact.value > 0 or kind == "flat_large"  # (all clamped)
