@@ -35,10 +35,6 @@ __constant__ double c_cos16[128] = {
 #include "cos_table.inc"
 };
 
-__constant__ float c_cos16f[128] = {
-#include "cos_table.inc"
-};
-
 constexpr double kFrac = 0.7071067811865476;  // FRAC_1_SQRT_2
 
 // The reference's binary64 8-8 direct sum for sample (y, x) (decoder.rs:520-548):
@@ -117,41 +113,48 @@ __device__ __forceinline__ uint8_t dv_flat_sample(const int32_t *c, bool mode248
 // ---------------------------------------------------------------------------
 // Eight threads per block: thread r takes column r in the vertical pass (with the
 // 2-4-8 butterfly, exact), then row r in the horizontal pass. The factors are fp32
-// products of the fp32 roundings, W[u][x] = (u ? 1 : FRAC) * cos16f[(2x+1)u] and
-// V4[yy][v] = (v ? 1 : FRAC) * cos16f[2(2yy+1)v]. Where the outputs x and 7 - x share
+// products of the fp32 roundings, W[u][x] = (u ? 1 : FRAC) * cos16[(2x+1)u] and
+// V4[yy][v] = (v ? 1 : FRAC) * cos16[2(2yy+1)v]. Where the outputs x and 7 - x share
 // an eight-term sum (W[u][7-x] = (-1)^u W[u][x]), one packed FMA per pair of terms
 // keeps the even and the odd sum side by side; a 2-4-8 column keeps its two fields
 // side by side. All in all 32 packed FMAs a thread in either mode.
 
-// Fills the tables (48 floats) cooperatively; callers synchronise before use. Row x < 4
-// of wt holds W[0..7][x], then row yy < 4 (of four) V4[yy][0..3]. (No second table any
-// more: the argument is for callers that have one.)
+// The factors, as operands of the FMAs straight from constant memory (from shared memory
+// they were 16 vector loads a thread: 1000 NTSC frames took 2.53 ms instead of 2.34). Row
+// x < 4 holds W[0..7][x], then row yy < 4 (of four) V4[yy][0..3].
 constexpr int kDvTable = 48;
 constexpr int kDvV4 = 32;  // offset of V4 in it
 
-__device__ __forceinline__ void dv_fill_tables(float *wt, float * = nullptr) {
-    for (int i = threadIdx.x; i < kDvTable; i += blockDim.x) {
-        if (i < kDvV4) {
-            const int x = i >> 3, u = i & 7;
-            wt[i] = (u == 0 ? (float)kFrac : 1.0f) * c_cos16f[(2 * x + 1) * u];
-        } else {
-            const int yy = (i - kDvV4) >> 2, v = (i - kDvV4) & 3;
-            wt[i] = (v == 0 ? (float)kFrac : 1.0f) * c_cos16f[2 * (2 * yy + 1) * v];
-        }
-    }
+struct DvFactors {
+    float w[kDvTable];
+};
+
+constexpr DvFactors dv_factors() {
+    constexpr double cs[128] = {
+#include "cos_table.inc"
+    };
+    DvFactors t{};
+    for (int i = 0; i < kDvV4; i++) t.w[i] = ((i & 7) == 0 ? (float)kFrac : 1.0f) * (float)cs[(2 * (i >> 3) + 1) * (i & 7)];
+    for (int i = 0; i < 16; i++)
+        t.w[kDvV4 + i] = ((i & 3) == 0 ? (float)kFrac : 1.0f) * (float)cs[2 * (2 * (i >> 2) + 1) * (i & 3)];
+    return t;
 }
 
+__constant__ DvFactors c_dv_factors = dv_factors();
+
+// (The passes take tables no more: for callers that have some.)
+__device__ __forceinline__ void dv_fill_tables(float *, float * = nullptr) {}
+
 // The eight-point sums out[i] = sum_u W[u][i] b[u], b as the pairs (b[0], b[1]), ...
-__device__ __forceinline__ void dv_eight_point(const F2 (&b)[4], const float *wt, float (&out)[8]) {
+__device__ __forceinline__ void dv_eight_point(const F2 (&b)[4], float (&out)[8]) {
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const float4 w0 = reinterpret_cast<const float4 *>(wt + i * 8)[0];
-        const float4 w1 = reinterpret_cast<const float4 *>(wt + i * 8)[1];
+        const float *w = c_dv_factors.w + i * 8;
         F2 s;  // (even, odd) terms
-        s = fma2(f2(w0.x, w0.y), b[0], s);
-        s = fma2(f2(w0.z, w0.w), b[1], s);
-        s = fma2(f2(w1.x, w1.y), b[2], s);
-        s = fma2(f2(w1.z, w1.w), b[3], s);
+        s = fma2(f2(w[0], w[1]), b[0], s);
+        s = fma2(f2(w[2], w[3]), b[1], s);
+        s = fma2(f2(w[4], w[5]), b[2], s);
+        s = fma2(f2(w[6], w[7]), b[3], s);
         float e, o;
         split2(s, e, o);
         out[i] = e + o;
@@ -161,7 +164,7 @@ __device__ __forceinline__ void dv_eight_point(const F2 (&b)[4], const float *wt
 
 // First pass, thread r: the vertical sums of column r, outputs y = 0..7 into hcol
 // (16-byte aligned). c: the block's 64 coefficients (natural order).
-__device__ __forceinline__ void dv_row_pass8(const int32_t *c, const float *wt, bool mode248, int r, float *hcol) {
+__device__ __forceinline__ void dv_row_pass8(const int32_t *c, const float *, bool mode248, int r, float *hcol) {
     float b[8], out[8];
 #pragma unroll
     for (int v = 0; v < 8; v++) b[v] = (float)c[v * 8 + r];
@@ -169,17 +172,17 @@ __device__ __forceinline__ void dv_row_pass8(const int32_t *c, const float *wt, 
         F2 s[4];  // (field 0, field 1) of row yy
 #pragma unroll
         for (int yy = 0; yy < 4; yy++) {
-            const float4 w = reinterpret_cast<const float4 *>(wt + kDvV4 + yy * 4)[0];
+            const float *w = c_dv_factors.w + kDvV4 + yy * 4;
             // the butterfly of each row pair is exact: |c| < 2^23
-            s[yy] = fma2(f2(w.x, w.x), f2(b[0] + b[1], b[0] - b[1]), s[yy]);
-            s[yy] = fma2(f2(w.y, w.y), f2(b[2] + b[3], b[2] - b[3]), s[yy]);
-            s[yy] = fma2(f2(w.z, w.z), f2(b[4] + b[5], b[4] - b[5]), s[yy]);
-            s[yy] = fma2(f2(w.w, w.w), f2(b[6] + b[7], b[6] - b[7]), s[yy]);
+            s[yy] = fma2(f2(w[0], w[0]), f2(b[0] + b[1], b[0] - b[1]), s[yy]);
+            s[yy] = fma2(f2(w[1], w[1]), f2(b[2] + b[3], b[2] - b[3]), s[yy]);
+            s[yy] = fma2(f2(w[2], w[2]), f2(b[4] + b[5], b[4] - b[5]), s[yy]);
+            s[yy] = fma2(f2(w[3], w[3]), f2(b[6] + b[7], b[6] - b[7]), s[yy]);
             split2(s[yy], out[2 * yy], out[2 * yy + 1]);
         }
     } else {
         const F2 p[4] = {f2(b[0], b[1]), f2(b[2], b[3]), f2(b[4], b[5]), f2(b[6], b[7])};
-        dv_eight_point(p, wt, out);
+        dv_eight_point(p, out);
     }
     reinterpret_cast<float4 *>(hcol)[0] = make_float4(out[0], out[1], out[2], out[3]);
     reinterpret_cast<float4 *>(hcol)[1] = make_float4(out[4], out[5], out[6], out[7]);
@@ -190,7 +193,7 @@ __device__ __forceinline__ void dv_row_pass8(const int32_t *c, const float *wt, 
 // (x). h: the first pass's outputs, column u's at h + 8 * u. For a flat block (no nonzero
 // AC coefficient) lane `flat_src` of the warp computes the one reference-order value and
 // broadcasts it (all eight lanes of the block's group call this together).
-__device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h, const float *wt, const float *,
+__device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h, const float *, const float *,
                                                 bool mode248, int y, float c1, bool flat, int flat_src,
                                                 unsigned group_mask, unsigned long long *row) {
     if (flat) {
@@ -202,7 +205,7 @@ __device__ __forceinline__ uint32_t dv_row_fp32(const int32_t *c, const float *h
     }
     const F2 p[4] = {f2(h[y], h[8 + y]), f2(h[16 + y], h[24 + y]), f2(h[32 + y], h[40 + y]), f2(h[48 + y], h[56 + y])};
     float value[8];
-    dv_eight_point(p, wt, value);
+    dv_eight_point(p, value);
 #pragma unroll
     for (int x = 0; x < 8; x++) value[x] *= 0.25f;  // (exact; 8-8's / 4.0, 2-4-8's two / 2.0)
     // A value is certain when no half-integer lies within delta = 2^-21 C1 + 2^-30 of

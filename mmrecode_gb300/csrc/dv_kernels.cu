@@ -34,16 +34,6 @@ __constant__ int32_t c_dv_w248[64] = MMR_DV_IWEIGHT_248_INIT;
 
 namespace {
 
-__device__ __forceinline__ uint32_t upper_index32(const uint32_t *first, uint32_t n, uint32_t x) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (first[mid] <= x) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // dif.rs:235-253 expected_id
 __device__ __forceinline__ void expected_id(uint32_t pos, uint32_t *section, uint32_t *number) {
     if (pos == 0) {
@@ -94,51 +84,52 @@ __device__ __forceinline__ void append_bits(uint32_t *dst, uint32_t &dn, const u
 
 struct DvBlock {
     uint8_t position;
-    uint8_t complete;
     uint8_t mode;     // 1 = 2-4-8
     uint8_t cls;
-    uint16_t pval;    // partial bits (< 16), right-aligned
     uint8_t plen;
-    uint8_t pad;
+    uint16_t pval;    // partial bits (< 16), right-aligned
 };
 
-// A CTA takes four video segments per step (dv/src/decoder.rs:152-317), in the
-// reference's three levels, each level's independent parts in parallel:
-//   1. a thread per block (120): DC/mode/class and the AC codes inside the
+// A warp takes a video segment at a time (dv/src/decoder.rs:152-317), in the
+// reference's three levels:
+//   1. a lane per block (30): DC/mode/class and the AC codes inside the
 //      block's own region of its macroblock's payload, the region's bits in registers;
-//   2. a thread per macroblock (20): the leftover bits of its complete blocks, in
+//   2. a lane per macroblock (5): the leftover bits of its complete blocks, in
 //      block order, make the macroblock pool, which its incomplete blocks
 //      consume in order (decode_macroblock, decoder.rs:193-243);
-//   3. a thread per segment (4): the macroblock pools' leftovers, in macroblock
-//      order, make the segment pool, which the segment's incomplete blocks
-//      consume in order (consume_pool_for_macroblocks, decoder.rs:225-233).
+//   3. one lane: the macroblock pools' leftovers, in macroblock order, make the segment
+//      pool, which the segment's incomplete blocks consume in order
+//      (consume_pool_for_macroblocks, decoder.rs:225-233).
 // Payload, pools and dequantised coefficients stay in shared memory; every
 // block's 64 coefficients (zeros included) then leave as 16-byte stores. CTAs are
 // persistent: the VLC table and the dequantisation tables, which the lanes index
 // freely, are copied to shared memory once (constant memory and L1 served such
 // lookups a lane at a time).
-constexpr int kSegPerCta = 4;
-constexpr int kSegBlocks = kSegPerCta * 30;
-constexpr int kSegMbs = kSegPerCta * 5;
+//
+// Each level is a chain of lookups, so warps go their own ways: with four segments to a
+// CTA and a thread per block, then per macroblock, then per segment, half of all warp time
+// was spent at the barriers between them (1000 NTSC frames, 270,000 segments: 1277 us, and
+// 1955 us now against 2325 with the transform). More CTAs per SM gain nothing.
 constexpr int kSegThreads = 128;
+constexpr int kSegWarps = kSegThreads / 32;
 constexpr int kSegCtasPerSm = 6;
 
+struct SegWarp {
+    __align__(16) int16_t coef[30][64];
+    uint32_t pay[5 * 19 + 5];  // payload words of the five macroblocks (+5: reads past the end)
+    uint32_t mbpool[5][20];
+    uint32_t segpool[5 * 19 + 2];
+    DvBlock blk[30];
+    uint16_t left_start[30], left_len[30];  // unused bits of a complete block's region
+    uint16_t mb_pos[5], mb_len[5];
+    uint8_t qno[5];
+};
+
 struct SegSmem {
-    __align__(16) int16_t coef[kSegBlocks][64];
     __align__(16) uint32_t vlc[kDvVlcEntries];
     uint32_t dequant[2][64];            // per mode and zigzag index: weight | natural index << 16 | 8 * area << 24
     uint32_t shifts[22];                // per quantiser row: the four areas' shifts, a byte each
-    uint32_t pay[kSegPerCta][5 * 19 + 5];  // payload words of the five macroblocks (+5: reads past the end)
-    uint32_t mbpool[kSegMbs][20];
-    uint32_t segpool[kSegPerCta][5 * 19 + 2];
-    DvBlock blk[kSegBlocks];
-    uint16_t left_start[kSegBlocks], left_len[kSegBlocks];  // unused bits of a complete block's region
-    uint16_t mb_pos[kSegMbs], mb_len[kSegMbs];
-    uint32_t dif_off[kSegMbs];  // byte offset of each macroblock's DIF block in the frame
-    uint32_t frame[kSegPerCta], local[kSegPerCta];
-    uint8_t qno[kSegMbs], damaged[kSegMbs];
-    uint8_t bad[kSegBlocks];
-    uint16_t kind[kSegPerCta];
+    SegWarp warp[kSegWarps];
 };
 
 // Entry of the next 16 bits. The codes of more than kDvVlcL1Bits bits are the last of
@@ -156,11 +147,11 @@ struct Dequant {
     int16_t *coef;
 };
 
-__device__ __forceinline__ Dequant dequant_of(SegSmem &S, const DvBlock &b, uint32_t block, uint32_t qno) {
+__device__ __forceinline__ Dequant dequant_of(const SegSmem &S, SegWarp &W, const DvBlock &b, uint32_t block, uint32_t qno) {
     Dequant d;
     d.table = S.dequant[b.mode];
     d.shifts = S.shifts[qno + (uint32_t)c_dv_qoff[b.cls]] + (b.cls == 3 ? 0x02020202u : 0x01010101u);
-    d.coef = S.coef[block];
+    d.coef = W.coef[block];
     return d;
 }
 
@@ -179,10 +170,12 @@ __device__ __forceinline__ bool take_level(const Dequant &d, uint32_t e, uint32_
 // consume_ac (decoder.rs:245-284) on a pool, the virtual stream (partial bits ++
 // buf[pos, end)). On completion pos is left after the EOB; otherwise the remaining
 // bits become the block's partial and pos == end.
-__device__ void consume_pool(SegSmem &S, uint32_t block, uint32_t qno, const uint32_t *buf, uint32_t &pos, uint32_t end,
-                             bool &bad_vlc) {
-    DvBlock &b = S.blk[block];
-    const Dequant d = dequant_of(S, b, block, qno);
+// Returns whether the block is complete.
+__device__ bool consume_pool(const SegSmem &S, SegWarp &W, uint32_t block, uint32_t qno, const uint32_t *buf,
+                             uint32_t &pos, uint32_t end, bool &bad_vlc) {
+    DvBlock &b = W.blk[block];
+    const Dequant d = dequant_of(S, W, b, block, qno);
+    bool complete = false;
     uint32_t p = b.position, plen = b.plen, avail = plen + (end - pos);
     uint32_t w16 = get32(buf, pos) >> 16;
     if (plen) w16 = (((uint32_t)b.pval << (16 - plen)) | (w16 >> plen)) & 0xffffu;
@@ -205,92 +198,98 @@ __device__ void consume_pool(SegSmem &S, uint32_t block, uint32_t qno, const uin
         pos += len - plen;  // (a partial never holds a whole code)
         plen = 0;
         if (take_level(d, e, p)) {
-            b.complete = 1;
-            p = 64;
+            complete = true;
             break;
         }
         w16 = get32(buf, pos) >> 16;
     }
     b.position = (uint8_t)p;
+    return complete;
+}
+
+// The frame of segment g: 32 probes a step.
+__device__ __forceinline__ uint32_t frame_of(const DvLaunch &L, uint32_t g) {
+    uint32_t lo = 0, hi = L.n_frames;
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32, at = lo + (threadIdx.x & 31) * step;
+        const uint32_t below = __ballot_sync(0xffffffffu, at < hi && L.seg_first[at] <= g);
+        lo += (uint32_t)(31 - __clz(below)) * step;  // (lane 0's probe always holds)
+        hi = min(lo + step, hi);
+    }
+    return lo;
 }
 
 __global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvLaunch L) {
     __shared__ SegSmem S;
-    const uint32_t t = threadIdx.x;
-    for (uint32_t i = t; i < (uint32_t)kDvVlcEntries; i += kSegThreads) S.vlc[i] = __ldg(L.vlc + i);
-    {
-        const uint32_t p = t & 63, m = t >> 6;  // kSegThreads = 2 x 64
+    for (uint32_t i = threadIdx.x; i < (uint32_t)kDvVlcEntries; i += kSegThreads) S.vlc[i] = __ldg(L.vlc + i);
+    for (uint32_t i = threadIdx.x; i < 128; i += kSegThreads) {
+        const uint32_t p = i & 63, m = i >> 6;
         const uint32_t area = p <= 5 ? 0 : p <= 20 ? 1 : p <= 42 ? 2 : 3;
         S.dequant[m][p] = (uint32_t)(m ? c_dv_w248[p] : c_dv_w88[p]) |
                           (uint32_t)(m ? c_dv_zz248[p] : c_dv_zz88[p]) << 16 | area << 27;
-        if (t < 22)
-            S.shifts[t] = c_dv_shifts[t * 4] | c_dv_shifts[t * 4 + 1] << 8 | c_dv_shifts[t * 4 + 2] << 16 |
-                          (uint32_t)c_dv_shifts[t * 4 + 3] << 24;
     }
-    for (uint32_t g0 = blockIdx.x * kSegPerCta; g0 < L.n_segments; g0 += gridDim.x * kSegPerCta) {
-        __syncthreads();  // the tables; the last step's results
+    if (threadIdx.x < 22) {
+        const uint32_t t = threadIdx.x;
+        S.shifts[t] = c_dv_shifts[t * 4] | c_dv_shifts[t * 4 + 1] << 8 | c_dv_shifts[t * 4 + 2] << 16 |
+                      (uint32_t)c_dv_shifts[t * 4 + 3] << 24;
+    }
+    __syncthreads();
+    const uint32_t t = threadIdx.x & 31;
+    SegWarp &W = S.warp[threadIdx.x >> 5];
+    for (uint32_t g = blockIdx.x * kSegWarps + (threadIdx.x >> 5); g < L.n_segments; g += gridDim.x * kSegWarps) {
+        const uint32_t f = frame_of(L, g);
+        const uint32_t local = g - L.seg_first[f], sequence = local / 27, slot = local % 27;
+        const uint8_t *in = L.frames[f].in;
         // macroblock records: DIF block, its identifier against the canonical layout
         // (dif.rs:181-253), quantiser
-        if (t < (uint32_t)kSegMbs) {
-            const uint32_t sg = t / 5, m = t % 5, g = g0 + sg;
-            if (g < L.n_segments) {
-                const uint32_t f = upper_index32(L.seg_first, L.n_frames, g);
-                const uint32_t local = g - L.seg_first[f], sequence = local / 27, slot = local % 27;
-                const uint32_t vn = slot * 5 + m, pos = 7 + (vn / 15) * 16 + vn % 15;  // DIF block of the sequence
-                const uint32_t off = (sequence * 150 + pos) * 80;
-                const uint8_t *b = L.frames[f].in + off;
-                uint32_t es, en;
-                expected_id(pos, &es, &en);
-                S.damaged[t] = (uint32_t)(b[0] >> 5) != es || (uint32_t)(b[1] >> 4) != sequence || (uint32_t)b[2] != en;
-                S.qno[t] = b[3] & 0x0f;
-                S.dif_off[t] = off;
-                if (m == 0) {
-                    S.frame[sg] = f;
-                    S.local[sg] = local;
-                }
-            }
+        uint32_t off = 0;  // byte offset of the lane's macroblock's DIF block in the frame
+        bool damaged = false;
+        if (t < 5) {
+            const uint32_t vn = slot * 5 + t, pos = 7 + (vn / 15) * 16 + vn % 15;  // DIF block of the sequence
+            off = (sequence * 150 + pos) * 80;
+            const uint8_t *b = in + off;
+            uint32_t es, en;
+            expected_id(pos, &es, &en);
+            damaged = (uint32_t)(b[0] >> 5) != es || (uint32_t)(b[1] >> 4) != sequence || (uint32_t)b[2] != en;
+            W.qno[t] = b[3] & 0x0f;
         }
-        for (uint32_t i = t; i < (uint32_t)kSegBlocks * 8; i += kSegThreads)
-            reinterpret_cast<int4 *>(&S.coef[0][0])[i] = make_int4(0, 0, 0, 0);
-        for (uint32_t i = t; i < (uint32_t)kSegMbs * 20; i += kSegThreads) (&S.mbpool[0][0])[i] = 0;
-        for (uint32_t i = t; i < (uint32_t)kSegPerCta * 97; i += kSegThreads) (&S.segpool[0][0])[i] = 0;
-        __syncthreads();
-        if (t < (uint32_t)kSegPerCta) {
-            uint16_t kind = g0 + t < L.n_segments ? kDiagNone : 0xffff;  // 0xffff: no segment
-            for (int m = 0; m < 5; m++)
-                if (kind == kDiagNone && S.damaged[t * 5 + m]) kind = kDvDamagedId;
-            S.kind[t] = kind;
-        }
+        damaged = __any_sync(0xffffffffu, damaged);
         // payload words (bytes 4..80 of each DIF block), big-endian
-        for (uint32_t i = t; i < (uint32_t)kSegPerCta * 100; i += kSegThreads) {
-            const uint32_t sg = i / 100, wi = i - sg * 100;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t wi = k * 32 + t, m = min(wi / 19, 4u);
+            const uint8_t *src = in + __shfl_sync(0xffffffffu, off, m) + 4 + (wi - m * 19) * 4;
             uint32_t v = 0;
-            if (wi < 95 && g0 + sg < L.n_segments) {
-                const uint32_t m = wi / 19;
-                const uint8_t *src = L.frames[S.frame[sg]].in + S.dif_off[sg * 5 + m] + 4 + (wi - m * 19) * 4;
+            if (wi < 95) {
                 if ((reinterpret_cast<uintptr_t>(src) & 3) == 0)
                     v = __byte_perm(__ldg(reinterpret_cast<const uint32_t *>(src)), 0, 0x0123);
                 else
                     v = ((uint32_t)src[0] << 24) | ((uint32_t)src[1] << 16) | ((uint32_t)src[2] << 8) | (uint32_t)src[3];
             }
-            S.pay[sg][wi] = v;
+            if (wi < 100) W.pay[wi] = v;
         }
-        __syncthreads();
-        // 1. a thread per block: its own region
-        if (t < (uint32_t)kSegBlocks) {
-            const uint32_t sg = t / 30, b = t % 30, m = b / 6, bi = b % 6;
-            DvBlock B{};
-            uint16_t ls = 0, ll = 0;
-            bool bad = false;
-            if (S.kind[sg] == kDiagNone) {
-                const uint32_t *w = S.pay[sg] + m * 19;
+        for (uint32_t i = t; i < 240; i += 32) reinterpret_cast<int4 *>(&W.coef[0][0])[i] = make_int4(0, 0, 0, 0);
+        for (uint32_t i = t; i < 100; i += 32) (&W.mbpool[0][0])[i] = 0;
+        for (uint32_t i = t; i < 97; i += 32) W.segpool[i] = 0;
+        __syncwarp();
+        uint16_t kind = kDvDamagedId;
+        uint32_t mode = 0;
+        if (!damaged) {  // (uniform)
+            // 1. a lane per block: its own region
+            bool complete = true, bad = false;
+            if (t < 30) {
+                const uint32_t m = t / 6, bi = t % 6;
+                DvBlock B{};
+                uint16_t ls = 0, ll = 0;
+                const uint32_t *w = W.pay + m * 19;
                 const uint32_t r0 = bi < 4 ? bi * 112 : 448 + (bi - 4) * 80, bits = bi < 4 ? 112 : 80;
                 const uint32_t head = get32(w, r0) >> 20;  // 12 bits: dc(9) mode(1) class(2)
                 int32_t dc = (int32_t)(head >> 3);
                 if (dc & 0x100) dc -= 512;
                 B.mode = (head >> 2) & 1;
                 B.cls = head & 3;
-                const Dequant d = dequant_of(S, B, t, S.qno[sg * 5 + m]);
+                mode = B.mode;
+                const Dequant d = dequant_of(S, W, B, t, W.qno[m]);
                 d.coef[0] = (int16_t)(dc * 4 + 1024);
                 // the region's bits after the header (at most 100), left-aligned
                 const uint32_t at = r0 + 12, i = at >> 5, o = at & 31;
@@ -303,6 +302,7 @@ __global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvL
                     if (len == 0 || len > left) {
                         B.pval = (uint16_t)(left < 16 ? a0 >> 16 >> (16 - left) : 0);  // the partial
                         B.plen = (uint8_t)(left < 16 ? left : 0);
+                        complete = false;
                         break;
                     }
                     a0 = __funnelshift_l(a1, a0, len);
@@ -311,73 +311,67 @@ __global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvL
                     a3 <<= len;
                     left -= len;
                     if (take_level(d, e, p)) {
-                        p = 64;
-                        B.complete = 1;
                         ls = (uint16_t)(r0 + bits - left);
                         ll = (uint16_t)left;
                         break;
                     }
                 }
                 B.position = (uint8_t)p;
+                W.blk[t] = B;
+                W.left_start[t] = ls;
+                W.left_len[t] = ll;
             }
-            S.blk[t] = B;
-            S.left_start[t] = ls;
-            S.left_len[t] = ll;
-            S.bad[t] = bad ? 1 : 0;
+            uint32_t open = __ballot_sync(0xffffffffu, !complete);  // incomplete blocks
+            __syncwarp();
+            // 2. a lane per macroblock: its pool
+            uint32_t mine = 0;
+            if (t < 5) {
+                const uint32_t *w = W.pay + t * 19;
+                const uint32_t j0 = t * 6;
+                mine = (open >> j0) & 63;
+                uint32_t pos = 0, mbn = 0;
+                for (uint32_t done = ~mine & 63; done; done &= done - 1) {
+                    const uint32_t j = j0 + __ffs(done) - 1;
+                    append_bits(W.mbpool[t], mbn, w, W.left_start[j], W.left_len[j]);
+                }
+                for (uint32_t left = mine; left && pos < mbn; left &= left - 1) {
+                    const uint32_t k = __ffs(left) - 1;
+                    if (consume_pool(S, W, j0 + k, W.qno[t], W.mbpool[t], pos, mbn, bad)) mine ^= 1u << k;
+                }
+                W.mb_pos[t] = (uint16_t)pos;
+                W.mb_len[t] = (uint16_t)mbn;
+                mine <<= j0;
+            }
+            open = __reduce_or_sync(0xffffffffu, mine);
+            __syncwarp();
+            // 3. one lane: the segment's pool
+            if (t == 0 && open) {
+                uint32_t pos = 0, segn = 0;
+                for (uint32_t m = 0; m < 5; m++)
+                    if (W.mb_pos[m] < W.mb_len[m])
+                        append_bits(W.segpool, segn, W.mbpool[m], W.mb_pos[m], W.mb_len[m] - W.mb_pos[m]);
+                for (uint32_t left = open; left && pos < segn; left &= left - 1) {
+                    const uint32_t j = __ffs(left) - 1;
+                    if (consume_pool(S, W, j, W.qno[j / 6], W.segpool, pos, segn, bad)) open ^= 1u << j;
+                }
+            }
+            open = __shfl_sync(0xffffffffu, open, 0);
+            kind = __any_sync(0xffffffffu, bad) ? kDvBadVlc : open ? kDvIncomplete : kDiagNone;
+            __syncwarp();
         }
-        __syncthreads();
-        // 2. a thread per macroblock: its pool
-        if (t < (uint32_t)kSegMbs) {
-            const uint32_t sg = t / 5, m = t % 5;
-            uint32_t pos = 0, mbn = 0;
-            if (S.kind[sg] == kDiagNone) {
-                const uint32_t *w = S.pay[sg] + m * 19;
-                const uint32_t j0 = sg * 30 + m * 6;
-                for (uint32_t j = j0; j < j0 + 6; j++)
-                    if (S.blk[j].complete) append_bits(S.mbpool[t], mbn, w, S.left_start[j], S.left_len[j]);
-                bool bad = false;
-                for (uint32_t j = j0; j < j0 + 6 && pos < mbn; j++)
-                    if (!S.blk[j].complete) consume_pool(S, j, S.qno[t], S.mbpool[t], pos, mbn, bad);
-                if (bad) S.bad[j0] = 1;
-            }
-            S.mb_pos[t] = (uint16_t)pos;
-            S.mb_len[t] = (uint16_t)mbn;
-        }
-        __syncthreads();
-        // 3. a thread per segment: its pool, then its result
-        if (t < (uint32_t)kSegPerCta && S.kind[t] == kDiagNone) {
-            uint32_t segn = 0;
-            for (uint32_t m = 0; m < 5; m++) {
-                const uint32_t k = t * 5 + m;
-                if (S.mb_pos[k] < S.mb_len[k])
-                    append_bits(S.segpool[t], segn, S.mbpool[k], S.mb_pos[k], S.mb_len[k] - S.mb_pos[k]);
-            }
-            uint32_t pos = 0;
-            bool bad = false, incomplete = false;
-            for (uint32_t j = 0; j < 30; j++) {
-                const uint32_t jj = t * 30 + j;
-                if (!S.blk[jj].complete && pos < segn)
-                    consume_pool(S, jj, S.qno[t * 5 + j / 6], S.segpool[t], pos, segn, bad);
-                bad |= S.bad[jj] != 0;
-                incomplete |= !S.blk[jj].complete;
-            }
-            S.kind[t] = bad ? kDvBadVlc : incomplete ? kDvIncomplete : kDiagNone;
-        }
-        __syncthreads();
-        // coefficients out (the CTA's segments are consecutive: blocks g0 * 30 ..), modes, results
-        const uint32_t n_seg = min((uint32_t)kSegPerCta, L.n_segments - g0);
-        int4 *dst = reinterpret_cast<int4 *>(L.coef + (uint64_t)g0 * 30 * 64);
-        const int4 *src = reinterpret_cast<const int4 *>(&S.coef[0][0]);
-        for (uint32_t i = t; i < n_seg * 30 * 8; i += kSegThreads) dst[i] = src[i];
-        if (t < n_seg * 30) L.modes[(uint64_t)g0 * 30 + t] = S.blk[t].mode;
-        if (t < n_seg) {
-            const uint16_t kind = S.kind[t];
-            L.seg_err[g0 + t] = (uint8_t)kind;
+        // coefficients out, modes, result
+        int4 *dst = reinterpret_cast<int4 *>(L.coef + (uint64_t)g * 30 * 64);
+        const int4 *src = reinterpret_cast<const int4 *>(&W.coef[0][0]);
+        for (uint32_t i = t; i < 240; i += 32) dst[i] = src[i];
+        if (t < 30) L.modes[(uint64_t)g * 30 + t] = (uint8_t)mode;
+        if (t == 0) {
+            L.seg_err[g] = (uint8_t)kind;
             if (kind != kDiagNone) {
-                atomicMin(&L.states[S.frame[t]].bad_segment, S.local[t]);
-                atomicAdd(&L.states[S.frame[t]].failed, 1u);
+                atomicMin(&L.states[f].bad_segment, local);
+                atomicAdd(&L.states[f].failed, 1u);
             }
         }
+        __syncwarp();  // the coefficients are read
     }
 }
 
@@ -393,7 +387,7 @@ __global__ void dv_resolve_kernel(DvLaunch L) {
     }
 }
 
-constexpr int kIdctBlocks = 16;                  // blocks per CTA
+constexpr int kIdctBlocks = 8;                   // blocks per CTA (1000 NTSC frames: 1.92 ms, with 16 1.96)
 constexpr int kIdctThreads = kIdctBlocks * 8;    // eight threads (rows) per block
 
 // Stores the eight bytes of `row` at dst (any alignment).
@@ -429,9 +423,6 @@ constexpr int kBlockStride = 72;  // ints or floats per block: four blocks' colu
 __global__ void __launch_bounds__(kIdctThreads) dv_idct_kernel(DvLaunch L) {
     __shared__ __align__(16) int32_t s_c[kIdctBlocks][kBlockStride];
     __shared__ __align__(16) float s_h[kIdctBlocks][kBlockStride];
-    __shared__ __align__(16) float s_wt[kDvTable];
-    dv_fill_tables(s_wt);
-    __syncthreads();
     const int lane = threadIdx.x & 31, lb = threadIdx.x >> 3, r = threadIdx.x & 7;
     const unsigned group_mask = 0xffu << (lane & 24);
     const uint32_t gb = blockIdx.x * kIdctBlocks + lb;
@@ -482,12 +473,12 @@ __global__ void __launch_bounds__(kIdctThreads) dv_idct_kernel(DvLaunch L) {
     const bool flat = (__ballot_sync(0xffffffffu, ac) & group_mask) == 0;
     const bool active = valid && !failed;
     __syncwarp();
-    if (active && !flat) dv_row_pass8(c, s_wt, mode, r, s_h[lb] + r * 8);
+    if (active && !flat) dv_row_pass8(c, nullptr, mode, r, s_h[lb] + r * 8);
     __syncwarp();
     unsigned long long row = 0;
     uint32_t und = 0;
     if (active)
-        und = dv_row_fp32(c, s_h[lb], s_wt, nullptr, mode, r, (float)c1, flat, lane & 24, group_mask, &row);
+        und = dv_row_fp32(c, s_h[lb], nullptr, nullptr, mode, r, (float)c1, flat, lane & 24, group_mask, &row);
     dv_resolve_row(und, row, c, mode, r, c1, L.fixw);  // every lane of the warp takes part
     if (!valid) return;
     const uint32_t e = __ldg(L.place + (F->pal ? kDvBlocks525 : 0) + local_blk);
@@ -506,7 +497,7 @@ __global__ void __launch_bounds__(kIdctThreads) dv_idct_kernel(DvLaunch L) {
 }  // namespace
 
 void launch_dv_decode(const DvLaunch &L, cudaStream_t s) {
-    const uint32_t steps = (L.n_segments + kSegPerCta - 1) / kSegPerCta;
+    const uint32_t steps = (L.n_segments + kSegWarps - 1) / kSegWarps;
     if (steps) segment_kernel<<<std::min<uint32_t>(steps, 152 * kSegCtasPerSm), kSegThreads, 0, s>>>(L);
     if (L.n_frames) dv_resolve_kernel<<<(L.n_frames + 127) / 128, 128, 0, s>>>(L);
 }
