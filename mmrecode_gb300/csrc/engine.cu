@@ -817,6 +817,9 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         uint64_t batch_blocks = 0;
         for (const JPlan &p : jplans) batch_blocks += p.n_blocks;
         const uint32_t fused_strips = batch_blocks >= (2u << 20) ? 8 : batch_blocks >= (1u << 20) ? 4 : 1;
+        // Planar output: tiles of 64 blocks per CTA, four once that still fills the GPU
+        // (608 CTAs at a time; 30 VGA frames: 352 us, with one tile 355)
+        const uint32_t idct_tiles = batch_blocks >= (128u << 10) ? 4 : 1;
         uint32_t most_paths = 1;
         std::vector<size_t> in_off(n, 0), out_off(n, 0), planes_off(n, SIZE_MAX);
         std::vector<std::array<size_t, 6>> plane_geom(n);  // (offset, bytes) of up to 3 planes
@@ -999,7 +1002,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                     r.comp = c;
                     if (p.comps[c].bw != 0 && p.comps[c].bh != 0) {
                         ranges.push_back(r);
-                        idct_cta.push_back(idct_cta.back() + idct_ctas(p.comps[c].bw * p.comps[c].bh));
+                        idct_cta.push_back(idct_cta.back() + idct_ctas(p.comps[c].bw * p.comps[c].bh, idct_tiles));
                     }
                 }
                 blocks += p.n_blocks;
@@ -1270,6 +1273,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         JL.n_ranges = (uint32_t)ranges.size();
         JL.idct_cta_first = reinterpret_cast<const uint32_t *>(db + o_idctcta);
         JL.n_idct_ctas = idct_cta.back();
+        JL.idct_tiles = idct_tiles;
         JL.n_blocks = blocks;
         JL.item_ok = reinterpret_cast<uint32_t *>(db + o_itemok);
         JL.fix = I.d_fix.as<ulonglong2>();
@@ -1386,7 +1390,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
             // states them so that no change of shape can replay a stale graph
             for (uintptr_t v : {(uintptr_t)jframes.size(), (uintptr_t)tile_first.back(), (uintptr_t)luts.size(), (uintptr_t)lut_meta.size(),
                                 (uintptr_t)items_small.size(), (uintptr_t)n_items, (uintptr_t)ranges.size(),
-                                (uintptr_t)idct_cta.back(), (uintptr_t)n_slots, (uintptr_t)most_paths,
+                                (uintptr_t)idct_cta.back(), (uintptr_t)idct_tiles, (uintptr_t)n_slots, (uintptr_t)most_paths,
                                 (uintptr_t)blocks, (uintptr_t)dframes.size(), (uintptr_t)seg_first.back(),
                                 (uintptr_t)dv_blocks, (uintptr_t)rgbjobs.size(),
                                 (uintptr_t)rgbcta.back()})

@@ -165,6 +165,33 @@ __device__ __forceinline__ BlockRows load_rows(const int16_t *levels, const int3
     return b;
 }
 
+// The same by way of shared memory, asynchronously: slot of thread tid of nt, whose copies
+// begin with copy_rows (once what the slot held has been used) and are waited for by
+// staged_rows. Only the thread itself reads what it copied. (The transforms waited longest
+// for their levels; loads a tile ahead into registers spilled.)
+struct RowSlots {
+    int4 *row;    // 2 * nt
+    int32_t *dc;  // nt
+};
+
+__device__ __forceinline__ void copy_rows(const int16_t *levels, const int32_t *dc, uint64_t g, uint32_t q,
+                                          const RowSlots &to, uint32_t tid, uint32_t nt) {
+    const int4 *src = reinterpret_cast<const int4 *>(levels + g * 64) + q;
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(to.row + tid), d = (uint32_t)__cvta_generic_to_shared(to.dc + tid);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(src) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a + 16 * nt), "l"(src + 4) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(dc + g) : "memory");
+}
+
+__device__ __forceinline__ BlockRows staged_rows(const RowSlots &from, uint32_t tid, uint32_t nt) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    BlockRows b;
+    b.row[0] = from.row[tid];
+    b.row[1] = from.row[tid + nt];
+    b.dc = from.dc[tid];
+    return b;
+}
+
 // Dequantises them into fp32 rows q and q+4 of `blk` (the product of an
 // int16 level and an 8-bit quantiser is exact in fp32; the DC is the decoder's
 // dequantised int32, rounded to fp32 like every c in the bound). Returns the
@@ -210,84 +237,127 @@ __device__ __forceinline__ bool clamped(float acc, float near) {
     return acc > 129.0f + delta || acc < -130.0f - delta;
 }
 
-// Two samples saturated to 0..255 in one instruction: a in byte 0, b in byte 1.
-__device__ __forceinline__ uint32_t sat_pair_u8(int32_t a, int32_t b) {
-    uint32_t d;
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(b), "r"(a), "r"(0));
-    return d;
-}
-
-// Transform of one staged block by its four threads; thread q produces output
-// columns q and 7 - q into out[row * stride + col]. Both passes use the even/odd
-// split of the basis: M[7-x][u] = (-1)^u M[x][u] holds for the fp32 roundings of
-// the reference's literals (the literals themselves differ from exact symmetry by
-// < 2e-15, far inside the fp32 rounding), so
-//   s[x] = E + O, s[7-x] = E - O,  E = sum_{u even} M[x][u] c[u], O = sum_{u odd},
-// E and O side by side in packed FMAs over the pairs (c[0], c[1]), (c[2], c[3]), ...
-// Per output this is 4 FMAs per half and one add: each pass's error is <= 5u of
-// the sum of |terms|, plus u for each rounded M and c, <= 13u B after both
-// passes (the bound above). |s| <= Mmax^2 C1 < C1/4, so the relative term
-// 2^-40 |s| of the bound is folded into 2^-42 C1. One comparison of the largest distance
-// to an integer decides the eight outputs of a column, but for one in a hundred.
+// Transform of one staged block by its four threads; thread q produces output rows
+// q and 7 - q as eight bytes each (the first sample in the low byte). Both passes use
+// the even/odd split of the basis: M[7-x][u] = (-1)^u M[x][u] holds for the fp32
+// roundings of the reference's literals (the literals themselves differ from exact
+// symmetry by < 2e-15, far inside the fp32 rounding), so
+//   s[x] = E + O, s[7-x] = E - O,  E = sum_{u even} M[x][u] c[u], O = sum_{u odd}.
+// The vertical pass comes first, two columns to a packed FMA, so that a thread has whole
+// rows of samples; the horizontal one keeps E and O side by side over the pairs (t[0],
+// t[1]), (t[2], t[3]), ... Per output this is 4 FMAs per half and one add: each pass's
+// error is <= 5u of the sum of |terms|, plus u for each rounded M and c, <= 13u B after
+// both passes (the bound above, which is the same in either order of the passes). |s| <=
+// Mmax^2 C1 < C1/4, so the relative term 2^-40 |s| of the bound is folded into 2^-42 C1.
+// One comparison of the largest distance to an integer decides the eight outputs of a
+// row, but for one in a hundred.
 // Returns the samples left to the exact pass as bits (row * 8 + column).
-__device__ __forceinline__ unsigned long long idct_block(const float *blk, uint32_t q, float c1, uint8_t *out,
-                                                         int stride) {
-    F2 mq[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) mq[u] = f2(c_idct32[q * 8 + 2 * u], c_idct32[q * 8 + 2 * u + 1]);
-    float t[2][8];  // columns q and 7 - q
+//
+// Shared memory's wavefronts are the scarcest: rows leave as two 8-byte stores where
+// columns took sixteen of a byte, and eight in a hundred instructions less (a step of 300
+// 1080p frames with RGB output: 5.92 -> 5.85 ms).
+// mrow: M[q][0..7], each twice.
+__device__ __forceinline__ unsigned long long idct_rows(const float *blk, const float4 *mrow, uint32_t q, float c1,
+                                                        unsigned long long (&row)[2]) {
+    F2 e[4], o[4];  // even and odd sums of the columns (0, 1), (2, 3), ...
 #pragma unroll
     for (int v = 0; v < 8; v++) {
-        const float4 c0 = reinterpret_cast<const float4 *>(blk + v * 8)[0];
-        const float4 c1v = reinterpret_cast<const float4 *>(blk + v * 8)[1];
-        F2 s = mul2(f2(c0.x, c0.y), mq[0]);
-        s = fma2(f2(c0.z, c0.w), mq[1], s);
-        s = fma2(f2(c1v.x, c1v.y), mq[2], s);
-        s = fma2(f2(c1v.z, c1v.w), mq[3], s);
-        float e, o;
-        split2(s, e, o);
-        t[0][v] = e + o;
-        t[1][v] = e - o;
+        const float4 mm = mrow[v >> 1];
+        const F2 m = v & 1 ? f2(mm.z, mm.w) : f2(mm.x, mm.y);
+        const float4 a = reinterpret_cast<const float4 *>(blk + v * 8)[0];
+        const float4 b = reinterpret_cast<const float4 *>(blk + v * 8)[1];
+        const F2 c[4] = {f2(a.x, a.y), f2(a.z, a.w), f2(b.x, b.y), f2(b.z, b.w)};
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            F2 &s = v & 1 ? o[p] : e[p];
+            s = v < 2 ? mul2(c[p], m) : fma2(c[p], m, s);
+        }
     }
     // delta = 2^-22 C1 >= 13u Mmax^2 C1 (margin 1.28), see the bound above
     const float near = 0.5f - (c1 * (0x1p-22f + 0x1p-42f) + 0x1p-30f);
     unsigned long long mask = 0;
 #pragma unroll
+    for (int p = 0; p < 4; p++) {
+        const F2 sum = add2(e[p], o[p]);
+        o[p] = sub2(e[p], o[p]);
+        e[p] = sum;
+    }
+    float all[2][8];
+#pragma unroll
+    for (int x = 0; x < 4; x++) {  // (both rows at a time: the factors take registers)
+        const float *f = c_idct32 + x * 8;
+        const F2 m[4] = {f2(f[0], f[1]), f2(f[2], f[3]), f2(f[4], f[5]), f2(f[6], f[7])};
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            const F2 *t = side ? o : e;
+            F2 s = mul2(t[0], m[0]);
+            s = fma2(t[1], m[1], s);
+            s = fma2(t[2], m[2], s);
+            s = fma2(t[3], m[3], s);
+            float ev, od;
+            split2(s, ev, od);
+            all[side][x] = ev + od;
+            all[side][7 - x] = ev - od;
+        }
+    }
+#pragma unroll
     for (int side = 0; side < 2; side++) {
-        float acc[8], far = 0.0f;
+        const float (&acc)[8] = all[side];
+        float far = 0.0f;
+        const uint32_t y = side ? 7 - q : q;
+        int32_t n[8];
 #pragma unroll
-        for (int y = 0; y < 4; y++) {
-            const float *m = c_idct32 + y * 8;
-            F2 s = mul2(f2(t[side][0], t[side][1]), f2(m[0], m[1]));
-            s = fma2(f2(t[side][2], t[side][3]), f2(m[2], m[3]), s);
-            s = fma2(f2(t[side][4], t[side][5]), f2(m[4], m[5]), s);
-            s = fma2(f2(t[side][6], t[side][7]), f2(m[6], m[7]), s);
-            float e, o;
-            split2(s, e, o);
-            acc[y] = e + o;
-            acc[7 - y] = e - o;
+        for (int x = 0; x < 8; x++) {
+            float r;
+            n[x] = round_nearest(acc[x], r) + 128;
+            far = fmaxf(far, fabsf(acc[x] - r));
         }
-        const uint32_t col = side ? 7 - q : q;
-#pragma unroll
-        for (int y = 0; y < 8; y += 2) {
-            float r0, r1;
-            const int32_t n0 = round_nearest(acc[y], r0), n1 = round_nearest(acc[y + 1], r1);
-            far = fmaxf(far, fmaxf(fabsf(acc[y] - r0), fabsf(acc[y + 1] - r1)));
-            const uint32_t pair = sat_pair_u8(n0 + 128, n1 + 128);
-            out[y * stride + col] = (uint8_t)pair;
-            out[(y + 1) * stride + col] = (uint8_t)(pair >> 8);
-        }
+        row[side] = (unsigned long long)sat_quad_u8(n[4], n[5], n[6], n[7]) << 32 | sat_quad_u8(n[0], n[1], n[2], n[3]);
         if (far < near) continue;
 #pragma unroll
-        for (int y = 0; y < 8; y++) {
+        for (int x = 0; x < 8; x++) {
             float r;
-            round_nearest(acc[y], r);
-            if (fabsf(acc[y] - r) < near) continue;
-            if (clamped(acc[y], near)) out[y * stride + col] = acc[y] > 0.0f ? 255 : 0;
-            else mask |= 1ull << (y * 8 + col);
+            round_nearest(acc[x], r);
+            if (fabsf(acc[x] - r) < near) continue;
+            if (clamped(acc[x], near)) {
+                const unsigned long long byte = 0xffull << (8 * x);
+                row[side] = acc[x] > 0.0f ? row[side] | byte : row[side] & ~byte;
+            } else {
+                mask |= 1ull << (y * 8 + x);
+            }
         }
     }
     return mask;
+}
+
+// The factors of thread q's vertical pass are rows[4 * q .. 4 * q + 3].
+__device__ __forceinline__ void idct_fill_rows(float4 *rows, uint32_t tid) {
+    if (tid < 16) {
+        const float a = c_idct32[2 * tid], b = c_idct32[2 * tid + 1];
+        rows[tid] = make_float4(a, a, b, b);
+    }
+}
+
+// The samples into out[row * stride + column] (rows 8-byte aligned).
+__device__ __forceinline__ unsigned long long idct_block(const float *blk, const float4 *mrow, uint32_t q, float c1,
+                                                         uint8_t *out, int stride) {
+    unsigned long long row[2];
+    const unsigned long long mask = idct_rows(blk, mrow, q, c1, row);
+    *reinterpret_cast<uint2 *>(out + q * stride) = make_uint2((uint32_t)row[0], (uint32_t)(row[0] >> 32));
+    *reinterpret_cast<uint2 *>(out + (7 - q) * stride) = make_uint2((uint32_t)row[1], (uint32_t)(row[1] >> 32));
+    return mask;
+}
+
+// With the factors in registers.
+__device__ __forceinline__ unsigned long long idct_block(const float *blk, uint32_t q, float c1, uint8_t *out,
+                                                         int stride) {
+    float4 mrow[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float a = c_idct32[q * 8 + 2 * i], b = c_idct32[q * 8 + 2 * i + 1];
+        mrow[i] = make_float4(a, a, b, b);
+    }
+    return idct_block(blk, mrow, q, c1, out, stride);
 }
 
 }  // namespace

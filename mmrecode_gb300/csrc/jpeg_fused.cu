@@ -63,6 +63,8 @@ struct FusedSmem {
     __align__(16) uint8_t c[2][8 * Sh::CW];
     __align__(16) uint8_t rgb[Sh::YH * Sh::RW];
     __align__(16) float q[3][64];
+    int4 row[2 * Sh::THREADS];        // the next strip's levels on their way, and its DCs
+    int32_t dc[Sh::THREADS];
     unsigned long long mask[Sh::NB];  // samples left to the exact pass, per block
     unsigned long long blk[Sh::NB];
     int32_t cx[Sh::THREADS / 32][64];  // per warp: exact coefficients of the block it settles
@@ -183,12 +185,12 @@ __device__ __forceinline__ void strip_to_rgb(const JFrame &F, const FusedJob &J,
 }
 
 // A CTA takes J.strips consecutive strips of an MCU row: it reads the job's and the
-// frame's records once for them (one strip per CTA took 7.33 ms for a step of 300 1080p
-// frames, eight 6.57). The time goes to shared memory (two thirds of its wavefronts) and
-// to waits at the barriers, so strips are narrow and the kernel keeps to 64 registers
-// (levels loaded a strip ahead, or 80 registers: 7.46 and 7.11 ms against 6.76 with four
-// wide strips). Undecided samples are settled before the colour conversion, a warp per
-// block (settle_samples).
+// frame's records once for them, and the next strip's levels are on their way to shared
+// memory while it works on one (a step of 300 1080p frames: one strip per CTA 7.33 ms,
+// eight 6.57; with the levels on their way 5.77 against 5.85). What is left goes to issue
+// (two thirds of the slots) and shared memory's wavefronts, so strips are narrow and the
+// kernel keeps to 64 registers (80 registers: 7.11 ms against 6.76). Undecided samples are
+// settled before the colour conversion, a warp per block (settle_samples).
 template <int HM, int VM, int NM>
 __global__ void __launch_bounds__(FusedShape<HM, VM, NM>::THREADS, 1024 / FusedShape<HM, VM, NM>::THREADS) idct_rgb_kernel(JpegLaunch L, FusedLaunch FL) {
     using Sh = FusedShape<HM, VM, NM>;
@@ -217,13 +219,16 @@ __global__ void __launch_bounds__(FusedShape<HM, VM, NM>::THREADS, 1024 / FusedS
     float *blk = S.f + lb * kFStride;
     uint8_t *out = comp == 0 ? S.y + (i / HM) * 8 * Sh::YW + (m * HM + i % HM) * 8 : S.c[comp - 1] + m * 8;
     const int stride = comp == 0 ? Sh::YW : Sh::CW;
+    const RowSlots slots{S.row, S.dc};
+    if (mine && mx0 + m < mx_end) copy_rows(L.coef, L.dc, g, q, slots, threadIdx.x, Sh::THREADS);
     __syncthreads();  // q
     for (; mx0 < mx_end; mx0 += NM, g += step) {
         const bool valid = mine && mx0 + m < mx_end;
-        float l1 = valid ? stage_rows(load_rows(L.coef + g * 64, L.dc, g, q), q, S.q[comp], blk) : 0.0f;
+        float l1 = valid ? stage_rows(staged_rows(slots, threadIdx.x, Sh::THREADS), q, S.q[comp], blk) : 0.0f;
 #pragma unroll
         for (int o = 1; o < 4; o <<= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
         __syncwarp();
+        if (mine && mx0 + NM + m < mx_end) copy_rows(L.coef, L.dc, g + step, q, slots, threadIdx.x, Sh::THREADS);
         unsigned long long mask = 0;
         if (valid) mask = idct_block(blk, q, l1, out, stride);
         if (__syncthreads_or(mask != 0)) {

@@ -41,6 +41,7 @@ struct JpegLaunch {
     uint32_t n_ranges;
     const uint32_t *idct_cta_first;  // n_ranges + 1 prefix of transform CTAs (idct_ctas per range)
     uint32_t n_idct_ctas;
+    uint32_t idct_tiles;         // tiles of 64 blocks per transform CTA
     uint64_t n_blocks;
     uint32_t *item_ok;           // per batch item: 1 while decoding has not failed
     ulonglong2 *fix;             // blocks the fp32 IDCT could not fully decide: (block, sample mask)
@@ -78,7 +79,7 @@ void launch_jpeg_entropy(const JpegLaunch &L, cudaStream_t s);   // frames with 
 void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks = nullptr, bool capturing = false);
 int jpeg_slice_launches(const JpegLaunch &L);
 void launch_jpeg_idct(const JpegLaunch &L, cudaStream_t s);
-uint32_t idct_ctas(uint32_t blocks);
+uint32_t idct_ctas(uint32_t blocks, uint32_t tiles);
 
 // MJPEG frames decoded straight to RGB24 (three components, chroma 1x1, luma
 // 1x1, 2x1 or 2x2): one launch per layout, a CTA per strip of MCUs.

@@ -34,6 +34,15 @@ __device__ __forceinline__ F2 mul2(const F2 &a, const F2 &b) {
     return r;
 }
 
+__device__ __forceinline__ F2 add2(const F2 &a, const F2 &b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// a - b (as a + -1.0 * b: one rounding)
+__device__ __forceinline__ F2 sub2(const F2 &a, const F2 &b) { return fma2(b, f2(-1.0f, -1.0f), a); }
+
 // Four values saturated to 0..255 and packed, b0 in the low byte
 // (cvt.pack.sat: d = c << 16 | sat(a) << 8 | sat(b)).
 __device__ __forceinline__ uint32_t sat_quad_u8(int32_t b0, int32_t b1, int32_t b2, int32_t b3) {
