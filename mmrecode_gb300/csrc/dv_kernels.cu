@@ -20,6 +20,7 @@
 #include "dv_idct_core.h"
 #include "dv_layout.h"
 #include "kernels.h"
+#include "launch.h"
 #include "rounding.h"
 #include "tables.h"
 
@@ -220,6 +221,7 @@ __device__ __forceinline__ uint32_t frame_of(const DvLaunch &L, uint32_t g) {
 }
 
 __global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvLaunch L) {
+    begin_kernel();
     __shared__ SegSmem S;
     for (uint32_t i = threadIdx.x; i < (uint32_t)kDvVlcEntries; i += kSegThreads) S.vlc[i] = __ldg(L.vlc + i);
     for (uint32_t i = threadIdx.x; i < 128; i += kSegThreads) {
@@ -376,6 +378,7 @@ __global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvL
 }
 
 __global__ void dv_resolve_kernel(DvLaunch L) {
+    begin_kernel();
     uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= L.n_frames) return;
     DvState *st = &L.states[f];
@@ -423,6 +426,7 @@ __device__ __forceinline__ void store_row4(uint8_t *dst, uint32_t row) {
 constexpr int kBlockStride = 72;  // ints or floats per block: four blocks' column accesses on distinct banks
 
 __global__ void __launch_bounds__(kIdctThreads, 28) dv_idct_kernel(DvLaunch L) {
+    begin_kernel();
     __shared__ __align__(16) int32_t s_c[kIdctBlocks][kBlockStride];
     __shared__ __align__(16) float s_h[kIdctBlocks][kBlockStride];
     const int lane = threadIdx.x & 31, lb = threadIdx.x >> 3, r = threadIdx.x & 7;
@@ -500,13 +504,13 @@ __global__ void __launch_bounds__(kIdctThreads, 28) dv_idct_kernel(DvLaunch L) {
 
 void launch_dv_decode(const DvLaunch &L, cudaStream_t s) {
     const uint32_t steps = (L.n_segments + kSegWarps - 1) / kSegWarps;
-    if (steps) segment_kernel<<<std::min<uint32_t>(steps, 152 * kSegCtasPerSm), kSegThreads, 0, s>>>(L);
-    if (L.n_frames) dv_resolve_kernel<<<(L.n_frames + 127) / 128, 128, 0, s>>>(L);
+    if (steps) launch_next(segment_kernel, std::min<uint32_t>(steps, 152 * kSegCtasPerSm), kSegThreads, s, L);
+    if (L.n_frames) launch_next(dv_resolve_kernel, (L.n_frames + 127) / 128, 128, s, L);
 }
 
 void launch_dv_idct(const DvLaunch &L, cudaStream_t s) {
     if (L.n_blocks == 0) return;
-    dv_idct_kernel<<<(unsigned)((L.n_blocks + kIdctBlocks - 1) / kIdctBlocks), kIdctThreads, 0, s>>>(L);
+    launch_next(dv_idct_kernel, (unsigned)((L.n_blocks + kIdctBlocks - 1) / kIdctBlocks), kIdctThreads, s, L);
 }
 
 }  // namespace mmr

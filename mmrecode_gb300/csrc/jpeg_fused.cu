@@ -17,6 +17,7 @@
 
 #include "idct_core.h"
 #include "kernels.h"
+#include "launch.h"
 #include "packed.h"
 
 namespace mmr {
@@ -193,6 +194,7 @@ __device__ __forceinline__ void strip_to_rgb(const JFrame &F, const FusedJob &J,
 // settled before the colour conversion, a warp per block (settle_samples).
 template <int HM, int VM, int NM>
 __global__ void __launch_bounds__(FusedShape<HM, VM, NM>::THREADS, 1024 / FusedShape<HM, VM, NM>::THREADS) idct_rgb_kernel(JpegLaunch L, FusedLaunch FL) {
+    begin_kernel();
     using Sh = FusedShape<HM, VM, NM>;
     __shared__ __align__(16) FusedSmem<HM, VM, NM> S;
     __shared__ uint32_t s_job;
@@ -289,7 +291,7 @@ uint32_t fused_groups_x(int slot, uint32_t mcu_cols, uint32_t strips) {
 template <int HM, int VM, int NM>
 static void launch_variant(const JpegLaunch &L, const FusedLaunch &FL, cudaStream_t s) {
     if (!FL.n_ctas) return;
-    idct_rgb_kernel<HM, VM, NM><<<FL.n_ctas, FusedShape<HM, VM, NM>::THREADS, 0, s>>>(L, FL);
+    launch_next(idct_rgb_kernel<HM, VM, NM>, FL.n_ctas, FusedShape<HM, VM, NM>::THREADS, s, L, FL);
 }
 
 int fused_launches(const FusedLaunch &FL) { return FL.n_ctas ? 1 : 0; }

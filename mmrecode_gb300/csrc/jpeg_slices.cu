@@ -51,6 +51,7 @@
 
 #include "entropy_core.h"
 #include "kernels.h"
+#include "launch.h"
 #include "tables.h"
 
 namespace mmr {
@@ -243,6 +244,7 @@ constexpr int kPlanThreads = 128;
 
 // The last n_luts CTAs make the skip tables (host code took 13 us for one).
 __global__ void __launch_bounds__(kPlanThreads) slice_plan_kernel(JpegLaunch L) {
+    begin_kernel();
     if (blockIdx.x + L.n_luts >= gridDim.x) {
         const LutMeta m = L.lut_meta[gridDim.x - 1 - blockIdx.x];
         for (uint32_t x = threadIdx.x; x < m.len; x += kPlanThreads)
@@ -466,6 +468,7 @@ __device__ __forceinline__ void spec_slice(const JpegLaunch &L, LeanSmem &S, con
 }
 
 __global__ void __launch_bounds__(kSliceThreads) slice_spec_kernel(JpegLaunch L) {
+    begin_kernel();
     __shared__ LeanSmem S;
     const uint32_t slot = blockIdx.x * kSliceThreads + threadIdx.x;
     SliceRef s;
@@ -574,6 +577,7 @@ __device__ __forceinline__ void resync_slice(const JpegLaunch &L, LeanSmem &S, c
 // what another CTA still changes there is the next pass's, and after the last pass
 // slice_fix_kernel's, from the interval's first such slice on.
 __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L, bool first_pass, bool last_pass) {
+    begin_kernel();
     __shared__ LeanSmem S;
     __shared__ unsigned long long s_exit[kSliceThreads + 1];  // of the slice before the CTA's first, then of each
     const uint32_t tid = threadIdx.x, slot = blockIdx.x * kSliceThreads + tid;
@@ -679,6 +683,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L,
 
 // One warp per interval that the sync passes left unsettled.
 __global__ void __launch_bounds__(kSliceThreads) slice_fix_kernel(JpegLaunch L) {
+    begin_kernel();
     __shared__ LeanSmem S;
     if (*L.sync_left == 0) return;
     const uint32_t lane = threadIdx.x & 31;
@@ -793,6 +798,7 @@ __device__ __forceinline__ void prefix_run(const JpegLaunch &L, const IvInfo &v,
 // consecutive slices (a run of slices per thread touched a line per lane and load: 250 us
 // against 147 in a step of 64 mixed frames).
 __global__ void __launch_bounds__(kPrefixThreads) slice_prefix_kernel(JpegLaunch L, uint32_t per_cta) {
+    begin_kernel();
     constexpr uint32_t kWarps = kPrefixThreads / 32;
     __shared__ SliceSums s_warp[kWarps];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1005,6 +1011,7 @@ __device__ __forceinline__ void decode_slices(const JpegLaunch &L, DecodeSmem &S
 }
 
 __global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch L) {
+    begin_kernel();
     __shared__ DecodeSmem S;
     const uint32_t tid = threadIdx.x, slot = blockIdx.x * kSliceThreads + tid;
     SliceRef s;
@@ -1081,6 +1088,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch 
 // --------------------------------------------------------------- resolve ---
 
 __global__ void slice_resolve_kernel(JpegLaunch L) {
+    begin_kernel();
     const uint32_t item = blockIdx.x * blockDim.x + threadIdx.x;
     if (item >= L.n_items_small) return;
     const IvInfo v = L.ivs[item];
@@ -1133,21 +1141,21 @@ void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks,
     const uint32_t grid = L.n_slots / kSliceThreads;  // (frames reserve whole CTAs of slots)
     auto per_item = [&](uint32_t items) { return (L.n_items_small + items - 1) / items; };
     if (run) {
-        slice_plan_kernel<<<per_item(kPlanThreads) + L.n_luts, kPlanThreads, 0, s>>>(L);
-        slice_spec_kernel<<<dim3(grid, L.paths), kSliceThreads, 0, s>>>(L);
+        launch_next(slice_plan_kernel, per_item(kPlanThreads) + L.n_luts, kPlanThreads, s, L);
+        launch_next(slice_spec_kernel, dim3(grid, L.paths), kSliceThreads, s, L);
     }
     mark(0);
     if (run) {
         const uint32_t passes = jpeg_sync_passes(L);
-        for (uint32_t p = 0; p < passes; p++) slice_sync_kernel<<<grid, kSliceThreads, 0, s>>>(L, p == 0, p + 1 == passes);
-        if (passes > 1) slice_fix_kernel<<<per_item(kSliceThreads / 32), kSliceThreads, 0, s>>>(L);
+        for (uint32_t p = 0; p < passes; p++) launch_next(slice_sync_kernel, grid, kSliceThreads, s, L, p == 0, p + 1 == passes);
+        if (passes > 1) launch_next(slice_fix_kernel, per_item(kSliceThreads / 32), kSliceThreads, s, L);
         const uint32_t per_cta = std::min<uint32_t>((L.n_items_small + kPrefixCtas - 1) / kPrefixCtas, kPrefixThreads / 32);
-        slice_prefix_kernel<<<per_item(per_cta), kPrefixThreads, 0, s>>>(L, per_cta);
+        launch_next(slice_prefix_kernel, per_item(per_cta), kPrefixThreads, s, L, per_cta);
     }
     mark(1);
-    if (run) slice_decode_kernel<<<grid, kSliceThreads, 0, s>>>(L);
+    if (run) launch_next(slice_decode_kernel, grid, kSliceThreads, s, L);
     mark(2);
-    if (run) slice_resolve_kernel<<<per_item(128), 128, 0, s>>>(L);
+    if (run) launch_next(slice_resolve_kernel, per_item(128), 128, s, L);
 }
 
 }  // namespace mmr

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "launch.h"
 
 namespace mmr {
 
@@ -46,6 +47,7 @@ __device__ __forceinline__ void cursor_step(Cursor &c, uint32_t pw, uint32_t w) 
 }
 
 __global__ void __launch_bounds__(kRgbThreads) rgb_kernel(RgbLaunch L) {
+    begin_kernel();
     __shared__ uint32_t s_job;
     __shared__ __align__(16) uint32_t s_out[kRgbThreads * kRgbPix * 3 / 4];
     if (threadIdx.x == 0) {
@@ -143,7 +145,7 @@ uint32_t rgb_ctas(uint32_t w, uint32_t h) { return (uint32_t)(((uint64_t)w * h +
 
 void launch_rgb(const RgbLaunch &L, cudaStream_t s) {
     if (L.n_ctas == 0) return;
-    rgb_kernel<<<L.n_ctas, kRgbThreads, 0, s>>>(L);
+    launch_next(rgb_kernel, L.n_ctas, kRgbThreads, s, L);
 }
 
 }  // namespace mmr
