@@ -119,6 +119,7 @@ constexpr int kEncBlocksPerTile = 32;                    // blocks per CTA step,
 constexpr int kEncThreads = 8 * kEncBlocksPerTile;
 constexpr int kTieQueue = kEncThreads;                   // packed binary64 work: a thread per entry
 constexpr int kRowStride = 12;                           // floats per row: 16-byte stores of 8 rows hit all banks
+constexpr int kOutStride = 80;                           // int16 per block: four blocks' scattered stores least alike
 constexpr int kTileStride = 8 * kRowStride + 8;          // per block: four blocks' column loads on distinct banks
 
 // Where block blk's samples come from.
@@ -175,14 +176,21 @@ __device__ __forceinline__ uint2 source_row(const BlockSource &B, uint32_t r) {
 // of an encode of 60 1080p 4:2:2 frames of integer content. They are listed in
 // shared memory instead and recomputed a thread each once about 256 are waiting
 // (363k of 249 M coefficients): 0.73 ms against 5.67 ms, with the even/odd passes.
-__global__ void __launch_bounds__(kEncThreads) fdct_kernel(EncLaunch L, uint64_t n_tiles) {
+//
+// A tile's samples are loaded while the one before it is transformed, and whether enough
+// coefficients are listed is agreed on at its one barrier; scattered 2-byte stores of a
+// warp's four blocks go to rows 40 words apart (with 32 each bank was taken four times):
+// 735 -> 598 us for those 60 frames, issue-bound now (63 % of the slots).
+__global__ void __launch_bounds__(kEncThreads, 4) fdct_kernel(EncLaunch L, uint64_t n_tiles) {
     __shared__ __align__(16) float s_t[kEncBlocksPerTile * kTileStride];
-    __shared__ __align__(16) int16_t s_out[kEncBlocksPerTile][64];  // blocks in zigzag order
+    __shared__ __align__(16) int16_t s_out[kEncBlocksPerTile][kOutStride];  // blocks in zigzag order
     __shared__ double s_m64[64];
+    __shared__ float s_rq[2][64];
     __shared__ unsigned long long s_tie[kTieQueue + 64 * kEncBlocksPerTile];  // block << 6 | v * 8 + u
-    __shared__ uint32_t s_ties, s_frame;
+    __shared__ uint32_t s_ties;
     const int lb = threadIdx.x >> 3, r = threadIdx.x & 7;
     if (threadIdx.x < 64) s_m64[threadIdx.x] = c_m64[threadIdx.x];
+    if (threadIdx.x < 128) s_rq[threadIdx.x >> 6][threadIdx.x & 63] = L.rq[threadIdx.x];
     if (threadIdx.x == 0) s_ties = 0;
     uint32_t zzcol[2];  // zigzag positions of this thread's column, byte v of the pair
     {
@@ -192,63 +200,22 @@ __global__ void __launch_bounds__(kEncThreads) fdct_kernel(EncLaunch L, uint64_t
         zzcol[0] = w[0];
         zzcol[1] = w[1];
     }
-    for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        if (threadIdx.x == 0) s_frame = frame_of_block(L, tile * kEncBlocksPerTile);
-        __syncthreads();
-        const uint64_t blk = tile * kEncBlocksPerTile + lb;
-        const bool valid = blk < L.n_blocks;
-        float *tb = s_t + lb * kTileStride;
-        float mag = 0.0f;
-        uint32_t tq = 0;
-        if (valid) {  // row pass: t[r][u] = sum_x M[x][u] S[r][x]
-            uint32_t f = s_frame;
-            while (f + 1 < L.n_frames && L.frames[f + 1].block_base <= blk) f++;
-            const BlockSource B = block_source(L.frames[f], blk);
-            tq = B.tq;
-            const uint2 w = source_row(B, r);
-            float s[8], t[8];
-#pragma unroll
-            for (int x = 0; x < 8; x++) {  // 2^23 + sample as a float, then centred
-                const uint32_t b = __byte_perm(x < 4 ? w.x : w.y, 0x4B00u, 0x5440 | (x & 3));
-                s[x] = __uint_as_float(b) - 8388736.0f;
-                mag += fabsf(s[x]);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) t[u] = fdct_row(s, u);
-            reinterpret_cast<float4 *>(tb + r * kRowStride)[0] = make_float4(t[0], t[1], t[2], t[3]);
-            reinterpret_cast<float4 *>(tb + r * kRowStride)[1] = make_float4(t[4], t[5], t[6], t[7]);
-        }
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) mag += __shfl_xor_sync(0xffffffffu, mag, o);
-        __syncwarp();  // a warp's blocks are its own
-        if (valid) {   // column pass of column u = r, quantisation
-            const int u = r;
-            const float *rq = L.rq + tq * 64;
-            const float b = mag * kFdctBound;
-            float t[8];
-#pragma unroll
-            for (int y = 0; y < 8; y++) t[y] = tb[y * kRowStride + u];
-            uint32_t open = 0;
-#pragma unroll
-            for (int v = 0; v < 8; v++) {
-                bool unsure;
-                int k = fdct_round(fdct_column(t, v), b, rq[v * 8 + u], unsure);
-                open |= (unsure ? 1u : 0u) << v;
-                if (v | u) k = min(max(k, -1023), 1023);  // encode_scan (encoder.rs:372-374)
-                s_out[lb][(zzcol[v >> 2] >> (8 * (v & 3))) & 63] = (int16_t)k;
-            }
-            if (open) {
-                uint32_t at = atomicAdd(&s_ties, (uint32_t)__popc(open));
-                for (; open; open &= open - 1) s_tie[at++] = blk << 6 | (uint32_t)((__ffs(open) - 1) * 8 + u);
-            }
-        }
-        __syncwarp();
-        if (valid)  // 16 bytes per thread: the block's 128 bytes in one coalesced row
-            reinterpret_cast<uint4 *>(L.coef + blk * 64)[r] = reinterpret_cast<const uint4 *>(s_out[lb])[r];
-        __syncthreads();  // the list is complete, the coefficients are written
+    // row r of the thread's block of a tile, and the block's quantisation table
+    uint64_t blk = (uint64_t)blockIdx.x * kEncBlocksPerTile + lb;
+    uint32_t f = blk < L.n_blocks ? frame_of_block(L, blk) : 0, next_tq = 0;
+    uint2 next = make_uint2(0, 0);
+    auto fetch = [&](uint64_t at) {
+        if (at >= L.n_blocks) return;
+        while (f + 1 < L.n_frames && L.frames[f + 1].block_base <= at) f++;
+        const BlockSource B = block_source(L.frames[f], at);
+        next_tq = B.tq;
+        next = source_row(B, r);
+    };
+    fetch(blk);
+    __syncthreads();
+    // recomputes the listed coefficients, a thread each
+    auto settle = [&]() {
         const uint32_t n = s_ties;
-        const bool last = tile + gridDim.x >= n_tiles;
-        if (n < (uint32_t)kTieQueue && !(last && n)) continue;
         for (uint32_t i = threadIdx.x; i < n; i += kEncThreads) {
             const uint64_t eb = s_tie[i] >> 6;
             const int nat = (int)(s_tie[i] & 63);
@@ -265,7 +232,63 @@ __global__ void __launch_bounds__(kEncThreads) fdct_kernel(EncLaunch L, uint64_t
             if (n) atomicAdd(L.exact, (unsigned long long)n);
             s_ties = 0;
         }
+        __syncthreads();
+    };
+    for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const bool valid = blk < L.n_blocks;
+        float *tb = s_t + lb * kTileStride;
+        float mag = 0.0f;
+        const uint32_t tq = next_tq;
+        const uint2 w = next;
+        fetch(blk + (uint64_t)gridDim.x * kEncBlocksPerTile);
+        if (valid) {  // row pass: t[r][u] = sum_x M[x][u] S[r][x]
+            float s[8], t[8];
+#pragma unroll
+            for (int x = 0; x < 8; x++) {  // 2^23 + sample as a float, then centred
+                const uint32_t b = __byte_perm(x < 4 ? w.x : w.y, 0x4B00u, 0x5440 | (x & 3));
+                s[x] = __uint_as_float(b) - 8388736.0f;
+                mag += fabsf(s[x]);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) t[u] = fdct_row(s, u);
+            reinterpret_cast<float4 *>(tb + r * kRowStride)[0] = make_float4(t[0], t[1], t[2], t[3]);
+            reinterpret_cast<float4 *>(tb + r * kRowStride)[1] = make_float4(t[4], t[5], t[6], t[7]);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) mag += __shfl_xor_sync(0xffffffffu, mag, o);
+        __syncwarp();  // a warp's blocks are its own
+        bool full = false;
+        if (valid) {   // column pass of column u = r, quantisation
+            const int u = r;
+            const float *rq = s_rq[tq];
+            const float b = mag * kFdctBound;
+            float t[8];
+#pragma unroll
+            for (int y = 0; y < 8; y++) t[y] = tb[y * kRowStride + u];
+            uint32_t open = 0;
+#pragma unroll
+            for (int v = 0; v < 8; v++) {
+                bool unsure;
+                int k = fdct_round(fdct_column(t, v), b, rq[v * 8 + u], unsure);
+                open |= (unsure ? 1u : 0u) << v;
+                if (v | u) k = min(max(k, -1023), 1023);  // encode_scan (encoder.rs:372-374)
+                s_out[lb][(zzcol[v >> 2] >> (8 * (v & 3))) & 63] = (int16_t)k;
+            }
+            if (open) {
+                const uint32_t more = (uint32_t)__popc(open);
+                uint32_t at = atomicAdd(&s_ties, more);
+                full = at + more >= (uint32_t)kTieQueue;
+                for (; open; open &= open - 1) s_tie[at++] = blk << 6 | (uint32_t)((__ffs(open) - 1) * 8 + u);
+            }
+        }
+        __syncwarp();
+        if (valid)  // 16 bytes per thread: the block's 128 bytes in one coalesced row
+            reinterpret_cast<uint4 *>(L.coef + blk * 64)[r] = reinterpret_cast<const uint4 *>(s_out[lb])[r];
+        blk += (uint64_t)gridDim.x * kEncBlocksPerTile;
+        // (the same answer for all: the entry that fills the queue is added once)
+        if (__syncthreads_or(full)) settle();  // the list is complete, the coefficients are written
     }
+    settle();
 }
 
 // ------------------------------------------------------------- Huffman ---
