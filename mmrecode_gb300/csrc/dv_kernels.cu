@@ -421,7 +421,7 @@ __device__ __forceinline__ void store_row4(uint8_t *dst, uint32_t row) {
 // of one frame (frames start at multiples of 4 blocks: 8100 and 9720 blocks per frame),
 // found by one division where all frames are of one system; the eight threads of a
 // block synchronise through their warp only. Issue-bound (two thirds) with waits for the
-// levels between: 36 registers for 28 CTAs of 64 per SM (1000 NTSC frames: 1.82 ms, with
+// levels between: 32 registers for 28 CTAs of 64 per SM (1000 NTSC frames: 1.82 ms, with
 // 52 registers 1.93).
 constexpr int kBlockStride = 72;  // ints or floats per block: four blocks' column accesses on distinct banks
 
@@ -504,7 +504,8 @@ __global__ void __launch_bounds__(kIdctThreads, 28) dv_idct_kernel(DvLaunch L) {
 
 void launch_dv_decode(const DvLaunch &L, cudaStream_t s) {
     const uint32_t steps = (L.n_segments + kSegWarps - 1) / kSegWarps;
-    if (steps) launch_next(segment_kernel, std::min<uint32_t>(steps, 152 * kSegCtasPerSm), kSegThreads, s, L);
+    // (an ordinary launch: what comes before it on the stream may be the caller's)
+    if (steps) segment_kernel<<<std::min<uint32_t>(steps, 152 * kSegCtasPerSm), kSegThreads, 0, s>>>(L);
     if (L.n_frames) launch_next(dv_resolve_kernel, (L.n_frames + 127) / 128, 128, s, L);
 }
 

@@ -1311,7 +1311,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                 launches_ += fused_launches(FL[v]);
             }
             launch_jpeg_idct_rgb(JL, FL, s);
-            launches_ += (JL.n_tiles ? 3 : 0) + (JL.n_slots ? jpeg_slice_launches(JL) : 0) +
+            launches_ += (JL.n_tiles ? 2 : 0) + (JL.n_slots ? jpeg_slice_launches(JL) : 0) +
                          (n_items > JL.n_items_small ? 1 : 0) + 1 + (JL.n_idct_ctas ? 2 : 0);
         } else {
             stamp(I.ev[2]);

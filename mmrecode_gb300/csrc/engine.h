@@ -93,8 +93,8 @@ struct EngineTimes {
     uint64_t idct_exact_samples = 0;  // MJPEG samples recomputed in exact binary64 order
     uint32_t graph_replays = 0;       // batches whose launches replayed a captured CUDA graph
     uint64_t slices = 0;              // slices of the chunked entropy decoder
-    uint64_t slices_redone = 0;       // of which the final decode pass redid (the rest were placed)
-    uint64_t slices_redone_whole = 0; // of those, redone from their start (no usable speculative part)
+    uint64_t slices_redone = 0;       // of which the sync passes decoded again
+    uint64_t slices_redone_whole = 0; // of those, to their end (no speculative decode was met)
 };
 
 class Engine {

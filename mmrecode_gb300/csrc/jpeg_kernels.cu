@@ -1,6 +1,6 @@
 // MJPEG decode kernels for sm_103a.
 //
-//   scan_count / scan_prefix / scan_emit  marker scan of the entropy-coded data
+//   scan_count / scan_emit  marker scan of the entropy-coded data
 //       (crates/codecs/mjpeg/src/parser.rs:373-414 and the byte-unstuffing of
 //       entropy.rs:143-165), parallel over 4 KiB tiles: finds the terminating
 //       marker, lists RSTn markers in order and writes the unstuffed bytes.
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(256) idct_fixup_kernel(JpegLaunch L) {
 void launch_jpeg_scan(const JpegLaunch &L, cudaStream_t s) {
     if (L.n_tiles == 0) return;
     const uint32_t ctas = (L.n_tiles + kScanThreads / 32 - 1) / (kScanThreads / 32);
-    launch_next(scan_count_kernel, ctas, kScanThreads, s, L);
+    scan_count_kernel<<<ctas, kScanThreads, 0, s>>>(L);  // (after the uploads)
     launch_next(scan_emit_kernel, ctas, kScanThreads, s, L);
 }
 

@@ -465,14 +465,14 @@ __device__ __forceinline__ void spec_slice(const JpegLaunch &L, LeanSmem &S, con
     L.sync[slot] = out;
 }
 
-__global__ void __launch_bounds__(kSliceThreads) slice_spec_kernel(JpegLaunch L) {
+__global__ void __launch_bounds__(kSliceThreads) slice_spec_kernel(JpegLaunch L, uint32_t spread) {
     begin_kernel();
     __shared__ LeanSmem S;
-    const uint32_t slot = blockIdx.x * kSliceThreads + threadIdx.x;
+    const uint32_t at = blockIdx.x * kSliceThreads + threadIdx.x, slot = at >> spread;
     SliceRef s;
     // (a last slice has no exit, and the decode pass takes its start from its predecessor)
     const uint32_t path = blockIdx.y;
-    bool work = slice_ref(L, slot, s) && !s.last;
+    bool work = slot << spread == at && slice_ref(L, slot, s) && !s.last;
     if (work) {
         S.frame = s.v.frame;  // the same for all
         work = path == 0 || (s.j != 0 && path < L.frames[s.v.frame].paths);
@@ -1009,13 +1009,13 @@ __device__ __forceinline__ void decode_slices(const JpegLaunch &L, DecodeSmem &S
 }
 
 template <int kSteps>
-__global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch L) {
+__global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch L, uint32_t spread) {
     begin_kernel();
     __shared__ DecodeSmem S;
-    const uint32_t tid = threadIdx.x, slot = blockIdx.x * kSliceThreads + tid;
+    const uint32_t tid = threadIdx.x, at = blockIdx.x * kSliceThreads + tid, slot = at >> spread;
     SliceRef s;
     s.item = 0;
-    const bool used = slice_ref(L, slot, s);
+    const bool used = slot << spread == at && slice_ref(L, slot, s);
     // the blocks this slice decodes
     uint32_t n = 0, base = 0;
     unsigned long long from = pack_state(0, 0);
@@ -1132,6 +1132,19 @@ int jpeg_slice_launches(const JpegLaunch &L) {
     return 5 + (int)passes + (passes > 1 ? 1 : 0);
 }
 
+// Small grids leave most of the GPU idle while each warp settles and writes its 32 lanes'
+// blocks one group after another: there one thread in 2^spread takes a slice, as long as
+// that makes no more than two CTAs per SM (320x240: one thread in four, 174 -> 164 us; 30 VGA
+// frames: one in two, 347 -> 342; with up to four CTAs per SM a single 1080p frame gains
+// nothing and 60 720p ones lose 3 %).
+constexpr uint32_t kSpreadCtas = 2 * 152, kMostSpread = 2;
+
+static uint32_t slice_spread(uint32_t ctas) {
+    uint32_t spread = 0;
+    while (spread < kMostSpread && ctas << (spread + 1) <= kSpreadCtas) spread++;
+    return spread;
+}
+
 void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks, bool capturing) {
     auto mark = [&](int k) {
         if (marks) capturing ? cudaEventRecordWithFlags(marks[k], s, cudaEventRecordExternal) : cudaEventRecord(marks[k], s);
@@ -1141,7 +1154,8 @@ void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks,
     auto per_item = [&](uint32_t items) { return (L.n_items_small + items - 1) / items; };
     if (run) {
         launch_next(slice_plan_kernel, per_item(kPlanThreads) + L.n_luts, kPlanThreads, s, L);
-        launch_next(slice_spec_kernel, dim3(grid, L.paths), kSliceThreads, s, L);
+        const uint32_t spread = slice_spread(grid * L.paths);
+        launch_next(slice_spec_kernel, dim3(grid << spread, L.paths), kSliceThreads, s, L, spread);
     }
     mark(0);
     if (run) {
@@ -1153,7 +1167,8 @@ void launch_jpeg_slices(const JpegLaunch &L, cudaStream_t s, cudaEvent_t *marks,
     }
     mark(1);
     // (one path per slice: the long slices of a large batch)
-    if (run) launch_next(L.paths == 1 ? slice_decode_kernel<kDecodeStepsLong> : slice_decode_kernel<kDecodeSteps>, grid, kSliceThreads, s, L);
+    const uint32_t spread = slice_spread(grid);
+    if (run) launch_next(L.paths == 1 ? slice_decode_kernel<kDecodeStepsLong> : slice_decode_kernel<kDecodeSteps>, grid << spread, kSliceThreads, s, L, spread);
     mark(2);
     if (run) launch_next(slice_resolve_kernel, per_item(128), 128, s, L);
 }

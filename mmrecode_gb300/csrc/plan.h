@@ -29,7 +29,8 @@ struct HuffLut {
     // fastv with two AC symbols in one entry where both lie whole within the next
     // 11 bits, the first not EOB, with levels in -64..63 and -32..31:
     //   level2 << 26 | level1 << 19 | advance2 << 14 | kFastPair | advance1 << 5 | total bits
-    // (advance2 0: the second is EOB). The same as fastv for DC tables.
+    // (advance2 0: the second is EOB). The same as fastv for DC tables. No kernel reads
+    // them any more (skip, below); the table tests check them with the rest of the record.
     uint32_t fastp[1 << kHuffFastBits];
     int32_t maxcode[18];   // largest code of each length 1..16, -1 if none
     int32_t valptr[18];    // symbol index of a length's first code, minus that code
@@ -58,8 +59,9 @@ struct HuffCanon {
 //         level, 16 for ZRL, kSymEob for EOB, so that a block ends with an index of 64
 //         or from 97 to 159 and an overrun lies between); 0 for bits no code matches
 //         and for symbols the reference rejects.
-//   skip  for decodes that only follow positions, made on the device (skip_entry_of). Byte 3: advance of the
-//         first symbol, byte 2: its bits, magnitude included; bytes 1 and 0: the same
+//   skip  for decodes that only follow positions, made on the device (skip_entry_of).
+//         Byte 3: advance of the first symbol, byte 2: its bits, magnitude included;
+//         bytes 1 and 0: the same
 //         of the first two where the second's code lies within the 11 bits too (else of
 //         the first); 0 where sym is 0.
 constexpr uint32_t kSymEob = 96;

@@ -334,9 +334,9 @@ uint64_t Server::estimate_bytes(const Item &it) {
     const Probe p = probe_packet(it.codec, it.data, it.len);
     const uint64_t planar = p.status == kOk ? p.planar_bytes : 0;
     const uint64_t out = p.status == kOk ? (it.output == kOutRgb24 ? p.rgb_bytes : planar) : 0;
-    // tokens and slice records (~8 B per compressed byte at the smallest automatic
-    // slice), coefficients in place and in the speculative decode's scratch
-    // (~4.5 B per sample), planes, fixed scratch
+    // tokens and slice records (~8 B per compressed byte), coefficients (~2.25 B per
+    // sample) and as much again for the records of small batches, whose slices are short
+    // and decoded from several guesses; planes, fixed scratch
     uint64_t b = 8 * (uint64_t)it.len + (planar * 9) / 2 + planar + 65536;
     if (!it.out_on_device) b += out;  // staged output
     return b;
