@@ -221,7 +221,7 @@ __device__ __forceinline__ uint32_t frame_of(const DvLaunch &L, uint32_t g) {
 }
 
 __global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ SegSmem S;
     for (uint32_t i = threadIdx.x; i < (uint32_t)kDvVlcEntries; i += kSegThreads) S.vlc[i] = __ldg(L.vlc + i);
     for (uint32_t i = threadIdx.x; i < 128; i += kSegThreads) {
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kSegThreads, kSegCtasPerSm) segment_kernel(DvL
 }
 
 __global__ void dv_resolve_kernel(DvLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= L.n_frames) return;
     DvState *st = &L.states[f];
@@ -426,7 +426,7 @@ __device__ __forceinline__ void store_row4(uint8_t *dst, uint32_t row) {
 constexpr int kBlockStride = 72;  // ints or floats per block: four blocks' column accesses on distinct banks
 
 __global__ void __launch_bounds__(kIdctThreads, 28) dv_idct_kernel(DvLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ __align__(16) int32_t s_c[kIdctBlocks][kBlockStride];
     __shared__ __align__(16) float s_h[kIdctBlocks][kBlockStride];
     const int lane = threadIdx.x & 31, lb = threadIdx.x >> 3, r = threadIdx.x & 7;

@@ -17,6 +17,7 @@
 #include "huffman_lut.h"
 #include "jpeg_syntax.h"
 #include "kernels.h"
+#include "launch.h"
 #include "plan.h"
 #include "tables.h"
 
@@ -1274,6 +1275,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         JL.idct_cta_first = reinterpret_cast<const uint32_t *>(db + o_idctcta);
         JL.n_idct_ctas = idct_cta.back();
         JL.idct_tiles = idct_tiles;
+        JL.early = blocks + dv_blocks <= kEarlyBlocks;
         JL.n_blocks = blocks;
         JL.item_ok = reinterpret_cast<uint32_t *>(db + o_itemok);
         JL.fix = I.d_fix.as<ulonglong2>();
@@ -1323,6 +1325,7 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         DL.frames = reinterpret_cast<const DvFrame *>(db + o_dframes);
         DL.states = reinterpret_cast<DvState *>(db + o_dstates);
         DL.n_frames = (uint32_t)dframes.size();
+        DL.early = blocks + dv_blocks <= kEarlyBlocks;
         DL.seg_first = reinterpret_cast<const uint32_t *>(db + o_segfirst);
         DL.n_segments = seg_first.back();
         DL.seg_err = I.d_segerr.as<uint8_t>();

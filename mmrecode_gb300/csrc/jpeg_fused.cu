@@ -194,7 +194,7 @@ __device__ __forceinline__ void strip_to_rgb(const JFrame &F, const FusedJob &J,
 // settled before the colour conversion, a warp per block (settle_samples).
 template <int HM, int VM, int NM>
 __global__ void __launch_bounds__(FusedShape<HM, VM, NM>::THREADS, 1024 / FusedShape<HM, VM, NM>::THREADS) idct_rgb_kernel(JpegLaunch L, FusedLaunch FL) {
-    begin_kernel();
+    begin_kernel(L.early);
     using Sh = FusedShape<HM, VM, NM>;
     __shared__ __align__(16) FusedSmem<HM, VM, NM> S;
     __shared__ uint32_t s_job;

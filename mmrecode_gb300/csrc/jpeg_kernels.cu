@@ -148,7 +148,7 @@ __device__ __forceinline__ uint32_t group_base(const JpegLaunch &L, uint32_t f) 
 }
 
 __global__ void __launch_bounds__(kScanThreads) scan_count_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     Tile T;
     if (!warp_tile(L, T)) return;
     const JFrame &F = L.frames[T.frame];
@@ -212,7 +212,7 @@ __device__ __forceinline__ uint4 drop_byte(const uint4 &v, uint32_t i) {
 }
 
 __global__ void __launch_bounds__(kScanThreads) scan_emit_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     // a warp's tokens, staged at their destination's offset within a 16-byte line
     constexpr uint32_t kLines = kScanTile / 16 + 1;
     __shared__ uint4 s_line[kScanThreads / 32][kLines + 1];  // (one more: a chunk is written as five words)
@@ -451,7 +451,7 @@ __device__ void decode_interval(const JpegLaunch &L, uint32_t item, int16_t *sta
 
 template <int MAXC>
 __global__ void __launch_bounds__(kEntropyThreads) entropy_kernel(JpegLaunch L, uint32_t first, uint32_t count) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ __align__(16) int16_t s_stage[kEntropyThreads * kStageStride];
     __shared__ uint8_t s_zz[64];
     int4 *mine = reinterpret_cast<int4 *>(s_stage + threadIdx.x * kStageStride);
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kEntropyThreads) entropy_kernel(JpegLaunch L, 
 }
 
 __global__ void resolve_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= L.n_frames) return;
     const JFrame &F = L.frames[f];
@@ -502,7 +502,7 @@ __device__ __forceinline__ uint32_t find_range(const JpegLaunch &L, uint64_t g) 
 // Per CTA and tile it waited for a search over the ranges, four more dependent loads and the
 // levels; now once for up to four tiles (60 720p frames: 218 -> 154 us, 30 VGA frames 34 -> 26).
 __global__ void __launch_bounds__(kIdctThreads, 4) idct_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ __align__(16) float s_f[kIdctBlocks * kIdctStride];
     __shared__ __align__(16) float s_q[64];
     __shared__ float4 s_m[16];
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kIdctThreads, 4) idct_kernel(JpegLaunch L) {
 // block: its exact coefficients into shared memory, then settle_samples
 // (fixed-point value, or the reference order for genuine near-ties).
 __global__ void __launch_bounds__(256) idct_fixup_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ int32_t s_c[8][64];
     const uint32_t n = *L.fix_count;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

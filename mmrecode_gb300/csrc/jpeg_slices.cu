@@ -242,7 +242,7 @@ constexpr int kPlanThreads = 128;
 
 // The last n_luts CTAs make the skip tables (host code took 13 us for one).
 __global__ void __launch_bounds__(kPlanThreads) slice_plan_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     if (blockIdx.x + L.n_luts >= gridDim.x) {
         const LutMeta m = L.lut_meta[gridDim.x - 1 - blockIdx.x];
         for (uint32_t x = threadIdx.x; x < m.len; x += kPlanThreads)
@@ -466,7 +466,7 @@ __device__ __forceinline__ void spec_slice(const JpegLaunch &L, LeanSmem &S, con
 }
 
 __global__ void __launch_bounds__(kSliceThreads) slice_spec_kernel(JpegLaunch L, uint32_t spread) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ LeanSmem S;
     const uint32_t at = blockIdx.x * kSliceThreads + threadIdx.x, slot = at >> spread;
     SliceRef s;
@@ -575,7 +575,7 @@ __device__ __forceinline__ void resync_slice(const JpegLaunch &L, LeanSmem &S, c
 // what another CTA still changes there is the next pass's, and after the last pass
 // slice_fix_kernel's, from the interval's first such slice on.
 __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L, bool first_pass, bool last_pass) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ LeanSmem S;
     __shared__ unsigned long long s_exit[kSliceThreads + 1];  // of the slice before the CTA's first, then of each
     const uint32_t tid = threadIdx.x, slot = blockIdx.x * kSliceThreads + tid;
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L,
 
 // One warp per interval that the sync passes left unsettled.
 __global__ void __launch_bounds__(kSliceThreads) slice_fix_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ LeanSmem S;
     if (*L.sync_left == 0) return;
     const uint32_t lane = threadIdx.x & 31;
@@ -796,7 +796,7 @@ __device__ __forceinline__ void prefix_run(const JpegLaunch &L, const IvInfo &v,
 // consecutive slices (a run of slices per thread touched a line per lane and load: 250 us
 // against 147 in a step of 64 mixed frames).
 __global__ void __launch_bounds__(kPrefixThreads) slice_prefix_kernel(JpegLaunch L, uint32_t per_cta) {
-    begin_kernel();
+    begin_kernel(L.early);
     constexpr uint32_t kWarps = kPrefixThreads / 32;
     __shared__ SliceSums s_warp[kWarps];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1010,7 +1010,7 @@ __device__ __forceinline__ void decode_slices(const JpegLaunch &L, DecodeSmem &S
 
 template <int kSteps>
 __global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch L, uint32_t spread) {
-    begin_kernel();
+    begin_kernel(L.early);
     __shared__ DecodeSmem S;
     const uint32_t tid = threadIdx.x, at = blockIdx.x * kSliceThreads + tid, slot = at >> spread;
     SliceRef s;
@@ -1087,7 +1087,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch 
 // --------------------------------------------------------------- resolve ---
 
 __global__ void slice_resolve_kernel(JpegLaunch L) {
-    begin_kernel();
+    begin_kernel(L.early);
     const uint32_t item = blockIdx.x * blockDim.x + threadIdx.x;
     if (item >= L.n_items_small) return;
     const IvInfo v = L.ivs[item];

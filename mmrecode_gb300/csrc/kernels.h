@@ -19,6 +19,7 @@ struct JpegLaunch {
     const JFrame *frames;        // device
     JState *states;              // device
     uint32_t n_frames;
+    bool early;                  // begin_kernel's (a small batch)
     const uint32_t *tile_first;  // n_frames + 1 prefix of marker-scan tiles
     uint32_t n_tiles;
     unsigned long long *tile_cnt;    // per tile: tokens, and restart markers << 32
@@ -120,6 +121,7 @@ struct DvLaunch {
     const uint32_t *vlc;         // two-level VLC table
     const long long *fixw;       // fixed-point transform weights: 8-8 then 2-4-8 (exact_fixed.h)
     const uint32_t *place;       // where blocks land (dv_layout.h)
+    bool early;                  // begin_kernel's (a small batch)
     uint64_t n_blocks;           // less than 2^32
     uint32_t frame_blocks;       // of every frame, 0 when they differ
     uint32_t *item_ok;

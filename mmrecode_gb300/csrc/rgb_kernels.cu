@@ -47,7 +47,7 @@ __device__ __forceinline__ void cursor_step(Cursor &c, uint32_t pw, uint32_t w) 
 }
 
 __global__ void __launch_bounds__(kRgbThreads) rgb_kernel(RgbLaunch L) {
-    begin_kernel();
+    begin_kernel(false);
     __shared__ uint32_t s_job;
     __shared__ __align__(16) uint32_t s_out[kRgbThreads * kRgbPix * 3 / 4];
     if (threadIdx.x == 0) {
