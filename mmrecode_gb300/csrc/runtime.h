@@ -73,6 +73,7 @@ public:
     int device() const { return device_; }
     Engine &engine(int k) { return *engines_[k]; }
     static constexpr size_t kMinChunk = 16;
+    static constexpr uint64_t kOneChunkBytes = 4ull << 30;
     static constexpr size_t kMinStagedChunk = 4, kStagedPartBytes = 48u << 20;
 
 private:
