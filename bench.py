@@ -760,7 +760,7 @@ def small_legs(args, local, pool, cores, m, _lib, peak, peak_kind, figures):
         if label == "mjpeg":
             blocks = stage[-1]["jpeg_blocks"]
             st = {k: avg(k + "_ms") for k in ("scan", "entropy", "idct", "slice_spec", "slice_sync", "slice_decode")}
-            ent_bytes = in_bytes + blocks * 130
+            ent_bytes = 2 * in_bytes + blocks * 132
             achieved = ent_bytes / (st["entropy"] / 1e3) / 1e9
             leg["stage_ms"] = st
             leg["roofline"] = {"bound": "issue", "kernel": "slice_spec_kernel+slice_sync+slice_decode (entropy stage)",
@@ -1003,11 +1003,12 @@ def main():
                                               "slice_spec", "slice_sync", "slice_decode")}
     # algorithmic bytes per launch of each kernel of the step (every kernel runs once per step)
     kernels = {
-        # reads the compressed tokens, stores the 64 int16 levels and the DC difference of
-        # every block it owns (the final levels of nearly all blocks)
-        "slice_spec_kernel": (stage_times["slice_spec"], in_bytes + blocks * 130),
-        # reads levels, dequantised DC and the block map entry, writes interleaved RGB
-        "idct_rgb_kernel": (stage_times["idct"], blocks * 136 + n * rgb_bytes),
+        # reads the compressed tokens, once per guess (one in a batch of this size)
+        "slice_spec_kernel": (stage_times["slice_spec"], in_bytes),
+        # reads them again from the true states, stores every block's levels and DC
+        "slice_decode_kernel": (stage_times["slice_decode"], in_bytes + blocks * 132),
+        # reads levels and dequantised DC, writes interleaved RGB
+        "idct_rgb_kernel": (stage_times["idct"], blocks * 132 + n * rgb_bytes),
     }
 
     def roof(name):

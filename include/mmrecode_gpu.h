@@ -118,12 +118,12 @@ typedef struct mmr_gpu_batch_stats {
     /* inside entropy_ms: speculative slice decode, slice synchronisation + block prefix, final decode */
     double slice_spec_ms, slice_sync_ms, slice_decode_ms;
     uint32_t graph_replays; /* parts of the batch whose launches replayed a captured CUDA graph */
-    /* slices of the chunked entropy decoder, and those whose levels the final decode
-       pass redid instead of taking the speculative decode's */
+    /* slices of the chunked entropy decoder, and those whose true start no speculative
+       decode began with: decoded again by the synchronisation passes */
     uint64_t slices, slices_redone;
-    /* inside dv_ms: DIF identifier check + segment (VLC) decode, then transform + placement */
+    /* inside dv_ms: segment (VLC) decode with the DIF identifier check, then transform + placement */
     double dv_segment_ms, dv_idct_ms;
-    /* of slices_redone, those the final decode redid from their start */
+    /* of slices_redone, those that met no speculative decode before their end */
     uint64_t slices_redone_whole;
 } mmr_gpu_batch_stats;
 
