@@ -35,6 +35,7 @@
 #include "encode.h"
 #include "encode_gpu.h"
 #include "fdct_core.h"
+#include "launch.h"
 #include "tables.h"
 
 namespace mmr {
@@ -402,6 +403,7 @@ __device__ __forceinline__ const EncFrame &frame_from(const EncLaunch &L, uint32
 }
 
 __global__ void __launch_bounds__(kSymThreads) bits_kernel(EncLaunch L) {
+    begin_kernel(false);
     __shared__ SymSmem<true> S;
     load_symbols(L, S);
     const uint64_t blk = (uint64_t)blockIdx.x * kSymThreads + threadIdx.x;
@@ -422,6 +424,7 @@ __device__ __forceinline__ uint64_t segment_block(const EncFrame &F, uint32_t j)
 }
 
 __global__ void segment_kernel(EncLaunch L) {
+    begin_kernel(false);
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= L.n_segs) return;
     const EncFrame &F = L.frames[frame_of_segment(L, s)];
@@ -522,6 +525,7 @@ __device__ __forceinline__ void chunk_of(const EncLaunch &L, const ChunkSmem &S,
 }
 
 __global__ void __launch_bounds__(256) ff_count_kernel(EncLaunch L, uint64_t n_chunks) {
+    begin_kernel(false);
     __shared__ ChunkSmem S;
     chunk_range(L, n_chunks, S);
     const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -579,6 +583,7 @@ __device__ __forceinline__ uint8_t *frame_dst(const EncLaunch &L, uint32_t f) {
 // followed by its marker (RSTn, or EOI after the last); the frame's header into a
 // device buffer. The last CTA to finish lays out the frames staged for host buffers.
 __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(EncLaunch L) {
+    begin_kernel(false);
     __shared__ uint64_t s_total;
     __shared__ bool s_last;
     const uint32_t f = blockIdx.x;
@@ -622,6 +627,7 @@ __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(EncLaunch L) {
 constexpr int kEmitThreads = 256;
 
 __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EncLaunch L, uint64_t n_chunks) {
+    begin_kernel(false);
     __shared__ ChunkSmem S;
     __shared__ __align__(16) uint8_t s_out[kEmitThreads * 34 + 32];
     __shared__ uint8_t *s_dst;
@@ -694,6 +700,7 @@ constexpr uint64_t kScanTile = (uint64_t)kScanThreads * kScanItems;
 // writes the grand total.
 __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_t *in, uint64_t n, uint64_t *part,
                                                                    uint64_t *total, uint32_t *done) {
+    begin_kernel(false);
     __shared__ uint64_t s_total;
     __shared__ bool s_last;
     const uint64_t base = blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
@@ -724,6 +731,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_
 
 __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t *in, uint64_t n,
                                                                     const uint64_t *part, uint64_t *out) {
+    begin_kernel(false);
     __shared__ uint64_t s_total;
     const uint64_t base = blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
@@ -746,8 +754,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
 // done: a zeroed counter); n > 0
 void exclusive_scan(const uint32_t *in, uint64_t n, uint64_t *out, uint64_t *part, uint32_t *done, cudaStream_t s) {
     const unsigned tiles = (unsigned)((n + kScanTile - 1) / kScanTile);
-    scan_reduce_kernel<<<tiles, kScanThreads, 0, s>>>(in, n, part, out + n, done);
-    scan_apply_kernel<<<tiles, kScanThreads, 0, s>>>(in, n, part, out);
+    launch_next(scan_reduce_kernel, tiles, kScanThreads, s, in, n, part, out + n, done);
+    launch_next(scan_apply_kernel, tiles, kScanThreads, s, in, n, part, out);
 }
 
 }  // namespace
@@ -1066,9 +1074,9 @@ int32_t GpuJpegEncoder::encode(EncodeItem *items, size_t n, const JpegEncodeOpti
         const uint64_t tiles = (blocks + kEncBlocksPerTile - 1) / kEncBlocksPerTile;
         // one wave of resident CTAs (64 registers: four per SM)
         fdct_kernel<<<(unsigned)std::min<uint64_t>(tiles, 152 * 4), kEncThreads, 0, I.s>>>(L, tiles);
-        bits_kernel<<<bgrid, kSymThreads, 0, I.s>>>(L);
+        launch_next(bits_kernel, bgrid, kSymThreads, I.s, L);
         exclusive_scan(L.block_bits, blocks, L.bit_off, I.part.as<uint64_t>(), done, I.s);
-        segment_kernel<<<(segs + 255) / 256, 256, 0, I.s>>>(L);
+        launch_next(segment_kernel, (segs + 255) / 256, 256, I.s, L);
         exclusive_scan(L.seg_chunks, segs, L.seg_chunk_off, I.part.as<uint64_t>(), done + 1, I.s);
         cudaMemcpyAsync(hb, L.seg_chunk_off + segs, 8, cudaMemcpyDeviceToHost, I.s);
         if (cudaStreamSynchronize(I.s) != cudaSuccess) throw std::runtime_error("GPU encoder: device failure");
@@ -1085,10 +1093,10 @@ int32_t GpuJpegEncoder::encode(EncodeItem *items, size_t n, const JpegEncodeOpti
         cudaMemsetAsync(L.raw, 0, words * 4, I.s);
         write_bits_kernel<<<bgrid, kSymThreads, 0, I.s>>>(L);
         const unsigned cgrid = (unsigned)((chunks + kEmitThreads - 1) / kEmitThreads);
-        ff_count_kernel<<<cgrid, kEmitThreads, 0, I.s>>>(L, chunks);
+        launch_next(ff_count_kernel, cgrid, kEmitThreads, I.s, L, chunks);
         exclusive_scan(L.chunk_ff, chunks, L.ff_off, I.part.as<uint64_t>(), done + 2, I.s);
-        layout_kernel<<<nf, kLayoutThreads, 0, I.s>>>(L);
-        emit_kernel<<<cgrid, kEmitThreads, 0, I.s>>>(L, chunks);
+        launch_next(layout_kernel, nf, kLayoutThreads, I.s, L);
+        launch_next(emit_kernel, cgrid, kEmitThreads, I.s, L, chunks);
         if (cudaGetLastError() != cudaSuccess) throw std::runtime_error("GPU encoder: launch failed");
         cudaMemcpyAsync(hb + b_len, L.frame_len, nf * 4, cudaMemcpyDeviceToHost, I.s);
         cudaMemcpyAsync(hb + b_off, L.frame_off, nf * 8, cudaMemcpyDeviceToHost, I.s);
