@@ -10,7 +10,8 @@
 //   bits_kernel        thread per block: Huffman bit count (DC difference against the
 //                      previous block of the component in its restart interval)
 //   scans              exclusive prefix of the bit counts of 128 blocks each, of the segment
-//                      chunks and of the 0xFF counts (two launches each)
+//                      chunks, and of the 0xFF counts of segments and of 256 chunks each
+//                      (two launches each)
 //   segment_kernel     warp per restart interval ("segment"): its bits and 16-byte chunks
 //   write_bits_kernel  thread per block: its codes into the segment's bit buffer
 //                      (interior words stored, the two shared edge words OR-ed)
@@ -74,8 +75,9 @@ struct EncLaunch {
     uint64_t *seg_bits;       // per segment
     uint64_t *seg_chunk_off;  // n_segs + 1
     uint32_t *raw;            // segment bit buffers, big-endian words, four per chunk
-    uint32_t *chunk_ff;       // per chunk
-    uint64_t *ff_off;         // n_chunks + 1
+    uint8_t *chunk_ff;        // per chunk: its 0xFF bytes
+    uint32_t *ff_sums;        // of them, per segment, then per kEmitThreads chunks
+    uint64_t *ff_off;         // their exclusive prefix
     uint32_t *seg_out;        // per segment: its offset in the frame's entropy bytes
     uint32_t *frame_len;      // per frame: entropy bytes, markers and EOI
     uint64_t *frame_off;      // per frame staged for a host buffer: its entropy bytes in `out`
@@ -488,6 +490,7 @@ __global__ void __launch_bounds__(kSymThreads) write_bits_kernel(EncLaunch L) {
     __shared__ SymSmem<false> S;
     // bits of the tile's blocks before the thread's
     const uint64_t blk = (uint64_t)blockIdx.x * kSymThreads + threadIdx.x;
+    if (blk < L.n_segs) L.ff_sums[blk] = 0;  // (for ff_count_kernel; a segment has a block at least)
     const uint32_t mine = blk < L.n_blocks ? L.block_bits[blk] : 0, warp = threadIdx.x >> 5;
     uint32_t before = mine;
 #pragma unroll
@@ -562,21 +565,43 @@ __device__ __forceinline__ void chunk_of(const EncLaunch &L, const ChunkSmem &S,
     *n = (uint32_t)min((uint64_t)16, bytes - 16 * *k);
 }
 
-__global__ void __launch_bounds__(256) ff_count_kernel(EncLaunch L, uint64_t n_chunks) {
+constexpr int kEmitThreads = 256;  // chunks per CTA of ff_count_kernel and emit_kernel
+
+// (Sums per segment and per CTA: a scan over all chunks' counts read and wrote 68 MB for
+// the 4.2 M chunks of 60 1080p frames, which emit_kernel read again: 1.429 ms an encode, now 1.403.)
+__global__ void __launch_bounds__(kEmitThreads) ff_count_kernel(EncLaunch L, uint64_t n_chunks) {
     begin_kernel(false);
     __shared__ ChunkSmem S;
+    __shared__ uint32_t s_sum[kEmitThreads / 32];
     chunk_range(L, n_chunks, S);
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_chunks) return;
-    uint32_t s, n;
-    uint64_t k;
-    chunk_of(L, S, c, &s, &k, &n);
-    const uint4 v = *reinterpret_cast<const uint4 *>(L.raw + 4 * c);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    uint32_t count = 0;
+    const uint64_t c = (uint64_t)blockIdx.x * kEmitThreads + threadIdx.x;
+    uint32_t s = 0, count = 0;
+    if (c < n_chunks) {
+        uint32_t n;
+        uint64_t k;
+        chunk_of(L, S, c, &s, &k, &n);
+        const uint4 v = *reinterpret_cast<const uint4 *>(L.raw + 4 * c);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int q = 0; q < 4; q++) count += __popc(zero_bytes(~w[q]) & lead_bytes_mask((int)n - 4 * q));
-    L.chunk_ff[c] = count;
+        for (int q = 0; q < 4; q++) count += __popc(zero_bytes(~w[q]) & lead_bytes_mask((int)n - 4 * q));
+        L.chunk_ff[c] = (uint8_t)count;
+    }
+    __syncwarp();
+    const uint32_t lane = threadIdx.x & 31, sum = __reduce_add_sync(0xffffffffu, count);
+    const uint32_t s0 = __shfl_sync(0xffffffffu, s, 0);
+    if (__all_sync(0xffffffffu, s == s0 || !count)) {
+        if (lane == 0 && sum) atomicAdd(L.ff_sums + s0, sum);
+    } else if (count) {
+        atomicAdd(L.ff_sums + s, count);
+    }
+    if (lane == 0) s_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t all = 0;
+#pragma unroll
+        for (int w = 0; w < kEmitThreads / 32; w++) all += s_sum[w];
+        L.ff_sums[L.n_segs + blockIdx.x] = all;
+    }
 }
 
 // Exclusive prefix of v over a CTA of NT threads; *total = the CTA's sum.
@@ -631,7 +656,7 @@ __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(EncLaunch L) {
         const uint32_t j = j0 + threadIdx.x, s = F.seg_base + j;
         uint64_t bytes = 0;
         if (j < F.nseg)
-            bytes = (L.seg_bits[s] + 7) / 8 + L.ff_off[L.seg_chunk_off[s + 1]] - L.ff_off[L.seg_chunk_off[s]] + 2;
+            bytes = (L.seg_bits[s] + 7) / 8 + L.ff_sums[s] + 2;
         const uint64_t ex = cta_exclusive<kLayoutThreads>(bytes, &s_total);
         if (j < F.nseg) L.seg_out[s] = (uint32_t)(pos + ex);
         pos += s_total;
@@ -662,23 +687,35 @@ __global__ void __launch_bounds__(kLayoutThreads) layout_kernel(EncLaunch L) {
 // encoder.rs:519-528), then the segment's marker after its last chunk. A CTA whose
 // chunks are of one frame collects its run of bytes in shared memory and stores it as
 // 16-byte vectors; byte stores took 0.20 ms for the 67 MB of 60 1080p frames.
-constexpr int kEmitThreads = 256;
 
 __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EncLaunch L, uint64_t n_chunks) {
     begin_kernel(false);
     __shared__ ChunkSmem S;
     __shared__ __align__(16) uint8_t s_out[kEmitThreads * 34 + 32];
     __shared__ uint8_t *s_dst;
-    __shared__ uint32_t s_frame[2], s_len;
-    chunk_range(L, n_chunks, S);
+    __shared__ uint32_t s_frame[2], s_len, s_ff[kEmitThreads / 32];
+    const uint64_t c = (uint64_t)blockIdx.x * kEmitThreads + threadIdx.x;
+    const bool valid = c < n_chunks;
+    // 0xFF bytes of the CTA's chunks before the thread's
+    const uint32_t mine = valid ? L.chunk_ff[c] : 0, warp = threadIdx.x >> 5;
+    uint32_t before = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, before, o);
+        if ((threadIdx.x & 31) >= (uint32_t)o) before += v;
+    }
+    if ((threadIdx.x & 31) == 31) s_ff[warp] = before;
+    before -= mine;
+    chunk_range(L, n_chunks, S);  // (a barrier)
+#pragma unroll
+    for (uint32_t w = 0; w + 1 < kEmitThreads / 32; w++)
+        if (w < warp) before += s_ff[w];
     if (threadIdx.x < 2) s_frame[threadIdx.x] = frame_of_segment(L, threadIdx.x ? S.hi : S.lo);
     __syncthreads();
     const bool one = s_frame[0] == s_frame[1];
     uint32_t f = s_frame[0];
     uint8_t *base = frame_dst(L, f);
     if (one && !base) return;  // (uniform: the frame's buffer is too small)
-    const uint64_t c = (uint64_t)blockIdx.x * kEmitThreads + threadIdx.x;
-    const bool valid = c < n_chunks;
     uint8_t *dst = base;
     uint32_t s = 0, n = 0;
     uint64_t k = 0;
@@ -688,7 +725,7 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(EncLaunch L, uint64_
             f = frame_of_segment(L, s);
             base = frame_dst(L, f);
         }
-        dst = base + L.seg_out[s] + 16 * k + (L.ff_off[c] - L.ff_off[L.seg_chunk_off[s]]);
+        dst = base + L.seg_out[s] + 16 * k + (L.ff_off[L.n_segs + blockIdx.x] - L.ff_off[L.n_segs] + before - L.ff_off[s]);
     }
     if (threadIdx.x == 0) s_dst = dst;
     __syncthreads();
@@ -779,7 +816,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
         v[k] = base + k < n ? in[base + k] : 0u;
         sum += v[k];
     }
-    uint64_t run = part[blockIdx.x] + cta_exclusive<kScanThreads>(sum, &s_total);
+    uint64_t run = (part ? part[blockIdx.x] : 0) + cta_exclusive<kScanThreads>(sum, &s_total);
+    if (!part && threadIdx.x == 0) out[n] = s_total;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++)
         if (base + k < n) {
@@ -792,6 +830,10 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
 // done: a zeroed counter); n > 0
 void exclusive_scan(const uint32_t *in, uint64_t n, uint64_t *out, uint64_t *part, uint32_t *done, cudaStream_t s) {
     const unsigned tiles = (unsigned)((n + kScanTile - 1) / kScanTile);
+    if (tiles == 1) {  // (12 719x405 frames: three launches less: 196.4 us a call, now 192.8)
+        launch_next(scan_apply_kernel, 1u, kScanThreads, s, in, n, nullptr, out);
+        return;
+    }
     launch_next(scan_reduce_kernel, tiles, kScanThreads, s, in, n, part, out + n, done);
     launch_next(scan_apply_kernel, tiles, kScanThreads, s, in, n, part, out);
 }
@@ -889,7 +931,7 @@ struct GpuJpegEncoder::Impl {
     cudaStream_t s = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::mutex mu;
-    DBuf plan, in, coef, block_bits, tile_bits, tile_off, part, seg_bits, seg_off, seg_chunks, seg_chunk_off, raw, chunk_ff, ff_off, seg_out,
+    DBuf plan, in, coef, block_bits, tile_bits, tile_off, part, seg_bits, seg_off, seg_chunks, seg_chunk_off, raw, chunk_ff, ff_sums, ff_off, seg_out,
         frame_len, frame_off, out, counters;
     PBuf up, back;
 };
@@ -1125,19 +1167,22 @@ int32_t GpuJpegEncoder::encode(EncodeItem *items, size_t n, const JpegEncodeOpti
         if (cudaStreamSynchronize(I.s) != cudaSuccess) throw std::runtime_error("GPU encoder: device failure");
         const uint64_t chunks = *reinterpret_cast<const uint64_t *>(hb), words = 4 * chunks;
         I.raw.ensure(std::max<uint64_t>(words, 4) * 4);
-        I.chunk_ff.ensure(std::max<uint64_t>(chunks, 1) * 4);
-        I.ff_off.ensure((chunks + 1) * 8);
-        I.part.ensure(((chunks + kScanTile - 1) / kScanTile + 1) * 8);
+        const unsigned cgrid = (unsigned)((chunks + kEmitThreads - 1) / kEmitThreads);
+        const uint64_t ff_sums = segs + (uint64_t)cgrid;
+        I.chunk_ff.ensure(std::max<uint64_t>(chunks, 1));
+        I.ff_sums.ensure(ff_sums * 4);
+        I.ff_off.ensure((ff_sums + 1) * 8);
+        I.part.ensure(((ff_sums + kScanTile - 1) / kScanTile + 1) * 8);
         I.out.ensure(std::max<uint64_t>(chunks * 32 + (uint64_t)segs * 2, 16));
         L.raw = I.raw.as<uint32_t>();
-        L.chunk_ff = I.chunk_ff.as<uint32_t>();
+        L.chunk_ff = I.chunk_ff.as<uint8_t>();
+        L.ff_sums = I.ff_sums.as<uint32_t>();
         L.ff_off = I.ff_off.as<uint64_t>();
         L.out = I.out.as<uint8_t>();
         cudaMemsetAsync(L.raw, 0, words * 4, I.s);
         write_bits_kernel<<<bgrid, kSymThreads, 0, I.s>>>(L);
-        const unsigned cgrid = (unsigned)((chunks + kEmitThreads - 1) / kEmitThreads);
         launch_next(ff_count_kernel, cgrid, kEmitThreads, I.s, L, chunks);
-        exclusive_scan(L.chunk_ff, chunks, L.ff_off, I.part.as<uint64_t>(), done + 2, I.s);
+        exclusive_scan(L.ff_sums, ff_sums, L.ff_off, I.part.as<uint64_t>(), done + 2, I.s);
         launch_next(layout_kernel, nf, kLayoutThreads, I.s, L);
         launch_next(emit_kernel, cgrid, kEmitThreads, I.s, L, chunks);
         if (cudaGetLastError() != cudaSuccess) throw std::runtime_error("GPU encoder: launch failed");
