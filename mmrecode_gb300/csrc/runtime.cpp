@@ -266,12 +266,18 @@ int32_t EnginePool::decode(Item *items, size_t n, EngineTimes *times) {
         status = engines_[0]->decode(items, n, &sum);
         launches_ = engines_[0]->last_launches();
     } else {
-        // One chunk per engine: fewer and larger launches (300 1080p frames 5.76 -> 5.64 ms
-        // against two, 1000 NTSC frames 1.82 -> 1.80; six gain nothing). Past kOneChunkBytes of
-        // outputs two, so that the engines' arenas hold half of the batch at a time.
+        // Frames of one size: one chunk per engine, fewer and larger launches (300 1080p
+        // frames 5.75 -> 5.64 ms against two, 1000 NTSC frames 1.82 -> 1.80; six gain
+        // nothing). Frames of many sizes: two, which even out (512 mixed frames 10.9 -> 10.5
+        // ms); as past kOneChunkBytes of outputs, so that the engines' arenas hold half of the
+        // batch at a time.
         uint64_t out_bytes = 0;
-        for (size_t i = 0; i < n; i++) out_bytes += std::min<uint64_t>(items[i].out_capacity, kOneChunkBytes);
-        size_t parts = std::min(out_bytes <= kOneChunkBytes ? k : 2 * k, n / kMinChunk);
+        bool alike = true;
+        for (size_t i = 0; i < n; i++) {
+            out_bytes += std::min<uint64_t>(items[i].out_capacity, kOneChunkBytes);
+            alike &= items[i].codec == items[0].codec && items[i].out_capacity == items[0].out_capacity;
+        }
+        size_t parts = std::min(alike && out_bytes <= kOneChunkBytes ? k : 2 * k, n / kMinChunk);
         Item *work = items;
         if (cudaSetDevice(device_) == cudaSuccess && stage(items, n)) {
             work = staged_.data();
