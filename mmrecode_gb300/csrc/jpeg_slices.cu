@@ -61,8 +61,8 @@ constexpr unsigned long long kStErr = ~0ull;        // no state: the decode fail
 constexpr unsigned long long kStGuess = ~0ull - 1;  // start not yet derived from the predecessor
 
 // Slices only ever take real states from their predecessors. After a true error the
-// slices that follow keep what they guessed: they may decode nonsense, but events count
-// by slice, so theirs come after the one that matters.
+// slices that follow keep what they guessed: they may decode nonsense, within their
+// interval (slice_share), but events count by slice, so theirs come after the one that matters.
 __device__ __forceinline__ bool is_state(unsigned long long x) { return x < kStGuess; }
 
 constexpr int kStride = 72;  // int16 per staged block: 64 levels, and 64.. for what EOB steps store
@@ -1041,7 +1041,8 @@ __global__ void __launch_bounds__(kSliceThreads) slice_decode_kernel(JpegLaunch 
                 redone = s.j != 0 && y.q != 0;
                 whole = y.q == kMatchNone;
             }
-            n = !is_state(from) || over || base >= s.v.blocks ? 0 : min(n, s.v.blocks - base);
+            n = !is_state(from) || over
+                    ? 0 : slice_share(n, base, s.v.blocks, (uint32_t)(from & 0xff), L.frames[s.v.frame].sched_len);
         }
     }
     const int n_used = __syncthreads_count(used), n_redone = __syncthreads_count(redone),

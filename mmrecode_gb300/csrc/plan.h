@@ -220,6 +220,17 @@ struct SliceSpec {
     SlicePoint cp[kSliceCheckpoints];
 };
 
+// Blocks that a slice decodes: of the n that start in it, those up to the interval's last
+// of `blocks`; the first is block `base` of the interval, block si of the MCU. After an
+// error in the scan, slices start where guesses met and base sums what those counted: one
+// whose si is not base's place in the MCU would go past the interval's last MCU (into
+// another component's blocks, another frame's, or past the arena) and decodes nothing. (For
+// true states the two agree, and what an error leaves behind is never shown.)
+MMR_HD uint32_t slice_share(uint32_t n, uint32_t base, uint32_t blocks, uint32_t si, uint32_t sched_len) {
+    if (base >= blocks || base % sched_len != si) return 0;
+    return n < blocks - base ? n : blocks - base;
+}
+
 // Block index and DC predictors at a slice's start (interval-relative).
 struct SlicePrefix {
     uint32_t base;
