@@ -582,11 +582,12 @@ __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L,
     SliceRef s;
     bool work = slice_ref(L, slot, s) && !s.last;
     unsigned long long start = 0, exit = 0, entry[kMostPaths], leave[kMostPaths];
+    unsigned long long stored = 0;  // the exit that the next CTA finds in L.sync
     if (work) {
         S.frame = s.v.frame;
         const uint32_t paths = L.frames[s.v.frame].paths;
         start = L.sync[slot].start;
-        exit = L.sync[slot].exit;
+        exit = stored = L.sync[slot].exit;
 #pragma unroll
         for (uint32_t h = 0; h < kMostPaths; h++) {
             entry[h] = leave[h] = kStGuess;  // (never an exit)
@@ -612,10 +613,9 @@ __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L,
     }
     work = work && s.j != 0;
     s_exit[tid + 1] = exit;
-    const unsigned long long exit_before = exit;
     __syncthreads();
     if (!first_pass && !__syncthreads_or(work && is_state(s_exit[tid]) && s_exit[tid] != start)) return;
-    bool loaded = false;
+    bool loaded = false, told = false;         // (whether another exit than `stored` was ever in L.sync)
     uint32_t met = kMostPaths;                 // the speculative decode the slice takes, if it changes
     unsigned long long refused = kStGuess;     // an exit no speculative decode fits
     for (;;) {
@@ -656,6 +656,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L,
             if (F.shared_tabs) resync_slice<true>(L, S, F, slot, s, from, y);
             else resync_slice<false>(L, S, F, slot, s, from, y);
             L.sync[slot] = y;
+            told |= y.exit != stored;
             met = kMostPaths;
             start = from;
             exit = y.exit;
@@ -673,7 +674,8 @@ __global__ void __launch_bounds__(kSliceThreads) slice_sync_kernel(JpegLaunch L,
         settle(sp, 0, y);
         L.sync[slot] = y;
     }
-    if (last_pass && tid == kSliceThreads - 1 && work && exit != exit_before && s.j + 2 < s.v.n_slices) {
+    // (`stored` is path 0's exit where the slice had no start yet, whatever most guesses agree on)
+    if (last_pass && tid == kSliceThreads - 1 && work && (told || exit != stored) && s.j + 2 < s.v.n_slices) {
         atomicAdd(L.sync_left, 1u);
         atomicMin(L.iv_pend + s.item, s.j + 1);
     }
