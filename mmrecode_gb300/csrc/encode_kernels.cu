@@ -22,6 +22,7 @@
 //   emit_kernel        thread per chunk: stuffed bytes, then RSTn or EOI after the
 //                      segment's last chunk, straight into device buffers
 // The header bytes (SOI .. SOS) are the host plan's (plan_jpeg_encode).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,6 +37,7 @@
 #include "encode_gpu.h"
 #include "fdct_core.h"
 #include "launch.h"
+#include "plane_uploads.h"
 #include "tables.h"
 
 namespace mmr {
@@ -904,25 +906,39 @@ struct PBuf {
     }
 };
 
-// Copies host planes up. Planes that follow one another in host memory go up as one
-// copy (a call per plane took a third of the encode of 12 small frames).
-struct PlaneUploads {
-    const uint8_t *src = nullptr;
-    uint8_t *dst = nullptr;
-    size_t bytes = 0;
+// The range that a host address was pinned or registered in.
+HostRange host_range(const uint8_t *p) {
+    using Query = CUresult(CUDAAPI *)(void *, CUpointer_attribute, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Query>(f);
+    }();
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return HostRange{p, p};  // unknown: continued by nothing
+    }
+    if (at.type == cudaMemoryTypeUnregistered) return HostRange{};
+    CUdeviceptr lo = 0;
+    size_t size = 0;
+    const CUdeviceptr at_p = reinterpret_cast<CUdeviceptr>(p);
+    if (!query || query(&lo, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at_p) != CUDA_SUCCESS ||
+        query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at_p) != CUDA_SUCCESS || at_p < lo || at_p >= lo + size)
+        return HostRange{p, p};
+    return HostRange{reinterpret_cast<const uint8_t *>(lo), reinterpret_cast<const uint8_t *>(lo + size)};
+}
 
-    void flush(cudaStream_t s) {
-        if (bytes && cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
-            throw std::runtime_error("GPU encoder: upload failed");
-        bytes = 0;
-    }
-    // Whether `more` at p continues the pending copy.
-    bool append(const uint8_t *p, size_t more) {
-        if (!bytes || p != src + bytes) return false;
-        bytes += more;
-        return true;
-    }
-};
+void flush(PlaneUploads &up, cudaStream_t s) {
+    if (up.bytes && cudaMemcpyAsync(up.dst, up.src, up.bytes, cudaMemcpyHostToDevice, s) != cudaSuccess)
+        throw std::runtime_error("GPU encoder: upload failed");
+    up.bytes = 0;
+}
 
 }  // namespace
 
@@ -1079,27 +1095,25 @@ int32_t GpuJpegEncoder::encode(EncodeItem *items, size_t n, const JpegEncodeOpti
                 const size_t bytes = pl.width * pl.height;
                 fr[k].stride[c] = pl.width;
                 const uint8_t *before = up.src;
-                if (pl.stride == pl.width && up.append(pl.data, bytes)) {  // packed right behind the last one
+                if (pl.stride == pl.width && up.append(pl.data, bytes, host_range)) {  // packed right behind the last one
                     fr[k].plane[c] = up.dst + (pl.data - before);
                     at += bytes;
                     continue;
                 }
-                up.flush(I.s);
+                flush(up, I.s);
                 at = (at + 255) / 256 * 256;
                 uint8_t *dst = I.in.as<uint8_t>() + at;
                 fr[k].plane[c] = dst;
                 at += bytes;
                 if (pl.stride == pl.width) {
-                    up.src = pl.data;
-                    up.dst = dst;
-                    up.bytes = bytes;
+                    up.start(pl.data, dst, bytes, host_range);
                 } else if (cudaMemcpy2DAsync(dst, pl.width, pl.data, pl.stride, pl.width, pl.height,
                                              cudaMemcpyHostToDevice, I.s) != cudaSuccess) {  // row by row
                     throw std::runtime_error("GPU encoder: upload failed");
                 }
             }
         }
-        up.flush(I.s);
+        flush(up, I.s);
         // the plan: frames | tables | headers, one copy
         const uint32_t nf = (uint32_t)live.size();
         const size_t o_tab = (nf * sizeof(EncFrame) + 255) / 256 * 256, o_hdr = o_tab + (kTabBytes + 255) / 256 * 256;
