@@ -32,6 +32,7 @@
 #include <string>
 #include <vector>
 
+#include "block_source.h"
 #include "common.h"
 #include "encode.h"
 #include "encode_gpu.h"
@@ -129,12 +130,6 @@ constexpr int kOutStride = 80;                           // int16 per block: fou
 constexpr int kTileStride = 8 * kRowStride + 8;          // per block: four blocks' column loads on distinct banks
 
 // Where block blk's samples come from.
-struct BlockSource {
-    const uint8_t *plane;
-    size_t stride;
-    uint32_t x0, y0, pw, ph, tq;
-};
-
 __device__ __forceinline__ BlockSource block_source(const EncFrame &F, uint64_t blk) {
     const uint32_t i = (uint32_t)(blk - F.block_base);
     const uint32_t mcu = i / F.bpm, k = i - mcu * F.bpm;
@@ -151,27 +146,9 @@ __device__ __forceinline__ BlockSource block_source(const EncFrame &F, uint64_t 
     return B;
 }
 
-// Row r of the block's samples, byte x in bits 8x (read_block, encoder.rs:392-402:
-// rows and columns past the plane repeat its last).
 __device__ __forceinline__ uint2 source_row(const BlockSource &B, uint32_t r) {
-    const uint8_t *row = B.plane + (size_t)min(B.y0 + r, B.ph - 1) * B.stride;
-    if (B.x0 + 8 <= B.pw) {  // one aligned 8-byte load, or the two that hold the eight samples
-        const uintptr_t a = reinterpret_cast<uintptr_t>(row + B.x0);
-        const uint2 *q = reinterpret_cast<const uint2 *>(a & ~(uintptr_t)7);
-        const uint32_t sh = (uint32_t)(a & 7) * 8;
-        const uint2 v = q[0];
-        if (sh == 0) return v;
-        const uint2 n = q[1];
-        const unsigned long long x = ((unsigned long long)v.y << 32 | v.x) >> sh | ((unsigned long long)n.y << 32 | n.x) << (64 - sh);
-        return make_uint2((uint32_t)x, (uint32_t)(x >> 32));
-    }
-    uint2 w = make_uint2(0, 0);
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-        w.x |= (uint32_t)row[min(B.x0 + x, B.pw - 1)] << (8 * x);
-        w.y |= (uint32_t)row[min(B.x0 + 4 + x, B.pw - 1)] << (8 * x);
-    }
-    return w;
+    return plane_row<uint2>(
+        B, r, [](const uint2 *p) { return *p; }, [](const uint8_t *p) { return *p; });
 }
 
 // Persistent CTAs, 32 blocks per step. Quotients too close to a half-integer (exact
