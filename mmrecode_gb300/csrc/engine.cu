@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "arena.h"
 #include "dv_layout.h"
 #include "dv_vlc.h"
 #include "exact_fixed.h"
@@ -138,27 +139,19 @@ uint32_t tune_class_of(const JPlan &p, size_t len) {
     return layout << 8 | lg;
 }
 
-// Slice size, and lead and number of the speculative decodes per slice of a batch.
-struct SlicePlan {
-    uint32_t bits, lead, paths;
-};
-
-// Small batches leave the GPU idle, so their time is that of one thread's slice: short
-// slices, and every block of the MCU guessed, which finds the true state after 250 to
-// 500 bits (99 % of starts) where one guess takes 1,000 to 5,000. Large batches are
-// bound by the instructions of all threads: long slices and one guess. Measured, us,
-// by slice bits / lead / paths:
-//   one 320x240 4:2:0 frame (0.13 Mbit)   256/384/6 307   512/384/6 317   1024/384/6 352
-//   one 1080p 4:2:2 frame (9 Mbit)        256/384/6 350   512/384/6 327   1024/384/6 359
-//   30 VGA 4:2:0 frames (14 Mbit)         512/384/6 471   1024/384/6 421  1024/1024/1 492   2048/768/1 544
-//   64 mixed frames (four of 106 Mbit)    1024/1024/1 3271   2048/768/1 3079   4096/768/1 3128
-//   300 1080p frames (eight of 341 Mbit)  2048/768/1 7930   4096/768/1 7469   2048/384/4 11003
-SlicePlan auto_slices(uint64_t total_bits) {
-    if (total_bits <= 2u << 20) return SlicePlan{256, 384, 6};
-    if (total_bits <= 12u << 20) return SlicePlan{512, 384, 6};
-    if (total_bits <= 32u << 20) return SlicePlan{1024, 384, 6};
-    if (total_bits <= 160u << 20) return SlicePlan{2048, 768, 1};
-    return SlicePlan{4096, 768, 1};
+// What the frame needs on the device for item `it`.
+FrameNeed frame_need(const JPlan &p, const Item &it) {
+    FrameNeed f;
+    f.len = it.len;
+    f.host_in = !it.dev_data;
+    if (!p.decode) return f;
+    f.planar = p.planar_bytes;
+    f.blocks = p.n_blocks;
+    f.intervals = p.n_intervals;
+    f.sliced = p.ncomp <= 4;
+    f.planes = it.output != kOutPlanar && fused_layout(p) < 0;
+    if (!it.out_on_device) f.host_out = it.output == kOutRgb24 ? 3 * (uint64_t)p.W * p.H : p.planar_bytes;
+    return f;
 }
 
 // Huffman LUT source: counts + symbols bytes (as in the DHT payload).
@@ -405,6 +398,13 @@ DvPlan plan_dv(const uint8_t *in, size_t len) {
     return p;
 }
 
+// Device bytes of a DV frame in a batch: packet, coefficients, modes, segment results, planes.
+uint64_t dv_bytes(const DvPlan &p, const Item &it) {
+    const uint64_t segments = p.sequences * 27, rgb = 3 * (uint64_t)p.W * p.H;
+    return (it.dev_data ? 0 : it.len) + segments * (30 * 129 + 1) + (it.output == kOutRgb24 ? p.planar_bytes : 0) +
+           (it.out_on_device ? 0 : it.output == kOutRgb24 ? rgb : p.planar_bytes) + 1024;
+}
+
 // Two-level DV VLC table (dv_vlc.h).
 std::vector<uint32_t> build_dv_vlc() {
     std::vector<uint32_t> t(kDvVlcMaxEntries);
@@ -584,6 +584,22 @@ uint32_t jpeg_tune_class(const uint8_t *data, size_t len) {
     plan_jpeg(data, len, p);
     if (!p.decode || p.ncomp > 4) return 0xffffffffu;
     return tune_class_of(p, len);
+}
+
+uint64_t request_bytes(const Item &it) {
+    if (it.codec == kCodecMjpeg) {
+        JPlan p;
+        plan_jpeg(it.data, it.len, p);
+        return reserved_bytes(frame_need(p, it));
+    }
+    FrameNeed f;
+    f.len = it.len;
+    const Probe p = probe_packet(it.codec, it.data, it.len);
+    if (p.status == kOk) {
+        f.planar = p.planar_bytes;
+        if (!it.out_on_device) f.host_out = it.output == kOutRgb24 ? p.rgb_bytes : p.planar_bytes;
+    }
+    return reserved_bytes(f);
 }
 
 Probe probe_packet(uint32_t codec, const uint8_t *data, size_t len) {
@@ -809,7 +825,29 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
         uint64_t total_bits = 0;  // compressed MJPEG bits of the batch
         for (size_t i = 0; i < n; i++)
             if (items[i].codec == kCodecMjpeg) total_bits += 8 * (uint64_t)items[i].len;
-        const SlicePlan auto_plan = auto_slices(total_bits);
+        // a frame's slices: the set size, its class's tuned one, or the plan's
+        auto frame_slice_bits = [&](const JPlan &p, size_t len, const SlicePlan &plan) {
+            if (slice_bits_) return slice_bits_;
+            uint32_t bits = plan.bits;
+            auto t = tuned.find(tune_class_of(p, len));
+            if (t != tuned.end()) bits = t->second;
+            // Intervals shorter than a slice are one slice each. An interval's slots start at
+            // its bits / S plus its number (slice_plan_kernel), so a larger S leaves fewer slots
+            // unused between them.
+            const uint64_t four = 4 * 8 * (uint64_t)len / p.n_intervals;
+            if (four < 4 * (uint64_t)bits && four > bits) bits = (uint32_t)align_up(four, 32);
+            return bits;
+        };
+        const SlicePlan plan = batch_slices(total_bits, memory_limit_, [&](const SlicePlan &s) {
+            uint64_t bytes = 0;
+            for (size_t k = 0; k < jplans.size(); k++) {
+                const Item &it = items[jitem[k]];
+                const FrameNeed f = frame_need(jplans[k], it);
+                bytes += frame_bytes(f, f.sliced ? frame_slice_bits(jplans[k], it.len, s) : s.bits, s.paths);
+            }
+            for (size_t k = 0; k < dplans.size(); k++) bytes += dv_bytes(dplans[k], items[ditem[k]]);
+            return bytes;
+        });
         // Strips per CTA of the fused transform: several where the batch fills the GPU
         // many times over anyway, one where every CTA counts. Measured with narrow (wide)
         // strips, ms: 300 1080p frames (eight parts of 2.5 M blocks) 4 strips 6.69 (6.76), 8
@@ -953,23 +991,14 @@ int32_t Engine::decode(Item *items, size_t n, EngineTimes *times) {
                 F.rst_off = rst_total;
                 rst_total += p.n_intervals;
                 if (p.ncomp <= 4) {
-                    uint32_t slice_bits = slice_bits_ ? slice_bits_ : auto_plan.bits;
-                    if (!slice_bits_) {
-                        auto t = tuned.find(tune_class_of(p, it.len));
-                        if (t != tuned.end()) slice_bits = t->second;
-                        // Intervals shorter than a slice are one slice each. An interval's slots start at
-                        // its bits / S plus its number (slice_plan_kernel), so a larger S leaves fewer slots
-                        // unused between them.
-                        const uint64_t four = 4 * 8 * (uint64_t)it.len / p.n_intervals;
-                        if (four < 4 * (uint64_t)slice_bits && four > slice_bits) slice_bits = (uint32_t)align_up(four, 32);
-                    }
+                    const uint32_t slice_bits = frame_slice_bits(p, it.len, plan);
                     F.slice_bits = slice_bits;
-                    F.lead = auto_plan.lead;
+                    F.lead = plan.lead;
                     // (with one block per MCU, or one interval per slice, all guesses are alike)
-                    F.paths = p.ri * F.sched_len > 1 ? std::min<uint32_t>(auto_plan.paths, F.sched_len) : 1;
+                    F.paths = p.ri * F.sched_len > 1 ? std::min<uint32_t>(plan.paths, F.sched_len) : 1;
                     most_paths = std::max(most_paths, F.paths);
                     F.slot_first = (uint32_t)n_slots;
-                    F.slot_count = (uint32_t)align_up((8 * (uint64_t)it.len + slice_bits - 1) / slice_bits + p.n_intervals, kSliceThreads);
+                    F.slot_count = (uint32_t)slice_slots(it.len, p.n_intervals, slice_bits);
                     n_slots += F.slot_count;
                 }
                 F.blk_off = blocks;

@@ -58,6 +58,9 @@ struct Probe {
 
 Probe probe_packet(uint32_t codec, const uint8_t *data, size_t len);
 
+// Device bytes to reserve for a request that may share a batch with others (arena.h).
+uint64_t request_bytes(const Item &item);
+
 // Tuning class of an MJPEG packet (restart layout, log2 compressed bits per
 // interval), UINT32_MAX when its headers fail or it has more than 4 components.
 uint32_t jpeg_tune_class(const uint8_t *data, size_t len);
@@ -130,6 +133,9 @@ public:
         slice_bits_ = bits;
         return true;
     }
+    // Device bytes that a batch's arenas should stay within, as far as slices have a choice
+    // (batch_slices; 0: no limit). Not while a batch decodes.
+    void set_memory_limit(uint64_t bytes) { memory_limit_ = bytes; }
     // Slice bits per tuning class, used when no fixed size is set.
     // (The tables may change while another thread decodes: a batch reads a copy
     // taken at its start.)
@@ -156,6 +162,7 @@ private:
     std::vector<cudaStream_t> streams_;  // one per priority level
     uint32_t launches_ = 0;
     uint32_t slice_bits_;
+    uint64_t memory_limit_ = 0;
     bool graphs_ = true;
     std::mutex tables_mu_;
     std::map<uint32_t, uint32_t> tuned_;

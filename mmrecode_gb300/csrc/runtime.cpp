@@ -339,24 +339,17 @@ int32_t EnginePool::decode(Item *items, size_t n, EngineTimes *times) {
 
 // ---------------------------------------------------------------- server ---
 
-uint64_t Server::estimate_bytes(const Item &it) {
-    const Probe p = probe_packet(it.codec, it.data, it.len);
-    const uint64_t planar = p.status == kOk ? p.planar_bytes : 0;
-    const uint64_t out = p.status == kOk ? (it.output == kOutRgb24 ? p.rgb_bytes : planar) : 0;
-    // tokens and slice records (~8 B per compressed byte), coefficients (~2.25 B per
-    // sample) and as much again for the records of small batches, whose slices are short
-    // and decoded from several guesses; planes, fixed scratch
-    uint64_t b = 8 * (uint64_t)it.len + (planar * 9) / 2 + planar + 65536;
-    if (!it.out_on_device) b += out;  // staged output
-    return b;
-}
+uint64_t Server::estimate_bytes(const Item &it) { return request_bytes(it); }
 
 Server::Server(const ServerConfig &cfg) : cfg_(cfg) {
     cfg_.engines = std::max(1, cfg_.engines);
     cfg_.max_batch = std::max<size_t>(1, cfg_.max_batch);
     share_ = cfg_.memory_budget ? cfg_.memory_budget / cfg_.engines : 0;
     window_start_ = std::chrono::steady_clock::now();
-    for (int k = 0; k < cfg_.engines; k++) engines_.emplace_back(new Engine(cfg_.device));
+    for (int k = 0; k < cfg_.engines; k++) {
+        engines_.emplace_back(new Engine(cfg_.device));
+        engines_.back()->set_memory_limit(share_);
+    }
     for (int k = 0; k < cfg_.engines; k++) threads_.emplace_back(&Server::worker, this, k);
 }
 

@@ -168,8 +168,9 @@ public:
     // Items the budget refuses complete at once with kInvalidArgument.
     void replay(Item *items, size_t n, const int64_t *arrival_ns, double *latency_ms, int64_t *max_lag_ns);
 
-    // Device bytes a request needs inside a batch (inputs, outputs, coefficient
-    // and slice arenas), from its headers.
+    // Device bytes reserved for a request inside a batch (inputs, outputs, coefficient
+    // and slice arenas), from its headers (arena.h). The engines decode with as many
+    // guesses per slice as fit the sum of a batch's.
     static uint64_t estimate_bytes(const Item &item);
 
 private:
