@@ -157,15 +157,7 @@ struct BlockRows {
     int32_t dc;
 };
 
-__device__ __forceinline__ BlockRows load_rows(const int16_t *levels, const int32_t *dc, uint64_t g, uint32_t q) {
-    BlockRows b;
-    b.row[0] = reinterpret_cast<const int4 *>(levels)[q];
-    b.row[1] = reinterpret_cast<const int4 *>(levels)[q + 4];
-    b.dc = dc[g];
-    return b;
-}
-
-// The same by way of shared memory, asynchronously: slot of thread tid of nt, whose copies
+// They come by way of shared memory, asynchronously: slot of thread tid of nt, whose copies
 // begin with copy_rows (once what the slot held has been used) and are waited for by
 // staged_rows. Only the thread itself reads what it copied. (The transforms waited longest
 // for their levels; loads a tile ahead into registers spilled.)
