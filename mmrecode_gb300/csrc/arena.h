@@ -26,6 +26,17 @@ struct SlicePlan {
 //   30 VGA 4:2:0 frames (14 Mbit)         512/384/6 471   1024/384/6 421  1024/1024/1 492   2048/768/1 544
 //   64 mixed frames (four of 106 Mbit)    1024/1024/1 3271   2048/768/1 3079   4096/768/1 3128
 //   300 1080p frames (eight of 341 Mbit)  2048/768/1 7930   4096/768/1 7469   2048/384/4 11003
+// and with the present kernels, near the lines between them (VGA 4:2:0 frames of 0.48 Mbit
+// to planes, 1080p 4:2:2 ones of 9 Mbit to RGB; the plan taken is the first):
+//   20 VGA (10 Mbit)     512/384/6 290    1024/384/6 292
+//   28 VGA (13 Mbit)     1024/384/6 318   512/384/6 330    1024/1024/1 384
+//   3 1080p (27 Mbit)    1024/384/6 290   2048/768/1 326   1024/1024/1 305
+//   4 1080p (36 Mbit)    2048/768/1 339   1024/384/6 353   2048/384/6 352
+//   5 1080p (45 Mbit)    2048/768/1 390   1024/384/6 372   2048/384/6 382
+//   16 1080p (144 Mbit)  2048/768/1 562   4096/768/1 705   2048/384/6 719
+//   20 1080p (180 Mbit)  4096/768/1 723   2048/768/1 599
+//   28 1080p (252 Mbit)  4096/768/1 815   2048/768/1 871
+// (so the last line could lie nearer 200 Mbit).
 inline SlicePlan auto_slices(uint64_t total_bits) {
     if (total_bits <= 2u << 20) return SlicePlan{256, 384, 6};
     if (total_bits <= 12u << 20) return SlicePlan{512, 384, 6};

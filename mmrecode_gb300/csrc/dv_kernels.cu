@@ -1,13 +1,13 @@
 // DV25 decode kernels for sm_103a.
 //
-//   segment    four video segments (5 macroblocks, 30 blocks each) per CTA step: DIF
+//   segment    a warp per video segment (5 macroblocks, 30 blocks), persistent CTAs: DIF
 //              identifiers vs the canonical layout (crates/codecs/dv/src/dif.rs:181-253),
 //              DC/mode/class fields, VLC decode and the three-level spill of
-//              unused bits -- block region (a thread per block), macroblock pool
-//              (a thread per macroblock), segment pool (a thread per segment)
+//              unused bits -- block region (a lane per block), macroblock pool
+//              (a lane per macroblock), segment pool (one lane)
 //              (dv/src/decoder.rs:152-317); writes every dequantised coefficient.
 //   resolve    first failing segment per frame (sequential semantics).
-//   idct       eight threads per block (one per output row), 16 blocks per CTA:
+//   idct       eight threads per block (one per output row), 8 blocks per CTA:
 //              fp32 separable 8-8 / 2-4-8 transform with a proven error bound;
 //              samples within it of a rounding boundary are settled by the warp in
 //              exact fixed point, or in the reference's binary64 order for genuine
@@ -109,8 +109,9 @@ struct DvBlock {
 //
 // Each level is a chain of lookups, so warps go their own ways: with four segments to a
 // CTA and a thread per block, then per macroblock, then per segment, half of all warp time
-// was spent at the barriers between them (1000 NTSC frames, 270,000 segments: 1277 us, and
-// 1955 us now against 2325 with the transform). More CTAs per SM gain nothing.
+// was spent at the barriers between them (a call of 1000 NTSC frames, 270,000 segments,
+// transform included: 2325 us, then 1955; 1775 with the transform's later steps). More CTAs
+// per SM gain nothing.
 constexpr int kSegThreads = 128;
 constexpr int kSegWarps = kSegThreads / 32;
 constexpr int kSegCtasPerSm = 6;
@@ -390,7 +391,7 @@ __global__ void dv_resolve_kernel(DvLaunch L) {
     }
 }
 
-constexpr int kIdctBlocks = 8;                   // blocks per CTA (1000 NTSC frames: 1.92 ms, with 16 1.96)
+constexpr int kIdctBlocks = 8;                   // blocks per CTA (1000 NTSC frames at the time: 1.92 ms, with 16 1.96)
 constexpr int kIdctThreads = kIdctBlocks * 8;    // eight threads (rows) per block
 
 // Stores the eight bytes of `row` at dst (any alignment).
@@ -422,7 +423,7 @@ __device__ __forceinline__ void store_row4(uint8_t *dst, uint32_t row) {
 // found by one division where all frames are of one system; the eight threads of a
 // block synchronise through their warp only. Issue-bound (two thirds) with waits for the
 // levels between: 32 registers for 28 CTAs of 64 per SM (1000 NTSC frames: 1.82 ms, with
-// 52 registers 1.93).
+// 52 registers 1.93; 1.78 with fewer and larger parts).
 constexpr int kBlockStride = 72;  // ints or floats per block: four blocks' column accesses on distinct banks
 
 __global__ void __launch_bounds__(kIdctThreads, 28) dv_idct_kernel(DvLaunch L) {

@@ -1,9 +1,10 @@
 // The reference's forward DCT and quantisation reproduced exactly
 // (crates/codecs/mjpeg/src/transform.rs:111-134 forward_dct_quantize): an fp32
-// evaluation with a per-coefficient error bound, and the binary64 reference
-// order for quotients within that bound of a half-integer. Used by fdct_kernel
-// (8 threads per block) and, with the same functions, by the block-level
-// transform tests.
+// evaluation with an error bound, and the binary64 reference
+// order for quotients within that bound of a half-integer. fdct_kernel (8 threads per
+// block) takes one bound per block (fdct_row, fdct_column, fdct_round, kFdctBound,
+// exact_coefficient), as does a block-level test; fdct_row_pass and fdct_quantise take the
+// tighter bound per coefficient and are the other block-level test's alone.
 #pragma once
 
 #include <cuda_runtime.h>
